@@ -7,10 +7,12 @@
 // with -fmad=false so its arithmetic rounds after every operation, like the
 // reference solver's float64 torch ops (hydrointel/solver/swe2d.py).
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
 #include "../../include/his_gb300.h"
+#include "f64_ops.cuh"
 
 namespace his {
 
@@ -159,16 +161,13 @@ inline StepParams step_params_from(const his_step_params& q) {
     return sp;
 }
 
-struct TileRef {
-    int member, x0, y0, local;
-};
-
 // The solver constants in the compute type R, converted on the host and passed by
 // value: converting float64 constants inside the kernels put the float32 kernels on
 // GB300's FP64 pipe (a small fraction of the float32 rate).
 template <class R>
 struct KC {
     R g, hg, nhg, h_dry, kp_eps;
+    R h_kp;                          // depths from here on have h^4 >= kp_eps: no desingularisation
     int order, hllc;
 };
 
@@ -180,6 +179,7 @@ inline KC<R> make_kc(const Consts& c) {
     k.nhg = R(-0.5 * c.g);
     k.h_dry = R(c.h_dry);
     k.kp_eps = R(c.kp_eps);
+    k.h_kp = R(std::sqrt(std::sqrt(c.kp_eps)) * (1.0 + 1e-12));
     k.order = c.order;
     k.hllc = c.hllc;
     return k;
@@ -232,18 +232,13 @@ template <class R> __device__ __forceinline__ R per_len(R x, R d, R inv_d) {
 __device__ __forceinline__ double dsqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float dsqrt(float x) { return sqrtf(x); }
 
-// h**4 as the reference computes it (a power call), in each precision.
-__device__ __forceinline__ double pow4(double h) { return pow(h, 4.0); }
-__device__ __forceinline__ float pow4(float h) { float h2 = h * h; return h2 * h2; }
-// hf**(4/3)
-__device__ __forceinline__ double pow43(double x) { return pow(x, 4.0 / 3.0); }
-__device__ __forceinline__ float pow43(float x) { return powf(x, 4.0f / 3.0f); }
-__device__ __forceinline__ double rexp(double x) { return exp(x); }
-__device__ __forceinline__ float rexp(float x) { return expf(x); }
 __device__ __forceinline__ double cbrt_pow(double x) { return pow(x, 1.0 / 3.0); }
 __device__ __forceinline__ float cbrt_pow(float x) { return powf(x, 1.0f / 3.0f); }
 
-// Kurganov-Petrova desingularised velocity (swe2d.py:161-167)
+// Kurganov-Petrova desingularised velocity (swe2d.py:161-167):
+// sqrt(2) h hu / sqrt(h^4 + max(h^4, eps)).  float64: where h^4 >= eps that is hu / h,
+// one reciprocal instead of a power, a root and two divisions (10 FP64 instructions
+// instead of 115, and four roundings fewer).
 template <class R>
 __device__ __forceinline__ void kp_velocity(const KC<R>& c, R h, R hu, R hv, R& u, R& v) {
     const R SQRT2 = R(1.4142135623730951);
@@ -253,16 +248,19 @@ __device__ __forceinline__ void kp_velocity(const KC<R>& c, R h, R hu, R hv, R& 
         const bool wet = h >= c.h_dry;
         u = wet ? hu * s : 0.0f;
         v = wet ? hv * s : 0.0f;
-        return;
-    }
-    R h4 = pow4(h);
-    R den = dsqrt(h4 + rmax(h4, c.kp_eps));
-    if (h >= c.h_dry) {
-        u = SQRT2 * h * hu / den;
-        v = SQRT2 * h * hv / den;
     } else {
-        u = R(0);
-        v = R(0);
+        u = v = 0.0;
+        if (!f64_ge_pos(h, c.h_dry)) return;
+        if (f64_ge_pos(h, c.h_kp)) {
+            const double r = __drcp_rn(h);
+            u = f64_div(hu, h, r);
+            v = f64_div(hv, h, r);
+        } else {
+            const double h2 = h * h, h4 = h2 * h2;
+            const double den = sqrt(h4 + (h4 > c.kp_eps ? h4 : c.kp_eps));
+            u = SQRT2 * h * hu / den;
+            v = SQRT2 * h * hv / den;
+        }
     }
 }
 
@@ -294,211 +292,120 @@ __device__ __forceinline__ void discharge_ghost(const KC<R>& c, R val, R h, R& h
     ut_o = R(0);
 }
 
-template <class R>
-__device__ __forceinline__ R minmod(R a, R b) {
-    // float32: the median of (a, b, 0) from four min/max (for finite a, b: the smaller
-    // magnitude with the common sign, zero when the signs differ)
-    if constexpr (sizeof(R) == 4) return fmaxf(fminf(a, b), fminf(fmaxf(a, b), 0.0f));
-    if (a * b > R(0)) {
-        R m = rmin(fabs(a), fabs(b));
-        return a > R(0) ? m : -m;
-    }
-    return R(0);
-}
+// minmod as the median of (a, b, 0) from four min/max (for finite a, b: the smaller
+// magnitude with the common sign, zero when the signs differ)
+__device__ __forceinline__ float minmod(float a, float b) { return fmaxf(fminf(a, b), fminf(fmaxf(a, b), 0.0f)); }
 
-// MUSCL face states of one cell along one axis (swe2d.py:205-219).  Inputs are the
-// cell and its two neighbours along the axis; outputs the minus (left face) and
-// plus (right face) reconstructions of h, normal and tangential velocity, and the
-// recovered bed z = eta - h.
-//
-// float64 (plain method): the reference's own formulation, eta = h + z formed per
-// cell and the bed recovered as Zm = Em - Hm, Zp = Ep - Hp.
-// float32 (production form): the same reconstruction in difference form.  The
-// surface-elevation differences are dE = dh + dz (never forming eta = h + z, whose
-// float32 rounding would be ulp(z) ~ 1e-6 m at tens of metres of terrain) and the
-// reconstructed bed enters only through the in-cell bed slope d = sE - sH
-// (Zp - Zm = d, Zm = z - d/2, Zp = z + d/2), so the hydrostatic reconstruction
-// and the bed source keep their exact cancellation at rest.
-template <class R>
+// MUSCL face states of one cell along one axis (swe2d.py:205-219), float32 production
+// form.  Inputs are the cell and its two neighbours along the axis; outputs the minus
+// (left face) and plus (right face) reconstructions of h, normal and tangential velocity.
+// The reconstruction is in difference form: the surface-elevation differences are
+// dE = dh + dz (never forming eta = h + z, whose float32 rounding would be ulp(z) ~ 1e-6 m
+// at tens of metres of terrain) and the reconstructed bed enters only through the in-cell
+// bed slope d = sE - sH (Zp - Zm = d, Zm = z - d/2, Zp = z + d/2), so the hydrostatic
+// reconstruction and the bed source keep their exact cancellation at rest.  (The float64
+// form, with eta = h + z, is face64 in swe2d_tile64.cuh.)
 struct Recon {
-    R Hm, Hp, Um, Up, Vm, Vp, Zm, Zp;   // Zm/Zp: float64 path
-    R z, d, h0, sE;                     // float32 path: cell bed, in-cell bed slope, depth, eta slope
+    float Hm, Hp, Um, Up, Vm, Vp;
+    float z, d, h0, sE;                 // cell bed, in-cell bed slope, depth, eta slope
 };
 
-template <class R>
-__device__ __forceinline__ Recon<R> reconstruct(const KC<R>& c, R hm, R h0, R hp, R um, R u0, R up, R vm, R v0, R vp,
-                                                R zm, R z0, R zp) {
-    Recon<R> r;
+__device__ __forceinline__ Recon reconstruct(const KC<float>& c, float hm, float h0, float hp, float um, float u0,
+                                             float up, float vm, float v0, float vp, float zm, float z0, float zp) {
+    Recon r;
     r.z = z0;
     r.h0 = h0;
-    r.sE = R(0);
+    r.sE = 0.0f;
     if (c.order == 2) {
-        R hmin = rmin(rmin(hm, h0), hp);
-        R ok = (hmin >= c.h_dry) ? R(1) : R(0);
-        R sH = minmod(h0 - hm, hp - h0) * ok;
-        R sU = minmod(u0 - um, up - u0) * ok;
-        R sV = minmod(v0 - vm, vp - v0) * ok;
-        r.Hm = h0 - R(0.5) * sH;
-        r.Hp = h0 + R(0.5) * sH;
-        r.Um = u0 - R(0.5) * sU;
-        r.Up = u0 + R(0.5) * sU;
-        r.Vm = v0 - R(0.5) * sV;
-        r.Vp = v0 + R(0.5) * sV;
-        if constexpr (sizeof(R) == 8) {
-            R em = hm + zm, e0 = h0 + z0, ep = hp + zp;
-            R sE = minmod(e0 - em, ep - e0) * ok;
-            R Em = e0 - R(0.5) * sE, Ep = e0 + R(0.5) * sE;
-            r.Zm = Em - r.Hm;
-            r.Zp = Ep - r.Hp;
-            r.d = R(0);
-        } else {
-            R sE = minmod((h0 - hm) + (z0 - zm), (hp - h0) + (zp - z0)) * ok;
-            r.d = sE - sH;
-            r.sE = sE;
-            r.Zm = r.Zp = R(0);
-        }
+        const float hmin = fminf(fminf(hm, h0), hp);
+        const float ok = (hmin >= c.h_dry) ? 1.0f : 0.0f;
+        const float sH = minmod(h0 - hm, hp - h0) * ok;
+        const float sU = minmod(u0 - um, up - u0) * ok;
+        const float sV = minmod(v0 - vm, vp - v0) * ok;
+        r.Hm = h0 - 0.5f * sH;
+        r.Hp = h0 + 0.5f * sH;
+        r.Um = u0 - 0.5f * sU;
+        r.Up = u0 + 0.5f * sU;
+        r.Vm = v0 - 0.5f * sV;
+        r.Vp = v0 + 0.5f * sV;
+        const float sE = minmod((h0 - hm) + (z0 - zm), (hp - h0) + (zp - z0)) * ok;
+        r.d = sE - sH;
+        r.sE = sE;
     } else {
         r.Hm = r.Hp = h0;
         r.Um = r.Up = u0;
         r.Vm = r.Vp = v0;
-        r.Zm = r.Zp = z0;
-        r.d = R(0);
+        r.d = 0.0f;
     }
     return r;
 }
 
-// HLLC / HLL flux with two-rarefaction wave speeds and dry-bed fixes (swe2d.py:61-101)
-template <class R>
-__device__ __forceinline__ void riemann(const KC<R>& c, R hL, R uL, R vL, R hR, R uR, R vR, R& F1o, R& F2o,
-                                        R& F3o) {
-    const R g = c.g, tiny = R(1e-14);
-    R cL = dsqrt(g * hL), cR = dsqrt(g * hR);
-    bool dryL = hL <= tiny, dryR = hR <= tiny;
-    R u_s = R(0.5) * (uL + uR) + cL - cR;
-    R c_s = R(0.5) * (cL + cR) + R(0.25) * (uL - uR);
-    R SL = rmin(uL - cL, u_s - c_s);
-    R SR = rmax(uR + cR, u_s + c_s);
-    if (dryL) { SL = uR - R(2) * cR; SR = uR + cR; }
-    if (dryR) { SL = uL - cL; SR = uL + R(2) * cL; }
-    const R hg = c.hg;
-    R qL = hL * uL, qR = hR * uR;
-    R FL1 = qL, FR1 = qR;
-    R FL2 = qL * uL + hg * hL * hL, FR2 = qR * uR + hg * hR * hR;
-    R den = SR - SL;
-    if (fabs(den) < tiny) den = R(1);
-    bool left = SL >= R(0), right = SR <= R(0);
-    R F1, F2, F3;
-    if (left) {
-        F1 = FL1; F2 = FL2;
-    } else if (right) {
-        F1 = FR1; F2 = FR2;
-    } else {
-        F1 = (SR * FL1 - SL * FR1 + SL * SR * (hR - hL)) / den;
-        F2 = (SR * FL2 - SL * FR2 + SL * SR * (qR - qL)) / den;
-    }
-    if (c.hllc) {
-        R num = SL * hR * (uR - SR) - SR * hL * (uL - SL);
-        R dd = hR * (uR - SR) - hL * (uL - SL);
-        R SM = fabs(dd) < tiny ? R(0.5) * (uL + uR) : num / dd;
-        F3 = F1 * (SM >= R(0) ? vL : vR);
-    } else {
-        R FL3 = qL * vL, FR3 = qR * vR;
-        F3 = left ? FL3 : (right ? FR3 : (SR * FL3 - SL * FR3 + SL * SR * (hR * vR - hL * vL)) / den);
-    }
-    if (dryL && dryR) { F1 = R(0); F2 = R(0); F3 = R(0); }
-    F1o = F1; F2o = F2; F3o = F3;
-}
-
-// The same HLLC/HLL flux in well-balanced deviation form (float32 production form).
-// Instead of the momentum flux F2 it returns, for each side s in {L, R},
+// HLLC / HLL flux with two-rarefaction wave speeds and dry-bed fixes (swe2d.py:61-101) in
+// well-balanced deviation form (float32 production form).  Instead of the momentum flux F2 it returns, for each side s in {L, R},
 //     D_s = F2 + corr_s - g/2 h_s^2 = F2 - g/2 h*_s^2
 // (corr_s = g/2 (h_s^2 - h*_s^2) is the hydrostatic-reconstruction correction), so
 // that the cell update -[(F2 + corrL)_east - (F2 + corrR)_west] + bed source becomes
 // -[D_L,east - D_R,west] - g/2 (H+ + H-) sE: every term is small at rest and no
 // O(g h^2 / 2) quantities cancel in float32.  The pressure difference across the face
 // is formed from the depth difference, dp = g/2 (h*_R - h*_L)(h*_R + h*_L).
-template <class R>
-__device__ __forceinline__ void riemann_wb(const KC<R>& c, R hL, R uL, R vL, R hR, R uR, R vR, R jump, R& F1o,
-                                           R& DLo, R& DRo, R& F3o) {
-    const R g = c.g, tiny = R(1e-14);
-    R cL = dsqrt(g * hL), cR = dsqrt(g * hR);
+__device__ __forceinline__ void riemann_wb(const KC<float>& c, float hL, float uL, float vL, float hR, float uR, float vR, float jump, float& F1o,
+                                           float& DLo, float& DRo, float& F3o) {
+    const float g = c.g, tiny = 1e-14f;
+    float cL = dsqrt(g * hL), cR = dsqrt(g * hR);
     bool dryL = hL <= tiny, dryR = hR <= tiny;
-    R u_s = R(0.5) * (uL + uR) + cL - cR;
-    R c_s = R(0.5) * (cL + cR) + R(0.25) * (uL - uR);
-    R SL = rmin(uL - cL, u_s - c_s);
-    R SR = rmax(uR + cR, u_s + c_s);
-    if (dryL) { SL = uR - R(2) * cR; SR = uR + cR; }
-    if (dryR) { SL = uL - cL; SR = uL + R(2) * cL; }
-    const R hg = c.hg;
-    R qL = hL * uL, qR = hR * uR;
-    R dp = hg * jump * (hR + hL);
-    R den = SR - SL;
-    if (fabs(den) < tiny) den = R(1);
-    bool left = SL >= R(0), right = SR <= R(0);
-    R F1, DL, DR, F3;
+    float u_s = 0.5f * (uL + uR) + cL - cR;
+    float c_s = 0.5f * (cL + cR) + 0.25f * (uL - uR);
+    float SL = rmin(uL - cL, u_s - c_s);
+    float SR = rmax(uR + cR, u_s + c_s);
+    if (dryL) { SL = uR - 2.0f * cR; SR = uR + cR; }
+    if (dryR) { SL = uL - cL; SR = uL + 2.0f * cL; }
+    const float hg = c.hg;
+    float qL = hL * uL, qR = hR * uR;
+    float dp = hg * jump * (hR + hL);
+    float den = SR - SL;
+    if (fabs(den) < tiny) den = 1.0f;
+    bool left = SL >= 0.0f, right = SR <= 0.0f;
+    float F1, DL, DR, F3;
     if (left) {
         F1 = qL; DL = qL * uL; DR = qL * uL - dp;
     } else if (right) {
         F1 = qR; DL = qR * uR + dp; DR = qR * uR;
     } else {
-        R inv = R(1) / den;
+        float inv = 1.0f / den;
         F1 = (SR * qL - SL * qR + SL * SR * jump) * inv;
-        R dyn = (SR * qL * uL - SL * qR * uR + SL * SR * (qR - qL)) * inv;
+        float dyn = (SR * qL * uL - SL * qR * uR + SL * SR * (qR - qL)) * inv;
         DL = dyn - SL * dp * inv;
         DR = dyn - SR * dp * inv;
     }
     if (c.hllc) {
-        R num = SL * hR * (uR - SR) - SR * hL * (uL - SL);
-        R dd = hR * (uR - SR) - hL * (uL - SL);
-        R SM = fabs(dd) < tiny ? R(0.5) * (uL + uR) : num / dd;
-        F3 = F1 * (SM >= R(0) ? vL : vR);
+        float num = SL * hR * (uR - SR) - SR * hL * (uL - SL);
+        float dd = hR * (uR - SR) - hL * (uL - SL);
+        float SM = fabs(dd) < tiny ? 0.5f * (uL + uR) : num / dd;
+        F3 = F1 * (SM >= 0.0f ? vL : vR);
     } else {
-        R FL3 = qL * vL, FR3 = qR * vR;
+        float FL3 = qL * vL, FR3 = qR * vR;
         F3 = left ? FL3 : (right ? FR3 : (SR * FL3 - SL * FR3 + SL * SR * (hR * vR - hL * vL)) / den);
     }
-    if (dryL && dryR) { F1 = R(0); DL = R(0); DR = R(0); F3 = R(0); }
+    if (dryL && dryR) { F1 = 0.0f; DL = 0.0f; DR = 0.0f; F3 = 0.0f; }
     F1o = F1; DLo = DL; DRo = DR; F3o = F3;
 }
 
-// Face flux between two reconstructed cells (swe2d.py:226-234): hydrostatic
+// Face flux between two reconstructed cells (swe2d.py:226-234), float32: hydrostatic
 // reconstruction z* = max(zL, zR), h* = max(0, h + z - z*); returns the mass flux,
 // the momentum flux plus the left and right pressure corrections, and the
 // tangential flux.
-template <class R>
-__device__ __forceinline__ void face_flux(const KC<R>& c, const Recon<R>& L, const Recon<R>& Rr, R& F1, R& F2L,
-                                          R& F2R, R& F3) {
-    R hL = L.Hp, uL = L.Up, vL = L.Vp;
-    R hR = Rr.Hm, uR = Rr.Um, vR = Rr.Vm;
-    R hLs, hRs;
-    if constexpr (sizeof(R) == 8) {
-        R zL = L.Zp, zR = Rr.Zm;
-        R zf = rmax(zL, zR);
-        hLs = clamp0(hL + zL - zf);
-        hRs = clamp0(hR + zR - zf);
-    } else {
-        // z* - zL = max(0, zR - zL), z* - zR = max(0, zL - zR), with
-        // zR - zL = (z_R - z_L) - (d_L + d_R) / 2 formed from the cell-bed difference
-        R dz = (Rr.z - L.z) - R(0.5) * (L.d + Rr.d);
-        R aL = hL - clamp0(dz), aR = hR - clamp0(-dz);
-        hLs = clamp0(aL);
-        hRs = clamp0(aR);
-        // surface jump h*_R - h*_L = (eta_R - eta_L) - (sE_L + sE_R)/2 when neither side is
-        // clamped, formed from cell differences rather than from two rounded depths
-        R jump = (aL > R(0) && aR > R(0))
-                     ? ((Rr.h0 - L.h0) + (Rr.z - L.z)) - R(0.5) * (L.sE + Rr.sE)
-                     : hRs - hLs;
-        riemann_wb(c, hLs, uL, vL, hRs, uR, vR, jump, F1, F2L, F2R, F3);
-        return;
-    }
-    if constexpr (sizeof(R) == 8) {
-        R F2;
-        riemann(c, hLs, uL, vL, hRs, uR, vR, F1, F2, F3);
-        const R hg = c.hg;
-        R corrL = hg * (hL * hL - hLs * hLs);
-        R corrR = hg * (hR * hR - hRs * hRs);
-        F2L = F2 + corrL;
-        F2R = F2 + corrR;
-    }
+__device__ __forceinline__ void face_flux(const KC<float>& c, const Recon& L, const Recon& Rr, float& F1, float& F2L,
+                                          float& F2R, float& F3) {
+    const float hL = L.Hp, hR = Rr.Hm;
+    // z* - zL = max(0, zR - zL), z* - zR = max(0, zL - zR), with
+    // zR - zL = (z_R - z_L) - (d_L + d_R) / 2 formed from the cell-bed difference
+    const float dz = (Rr.z - L.z) - 0.5f * (L.d + Rr.d);
+    const float aL = hL - clamp0(dz), aR = hR - clamp0(-dz);
+    const float hLs = clamp0(aL), hRs = clamp0(aR);
+    // surface jump h*_R - h*_L = (eta_R - eta_L) - (sE_L + sE_R)/2 when neither side is
+    // clamped, formed from cell differences rather than from two rounded depths
+    const float jump = (aL > 0.0f && aR > 0.0f) ? ((Rr.h0 - L.h0) + (Rr.z - L.z)) - 0.5f * (L.sE + Rr.sE) : hRs - hLs;
+    riemann_wb(c, hLs, L.Up, L.Vp, hRs, Rr.Um, Rr.Vm, jump, F1, F2L, F2R, F3);
 }
 
 // ------------------------------------------------------------ block reductions

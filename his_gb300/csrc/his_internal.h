@@ -28,7 +28,7 @@ struct his_grid {
     std::vector<his_grid_desc> desc;
     std::vector<int> tile0, ntile;
     void* d_grids = nullptr;                 // his::Grid<R>[n]
-    his::TileRef* d_tiles = nullptr;
+    void* d_tiles = nullptr;                 // his::StripRef[n_tiles]
     int n_tiles = 0;
     his::StepParams* d_params = nullptr;
     double* d_partials = nullptr;            // n_tiles x NPART
@@ -37,6 +37,7 @@ struct his_grid {
     void* d_scratch = nullptr;               // stage buffers of every member
     size_t scratch_bytes = 0;
     size_t table_bytes = 0;
+    size_t stage_smem = 0;                   // dynamic shared memory of a stage CTA
     HostStage params_stage;                  // his_grid_step_async parameters
     // The 2-D stages of a grid step run as n_parts launches over whole members' tiles
     // [part_t[k], part_t[k + 1]), part 0 on the caller's stream and part k >= 1 on

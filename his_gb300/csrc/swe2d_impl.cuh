@@ -9,15 +9,46 @@
 #include "his_internal.h"
 #include "net1d_kernels.cuh"
 #include "swe2d_strip.cuh"
+#include "swe2d_tile64.cuh"
 
 namespace his {
 
+// Launch of one stage over `count` strip-chunks: float32 marches strips with NT threads,
+// float64 works off sub-tiles (`smem` bytes each, stage_smem).
+template <class R, int NT, int STAGE>
+void launch_stage(const Grid<R>* grids, const StripRef* strips, const StepParams* params, const KC<R>& kc, double* part,
+                  int count, size_t smem, cudaStream_t s) {
+    if constexpr (sizeof(R) == 8)
+        tile64_kernel<STAGE><<<count, TILE64_THREADS, smem, s>>>(grids, strips, params, kc, part);
+    else
+        strip_kernel<R, NT, STAGE><<<count, NT, smem, s>>>(grids, strips, params, kc, part);
+}
+
+// Strip-chunk of a member whose full chunks are w x rows cells.
+inline StripRef strip_ref(int member, int x0, int wc, int y0, int y1, int w, int rows) {
+    return StripRef{member, x0, wc, y0, y1, (short)tile64_part(w, TILE64_W), (short)tile64_part(rows, TILE64_H)};
+}
+
+// Dynamic shared memory of a stage CTA over strip-chunks of at most w x rows cells.
 template <class R, int NT>
-int set_strip_attrs() {
-    const int bytes = (int)StripGeom<R, NT>::smem_bytes;
-    HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+size_t stage_smem(int w, int rows, int order) {
+    if constexpr (sizeof(R) == 8) return tile64_smem(tile64_part(w, TILE64_W), tile64_part(rows, TILE64_H), order == 2);
+    else return StripGeom<R, NT>::smem_bytes;
+}
+
+template <class R, int NT>
+int set_stage_attrs() {
+    if constexpr (sizeof(R) == 8) {
+        const int bytes = (int)tile64_smem(TILE64_W, TILE64_H, true);
+        HIS_CK(cudaFuncSetAttribute(tile64_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        HIS_CK(cudaFuncSetAttribute(tile64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        HIS_CK(cudaFuncSetAttribute(tile64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    } else {
+        const int bytes = (int)StripGeom<R, NT>::smem_bytes;
+        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    }
     return HIS_OK;
 }
 
@@ -25,7 +56,6 @@ int set_strip_attrs() {
 // (default: all); a tile's partials sit at its global index.
 template <class R, int NT>
 int launch_stages(his_grid* g, cudaStream_t s, int t0 = 0, int count = -1) {
-    using G = StripGeom<R, NT>;
     if (count < 0) count = g->n_tiles - t0;
     if (count == 0) return HIS_OK;
     auto* grids = reinterpret_cast<const Grid<R>*>(g->d_grids);
@@ -33,11 +63,11 @@ int launch_stages(his_grid* g, cudaStream_t s, int t0 = 0, int count = -1) {
     auto* strips = reinterpret_cast<const StripRef*>(g->d_tiles) + t0;
     double* part = g->d_partials + (size_t)t0 * NPART;
     if (g->c.order == 2) {
-        strip_kernel<R, NT, 1><<<count, NT, G::smem_bytes, s>>>(grids, strips, g->d_params, kc, part);
-        strip_kernel<R, NT, 2><<<count, NT, G::smem_bytes, s>>>(grids, strips, g->d_params, kc, part);
+        launch_stage<R, NT, 1>(grids, strips, g->d_params, kc, part, count, g->stage_smem, s);
+        launch_stage<R, NT, 2>(grids, strips, g->d_params, kc, part, count, g->stage_smem, s);
     } else {
-        strip_kernel<R, NT, 0><<<count, NT, G::smem_bytes, s>>>(grids, strips, g->d_params, kc, part);
-        stage_copy_kernel<R, NT><<<count, NT, 0, s>>>(grids, strips, g->d_params);
+        launch_stage<R, NT, 0>(grids, strips, g->d_params, kc, part, count, g->stage_smem, s);
+        stage_copy_kernel<R><<<count, CHUNK_THREADS, 0, s>>>(grids, strips, g->d_params);
     }
     HIS_CK(cudaGetLastError());
     return HIS_OK;
@@ -72,26 +102,28 @@ int launch_step_nt(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
     return HIS_OK;
 }
 
-template <class R, int NT>
-int launch_reduce_nt(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
+template <class R>
+int launch_reduce(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
     auto* grids = reinterpret_cast<const Grid<R>*>(g->d_grids);
     auto* strips = reinterpret_cast<const StripRef*>(g->d_tiles);
     if (rate_only)
-        strip_rate_kernel<R, NT><<<g->n_tiles, NT, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
+        strip_rate_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
     else
-        strip_reduce_kernel<R, NT><<<g->n_tiles, NT, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
+        strip_reduce_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
     finalize_kernel<R><<<g->n, 32, 0, s>>>(grids, g->d_params, g->c, g->d_partials, g->d_out, rate_only ? 2 : 1,
                                            ext);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
 }
 
+// float64 has one CTA size, whatever the strip width
 #define HIS_NT_DISPATCH(FN, R, g, ...)                           \
     do {                                                         \
-        if (g->nt == 64) return FN<R, 64>(g, __VA_ARGS__);       \
-        if (g->nt == 128) return FN<R, 128>(g, __VA_ARGS__);     \
-        if (g->nt == 224) return FN<R, 224>(g, __VA_ARGS__);     \
-        if (g->nt == 352) return FN<R, 352>(g, __VA_ARGS__);     \
+        if constexpr (sizeof(R) == 8) return FN<R, 0>(g, __VA_ARGS__); \
+        else if (g->nt == 64) return FN<R, 64>(g, __VA_ARGS__);       \
+        else if (g->nt == 128) return FN<R, 128>(g, __VA_ARGS__); \
+        else if (g->nt == 224) return FN<R, 224>(g, __VA_ARGS__); \
+        else if (g->nt == 352) return FN<R, 352>(g, __VA_ARGS__); \
         set_error("unsupported strip width (threads per CTA)");  \
         return HIS_ERR_BAD_ARG;                                  \
     } while (0)
@@ -101,10 +133,14 @@ int launch_reduce_nt(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
 template <class R>
 int grid_init_impl(his_grid* g) {
     int rc;
-    if ((rc = set_strip_attrs<R, 64>()) != HIS_OK) return rc;
-    if ((rc = set_strip_attrs<R, 128>()) != HIS_OK) return rc;
-    if ((rc = set_strip_attrs<R, 224>()) != HIS_OK) return rc;
-    if ((rc = set_strip_attrs<R, 352>()) != HIS_OK) return rc;
+    if constexpr (sizeof(R) == 8) {
+        if ((rc = set_stage_attrs<R, 0>()) != HIS_OK) return rc;
+    } else {
+        if ((rc = set_stage_attrs<R, 64>()) != HIS_OK) return rc;
+        if ((rc = set_stage_attrs<R, 128>()) != HIS_OK) return rc;
+        if ((rc = set_stage_attrs<R, 224>()) != HIS_OK) return rc;
+        if ((rc = set_stage_attrs<R, 352>()) != HIS_OK) return rc;
+    }
     const int n = g->n;
     std::vector<Grid<R>> H(n);
     std::vector<StripRef> strips;
@@ -143,13 +179,15 @@ int grid_init_impl(his_grid* g) {
         G.tiles_x = ns;
         G.tiles_y = nch;
         G.n_tiles = ns * nch;
+        if constexpr (sizeof(R) == 8)
+            g->stage_smem = std::max(g->stage_smem, stage_smem<R, 0>(w, hch, g->c.order));
         G.tile0 = (int)strips.size();
         g->tile0[m] = G.tile0;
         g->ntile[m] = G.n_tiles;
         for (int cy = 0; cy < nch; ++cy)
             for (int sx = 0; sx < ns; ++sx) {
                 const int x0 = sx * w, y0 = cy * hch;
-                strips.push_back(StripRef{m, x0, std::min(w, d.nx - x0), y0, std::min(y0 + hch, d.ny), 0});
+                strips.push_back(strip_ref(m, x0, std::min(w, d.nx - x0), y0, std::min(y0 + hch, d.ny), w, hch));
             }
         G.h = (R*)d.h; G.hu = (R*)d.hu; G.hv = (R*)d.hv; G.sf = (R*)d.s_filled; G.ic = (R*)d.infil_cum;
         size_t plane = ((size_t)d.ny * d.nx * sizeof(R) + 255) & ~size_t(255);
@@ -160,6 +198,9 @@ int grid_init_impl(his_grid* g) {
         G.pk = (R*)d.peak_h; G.ps = (R*)d.peak_speed;
     }
     g->n_tiles = (int)strips.size();
+    if constexpr (sizeof(R) == 4)
+        g->stage_smem = g->nt == 64 ? stage_smem<R, 64>(0, 0, 0) : g->nt == 128 ? stage_smem<R, 128>(0, 0, 0)
+                      : g->nt == 224 ? stage_smem<R, 224>(0, 0, 0) : stage_smem<R, 352>(0, 0, 0);
     HIS_CK(cudaMalloc(&g->d_grids, sizeof(Grid<R>) * n));
     HIS_CK(cudaMemcpy(g->d_grids, H.data(), sizeof(Grid<R>) * n, cudaMemcpyHostToDevice));
     HIS_CK(cudaMalloc(&g->d_tiles, sizeof(StripRef) * strips.size()));
@@ -177,7 +218,7 @@ int grid_step_impl(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
 
 template <class R>
 int grid_reduce_impl(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
-    HIS_NT_DISPATCH(launch_reduce_nt, R, g, s, ext, rate_only);
+    return launch_reduce<R>(g, s, ext, rate_only);
 }
 
 template <class R>
@@ -247,7 +288,6 @@ int engine_take_rate_impl(his_engine* E) {
 // kernel class on its own stream; accumulates device milliseconds into ms[6].
 template <class R, int NT>
 int eng_profile_nt(his_grid* g, his_engine* E, int n_steps, double* ms) {
-    using G = StripGeom<R, NT>;
     auto* grids = reinterpret_cast<const Grid<R>*>(g->d_grids);
     const Net* nets = E->net ? E->net->d_nets : nullptr;
     const Lnk* links = E->links ? E->links->d_links : nullptr;
@@ -269,16 +309,13 @@ int eng_profile_nt(his_grid* g, his_engine* E, int n_steps, double* ms) {
             cudaEventRecord(ev[5], E->s1);
         }
         if (g->c.order == 2) {
-            strip_kernel<R, NT, 1><<<g->n_tiles, NT, G::smem_bytes, E->s0>>>(grids, strips, g->d_params, kc,
-                                                                            g->d_partials);
+            launch_stage<R, NT, 1>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, g->stage_smem, E->s0);
             cudaEventRecord(ev[2], E->s0);
-            strip_kernel<R, NT, 2><<<g->n_tiles, NT, G::smem_bytes, E->s0>>>(grids, strips, g->d_params, kc,
-                                                                            g->d_partials);
+            launch_stage<R, NT, 2>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, g->stage_smem, E->s0);
         } else {
             cudaEventRecord(ev[2], E->s0);
-            strip_kernel<R, NT, 0><<<g->n_tiles, NT, G::smem_bytes, E->s0>>>(grids, strips, g->d_params, kc,
-                                                                            g->d_partials);
-            stage_copy_kernel<R, NT><<<g->n_tiles, NT, 0, E->s0>>>(grids, strips, g->d_params);
+            launch_stage<R, NT, 0>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, g->stage_smem, E->s0);
+            stage_copy_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, E->s0>>>(grids, strips, g->d_params);
         }
         cudaEventRecord(ev[3], E->s0);
         if (E->net) cudaStreamWaitEvent(E->s0, ev[5], 0);
@@ -319,7 +356,8 @@ __global__ void noalloc_setup_kernel(Grid<R> G, StepParams P, NoallocPlan L, uns
     for (int b = i; b < L.n_strips; b += stride) {
         const int sx = b % L.ns, cy = b / L.ns;
         const int x0 = sx * L.w, y0 = cy * L.hch;
-        strips[b] = StripRef{0, x0, min(L.w, G.nx - x0), y0, min(y0 + L.hch, G.ny), 0};
+        strips[b] = StripRef{0, x0, min(L.w, G.nx - x0), y0, min(y0 + L.hch, G.ny),
+                             (short)tile64_part(L.w, TILE64_W), (short)tile64_part(L.hch, TILE64_H)};
     }
     for (int j = i; j < NPART * L.n_strips; j += stride) part[j] = 0.0;
     if (i < 8) reinterpret_cast<double*>(base + L.o_out)[i] = 0.0;
@@ -335,9 +373,9 @@ __global__ void noalloc_setup_kernel(Grid<R> G, StepParams P, NoallocPlan L, uns
 template <class R>
 int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_params& p, const NoallocPlan& L,
                       unsigned char* base, cudaStream_t s) {
-    constexpr int NT = 64;
+    constexpr int NT = sizeof(R) == 8 ? 0 : 64;
     static_assert(sizeof(Grid<R>) <= 256 && sizeof(StepParams) <= 256, "records exceed their scratch slots");
-    int rc = set_strip_attrs<R, NT>();
+    int rc = set_stage_attrs<R, NT>();
     if (rc) return rc;
     Grid<R> G{};
     G.ny = d.ny;
@@ -371,13 +409,13 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
     auto* part = reinterpret_cast<double*>(base + L.o_part);
     auto* out = reinterpret_cast<double*>(base + L.o_out);
     const KC<R> kc = make_kc<R>(c);
-    const size_t smem = StripGeom<R, NT>::smem_bytes;
+    const size_t smem = stage_smem<R, NT>(L.w, L.hch, c.order);
     if (c.order == 2) {
-        strip_kernel<R, NT, 1><<<L.n_strips, NT, smem, s>>>(grid, strips, params, kc, part);
-        strip_kernel<R, NT, 2><<<L.n_strips, NT, smem, s>>>(grid, strips, params, kc, part);
+        launch_stage<R, NT, 1>(grid, strips, params, kc, part, L.n_strips, smem, s);
+        launch_stage<R, NT, 2>(grid, strips, params, kc, part, L.n_strips, smem, s);
     } else {
-        strip_kernel<R, NT, 0><<<L.n_strips, NT, smem, s>>>(grid, strips, params, kc, part);
-        stage_copy_kernel<R, NT><<<L.n_strips, NT, 0, s>>>(grid, strips, params);
+        launch_stage<R, NT, 0>(grid, strips, params, kc, part, L.n_strips, smem, s);
+        stage_copy_kernel<R><<<L.n_strips, CHUNK_THREADS, 0, s>>>(grid, strips, params);
     }
     finalize_kernel<R><<<1, 32, 0, s>>>(grid, params, c, part, out, 0, nullptr);
     HIS_CK(cudaGetLastError());

@@ -1,4 +1,6 @@
-// 2-D finite-volume step kernels: row-marching strips.
+// 2-D finite-volume step kernels of the float32 production form: row-marching strips
+// (the float64 method's are in swe2d_tile64.cuh), and the per-strip-chunk reductions of
+// both precisions.
 //
 // A CTA of NT threads owns a strip of W <= NT - 6 columns of one member and marches
 // up a chunk of rows [y0, y1).  Thread t works on column cx = x0 - 3 + t.  Per new
@@ -24,12 +26,13 @@
 namespace his {
 
 struct StripRef {
-    int member, x0, w, y0, y1, pad;
+    int member, x0, w, y0, y1;
+    short sub_w, sub_h;              // float64: largest sub-tile (swe2d_tile64.cuh)
 };
 
 // Four values of one cell or face kept together in shared memory, so that one
 // vector access moves them: cells {h, u, v, z}, faces {F1, F2L, F2R, F3}, and the
-// x-reconstruction as {Hm, Hp, Um, Up} and {Vm, Vp, Zm, Zp} (float32: {Vm, Vp, d, sE}).
+// plus side of the x-reconstruction.
 template <class R>
 struct alignas(4 * sizeof(R)) Q4 {
     R a, b, c, d;
@@ -52,23 +55,18 @@ struct StripGeom {
     static constexpr size_t scalars = (size_t)(1 + RING) * P;
     static_assert((size_t)4 * RING * P >= (size_t)(NT / 32) * NRED, "reduction scratch must fit in the cell ring");
     static constexpr size_t smem_bytes = sizeof(Q4<R>) * quads + sizeof(R) * scalars;
-    // resident CTAs per SM the float32 kernels are register-capped for; float64 keeps
-    // the compiler's choice (one CTA of any width must fit the register file)
+    // resident CTAs per SM the kernels are register-capped for
     static constexpr int min_ctas(int stage) {
-        return sizeof(R) == 4 ? ((stage == 1 ? 768 : 640) / NT > 0 ? (stage == 1 ? 768 : 640) / NT : 1) : 1;
+        return (stage == 1 ? 768 : 640) / NT > 0 ? (stage == 1 ? 768 : 640) / NT : 1;
     }
 };
 
 // Centred bed source of one cell along one axis (swe2d.py:220), from the cell's own
-// reconstruction: -g/2 (H- + H+)(Z+ - Z-).  float32: Z+ - Z- is the in-cell surface
+// reconstruction: -g/2 (H- + H+)(Z+ - Z-), with Z+ - Z- replaced by the in-cell surface
 // slope sE (the hydrostatic part of the face momentum fluxes is carried by riemann_wb).
 // The row loop computes it where the reconstruction is formed and carries it in
 // registers to the update of that cell.
-template <class R>
-__device__ __forceinline__ R bed_term(const KC<R>& c, const Recon<R>& r) {
-    if constexpr (sizeof(R) == 8) return c.nhg * (r.Hm + r.Hp) * (r.Zp - r.Zm);
-    else return c.nhg * (r.Hm + r.Hp) * r.sE;
-}
+__device__ __forceinline__ float bed_term(const KC<float>& c, const Recon& r) { return c.nhg * (r.Hm + r.Hp) * r.sE; }
 
 // One halo position: an interior cell, or the ghost that the x-sweep (outside in x)
 // or the y-sweep (outside in y) would see (boundaries.py:81-128), in two parts for
@@ -231,40 +229,24 @@ __device__ __forceinline__ void block_reduce_store(T (&v)[NV], const bool* is_ma
 }
 
 // One side of a reconstructed cell as a face sees it: depth, normal and tangential
-// velocity, and X = the recovered bed (float64) or the in-cell bed slope d (float32),
-// S = the in-cell surface slope sE (float32).  The cell's own bed z and depth h0 (the
-// float32 flux's difference form) come with the cell record.
-template <class R>
+// velocity, X = the in-cell bed slope d and S = the in-cell surface slope sE.  The cell's
+// own bed z and depth h0 (the flux's difference form) come with the cell record.
 struct Side {
-    R H, U, V, X, S;
+    float H, U, V, X, S;
 };
-template <class R>
-__device__ __forceinline__ Side<R> side_plus(const Recon<R>& r) {
-    if constexpr (sizeof(R) == 8) return Side<R>{r.Hp, r.Up, r.Vp, r.Zp, R(0)};
-    else return Side<R>{r.Hp, r.Up, r.Vp, r.d, r.sE};
-}
-template <class R>
-__device__ __forceinline__ Side<R> side_minus(const Recon<R>& r) {
-    if constexpr (sizeof(R) == 8) return Side<R>{r.Hm, r.Um, r.Vm, r.Zm, R(0)};
-    else return Side<R>{r.Hm, r.Um, r.Vm, r.d, r.sE};
-}
+__device__ __forceinline__ Side side_plus(const Recon& r) { return Side{r.Hp, r.Up, r.Vp, r.d, r.sE}; }
+__device__ __forceinline__ Side side_minus(const Recon& r) { return Side{r.Hm, r.Um, r.Vm, r.d, r.sE}; }
 
 // Face flux from the plus side of the cell below / west of the face (bed zl, depth hl)
 // and the minus side of the cell above / east of it: face_flux's arithmetic exactly.
-template <class R>
-__device__ __forceinline__ Q4<R> side_flux(const KC<R>& c, const Side<R>& L, R zl, R hl, const Side<R>& Rt, R zr,
-                                           R hr) {
-    Recon<R> a, b;
+__device__ __forceinline__ Q4<float> side_flux(const KC<float>& c, const Side& L, float zl, float hl, const Side& Rt,
+                                               float zr, float hr) {
+    Recon a, b;
     a.Hp = L.H; a.Up = L.U; a.Vp = L.V;
     b.Hm = Rt.H; b.Um = Rt.U; b.Vm = Rt.V;
-    if constexpr (sizeof(R) == 8) {
-        a.Zp = L.X; b.Zm = Rt.X;
-    } else {
-        a.d = L.X; a.sE = L.S; a.z = zl; a.h0 = hl;
-        b.d = Rt.X; b.sE = Rt.S; b.z = zr; b.h0 = hr;
-    }
-    (void)zl; (void)hl; (void)zr; (void)hr;
-    Q4<R> f;
+    a.d = L.X; a.sE = L.S; a.z = zl; a.h0 = hl;
+    b.d = Rt.X; b.sE = Rt.S; b.z = zr; b.h0 = hr;
+    Q4<float> f;
     face_flux(c, a, b, f.a, f.b, f.c, f.d);
     return f;
 }
@@ -284,6 +266,7 @@ __device__ __forceinline__ Q4<R> side_flux(const KC<R>& c, const Side<R>& L, R z
 // pipeline fill at the chunk's start, the drain at its end and the grid's edges.
 template <class R, int NT, int STAGE>
 struct StripPipe {
+    static_assert(sizeof(R) == 4, "the float64 step is tile64_kernel's");
     using G = StripGeom<R, NT>;
     static constexpr int P = G::P;
     static constexpr int RM = G::RING - 1;
@@ -306,7 +289,7 @@ struct StripPipe {
     R dt, rdx, rdy, idx, idy, rdt, tt;
     // carried state of this thread's column
     HaloRaw<R> ra;                     // raw row r (prefetched one row ahead)
-    Side<R> ylow;                      // plus side of the y-reconstruction of row r-2
+    Side ylow;                      // plus side of the y-reconstruction of row r-2
     R by1, by2, bx1;                   // bed terms: y of rows r-2, r-3; x of row r-3
     CellIn<R> cin;
     R acc_clip, xin, xout, yin, yout, infil, rainw, rate, hsum, ssum, hmax;
@@ -356,23 +339,23 @@ struct StripPipe {
         // y-reconstruction of row r-1 (normal velocity v, tangential u); its face with
         // row r-2 is formed in phase B beside the x-face, two independent chains
         const bool yact = FULL || r >= y0 - 1;
-        Side<R> ylo = ylow, yum;
+        Side ylo = ylow, yum;
         if (yact) {
-            const Recon<R> yup = reconstruct(c, c2.a, c1.a, c0.a, c2.c, c1.c, c0.c, c2.b, c1.b, c0.b, c2.d, c1.d, c0.d);
+            const Recon yup = reconstruct(c, c2.a, c1.a, c0.a, c2.c, c1.c, c0.c, c2.b, c1.b, c0.b, c2.d, c1.d, c0.d);
             yum = side_minus(yup);
             ylow = side_plus(yup);
             if (c.order == 2) by0 = bed_term(c, yup);
         }
         const bool xact = FULL || (r >= y0 + 1 && (unsigned)row < (unsigned)ny);
         Q4<R> cl;
-        Side<R> xm;
+        Side xm;
         if (xact) {
             cl = s_cell[k2 + ts - 1];
             const Q4<R> cr = s_cell[k2 + ts + 1];
-            const Recon<R> xr = reconstruct(c, cl.a, c2.a, cr.a, cl.b, c2.b, cr.b, cl.c, c2.c, cr.c, cl.d, c2.d, cr.d);
-            const Side<R> xp_ = side_plus(xr);
+            const Recon xr = reconstruct(c, cl.a, c2.a, cr.a, cl.b, c2.b, cr.b, cl.c, c2.c, cr.c, cl.d, c2.d, cr.d);
+            const Side xp_ = side_plus(xr);
             s_rp[ts] = Q4<R>{xp_.H, xp_.U, xp_.V, xp_.X};
-            if constexpr (sizeof(R) == 4) s_rs[ts] = xp_.S;
+            s_rs[ts] = xp_.S;
             xm = side_minus(xr);
             if (c.order == 2) bx0 = bed_term(c, xr);
         }
@@ -387,8 +370,7 @@ struct StripPipe {
         Q4<R> xf0{R(0), R(0), R(0), R(0)};
         if (xact) {
             const Q4<R> lp = s_rp[ts - 1];
-            Side<R> L{lp.a, lp.b, lp.c, lp.d, R(0)};
-            if constexpr (sizeof(R) == 4) L.S = s_rs[ts - 1];
+            const Side L{lp.a, lp.b, lp.c, lp.d, s_rs[ts - 1]};
             xf0 = side_flux(c, L, cl.d, cl.a, xm, c2.d, c2.a);
             s_xf[xo + ts] = xf0;
         }
@@ -472,7 +454,7 @@ struct StripPipe {
             hn = hn + rdt;
         }
         if (feat & FEAT_HORTON) {
-            const R rate_f = cin.fc + (cin.f0 - cin.fc) * rexp(-cin.k * tt);
+            const R rate_f = cin.fc + (cin.f0 - cin.fc) * expf(-cin.k * tt);
             const R pot = rate_f * dt;
             const R take = rmin(pot, hn);
             const R safe = hn > R(0) ? hn : R(1);
@@ -501,20 +483,14 @@ struct StripPipe {
             gd.sf[i] = sf;
         }
         // ---- semi-implicit Manning friction (swe2d.py:362-370)
-        R u, v, ks = R(0);
-        if constexpr (sizeof(R) == 4) {
-            // KP factor of the new depth, kept for the CFL velocity below
-            const float h2 = hn * hn, h4 = h2 * h2;
-            ks = hn >= c.h_dry ? 1.4142135623730951f * hn * rsqrtf(h4 + fmaxf(h4, c.kp_eps)) : 0.0f;
-            u = hun * ks;
-            v = hvn * ks;
-        } else {
-            kp_velocity(c, hn, hun, hvn, u, v);
-        }
+        // KP factor of the new depth, kept for the CFL velocity below
+        const R h2 = hn * hn, h4 = h2 * h2;
+        const R ks = hn >= c.h_dry ? 1.4142135623730951f * hn * rsqrtf(h4 + fmaxf(h4, c.kp_eps)) : 0.0f;
+        R u = hun * ks, v = hvn * ks;
         const R speed = dsqrt(u * u + v * v);
         const R hf = rmax(hn, c.h_dry);
         const R nm = cin.n;
-        const R denom = R(1) + dt * c.g * nm * nm * speed / pow43(hf);
+        const R denom = R(1) + dt * c.g * nm * nm * speed / powf(hf, 4.0f / 3.0f);
         u = u / denom;
         v = v / denom;
         const bool wet = hn >= c.h_dry;
@@ -527,13 +503,7 @@ struct StripPipe {
         }
         if (feat & FEAT_PEAK) gd.pk[i] = rmax(gd.pk[i], hn);
         // ---- CFL rate of the new state for the next step (swe2d.py:179-184)
-        R u2, v2;
-        if constexpr (sizeof(R) == 4) {
-            u2 = hun * ks;
-            v2 = hvn * ks;
-        } else {
-            kp_velocity(c, hn, hun, hvn, u2, v2);
-        }
+        const R u2 = hun * ks, v2 = hvn * ks;
         // running peak speed and output use the KP velocities of the new state, as the
         // reference's snapshots do (swe2d.py:161-167, coupling.py:229-242)
         if (feat & FEAT_PSPEED) gd.ps[i] = rmax(gd.ps[i], dsqrt(u2 * u2 + v2 * v2));
@@ -675,83 +645,95 @@ __global__ void __launch_bounds__(NT, StripGeom<R, NT>::min_ctas(STAGE)) strip_k
     }
 }
 
+// Cells of a strip-chunk in row order, spread over the threads of a CTA: consecutive
+// threads take consecutive cells, and a chunk of any shape keeps every thread busy (one
+// column per thread left most of a GPU idle behind a march of up to 48 rows).
+constexpr int CHUNK_THREADS = 256;
+template <class F>
+__device__ __forceinline__ void for_chunk_cells(const StripRef& sr, int nx, F f) {
+    const int n = sr.w * (sr.y1 - sr.y0);
+    for (int i = threadIdx.x; i < n; i += CHUNK_THREADS) {
+        const int y = i / sr.w;
+        f((size_t)(sr.y0 + y) * nx + (sr.x0 + (i - y * sr.w)));
+    }
+}
+
 // First-order step: move the result from the stage buffers back to the state.
-template <class R, int NT>
-__global__ void __launch_bounds__(NT) stage_copy_kernel(const Grid<R>* __restrict__ grids,
-                                                         const StripRef* __restrict__ strips,
-                                                         const StepParams* __restrict__ params) {
+template <class R>
+__global__ void __launch_bounds__(CHUNK_THREADS) stage_copy_kernel(const Grid<R>* __restrict__ grids,
+                                                                   const StripRef* __restrict__ strips,
+                                                                   const StepParams* __restrict__ params) {
     const StripRef sr = strips[blockIdx.x];
     const Grid<R>& gd = grids[sr.member];
     if (!params[sr.member].active) return;
-    const int cx = sr.x0 + threadIdx.x;
-    if ((int)threadIdx.x >= sr.w || cx >= gd.nx) return;
-    for (int y = sr.y0; y < sr.y1; ++y) {
-        const size_t i = (size_t)y * gd.nx + cx;
-        gd.h[i] = gd.h1[i];
-        gd.hu[i] = gd.hu1[i];
-        gd.hv[i] = gd.hv1[i];
-    }
+    R *__restrict__ h = gd.h, *__restrict__ hu = gd.hu, *__restrict__ hv = gd.hv;
+    const R *__restrict__ h1 = gd.h1, *__restrict__ hu1 = gd.hu1, *__restrict__ hv1 = gd.hv1;
+    for_chunk_cells(sr, gd.nx, [&](size_t i) {
+        h[i] = h1[i];
+        hu[i] = hu1[i];
+        hv[i] = hv1[i];
+    });
+}
+
+// CFL rate of one cell's state (swe2d.py:179-184); float64: rate64, as in the step.
+__device__ __forceinline__ float cell_rate(const KC<float>& c, float h, float hu, float hv, const Grid<float>& gd) {
+    float u, v;
+    kp_velocity(c, h, hu, hv, u, v);
+    const float cw = sqrtf(c.g * h);
+    return h > c.h_dry ? per_len(fabsf(u) + cw, gd.rdx, gd.idx) + per_len(fabsf(v) + cw, gd.rdy, gd.idy) : 0.0f;
+}
+__device__ __forceinline__ double rate64(const KC<double>& c, double h, double u, double v, double dx, double dy,
+                                         double idx, double idy) {
+    const double cw = sqrt(c.g * h);
+    return f64_div(fabs(u) + cw, dx, idx) + f64_div(fabs(v) + cw, dy, idy);
+}
+__device__ __forceinline__ double cell_rate(const KC<double>& c, double h, double hu, double hv,
+                                            const Grid<double>& gd) {
+    if (!f64_ge_pos(h, c.h_dry) || f64_bits(h) == f64_bits(c.h_dry)) return 0.0;
+    double u, v;
+    kp_velocity(c, h, hu, hv, u, v);
+    return rate64(c, h, u, v, gd.rdx, gd.rdy, gd.idx, gd.idy);
 }
 
 // Per strip-chunk CFL rate, surface and retained water of the current state (float64 sums).
-template <class R, int NT>
-__global__ void __launch_bounds__(NT) strip_reduce_kernel(const Grid<R>* __restrict__ grids,
-                                                           const StripRef* __restrict__ strips, const KC<R> c,
-                                                           double* __restrict__ partials) {
+template <class R>
+__global__ void __launch_bounds__(CHUNK_THREADS) strip_reduce_kernel(const Grid<R>* __restrict__ grids,
+                                                                     const StripRef* __restrict__ strips, const KC<R> c,
+                                                                     double* __restrict__ partials) {
     __shared__ double red[32 * 3];
     const StripRef sr = strips[blockIdx.x];
     const Grid<R>& gd = grids[sr.member];
-    double rate = 0, hs = 0, ss = 0;
-    const int cx = sr.x0 + threadIdx.x;
-    if ((int)threadIdx.x < sr.w && cx < gd.nx) {
-        for (int y = sr.y0; y < sr.y1 && y < gd.ny; ++y) {
-            const size_t i = (size_t)y * gd.nx + cx;
-            R h = gd.h[i], u, v;
-            kp_velocity(c, h, gd.hu[i], gd.hv[i], u, v);
-            const R cw = dsqrt(c.g * h);
-            const R r = h > c.h_dry ? per_len(fabs(u) + cw, gd.rdx, gd.idx) + per_len(fabs(v) + cw, gd.rdy, gd.idy)
-                                    : R(0);
-            rate = fmax(rate, (double)r);
-            hs += (double)h;
-            ss += (double)gd.sf[i];
-        }
-    }
-    double v[3] = {rate, hs, ss};
+    R rate = R(0);
+    double hs = 0, ss = 0;
+    for_chunk_cells(sr, gd.nx, [&](size_t i) {
+        const R h = gd.h[i];
+        rate = rmax(rate, cell_rate(c, h, gd.hu[i], gd.hv[i], gd));
+        hs += (double)h;
+        ss += (double)gd.sf[i];
+    });
+    double v[3] = {(double)rate, hs, ss};
     const bool mx[3] = {true, false, false};
     const int sl[3] = {P_RATE, P_HSUM, P_SSUM};
-    block_reduce_store<3>(v, mx, red, partials + (size_t)blockIdx.x * NPART, sl, NT);
+    block_reduce_store<3>(v, mx, red, partials + (size_t)blockIdx.x * NPART, sl, CHUNK_THREADS);
 }
 
 // Per strip-chunk CFL rate alone (swe2d.py:179-184), for the step's dt: the maximum
-// is exact in the compute type, so the cells need no float64 work (slow on this GPU)
-// and the result equals strip_reduce_kernel's; rows are unrolled to keep loads in
-// flight.  Writes only the P_RATE partial.
-template <class R, int NT>
-__global__ void __launch_bounds__(NT) strip_rate_kernel(const Grid<R>* __restrict__ grids,
-                                                         const StripRef* __restrict__ strips, const KC<R> c,
-                                                         double* __restrict__ partials) {
+// is exact in the compute type, so the result equals strip_reduce_kernel's.  Writes only
+// the P_RATE partial.
+template <class R>
+__global__ void __launch_bounds__(CHUNK_THREADS) strip_rate_kernel(const Grid<R>* __restrict__ grids,
+                                                                   const StripRef* __restrict__ strips, const KC<R> c,
+                                                                   double* __restrict__ partials) {
     __shared__ R red[32];
     const StripRef sr = strips[blockIdx.x];
     const Grid<R>& gd = grids[sr.member];
+    const R *__restrict__ h = gd.h, *__restrict__ hu = gd.hu, *__restrict__ hv = gd.hv;
     R rate = R(0);
-    const int cx = sr.x0 + threadIdx.x;
-    if ((int)threadIdx.x < sr.w && cx < gd.nx) {
-        const int y1 = min(sr.y1, gd.ny);
-#pragma unroll 4
-        for (int y = sr.y0; y < y1; ++y) {
-            const size_t i = (size_t)y * gd.nx + cx;
-            R h = gd.h[i], u, v;
-            kp_velocity(c, h, gd.hu[i], gd.hv[i], u, v);
-            const R cw = dsqrt(c.g * h);
-            const R r = h > c.h_dry ? per_len(fabs(u) + cw, gd.rdx, gd.idx) + per_len(fabs(v) + cw, gd.rdy, gd.idy)
-                                    : R(0);
-            rate = rmax(rate, r);
-        }
-    }
+    for_chunk_cells(sr, gd.nx, [&](size_t i) { rate = rmax(rate, cell_rate(c, h[i], hu[i], hv[i], gd)); });
     R v[1] = {rate};
     const bool mx[1] = {true};
     const int sl[1] = {P_RATE};
-    block_reduce_store<1>(v, mx, red, partials + (size_t)blockIdx.x * NPART, sl, NT);
+    block_reduce_store<1>(v, mx, red, partials + (size_t)blockIdx.x * NPART, sl, CHUNK_THREADS);
 }
 
 // Per-member totals from the strip-chunk partials, in a fixed order.  out: 8 per
