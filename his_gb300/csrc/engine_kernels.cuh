@@ -9,7 +9,7 @@
 //   stage 1, stage 2 (tiles of every member)              (swe2d.py:305-371)
 //   net substeps (one CTA per member, concurrent with the 2-D stages)
 //                                                         (coupling.py:216-221)
-//   eng_post  (one warp per member)  step volumes summed in tile order into the
+//   eng_post  (one CTA per member)  step volumes summed in tile order into the
 //             float64 accumulators, t += dt, plausibility (coupling.py:213-227, :169-192)
 #pragma once
 #include "net1d_kernels.cuh"
@@ -127,69 +127,63 @@ __global__ void eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restric
 }
 
 template <class R>
-__global__ void eng_post_kernel(EngMember* __restrict__ em, const StepParams* __restrict__ params,
-                                const Grid<R>* __restrict__ grids, Consts c, const double* __restrict__ partials,
-                                const double* __restrict__ vol1d, double* __restrict__ out, int m0) {
-    const int m = m0 + blockIdx.x, lane = threadIdx.x;
+__global__ void __launch_bounds__(FIN_THREADS) eng_post_kernel(EngMember* __restrict__ em,
+                                                               const StepParams* __restrict__ params,
+                                                               const Grid<R>* __restrict__ grids, Consts c,
+                                                               const double* __restrict__ partials,
+                                                               const double* __restrict__ vol1d,
+                                                               double* __restrict__ out, int m0) {
+    __shared__ double S[NPART];
+    const int m = m0 + blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (!params[m].active) return;
     const Grid<R>& gd = grids[m];
-    double s[NPART];
-#pragma unroll
-    for (int j = 0; j < NPART; ++j) s[j] = 0.0;
-    for (int t = lane; t < gd.n_tiles; t += 32) {
-        const double* p = partials + (size_t)(gd.tile0 + t) * NPART;
-#pragma unroll
-        for (int j = 0; j < NPART; ++j) s[j] = (j == P_RATE || j == P_HMAX) ? fmax(s[j], p[j]) : s[j] + p[j];
-    }
-#pragma unroll
-    for (int j = 0; j < NPART; ++j) s[j] = (j == P_RATE || j == P_HMAX) ? warp_max(s[j]) : warp_sum(s[j]);
+    sum_partials(partials, gd.tile0, gd.n_tiles, S);
     if (lane != 0) return;
+    // one thread per accumulated term, clock and status on another: each in its own warp
     EngMember& E = em[m];
     const StepParams& pr = params[m];
-    const double dt = (double)R(pr.dt);
-    double qin = s[P_XIN1] * gd.dy + s[P_YIN1] * gd.dx;
-    double qout = s[P_XOUT1] * gd.dy + s[P_YOUT1] * gd.dx;
-    double clip = s[P_CLIP1] * gd.area;
-    if (c.order == 2) {
-        qin = 0.5 * (qin + (s[P_XIN2] * gd.dy + s[P_YIN2] * gd.dx));
-        qout = 0.5 * (qout + (s[P_XOUT2] * gd.dy + s[P_YOUT2] * gd.dx));
-        clip = clip + s[P_CLIP2] * gd.area;
-    }
-    const double rain = gd.rw ? s[P_RAINW] * gd.area
-                              : (double)(R(pr.rain) * R(pr.dt)) * ((double)((long long)gd.nx * gd.ny) * gd.area);
-    const double infil = s[P_INFIL] * gd.area;
-    E.acc[0] += rain;
-    E.acc[1] += infil;
-    E.acc[2] += qin * dt;
-    E.acc[3] += qout * dt;
-    E.acc[6] += clip;
-    if (vol1d && E.n_sub > 0) {
-        E.acc[4] += vol1d[m * 3 + 0];
-        E.acc[5] += vol1d[m * 3 + 1];
-        E.acc[6] += vol1d[m * 3 + 2];
-    }
-    E.rate = s[P_RATE];
-    E.t = E.t + E.dt;
-    if (pr.snap_k >= 0) {
-        E.snap_t[pr.snap_k] = E.t;
-        E.k_out = pr.snap_k + 1;
-        if (double* L = pr.snap_ledger) {        // the 1-D kernel writes L[L_V1D]
-            L[L_V2D] = s[P_HSUM] * gd.area;
-            L[L_STORE] = s[P_SSUM] * gd.area;
-            L[L_RAIN] = E.acc[0]; L[L_INFIL] = E.acc[1]; L[L_BND2_IN] = E.acc[2]; L[L_BND2_OUT] = E.acc[3];
-            L[L_BND1_IN] = E.acc[4]; L[L_BND1_OUT] = E.acc[5]; L[L_CLIP] = E.acc[6];
-        }
-    }
-    E.steps += 1;
-    E.dt_min = fmin(E.dt_min, E.dt);
-    E.dt_max = fmax(E.dt_max, E.dt);
-    E.n_sub_max = max(E.n_sub_max, E.n_sub);
     double* o = out + (size_t)m * 8;
-    o[0] = qin * dt; o[1] = qout * dt; o[2] = rain; o[3] = infil; o[4] = clip;
-    o[5] = s[P_RATE]; o[6] = s[P_HSUM] * gd.area; o[7] = s[P_SSUM] * gd.area;
-    if (!isfinite(s[P_HSUM]) || !isfinite(s[P_RATE])) E.status = ST_NONFINITE;
-    else if (s[P_HMAX] > MAX_PLAUSIBLE_DEPTH_2D) E.status = ST_IMPLAUSIBLE;
-    else if (E.t >= E.t_end - 1e-9) E.status = ST_DONE;
+    double* L = pr.snap_k >= 0 ? pr.snap_ledger : nullptr;      // the 1-D kernel writes L[L_V1D]
+    const bool net = vol1d && E.n_sub > 0;
+    if (warp <= 4) {
+        const double v = step_term(warp, gd, pr, c.order, S);
+        o[warp] = v;
+        const int a = warp == 0 ? 2 : warp == 1 ? 3 : warp == 2 ? 0 : warp == 3 ? 1 : 6;
+        double acc = E.acc[a] + v;
+        if (warp == 4 && net) acc += vol1d[m * 3 + 2];
+        E.acc[a] = acc;
+        if (L) L[L_RAIN + a] = acc;
+    } else if (warp == 5) {
+        for (int k = 0; k < 2; ++k) {
+            const double acc = net ? E.acc[4 + k] + vol1d[m * 3 + k] : E.acc[4 + k];
+            E.acc[4 + k] = acc;
+            if (L) L[L_BND1_IN + k] = acc;
+        }
+    } else if (warp == 6) {
+        const double v2 = S[P_HSUM] * gd.area, vs = S[P_SSUM] * gd.area;
+        o[6] = v2;
+        o[7] = vs;
+        if (L) {
+            L[L_V2D] = v2;
+            L[L_STORE] = vs;
+        }
+        E.dt_min = fmin(E.dt_min, E.dt);
+        E.dt_max = fmax(E.dt_max, E.dt);
+    } else {
+        o[5] = S[P_RATE];
+        E.rate = S[P_RATE];
+        const double t = E.t + E.dt;
+        E.t = t;
+        if (pr.snap_k >= 0) {
+            E.snap_t[pr.snap_k] = t;
+            E.k_out = pr.snap_k + 1;
+        }
+        E.steps += 1;
+        E.n_sub_max = max(E.n_sub_max, E.n_sub);
+        if (!isfinite(S[P_HSUM]) || !isfinite(S[P_RATE])) E.status = ST_NONFINITE;
+        else if (S[P_HMAX] > MAX_PLAUSIBLE_DEPTH_2D) E.status = ST_IMPLAUSIBLE;
+        else if (t >= E.t_end - 1e-9) E.status = ST_DONE;
+    }
 }
 
 // Copy the rate of the current state (finalize output, mode 1) into the engine records.

@@ -96,7 +96,7 @@ template <class R, int NT>
 int launch_step_nt(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
     int rc = launch_stages_parted<R, NT>(g, s);
     if (rc) return rc;
-    finalize_kernel<R><<<g->n, 32, 0, s>>>(reinterpret_cast<const Grid<R>*>(g->d_grids), g->d_params, g->c,
+    finalize_kernel<R><<<g->n, FIN_THREADS, 0, s>>>(reinterpret_cast<const Grid<R>*>(g->d_grids), g->d_params, g->c,
                                            g->d_partials, g->d_out, 0, ext, ledger);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
@@ -110,7 +110,7 @@ int launch_reduce(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
         strip_rate_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
     else
         strip_reduce_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
-    finalize_kernel<R><<<g->n, 32, 0, s>>>(grids, g->d_params, g->c, g->d_partials, g->d_out, rate_only ? 2 : 1,
+    finalize_kernel<R><<<g->n, FIN_THREADS, 0, s>>>(grids, g->d_params, g->c, g->d_partials, g->d_out, rate_only ? 2 : 1,
                                            ext);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
@@ -259,7 +259,7 @@ int eng_enqueue_nt(his_grid* g, his_engine* E, int chain, int n_steps) {
         int rc = launch_stages<R, NT>(g, s_main, t0, tc);
         if (rc) return rc;
         if (E->net) HIS_CK(cudaStreamWaitEvent(s_main, join, 0));
-        eng_post_kernel<R><<<mc, 32, 0, s_main>>>(E->d_em, g->d_params, grids, g->c, g->d_partials,
+        eng_post_kernel<R><<<mc, FIN_THREADS, 0, s_main>>>(E->d_em, g->d_params, grids, g->c, g->d_partials,
                                                   E->net ? E->d_vol1d : nullptr, g->d_out, m0);
         HIS_CK(cudaGetLastError());
     }
@@ -319,7 +319,7 @@ int eng_profile_nt(his_grid* g, his_engine* E, int n_steps, double* ms) {
         }
         cudaEventRecord(ev[3], E->s0);
         if (E->net) cudaStreamWaitEvent(E->s0, ev[5], 0);
-        eng_post_kernel<R><<<E->n, 32, 0, E->s0>>>(E->d_em, g->d_params, grids, g->c, g->d_partials,
+        eng_post_kernel<R><<<E->n, FIN_THREADS, 0, E->s0>>>(E->d_em, g->d_params, grids, g->c, g->d_partials,
                                                    E->net ? E->d_vol1d : nullptr, g->d_out, 0);
         cudaEventRecord(ev[6], E->s0);
         cudaError_t ce = cudaEventSynchronize(ev[6]);
@@ -368,8 +368,8 @@ __global__ void noalloc_setup_kernel(Grid<R> G, StepParams P, NoallocPlan L, uns
 }
 
 // One step of one grid with every table and stage buffer in the scratch at `base`
-// (laid out by L): the same strip kernels, decomposition (58-column strips, 48-row
-// chunks) and fixed-order totals as a one-member set created with default tiles.
+// (laid out by L): the same stage kernels, decomposition and fixed-order totals as a
+// one-member set created with default tiles.
 template <class R>
 int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_params& p, const NoallocPlan& L,
                       unsigned char* base, cudaStream_t s) {
@@ -417,7 +417,7 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
         launch_stage<R, NT, 0>(grid, strips, params, kc, part, L.n_strips, smem, s);
         stage_copy_kernel<R><<<L.n_strips, CHUNK_THREADS, 0, s>>>(grid, strips, params);
     }
-    finalize_kernel<R><<<1, 32, 0, s>>>(grid, params, c, part, out, 0, nullptr);
+    finalize_kernel<R><<<1, FIN_THREADS, 0, s>>>(grid, params, c, part, out, 0, nullptr);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
 }
