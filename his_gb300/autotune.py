@@ -1,7 +1,7 @@
 """Work-decomposition tuner of the 2-D stage kernels.
 
 The strip kernels split every member's grid into strips of at most ``tile_x``
-columns (CTAs of 64, 128, 224 or 352 threads for up to 58, 122, 218 or 346
+columns (float32: CTAs of 64, 128, 224 or 352 threads for up to 58, 122, 218 or 346
 columns) and chunks of at most ``tile_y`` rows (``his_grid_create``).  The fastest split depends on the
 grid sizes, the batch and the precision: narrow strips recompute more halo
 columns, short chunks more halo rows, and the number of strip-chunks decides how
@@ -241,7 +241,7 @@ def choose_tile_engine(storms, cfg, precision: str, device: torch.device, couple
     dtype = torch.float64 if precision == "fp64" else torch.float32
     prec = _lib.PREC_F64 if precision == "fp64" else _lib.PREC_F32
     shapes = [(int(s.terrain.ny), int(s.terrain.nx)) for s in storms]
-    key = tune_key(device, prec, int(cfg.spatial_order), shapes) + f"|engine|coupled{int(bool(couple))}"
+    key = tune_key(device, prec, int(cfg.spatial_order), shapes) + f"|engine|coupled{int(bool(couple))}|library"
     with _LOCK:
         if use_cache:
             if key in _MEM:
@@ -250,7 +250,8 @@ def choose_tile_engine(storms, cfg, precision: str, device: torch.device, couple
             if hit:
                 _MEM[key] = tuple(hit["tile"])
                 return _MEM[key]
-    cands = [t for t in candidates(shapes) if t[0] in ENGINE_CANDIDATES_X]
+    # (0, 0): the library's own choice, finer than the listed ones for small batches
+    cands = [(0, 0)] + [t for t in candidates(shapes) if t[0] in ENGINE_CANDIDATES_X]
     zcache: dict = {}
     members = [Member(s, dtype, device, couple, False, zcache) for s in storms]
     stream = torch.cuda.current_stream(device)

@@ -93,6 +93,50 @@ static int check_async_out(const void* p, const char* what, bool* direct) {
 // 128, 224 or 352 threads, see strip_threads), chunks of ty rows.
 bool tile_supported(int tx, int ty) { return tx >= 1 && strip_threads(tx) > 0 && ty >= 1 && ty <= 1 << 20; }
 
+// The decomposition is the one with the smallest estimated step time, from two models
+// fitted to measured sweeps of 100 x 81 to 1601 x 1301 grids, 1 to 64 members (a fixed
+// 58 x 48 left most SMs without work below about 20 members of 400 x 325 cells):
+//  * float64 (sub-tiles): an SM works off its strip-chunks one after the other at the rate
+//    of its FP64 pipe, so the time is that of the SM with the most chunks: FP64
+//    instructions of a chunk (faces, halo cells, slopes, updates) x ceil(chunks / 152).
+//    Picks 10 x 6 for 100 x 81 (56 us per step against 516 with 58 x 48), 25 x 10 for
+//    163 x 201, 58 x 16 for 400 x 325 (249 against 690);
+//  * float32 (marching strips): a chunk takes (rows + 6) row times, a row 1.6 us while an
+//    SM holds few CTAs and 0.4 + 0.28 us x CTAs per SM beyond.  Picks 58 x 2 for 100 x 81
+//    (31 us against 95), 58 x 4 for 400 x 325 (43 against 106), 58 x 8 for 4 members (58
+//    against 107), 58 x 24 to 64 for 16 to 64.
+void default_tile(int prec, int order, int n, const his_grid_desc* grids, int* tx, int* ty) {
+    constexpr double SMS = 152.0;
+    const int w64[] = {58, 50, 41, 34, 29, 25, 20, 17, 13, 10, 8}, w32[] = {58};
+    const int h64[] = {16, 12, 10, 8, 6, 4, 3, 2};
+    const int h32[] = {64, 48, 40, 32, 28, 24, 20, 16, 14, 12, 10, 8, 6, 4, 3, 2};
+    const bool f64 = prec == HIS_PREC_F64;
+    const int nw = f64 ? 11 : 1, nh = f64 ? 8 : 16;
+    double best = INFINITY;
+    for (int a = 0; a < nw; ++a)
+        for (int b = 0; b < nh; ++b) {
+            const int tw = f64 ? w64[a] : w32[a], th = f64 ? h64[b] : h32[b];
+            double chunks = 0.0, work = 0.0, t;
+            int hmax = 0;
+            for (int m = 0; m < n; ++m) {
+                const int ns = (grids[m].nx + tw - 1) / tw, nch = (grids[m].ny + th - 1) / th;
+                const double w = (grids[m].nx + ns - 1) / ns, h = (grids[m].ny + nch - 1) / nch;
+                const double faces = (w + 3) * h + (w + 1) * 2 + (h + 3) * w + (h + 1) * 2;
+                const double slopes = order == 2 ? (w + 4) * (h + 2) + (w + 2) * (h + 4) : 0.0;
+                chunks += (double)ns * nch;
+                work += (double)ns * nch * (order * (90 * faces + 12 * (w + 6) * (h + 6)) + 8 * slopes + 190 * w * h);
+                hmax = std::max(hmax, (int)h);
+            }
+            if (f64) t = std::ceil(chunks / SMS) * (work / chunks);
+            else t = (hmax + 6) * std::max(1.6, 0.4 + 0.28 * chunks / SMS);
+            if (t < best) {
+                best = t;
+                *tx = tw;
+                *ty = th;
+            }
+        }
+}
+
 Consts to_consts(const his_solver_cfg* c) {
     Consts k{};
     k.g = c->g; k.h_dry = c->h_dry; k.kp_eps = c->kp_eps; k.cfl = c->cfl; k.dt_min = c->dt_min; k.dt_max = c->dt_max;
@@ -155,6 +199,7 @@ int32_t his_grid_create(int32_t precision, const his_solver_cfg* cfg, int32_t n_
     if (rc) return rc;
     if (precision != HIS_PREC_F64 && precision != HIS_PREC_F32) return bad("precision must be 0 (f64) or 1 (f32)");
     if (n_members <= 0 || !grids) return bad("need at least one grid member");
+    const bool own_tile = tile_x == 0 && tile_y == 0;       // chosen below, once the sizes are checked
     if (tile_x == 0) tile_x = 58;
     if (tile_y == 0) tile_y = 48;
     if (!tile_supported(tile_x, tile_y)) return bad("unsupported work decomposition (strip width 1..346, rows >= 1)");
@@ -171,6 +216,7 @@ int32_t his_grid_create(int32_t precision, const his_solver_cfg* cfg, int32_t n_
         int nh = (d.f0 != nullptr) + (d.fc != nullptr) + (d.k != nullptr);
         if (nh != 0 && nh != 3) return bad(who + "f0, fc and k must be given together");
     }
+    if (own_tile) default_tile(precision, cfg->order, n_members, grids, &tile_x, &tile_y);
     his_grid* g = new his_grid();
     g->prec = precision;
     g->c = to_consts(cfg);

@@ -24,7 +24,7 @@ struct HostStage {
 struct his_grid {
     int prec = 0;
     his::Consts c{};
-    int n = 0, tx = 58, ty = 48, nt = 64, device = 0;   // strip width, rows per chunk, threads per CTA
+    int n = 0, tx = 0, ty = 0, nt = 64, device = 0;     // strip width, rows per chunk, threads per CTA
     std::vector<his_grid_desc> desc;
     std::vector<int> tile0, ntile;
     void* d_grids = nullptr;                 // his::Grid<R>[n]
@@ -147,12 +147,13 @@ bool tile_supported(int tx, int ty);
 inline int strip_threads(int tx) {
     return tx <= 58 ? 64 : tx <= 122 ? 128 : tx <= 218 ? 224 : tx <= 346 ? 352 : 0;
 }
+// Work decomposition for these grids where the caller leaves it to the library (capi.cu)
+void default_tile(int prec, int order, int n, const his_grid_desc* grids, int* tx, int* ty);
 int check_cfg(const his_solver_cfg* c);
 Consts to_consts(const his_solver_cfg* c);
 
-// Layout of the no-allocation 2-D step's scratch (noalloc.cu): one grid in strips of
-// up to 58 columns and chunks of up to 48 rows, every offset a multiple of 256 bytes
-// from the scratch base.
+// Layout of the no-allocation 2-D step's scratch (noalloc.cu): one grid in the strips and
+// chunks of a one-member set, every offset a multiple of 256 bytes from the scratch base.
 struct NoallocPlan {
     int ns, w, nch, hch, n_strips, pad;
     size_t plane;                       // one (ny, nx) plane of the compute type

@@ -110,14 +110,15 @@ static int noalloc_base(unsigned char** out) {
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Strips of up to 58 columns and chunks of up to 48 rows (the grid set's defaults),
-// then the scratch regions: three stage planes, partial sums, strip table, grid
-// record, step parameters, totals.
-static NoallocPlan noalloc_plan(int ny, int nx, size_t elem) {
+// The decomposition of a one-member grid set (default_tile), or, where its partial sums and
+// strip records would not fit the scratch beside the stage planes, strips of up to 58
+// columns and chunks of up to 48 rows; then the scratch regions: three stage planes,
+// partial sums, strip table, grid record, step parameters, totals.
+static NoallocPlan noalloc_plan(int ny, int nx, size_t elem, int tx, int ty) {
     NoallocPlan L{};
-    L.ns = (nx + 57) / 58;
+    L.ns = (nx + tx - 1) / tx;
     L.w = (nx + L.ns - 1) / L.ns;
-    L.nch = (ny + 47) / 48;
+    L.nch = (ny + ty - 1) / ty;
     L.hch = (ny + L.nch - 1) / L.nch;
     L.n_strips = L.ns * L.nch;
     L.plane = align256((size_t)ny * (size_t)nx * elem);
@@ -166,7 +167,10 @@ extern "C" int32_t his_grid_step_noalloc(int32_t precision, const his_solver_cfg
                   "-byte scratch; use his_grid_create for larger grids");
         return HIS_ERR_BAD_ARG;
     }
-    const NoallocPlan L = noalloc_plan(d.ny, d.nx, elem);
+    int tx = 0, ty = 0;
+    default_tile(precision, cfg->order, 1, &d, &tx, &ty);
+    NoallocPlan L = noalloc_plan(d.ny, d.nx, elem, tx, ty);
+    if (L.total > (size_t)HIS_NOALLOC_SCRATCH_BYTES) L = noalloc_plan(d.ny, d.nx, elem, 58, 48);
     if (L.total > (size_t)HIS_NOALLOC_SCRATCH_BYTES) {
         set_error("his_grid_step_noalloc: a " + std::to_string(d.ny) + " x " + std::to_string(d.nx) +
                   " grid needs " + std::to_string(L.total) + " bytes of scratch, more than the " +

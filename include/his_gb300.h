@@ -79,8 +79,8 @@ int32_t his_version(void);
 const char* his_last_error(void);
 
 /* Create a set of n_members 2-D grids computed in `precision`.  The stencil kernels
- * march up strips of at most tile_x columns (1..346) in chunks of tile_y rows
- * (0, 0 = defaults 58 x 48); the set allocates its own stage scratch.
+ * work on strips of at most tile_x columns (1..346) in chunks of at most tile_y rows
+ * (0, 0 = chosen by the grids' sizes, their number and the precision); the set allocates its own stage scratch.
  * Replaces hydrointel/solver/swe2d.py:113-146 (SWE2D constructor, batched form). */
 int32_t his_grid_create(int32_t precision, const his_solver_cfg* cfg, int32_t n_members, const his_grid_desc* grids,
                         int32_t tile_x, int32_t tile_y, his_grid** out);
@@ -158,7 +158,9 @@ int32_t his_grid_volumes(his_grid* grid, double* vols, void* stream);
  * for his_grid_create, in `precision`; params is one step's forcing; the stage buffers,
  * partial sums and tables live in a fixed library array of HIS_NOALLOC_SCRATCH_BYTES
  * bytes.  Same kernels, decomposition and results as a one-member grid set created
- * with default tiles.  Grids too large for the array return HIS_ERR_BAD_ARG.  The first
+ * with default tiles (58 x 48 chunks where the tables of finer ones would not fit beside
+ * the stage buffers: the totals' summation order then differs, no cell's value does).
+ * Grids too large for the array return HIS_ERR_BAD_ARG.  The first
  * call in each CUDA context (the device's primary context, or one the application made
  * current itself; a context made after cudaDeviceReset counts as new) looks up the
  * array's address in that context and should come before any stream capture.  Calls
