@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "his_internal.h"
@@ -717,9 +718,9 @@ int32_t his_links_create(his_grid* grid, his_net* net, int32_t n_members, const 
     if (n_members != grid->n || n_members != net->n)
         return bad("links, grid and network must have the same number of members");
     Arena ar;
-    struct Offs { size_t c1, inv, uq, zb, len, z2, us, ui, cs, ci, zbf, lenf, z2f; };
+    struct Offs { size_t c1, inv, uq, orig, zb, len, z2, us, ui, uf, cs, zbf, lenf, z2f; };
     std::vector<Offs> offs(n_members);
-    size_t smem = 0;
+    size_t smem = 0, smem64 = 0, smem32 = 0;
     int total = 0;
     for (int mb = 0; mb < n_members; ++mb) {
         const his_links_desc& d = links[mb];
@@ -741,25 +742,37 @@ int32_t his_links_create(his_grid* grid, his_net* net, int32_t n_members, const 
         std::vector<int> us, ui, cs, ci;
         build_csr(d.inv, d.n_links, d.n_unique, us, ui);
         build_csr(d.cell1d, d.n_links, nc, cs, ci);
-        Offs& o = offs[mb];
-        const size_t L = sizeof(double) * d.n_links;
-        o.c1 = ar.add(d.cell1d, sizeof(int32_t) * d.n_links);
-        o.inv = ar.add(d.inv, sizeof(int32_t) * d.n_links);
-        o.uq = ar.add(uq.data(), sizeof(int32_t) * uq.size());
-        o.zb = ar.add(d.zbank, L); o.len = ar.add(d.length, L); o.z2 = ar.add(d.z2, L);
-        auto addf = [&](const double* a) {
-            std::vector<float> f(a, a + d.n_links);
-            return ar.add(f.data(), sizeof(float) * f.size());
+        // links in the order of their 1-D cell; a 2-D cell's links keep the caller's order
+        std::vector<int> pos(d.n_links);
+        for (int p = 0; p < d.n_links; ++p) pos[ci[p]] = p;
+        for (int& l : ui) l = pos[l];
+        auto by_cell = [&](const auto* a) {
+            std::vector<std::decay_t<decltype(*a)>> v(d.n_links);
+            for (int p = 0; p < d.n_links; ++p) v[p] = a[ci[p]];
+            return v;
         };
-        o.zbf = addf(d.zbank); o.lenf = addf(d.length); o.z2f = addf(d.z2);
-        o.us = ar.add(us.data(), sizeof(int) * us.size()); o.ui = ar.add(ui.data(), sizeof(int) * ui.size());
-        o.cs = ar.add(cs.data(), sizeof(int) * cs.size()); o.ci = ar.add(ci.data(), sizeof(int) * ci.size());
-        smem = std::max(smem, exchange_smem_bytes(d.n_links, d.n_unique, nc));
+        auto put = [&](const auto& v) { return ar.add(v.data(), sizeof(v[0]) * v.size()); };
+        auto put_f = [&](const std::vector<double>& v) { return put(std::vector<float>(v.begin(), v.end())); };
+        Offs& o = offs[mb];
+        const std::vector<double> zb = by_cell(d.zbank), len = by_cell(d.length), z2 = by_cell(d.z2);
+        o.c1 = put(by_cell(d.cell1d)); o.inv = put(by_cell(d.inv));
+        o.uq = put(uq); o.orig = put(ci);
+        o.zb = put(zb); o.len = put(len); o.z2 = put(z2);
+        o.zbf = put_f(zb); o.lenf = put_f(len); o.z2f = put_f(z2);
+        std::vector<int> uf(d.n_unique);
+        for (int k = 0; k < d.n_unique; ++k) uf[k] = us[k + 1] - us[k] == 1 ? ui[us[k]] : -1;
+        o.us = put(us); o.ui = put(ui); o.uf = put(uf); o.cs = put(cs);
+        // (links per member are limited by one block's shared memory, as they were when sign
+        // and volume of a link were separate)
+        smem = std::max(smem, sizeof(double) * (2 * (size_t)d.n_links + 2 * (size_t)d.n_unique + (size_t)nc + 64));
+        smem64 = std::max(smem64, exchange_smem_bytes(d.n_links, d.n_unique, nc, 8));
+        smem32 = std::max(smem32, exchange_smem_bytes(d.n_links, d.n_unique, nc, 4));
         total += d.n_links;
     }
     if (smem > 200 * 1024) return bad("too many links for one thread block's shared memory");
     his_links* Lk = new his_links();
-    Lk->grid = grid; Lk->net = net; Lk->n = n_members; Lk->total_links = total; Lk->smem = smem;
+    Lk->grid = grid; Lk->net = net; Lk->n = n_members; Lk->total_links = total;
+    Lk->smem64 = smem64; Lk->smem32 = smem32;
     auto fail = [&](cudaError_t e, const char* w) { int r = cuda_fail(e, w); his_links_destroy(Lk); return r; };
     cudaError_t e = cudaMalloc(&Lk->d_arena, ar.host.size() ? ar.host.size() : 256);
     if (e == cudaSuccess) e = cudaMemcpy(Lk->d_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice);
@@ -779,7 +792,8 @@ int32_t his_links_create(his_grid* grid, his_net* net, int32_t n_members, const 
         L.zbank_f = (const float*)(base + o.zbf); L.length_f = (const float*)(base + o.lenf);
         L.z2_f = (const float*)(base + o.z2f);
         L.ustart = (const int*)(base + o.us); L.uidx = (const int*)(base + o.ui);
-        L.cstart = (const int*)(base + o.cs); L.cidx = (const int*)(base + o.ci);
+        L.ufirst = (const int*)(base + o.uf);
+        L.cstart = (const int*)(base + o.cs); L.orig = (const int*)(base + o.orig);
     }
     e = cudaMalloc(&Lk->d_links, sizeof(Lnk) * n_members);
     if (e == cudaSuccess) e = cudaMemcpy(Lk->d_links, H.data(), sizeof(Lnk) * n_members, cudaMemcpyHostToDevice);
@@ -978,7 +992,7 @@ int32_t his_engine_create(his_grid* grid, his_net* net, his_links* links, int32_
     his_engine* E = new his_engine();
     E->grid = grid; E->net = net; E->links = links; E->n = n_members; E->max_sub = max_sub;
     E->graph_steps = graph_steps;
-    E->pre_smem = std::max<size_t>(links ? links->smem : 0, sizeof(double) * 64);
+    E->pre_smem = links ? links->smem_of(grid->prec == HIS_PREC_F64 ? 8 : 4) : 0;
     auto fail = [&](cudaError_t e, const char* w) { int r = cuda_fail(e, w); his_engine_destroy(E); return r; };
     cudaError_t e = cudaMalloc(&E->d_arena, std::max<size_t>(ar.host.size(), 256));
     if (e == cudaSuccess && ar.host.size())

@@ -17,101 +17,135 @@
 
 namespace his {
 
-// threads of the per-member pre-step CTA.  1024 cut the pre kernel of a 400 x 325
-// member from 38.6 to 28.7 us, but a CTA that size holds a whole SM's registers while
-// it runs, and with member chains side by side the step got slower (0.509 against
-// 0.466 ms); threads 32..40 evaluate the step parameters
-constexpr int ENG_PRE_THREADS = 512;
-static_assert(ENG_PRE_THREADS >= 64 && ENG_PRE_THREADS <= 1024, "pre-step CTA size");
-
-__host__ __device__ inline size_t eng_pre_smem_bytes(size_t exchange_bytes) {
-    size_t r = sizeof(double) * 64;
-    return exchange_bytes > r ? exchange_bytes : r;
-}
+// The per-member pre-step CTA: warps 0 .. 13 exchange water with the channel, warp 14 chooses
+// dt and the substep count and evaluates the substep forcing, warp 15 the step's
+// parameters, side by side (a float64 cosine or division is a chain of hundreds to
+// thousands of cycles, and the exchange is a chain of load latencies).
+constexpr int ENG_PRE_THREADS = 512, ENG_EXCH_THREADS = 448, ENG_EXCH_WARPS = ENG_EXCH_THREADS / 32;
 
 template <class R>
-__global__ void eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params,
-                               const Grid<R>* __restrict__ grids, const Net* __restrict__ nets,
-                               const Lnk* __restrict__ links, Consts c, double* __restrict__ netf, int max_sub,
-                               double* __restrict__ exch, int m0) {
+__global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_pre_kernel(EngMember* __restrict__ em,
+                                                                  StepParams* __restrict__ params,
+                                                                  const Grid<R>* __restrict__ grids,
+                                                                  const Net* __restrict__ nets,
+                                                                  const Lnk* __restrict__ links, Consts c, ExchK<R> K,
+                                                                  double* __restrict__ netf, int max_sub,
+                                                                  double* __restrict__ exch, int m0) {
     extern __shared__ double sm[];
-    __shared__ int s_go, s_nsub, s_snap;
+    __shared__ Lnk s_L;
+    __shared__ Net s_N;
+    __shared__ int s_nsub, s_snap;
     __shared__ double s_dt;
-    const int m = m0 + blockIdx.x;
+    __shared__ R s_dtr, s_rate[ENG_EXCH_WARPS];
+    const int m = m0 + blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     EngMember& E = em[m];
-    if (threadIdx.x == 0) {
-        s_go = E.status == ST_RUNNING;
-        if (!s_go) params[m].active = 0;
-        double rate = E.rate;
-        double dt = rate > 0.0 ? c.cfl / rate : c.dt_max;
-        if (dt < c.dt_min || dt > c.dt_max) {
-            if (dt < c.dt_min && s_go) E.n_clamped++;
-            dt = fmin(fmax(dt, c.dt_min), c.dt_max);
-        }
-        // the step ends at the member's end or its next output time (coupling.py:255-262)
-        double limit = E.t_end;
-        const bool out_on = E.n_out > 0 && E.k_out < E.n_out;
-        const double t_next = out_on ? E.out_dt * E.k_out : 0.0;
-        if (out_on) limit = fmin(limit, t_next);
-        s_dt = fmin(dt, limit - E.t);
-        s_snap = out_on && E.t + s_dt >= t_next - 1e-9 ? E.k_out : -1;
-        s_nsub = 0;
+    StepParams& P = params[m];
+    if (E.status != ST_RUNNING) {              // (every thread reads it before any barrier)
+        if (tid == 0) P.active = 0;
+        return;
     }
-    __syncthreads();
-    if (!s_go) return;
-    const double dt = s_dt;
-    if (nets) {
-        double r1 = 0.0;
-        bool wet = false;
-        if constexpr (sizeof(R) == 4) net_rate_dev_f32(nets[m], c, r1, wet, sm);
-        else net_rate_dev(nets[m], c, r1, wet, sm);
-        if (threadIdx.x == 0) {
-            const double dt1 = wet ? fmin(c.cfl_1d / r1, c.dt_max) : c.dt_max;
-            const double ns = ceil(dt / dt1 - 1e-9);
-            s_nsub = ns < 1.0 ? 1 : (ns > (double)max_sub ? max_sub + 1 : (int)ns);
+    if (nets) stage_record(&s_N, nets + m);
+    if (links) stage_record(&s_L, links + m);
+    // barriers of the whole CTA, reached from the roles' own code
+    auto all = [] { bar_group(1, ENG_PRE_THREADS); };
+    all();
+    if (tid < ENG_EXCH_THREADS) {
+        auto ready = [&] { all(); return s_dtr; };
+        auto go = [&] { all(); return s_nsub <= max_sub; };
+        if (links) {
+            exchange_dev<R>(s_L, s_N, grids[m], K, nullptr, exch, m, sm, tid, ENG_EXCH_THREADS, s_rate,
+                            [] { bar_group(2, ENG_EXCH_THREADS); }, ready, go);
+        } else {
+            R rate = R(-1);
+            if (nets)
+                for (int i = tid; i < s_N.n_cells; i += ENG_EXCH_THREADS) {
+                    const CellLevel<R> o = cell_level(s_N, i, K.g, K.h_dry, true);
+                    if (o.wet) rate = rate > o.rate ? rate : o.rate;
+                }
+            for (int o = 16; o > 0; o >>= 1) {
+                const R w = __shfl_xor_sync(0xffffffffu, rate, o);
+                rate = w > rate ? w : rate;
+            }
+            if (lane == 0) s_rate[tid >> 5] = rate;
+            ready();
+            go();
         }
-        __syncthreads();
-        if (s_nsub > max_sub) {
-            if (threadIdx.x == 0) {
+        return;
+    }
+    if (tid < ENG_EXCH_THREADS + 32) {
+        if (lane == 0) {
+            const double rate = E.rate;
+            double dt = rate > 0.0 ? c.cfl / rate : c.dt_max;
+            if (dt < c.dt_min || dt > c.dt_max) {
+                if (dt < c.dt_min) E.n_clamped++;
+                dt = fmin(fmax(dt, c.dt_min), c.dt_max);
+            }
+            // the step ends at the member's end or its next output time (coupling.py:255-262)
+            double limit = E.t_end;
+            const bool out_on = E.n_out > 0 && E.k_out < E.n_out;
+            const double t_next = out_on ? E.out_dt * E.k_out : 0.0;
+            if (out_on) limit = fmin(limit, t_next);
+            dt = fmin(dt, limit - E.t);
+            s_dt = dt;
+            s_dtr = (R)dt;
+            s_snap = out_on && E.t + dt >= t_next - 1e-9 ? E.k_out : -1;
+        }
+        __syncwarp();
+        all();                                   // dt is chosen, the channel rates are in s_rate
+        if (lane == 0) {
+            int n = 0;
+            if (nets) {
+                R r1 = s_rate[0];
+                for (int w = 1; w < ENG_EXCH_WARPS; ++w) r1 = s_rate[w] > r1 ? s_rate[w] : r1;
+                const double dt1 = r1 >= R(0) ? fmin(c.cfl_1d / (double)r1, c.dt_max) : c.dt_max;
+                const double ns = ceil(s_dt / dt1 - 1e-9);
+                n = ns < 1.0 ? 1 : (ns > (double)max_sub ? max_sub + 1 : (int)ns);
+            }
+            s_nsub = n;
+        }
+        __syncwarp();
+        all();                                   // the substep count is known
+        const int n = s_nsub;
+        if (n > max_sub) {
+            if (lane == 0) {
                 E.status = ST_SUBSTEPS;
-                params[m].active = 0;
+                P.active = 0;
             }
             return;
         }
-        if (links) exchange_dev<R>(links[m], nets[m], grids[m], c, dt, nullptr, exch, m, sm);
-        const double sub = dt / s_nsub;
-        for (int k = threadIdx.x; k < s_nsub; k += blockDim.x) {
+        const double sub = s_dt / n;
+        for (int k = lane; k < n; k += 32) {
             const double tk = E.t + k * sub;
             netf[((size_t)m * max_sub + k) * 2 + 0] = eng_inflow(E, tk);
             netf[((size_t)m * max_sub + k) * 2 + 1] = eng_tide(E, tk);
         }
+        return;
     }
-    // the step's parameters, spread over threads that each write their own fields, so
-    // the float64 forcing (harmonic tides) is evaluated side by side rather than by
-    // one thread: threads 32..35 the edge values at t, 36..39 at t + dt, 40 the rain
-    // (a warp apart from the substep forcing above), thread 0 the rest
-    StepParams& P = params[m];
-    const int tid = threadIdx.x;
-    if (tid >= 32 && tid < 40) {
-        const int e = tid & 3;
-        if (tid < 36) {
-            const double v = eng_edge(E, e, E.t);
-            P.bc0[e] = v;
-            P.bc0_f[e] = (float)v;
-        } else {
-            const double v = eng_edge(E, e, E.t + dt);
-            P.bc1[e] = v;
-            P.bc1_f[e] = (float)v;
-        }
-    } else if (tid == 40) {
-        const double r = eng_rain(E, E.t);
-        P.rain = r;
-        P.rain_f = (float)r;
-    } else if (tid == 0) {
+    all();
+    const double dt = s_dt;
+    // edge values at t by lanes 0..3 and at t + dt by lanes 4..7, rain by lane 8
+    double v = 0.0;
+    if (lane < 8) v = eng_edge(E, lane & 3, lane < 4 ? E.t : E.t + dt);
+    else if (lane == 8) v = eng_rain(E, E.t);
+    __syncwarp();
+    all();
+    if (s_nsub > max_sub) return;
+    if (lane < 4) {
+        P.bc0[lane] = v;
+        P.bc0_f[lane] = (float)v;
+    } else if (lane < 8) {
+        P.bc1[lane & 3] = v;
+        P.bc1_f[lane & 3] = (float)v;
+    } else if (lane == 8) {
+        P.rain = v;
+        P.rain_f = (float)v;
+    } else if (lane == 9) {
         P.dt = dt;
         P.t = E.t;
         P.dt_f = (float)dt;
         P.t_f = (float)E.t;
+        E.dt = dt;
+        E.n_sub = s_nsub;
         P.active = 1;
         const int k = s_snap;
         P.snap_k = k;
@@ -121,8 +155,6 @@ __global__ void eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restric
         P.snap_eta = k >= 0 && E.snap_eta ? E.snap_eta + (size_t)k * E.n1d : nullptr;
         P.snap_q = k >= 0 && E.snap_q ? E.snap_q + (size_t)k * E.n1d : nullptr;
         P.snap_ledger = k >= 0 && E.snap_ledger ? E.snap_ledger + (size_t)k * LEDGER_N : nullptr;
-        E.dt = dt;
-        E.n_sub = s_nsub;
     }
 }
 

@@ -118,6 +118,7 @@ struct Grid {
     R *pk, *ps;                      // optional running peak depth and speed
     R rdx, rdy, rt0;                 // dx, dy, Horton t0 in the compute type
     R idx, idy;                      // 1/dx, 1/dy (the float32 kernels multiply instead of dividing)
+    R rarea;                         // 1 / cell area
 };
 
 // Per-member step parameters, in float64 and (for the float32 kernels, which must not
@@ -412,6 +413,10 @@ __device__ __forceinline__ void face_flux(const KC<float>& c, const Recon& L, co
 __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
+}
+// The same sum at the price of one vote where every lane holds zero
+__device__ __forceinline__ double warp_sum_sparse(double v) {
+    return __any_sync(0xffffffffu, f64_bits(v) << 1 != 0) ? warp_sum(v) : 0.0;
 }
 __device__ __forceinline__ double warp_max(double v) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));

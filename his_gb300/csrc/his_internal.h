@@ -84,7 +84,8 @@ struct his_links {
     double* d_V = nullptr;
     double* h_V = nullptr;
     double* d_exch = nullptr;                // n x 2 running exchange totals
-    size_t smem = 0;
+    size_t smem64 = 0, smem32 = 0;           // shared memory of one member's exchange, by precision
+    size_t smem_of(size_t size) const { return size == 8 ? smem64 : smem32; }
 };
 
 struct his_engine {

@@ -37,12 +37,15 @@ struct Net {
 };
 
 struct Lnk {
+    // Links in the order of their 1-D cell (within a cell in the caller's order), so that a
+    // cell's links are contiguous; orig: the caller's index
     int n_links, n_unique, v_offset, pad;
-    const int *cell1d, *inv, *uniq;
+    const int *cell1d, *inv, *uniq, *orig;
     const double *zbank, *length, *z2;
     const float *zbank_f, *length_f, *z2_f;        // float32 copies for the production form
-    const int *ustart, *uidx;                      // unique 2-D cell -> links (link order)
-    const int *cstart, *cidx;                      // 1-D cell -> links (link order)
+    const int *ustart, *uidx;                      // unique 2-D cell -> links (caller's order)
+    const int *ufirst;                             // its link where it has exactly one, else -1
+    const int *cstart;                             // 1-D cell -> its links
 };
 
 // ---------------------------------------------------------------- sections (swe1d.py:51-84)
@@ -520,279 +523,279 @@ __device__ __forceinline__ void net_substeps_f32_dev(const Net& N, const Consts&
     }
 }
 
-__host__ __device__ inline size_t exchange_smem_bytes(int n_links, int n_unique, int n_cells) {
-    const size_t f64 = sizeof(double) * (2 * (size_t)n_links + 2 * (size_t)n_unique + (size_t)n_cells + 32 * 2);
-    const size_t f32 = sizeof(float) * (2 * (size_t)n_links + 2 * (size_t)n_unique + 4 * (size_t)n_cells) +
-                       sizeof(double) * 32 * 2;
-    return f64 > f32 ? f64 : f32;
+// Shared memory the exchange of one member uses: volumes per link, depth and limit per
+// unique 2-D cell, level (then limit) and storage per 1-D cell, and the reductions.
+__host__ __device__ inline size_t exchange_smem_bytes(int n_links, int n_unique, int n_cells, size_t size) {
+    return sizeof(double) * 96 + size * ((size_t)n_links + 2 * (size_t)n_unique + 2 * (size_t)n_cells);
 }
 
-// Production-form exchange (2-D state in float32): the same steps as the float64
-// form below, in float32 arithmetic from float32 copies of the static link and
-// section tables.  Per 1-D cell the level, plan width and donor volume are formed
-// once; the 1-D area update and the tallies accumulate in float64.
-__device__ __forceinline__ void exchange_dev_f32(const Lnk& L, const Net& N, const Grid<float>& gd, const Consts& c,
-                                                 double dt, double* __restrict__ Vout, double* __restrict__ exch,
-                                                 int mb, double* sm) {
-    const int nl = L.n_links, nu = L.n_unique, nc = N.n_cells, tid = threadIdx.x, nt = blockDim.x;
-    double* red = sm;                                   // 64 doubles
-    float* V = reinterpret_cast<float*>(sm + 64);
-    float *sg = V + nl, *hu_ = sg + nl, *f2 = hu_ + nu, *eta1 = f2 + nu, *plan1 = eta1 + nc, *f1 = plan1 + nc,
-          *avail1 = f1 + nc;
-    __shared__ float s_k[6];
-    if (tid == 0) {
-        s_k[0] = (float)dt;
-        s_k[1] = (float)c.weir_cw;
-        s_k[2] = (float)c.exchange_relax;
-        s_k[3] = (float)c.exchange_limit;
-        s_k[4] = (float)gd.area;
-        s_k[5] = (float)(1.0 / gd.area);
+// Barrier `id` among n threads (whole warps) of a CTA
+__device__ __forceinline__ void bar_group(int id, int n) { asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// What the exchange and the CFL reduction need of one 1-D cell: water level, plan area,
+// volume above the bank, and the wave rate of a wet interior cell (0 otherwise).
+template <class R>
+struct CellLevel {
+    R eta, plan, avail, rate;
+    bool wet;
+};
+
+// Production form: float32 from float32 copies of the section tables.
+__device__ __forceinline__ CellLevel<float> cell_level(const Net& N, int i, float g, float h_dry, bool rate) {
+    CellLevel<float> o;
+    const float A = fmaxf((float)N.A[i], 0.0f);
+    const float b = N.bf[i], m = N.mf[i], yb = N.ybf[i], ts = N.tsf[i], dx = N.dxf[i];
+    const float ab = yb * (b + m * yb);
+    const float y = A <= ab ? 2.0f * A / (b + sqrtf(b * b + 4.0f * m * A)) : yb + (A - ab) / ts;
+    const float top = y <= yb ? b + 2.0f * m * y : ts;
+    o.eta = N.zf[i] + y;
+    o.plan = top * dx;
+    o.avail = fmaxf(A - ab, 0.0f) * dx;
+    o.wet = rate && N.kind[i] <= 1 && y > h_dry;
+    o.rate = o.wet ? (fabsf((float)N.Q[i] / fmaxf(A, 1e-12f)) + sqrtf(g * A / top)) / dx : 0.0f;
+    return o;
+}
+__device__ __forceinline__ CellLevel<double> cell_level(const Net& N, int i, double g, double h_dry, bool rate) {
+    CellLevel<double> o;
+    const Sec s{N.b, N.m, N.yb, N.ts};
+    const double A = N.A[i], dx = N.dx[i];
+    const double y = sec_depth(s, i, A), top = sec_top(s, i, y);
+    o.eta = N.z[i] + y;
+    o.plan = top * dx;
+    o.avail = clamp0(A - sec_bank_area(s, i)) * dx;
+    o.wet = rate && N.kind[i] <= 1 && y > h_dry;
+    o.rate = o.wet ? (fabs(N.Q[i] / fmax(A, 1e-12)) + sqrt(g * A / top)) / dx : 0.0;
+    return o;
+}
+
+// Signed volume of one link over dt before the donor limits (coupling.py:78-97): positive
+// from the 2-D to the 1-D side.  rp: 1 / (2-D cell area) + 1 / (1-D plan area).
+__device__ __forceinline__ float link_volume(float eta1, float eta2, float zb, float len, float rp, float dt, float cw,
+                                             float relax) {
+    const float up = fmaxf(eta1, eta2), dn = fminf(eta1, eta2);
+    const float d_up = fmaxf(up - zb, 0.0f), d_dn = fmaxf(dn - zb, 0.0f);
+    const float ratio = d_up > 0.0f ? d_dn / d_up : 0.0f;
+    const float sub = powf(fmaxf(1.0f - ratio * sqrtf(ratio), 0.0f), 0.385f);
+    const float q = cw * len * (d_up * sqrtf(d_up)) * sub;
+    const float v = fminf(q * dt, relax * ((up - dn) / rp));
+    return eta2 > eta1 ? v : -v;
+}
+// float64: a link whose water stands below its bank moves nothing, so the powers of the
+// weir formula (d^1.5 = d sqrt(d), and pow(., 0.385) only where the weir is submerged) are
+// left to the few links that overtop.
+__device__ __forceinline__ double link_volume(double eta1, double eta2, double zb, double len, double rp, double dt,
+                                              double cw, double relax) {
+    const double up = rmax(eta1, eta2), dn = rmin(eta1, eta2);
+    const double d_up = f64_clamp0(up - zb);
+    if (f64_bits(d_up) == 0) return 0.0;
+    const double d_dn = f64_clamp0(dn - zb);
+    double q = cw * len * (d_up * sqrt(d_up));
+    if (f64_bits(d_dn) != 0) {
+        const double ratio = d_dn / d_up;
+        q = q * pow(f64_clamp0(1.0 - ratio * sqrt(ratio)), 0.385);
     }
-    for (int k = tid; k < nu; k += nt) hu_[k] = gd.h[L.uniq[k]];
+    const double v = rmin(q * dt, relax * ((up - dn) / rp));
+    return eta2 > eta1 ? v : -v;
+}
+
+__device__ __forceinline__ float pos_part(float x) { return fmaxf(x, 0.0f); }
+__device__ __forceinline__ double pos_part(double x) { return f64_relu(x); }
+
+// Constants of the exchange and the channel rate in the compute type, formed on the host
+template <class R>
+struct ExchK {
+    R g, h_dry, cw, relax, limit;
+};
+template <class R>
+inline ExchK<R> make_exch_k(const Consts& c) {
+    return ExchK<R>{(R)c.g, (R)c.h_dry, (R)c.weir_cw, (R)c.exchange_relax, (R)c.exchange_limit};
+}
+
+// A member record copied to shared memory by the CTA (its pointers are read many times)
+template <class T>
+__device__ __forceinline__ void stage_record(T* dst, const T* src) {
+    static_assert(sizeof(T) % 4 == 0, "copied as 32-bit words");
+    for (int k = threadIdx.x; k < (int)(sizeof(T) / 4); k += blockDim.x)
+        reinterpret_cast<unsigned*>(dst)[k] = reinterpret_cast<const unsigned*>(src)[k];
+}
+
+// Weir exchange of one member by nt threads (whole warps, this one tid) of a CTA
+// (coupling.py:73-124), with the 1-D CFL rate of the same cells.  float64 plain method;
+// float32 in the production form (GB300's float64 pipe runs at a small fraction of the
+// float32 rate), with the 1-D area update and the tallies in float64.
+//
+// It is a chain of dependent phases on one SM, bound by the latency of their loads.  So
+// every static table entry and 2-D depth a thread needs is fetched before the first
+// barrier, for EXCH_SLOTS links and 2-D cells per thread at once (more in a loop), and the
+// later phases run from registers and shared memory; links lie in the order of their 1-D
+// cell, so a cell's sum walks contiguous shared memory.  Measured with the pre kernel
+// below, a step of six served storms in float32 89 -> 78 us, one of a 400 x 325 storm in
+// float64 444 -> 313 us.
+//
+// sync: barrier of the nt threads.  ready(): barrier with whoever chooses dt; returns it.
+//  go(): barrier before the states are changed; false leaves them as they are.
+// s_rate (optional): per warp the largest rate of a wet cell, -1 where none is wet.
+constexpr int EXCH_SLOTS = 3;
+template <class R, class Sync, class Ready, class Go>
+__device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const Grid<R>& gd, const ExchK<R>& K,
+                                             double* __restrict__ Vout, double* __restrict__ exch, int mb, double* sm,
+                                             int tid, int nt, R* s_rate, Sync sync, Ready ready, Go go) {
+    constexpr int S = EXCH_SLOTS;
+    constexpr bool F32 = sizeof(R) == 4;
+    const int nl = L.n_links, nu = L.n_unique, nc = N.n_cells;
+    const R area = R(gd.area);
+    double* red = sm;                                   // 64 doubles used
+    R* V = reinterpret_cast<R*>(sm + 96);
+    R *hq = V + nl, *f2 = hq + nu, *eta1 = f2 + nu, *rp = eta1 + nc, *f1 = eta1;
+    auto zbank = [&](int l) -> R { if constexpr (F32) return L.zbank_f[l]; else return L.zbank[l]; };
+    auto length = [&](int l) -> R { if constexpr (F32) return L.length_f[l]; else return L.length[l]; };
+    auto z2 = [&](int l) -> R { if constexpr (F32) return L.z2_f[l]; else return L.z2[l]; };
+
+    int c1[S], q2[S], cell[S], u0[S];
+    R zb[S], len[S], zz[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+        const int k = tid + j * nt;
+        cell[j] = u0[j] = 0;
+        if (k < nu) { cell[j] = L.uniq[k]; u0[j] = L.ufirst[k]; }
+        c1[j] = q2[j] = 0;
+        zb[j] = len[j] = zz[j] = R(0);
+        if (k < nl) { c1[j] = L.cell1d[k]; q2[j] = L.inv[k]; zb[j] = zbank(k); len[j] = length(k); zz[j] = z2(k); }
+    }
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+        const int k = tid + j * nt;
+        if (k < nu) hq[k] = gd.h[cell[j]];
+    }
+    for (int k = tid + S * nt; k < nu; k += nt) hq[k] = gd.h[L.uniq[k]];
+    R rate = R(-1);
     for (int i = tid; i < nc; i += nt) {
-        const float A = fmaxf((float)N.A[i], 0.0f);
-        const float b = N.bf[i], m = N.mf[i], yb = N.ybf[i], ts = N.tsf[i];
-        const float ab = yb * (b + m * yb);
-        const float y = A <= ab ? 2.0f * A / (b + sqrtf(b * b + 4.0f * m * A)) : yb + (A - ab) / ts;
-        eta1[i] = N.zf[i] + y;
-        plan1[i] = (y <= yb ? b + 2.0f * m * y : ts) * N.dxf[i];
-        avail1[i] = fmaxf(A - ab, 0.0f) * N.dxf[i];
+        const CellLevel<R> o = cell_level(N, i, K.g, K.h_dry, s_rate != nullptr);
+        eta1[i] = o.eta;
+        rp[i] = gd.rarea + R(1) / o.plan;
+        if (o.wet) rate = rate > o.rate ? rate : o.rate;
     }
-    __syncthreads();
-    const float dtf = s_k[0], cw = s_k[1], relax = s_k[2], limit = s_k[3], area2 = s_k[4], rarea2 = s_k[5];
-    for (int l = tid; l < nl; l += nt) {
-        const int c1 = L.cell1d[l];
-        const float eta2 = L.z2_f[l] + hu_[L.inv[l]];
-        const float e1 = eta1[c1];
-        const float zb = L.zbank_f[l];
-        const float up = fmaxf(e1, eta2), dn = fminf(e1, eta2);
-        const float d_up = fmaxf(up - zb, 0.0f), d_dn = fmaxf(dn - zb, 0.0f);
-        const float ratio = d_up > 0.0f ? d_dn / d_up : 0.0f;
-        const float sub = powf(fmaxf(1.0f - ratio * sqrtf(ratio), 0.0f), 0.385f);
-        const float q = cw * L.length_f[l] * (d_up * sqrtf(d_up)) * sub;
-        sg[l] = eta2 > e1 ? 1.0f : -1.0f;
-        const float v_eq = (up - dn) / (rarea2 + 1.0f / plan1[c1]);
-        V[l] = fminf(q * dtf, relax * v_eq);
+    if (s_rate) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const R w = __shfl_xor_sync(0xffffffffu, rate, o);
+            rate = w > rate ? w : rate;
+        }
+        if ((tid & 31) == 0) s_rate[tid >> 5] = rate;
     }
-    __syncthreads();
-    // donor limits, aggregated per donor in link order (coupling.py:98-107)
-    for (int k = tid; k < nu; k += nt) {
-        float tot = 0.0f;
-        for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) { int l = L.uidx[j]; tot += sg[l] > 0.0f ? V[l] : 0.0f; }
-        const float avail = limit * hu_[k] * area2;
-        f2[k] = tot > avail ? avail / (tot > 0.0f ? tot : 1.0f) : 1.0f;
+    const R dt = ready();
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+        const int l = tid + j * nt;
+        if (l < nl) V[l] = link_volume(eta1[c1[j]], zz[j] + hq[q2[j]], zb[j], len[j], rp[c1[j]], dt, K.cw, K.relax);
     }
+    for (int l = tid + S * nt; l < nl; l += nt) {
+        const int c = L.cell1d[l];
+        V[l] = link_volume(eta1[c], z2(l) + hq[L.inv[l]], zbank(l), length(l), rp[c], dt, K.cw, K.relax);
+    }
+    sync();
+    // donor limits, aggregated per donor in the caller's link order (coupling.py:98-107)
+    auto limit2 = [&](int k, int one) {
+        R tot = R(0);
+        if (one >= 0) tot = pos_part(V[one]);
+        else
+            for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) tot += pos_part(V[L.uidx[j]]);
+        const R avail = K.limit * hq[k] * area;
+        f2[k] = tot > avail ? avail / (tot > R(0) ? tot : R(1)) : R(1);
+    };
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+        if (tid + j * nt < nu) limit2(tid + j * nt, u0[j]);
+    for (int k = tid + S * nt; k < nu; k += nt) limit2(k, L.ufirst[k]);
     for (int i = tid; i < nc; i += nt) {
-        float tot = 0.0f;
-        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) { int l = L.cidx[j]; tot += sg[l] < 0.0f ? V[l] : 0.0f; }
-        const float avail = limit * avail1[i];
-        f1[i] = tot > avail ? avail / (tot > 0.0f ? tot : 1.0f) : 1.0f;
+        R tot = R(0);
+        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) tot += pos_part(-V[j]);
+        const R avail = K.limit * (tot > R(0) ? cell_level(N, i, K.g, K.h_dry, false).avail : R(0));
+        f1[i] = tot > avail ? avail / (tot > R(0) ? tot : R(1)) : R(1);
     }
-    __syncthreads();
-    float ex0 = 0.0f, ex1 = 0.0f;
-    for (int l = tid; l < nl; l += nt) {
-        const float v = (sg[l] > 0.0f ? V[l] * f2[L.inv[l]] : V[l] * f1[L.cell1d[l]]) * sg[l];
+    sync();
+    R ex0 = R(0), ex1 = R(0);
+    auto settle = [&](int l, int k, int c) {
+        const R v0 = V[l], v = v0 > R(0) ? v0 * f2[k] : v0 * f1[c];
         V[l] = v;
-        if (Vout) Vout[L.v_offset + l] = (double)v;
-        ex0 += fmaxf(v, 0.0f);
-        ex1 += fmaxf(-v, 0.0f);
-    }
-    __syncthreads();
-    // apply: 2-D through the unique cells, momentum kept only for water that stays
-    for (int k = tid; k < nu; k += nt) {
-        float d = 0.0f;
-        for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) d += V[L.uidx[j]];
-        const float hu0 = hu_[k];
-        const float hn = hu0 - d * rarea2;
-        const float keep = hu0 > 0.0f ? fminf(hn / hu0, 1.0f) : 0.0f;
-        const int idx = L.uniq[k];
+        if (Vout) Vout[L.v_offset + L.orig[l]] = (double)v;
+        ex0 += pos_part(v);
+        ex1 += pos_part(-v);
+    };
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+        if (tid + j * nt < nl) settle(tid + j * nt, q2[j], c1[j]);
+    for (int l = tid + S * nt; l < nl; l += nt) settle(l, L.inv[l], L.cell1d[l]);
+    if (!go()) return;
+    // apply: 2-D through the unique cells, momentum kept only for water that stays (a cell
+    // that gains and loses nothing keeps what it has)
+    auto apply = [&](int k, int idx, int one) {
+        R d = R(0);
+        if (one >= 0) d = V[one];
+        else
+            for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) d += V[L.uidx[j]];
+        const R h0 = hq[k];
+        if (d == R(0) && h0 > R(0)) return;
+        R hn, keep;
+        if constexpr (F32) {
+            hn = h0 - d * gd.rarea;
+            keep = h0 > 0.0f ? fminf(hn / h0, 1.0f) : 0.0f;
+        } else {
+            hn = h0 - d / area;
+            keep = h0 > 0.0 ? fmin(hn / h0, 1.0) : 0.0;
+        }
         gd.h[idx] = hn;
         gd.hu[idx] = gd.hu[idx] * keep;
         gd.hv[idx] = gd.hv[idx] * keep;
-    }
+    };
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+        if (tid + j * nt < nu) apply(tid + j * nt, cell[j], u0[j]);
+    for (int k = tid + S * nt; k < nu; k += nt) apply(k, L.uniq[k], L.ufirst[k]);
     for (int i = tid; i < nc; i += nt) {
-        float d = 0.0f;
-        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) d += V[L.cidx[j]];
-        if (d != 0.0f) N.A[i] = N.A[i] + (double)(d / N.dxf[i]);
+        R d = R(0);
+        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) d += V[j];
+        if (d != R(0)) {
+            if constexpr (F32) N.A[i] = N.A[i] + (double)(d / N.dxf[i]);
+            else N.A[i] = N.A[i] + d / N.dx[i];
+        }
     }
-    double ex[2] = {(double)ex0, (double)ex1};
-    block_sum<2>(ex, red);
-    if (tid == 0 && exch) {
-        exch[mb * 2 + 0] += ex[0];
-        exch[mb * 2 + 1] += ex[1];
+    if (!exch) return;
+    // tallies in float64: lanes, then warps in order
+    const double e0 = warp_sum_sparse((double)ex0), e1 = warp_sum_sparse((double)ex1);
+    if ((tid & 31) == 0) {
+        red[2 * (tid >> 5)] = e0;
+        red[2 * (tid >> 5) + 1] = e1;
     }
-    __syncthreads();
-}
-
-// Weir exchange for one member per CTA, float64 plain method (coupling.py:73-124).
-// V: per-link volumes at lnk.v_offset; exch: per member (2-D -> 1-D total,
-// 1-D -> 2-D total).
-__device__ __forceinline__ void exchange_dev_f64(const Lnk& L, const Net& N, const Grid<double>& gd, const Consts& c,
-                                                 double dt, double* __restrict__ Vout, double* __restrict__ exch,
-                                                 int mb, double* sm) {
-    using R = double;
-    const int nl = L.n_links, nu = L.n_unique, nc = N.n_cells, tid = threadIdx.x, nt = blockDim.x;
-    double *V = sm, *sg = V + nl, *hu_ = sg + nl, *f2 = hu_ + nu, *f1 = f2 + nu, *red = f1 + nc;
-    const Sec s{N.b, N.m, N.yb, N.ts};
-    const double area2 = gd.area;
-    for (int k = tid; k < nu; k += nt) hu_[k] = (double)gd.h[L.uniq[k]];
-    __syncthreads();
-    for (int l = tid; l < nl; l += nt) {
-        const int c1 = L.cell1d[l];
-        const double h2 = hu_[L.inv[l]];
-        const double eta2 = L.z2[l] + h2;
-        const double y1 = sec_depth(s, c1, N.A[c1]);
-        const double eta1 = N.z[c1] + y1;
-        const double zb = L.zbank[l];
-        const double up = rmax(eta1, eta2), dn = rmin(eta1, eta2);
-        const double d_up = clamp0(up - zb), d_dn = clamp0(dn - zb);
-        const double ratio = d_up > 0.0 ? d_dn / d_up : 0.0;
-        const double q = c.weir_cw * L.length[l] * pow(d_up, 1.5) * pow(clamp0(1.0 - pow(ratio, 1.5)), 0.385);
-        sg[l] = eta2 > eta1 ? 1.0 : -1.0;
-        double v = q * dt;
-        const double plan1 = (y1 <= N.yb[c1] ? N.b[c1] + 2.0 * N.m[c1] * y1 : N.ts[c1]) * N.dx[c1];
-        const double v_eq = (up - dn) / (1.0 / area2 + 1.0 / plan1);
-        V[l] = rmin(v, c.exchange_relax * v_eq);
+    sync();
+    if (tid < 2) {
+        double a = red[tid];
+        for (int w = 1; w < nt / 32; ++w) {
+            const double b = red[2 * w + tid];
+            if (f64_bits(b) << 1 != 0) a += b;
+        }
+        if (f64_bits(a) << 1 != 0) exch[mb * 2 + tid] += a;
     }
-    __syncthreads();
-    // donor limits, aggregated per donor in link order (coupling.py:98-107)
-    for (int k = tid; k < nu; k += nt) {
-        double tot = 0.0;
-        for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) { int l = L.uidx[j]; tot += sg[l] > 0.0 ? V[l] : 0.0; }
-        const double avail = c.exchange_limit * hu_[k] * area2;
-        f2[k] = tot > avail ? avail / (tot > 0.0 ? tot : 1.0) : 1.0;
-    }
-    for (int i = tid; i < nc; i += nt) {
-        double tot = 0.0;
-        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) { int l = L.cidx[j]; tot += sg[l] < 0.0 ? V[l] : 0.0; }
-        const double avail = c.exchange_limit * clamp0(N.A[i] - sec_bank_area(s, i)) * N.dx[i];
-        f1[i] = tot > avail ? avail / (tot > 0.0 ? tot : 1.0) : 1.0;
-    }
-    __syncthreads();
-    double ex[2] = {0.0, 0.0};
-    for (int l = tid; l < nl; l += nt) {
-        const double v = (sg[l] > 0.0 ? V[l] * f2[L.inv[l]] : V[l] * f1[L.cell1d[l]]) * sg[l];
-        V[l] = v;
-        if (Vout) Vout[L.v_offset + l] = v;
-        ex[0] += clamp0(v);
-        ex[1] += clamp0(-v);
-    }
-    __syncthreads();
-    // apply: 2-D through the unique cells, momentum kept only for water that stays
-    for (int k = tid; k < nu; k += nt) {
-        double d = 0.0;
-        for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) d += V[L.uidx[j]];
-        const double hu0 = hu_[k];
-        const double hn = hu0 - d / area2;
-        const double keep = hu0 > 0.0 ? fmin(hn / (hu0 > 0.0 ? hu0 : 1.0), 1.0) : 0.0;
-        const int idx = L.uniq[k];
-        const R kr = R(keep);
-        gd.h[idx] = R(hn);
-        gd.hu[idx] = gd.hu[idx] * kr;
-        gd.hv[idx] = gd.hv[idx] * kr;
-    }
-    for (int i = tid; i < nc; i += nt) {
-        double d = 0.0;
-        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) d += V[L.cidx[j]];
-        N.A[i] = N.A[i] + d / N.dx[i];
-    }
-    block_sum<2>(ex, red);
-    if (tid == 0 && exch) {
-        exch[mb * 2 + 0] += ex[0];
-        exch[mb * 2 + 1] += ex[1];
-    }
-    __syncthreads();
-}
-
-template <class R>
-__device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const Grid<R>& gd, const Consts& c, double dt,
-                                             double* __restrict__ Vout, double* __restrict__ exch, int mb, double* sm) {
-    if constexpr (sizeof(R) == 4) exchange_dev_f32(L, N, gd, c, dt, Vout, exch, mb, sm);
-    else exchange_dev_f64(L, N, gd, c, dt, Vout, exch, mb, sm);
 }
 
 // One CTA of EXCHANGE_THREADS per member.  The drop-in step runs it alone between
-// its CFL wait and the 2-D stages, so more threads (fewer dependent rounds over the
-// ~1,200 links per phase) shorten the step directly.
-constexpr int EXCHANGE_THREADS = 1024;
+// its CFL wait and the 2-D stages.
+constexpr int EXCHANGE_THREADS = 512;
 
 template <class R>
-__global__ void __launch_bounds__(EXCHANGE_THREADS) exchange_kernel(const Lnk* __restrict__ links, const Net* __restrict__ nets,
-                                const Grid<R>* __restrict__ grids, Consts c, double dt, double* __restrict__ Vout,
-                                double* __restrict__ exch) {
+__global__ void __launch_bounds__(EXCHANGE_THREADS, sizeof(R) == 4 ? 2 : 1) exchange_kernel(const Lnk* __restrict__ links,
+                                                                    const Net* __restrict__ nets,
+                                                                    const Grid<R>* __restrict__ grids, ExchK<R> K, R dt,
+                                                                    double* __restrict__ Vout,
+                                                                    double* __restrict__ exch) {
     extern __shared__ double sm[];
+    __shared__ Lnk L;
+    __shared__ Net N;
     const int mb = blockIdx.x;
-    exchange_dev(links[mb], nets[mb], grids[mb], c, dt, Vout, exch, mb, sm);
-}
-
-// 1-D CFL rate over wet interior cells and whether any is wet (swe1d.py:253-262);
-// results valid in thread 0.  red: 64 doubles of shared memory.
-__device__ __forceinline__ void net_rate_dev(const Net& N, const Consts& c, double& rate_o, bool& wet_o, double* red) {
-    const Sec s{N.b, N.m, N.yb, N.ts};
-    double rate = 0.0, wet_any = 0.0;
-    for (int i = threadIdx.x; i < N.n_cells; i += blockDim.x) {
-        if (N.kind[i] > 1) continue;
-        const double A = N.A[i];
-        const double y = sec_depth(s, i, A);
-        if (!(y > c.h_dry)) continue;
-        wet_any = 1.0;
-        const double cc = sqrt(c.g * A / sec_top(s, i, y));
-        const double u = vel1d(c, s, i, A, N.Q[i]);
-        rate = fmax(rate, (fabs(u) + cc) / N.dx[i]);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    rate = warp_max(rate);
-    wet_any = warp_max(wet_any);
-    if (lane == 0) { red[warp * 2] = rate; red[warp * 2 + 1] = wet_any; }
+    stage_record(&L, links + mb);
+    stage_record(&N, nets + mb);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = red[0], w = red[1];
-        for (int k = 1; k < nw; ++k) { r = fmax(r, red[k * 2]); w = fmax(w, red[k * 2 + 1]); }
-        rate_o = r;
-        wet_o = w > 0.0;
-    }
-    __syncthreads();
-}
-
-// The same rate in float32 arithmetic (production form: it only sets the substep count).
-__device__ __forceinline__ void net_rate_dev_f32(const Net& N, const Consts& c, double& rate_o, bool& wet_o,
-                                                 double* red) {
-    __shared__ float s_c[2];
-    if (threadIdx.x == 0) {
-        s_c[0] = (float)c.g;
-        s_c[1] = (float)c.h_dry;
-    }
-    __syncthreads();
-    const float g = s_c[0], h_dry = s_c[1];
-    float rate = 0.0f, wet_any = 0.0f;
-    for (int i = threadIdx.x; i < N.n_cells; i += blockDim.x) {
-        if (N.kind[i] > 1) continue;
-        const float A = fmaxf((float)N.A[i], 0.0f);
-        const float b = N.bf[i], m = N.mf[i], yb = N.ybf[i], ts = N.tsf[i];
-        const float ab = yb * (b + m * yb);
-        const float y = A <= ab ? 2.0f * A / (b + sqrtf(b * b + 4.0f * m * A)) : yb + (A - ab) / ts;
-        if (!(y > h_dry)) continue;
-        wet_any = 1.0f;
-        const float top = y <= yb ? b + 2.0f * m * y : ts;
-        const float cc = sqrtf(g * A / top);
-        const float u = (float)N.Q[i] / fmaxf(A, 1e-12f);
-        rate = fmaxf(rate, (fabsf(u) + cc) / N.dxf[i]);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        rate = fmaxf(rate, __shfl_xor_sync(0xffffffffu, rate, o));
-        wet_any = fmaxf(wet_any, __shfl_xor_sync(0xffffffffu, wet_any, o));
-    }
-    float* redf = reinterpret_cast<float*>(red);
-    if (lane == 0) { redf[warp * 2] = rate; redf[warp * 2 + 1] = wet_any; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float r = redf[0], w = redf[1];
-        for (int k = 1; k < nw; ++k) { r = fmaxf(r, redf[k * 2]); w = fmaxf(w, redf[k * 2 + 1]); }
-        rate_o = (double)r;
-        wet_o = w > 0.0f;
-    }
-    __syncthreads();
+    exchange_dev<R>(L, N, grids[mb], K, Vout, exch, mb, sm, threadIdx.x, EXCHANGE_THREADS, nullptr,
+                    [] { __syncthreads(); }, [&] { __syncthreads(); return dt; }, [] { __syncthreads(); return true; });
 }
 
 }  // namespace his

@@ -172,6 +172,7 @@ int grid_init_impl(his_grid* g) {
         G.rt0 = R(d.horton_t0);
         G.idx = R(1.0 / d.dx);
         G.idy = R(1.0 / d.dy);
+        G.rarea = R(1.0 / G.area);
         const int ns = (d.nx + wmax - 1) / wmax;
         const int w = (d.nx + ns - 1) / ns;
         const int nch = (d.ny + g->ty - 1) / g->ty;
@@ -223,11 +224,12 @@ int grid_reduce_impl(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
 
 template <class R>
 int exchange_impl(his_links* l, const Consts& c, double dt, cudaStream_t s) {
-    if (l->smem > 48 * 1024)
-        HIS_CK(cudaFuncSetAttribute(exchange_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l->smem));
-    exchange_kernel<R><<<l->n, EXCHANGE_THREADS, l->smem, s>>>(l->d_links, l->net->d_nets,
-                                                  reinterpret_cast<const Grid<R>*>(l->grid->d_grids), c, dt, l->d_V,
-                                                  l->d_exch);
+    const size_t smem = l->smem_of(sizeof(R));
+    if (smem > 48 * 1024)
+        HIS_CK(cudaFuncSetAttribute(exchange_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    exchange_kernel<R><<<l->n, EXCHANGE_THREADS, smem, s>>>(l->d_links, l->net->d_nets,
+                                                            reinterpret_cast<const Grid<R>*>(l->grid->d_grids),
+                                                            make_exch_k<R>(c), (R)dt, l->d_V, l->d_exch);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
 }
@@ -248,7 +250,8 @@ int eng_enqueue_nt(his_grid* g, his_engine* E, int chain, int n_steps) {
     if (mc == 0) return HIS_OK;
     for (int k = 0; k < n_steps; ++k) {
         eng_pre_kernel<R><<<mc, ENG_PRE_THREADS, E->pre_smem, s_main>>>(E->d_em, g->d_params, grids, nets, links, g->c,
-                                                                        E->d_netf, E->max_sub, exch, m0);
+                                                                        make_exch_k<R>(g->c), E->d_netf, E->max_sub,
+                                                                        exch, m0);
         if (E->net) {
             HIS_CK(cudaEventRecord(fork, s_main));
             HIS_CK(cudaStreamWaitEvent(s_side, fork, 0));
@@ -300,7 +303,7 @@ int eng_profile_nt(his_grid* g, his_engine* E, int n_steps, double* ms) {
     for (int k = 0; k < n_steps && rc == HIS_OK; ++k) {
         cudaEventRecord(ev[0], E->s0);
         eng_pre_kernel<R><<<E->n, ENG_PRE_THREADS, E->pre_smem, E->s0>>>(E->d_em, g->d_params, grids, nets, links, g->c,
-                                                             E->d_netf, E->max_sub, exch, 0);
+                                                             make_exch_k<R>(g->c), E->d_netf, E->max_sub, exch, 0);
         cudaEventRecord(ev[1], E->s0);
         if (E->net) {
             cudaStreamWaitEvent(E->s1, ev[1], 0);
@@ -390,6 +393,7 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
     G.rt0 = R(d.horton_t0);
     G.idx = R(1.0 / d.dx);
     G.idy = R(1.0 / d.dy);
+    G.rarea = R(1.0 / G.area);
     G.tile0 = 0;
     G.tiles_x = L.ns;
     G.tiles_y = L.nch;

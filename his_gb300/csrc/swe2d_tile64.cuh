@@ -118,10 +118,6 @@ __device__ __forceinline__ Q4<double> face64(const KC<double>& c, const Q4<doubl
     return Q4<double>{F1, F2 + corrL, F2 + corrR, F3};
 }
 
-// Warp sum (lane 0) that costs one vote where every lane holds zero
-__device__ __forceinline__ double warp_sum_sparse(double v) {
-    return __any_sync(0xffffffffu, f64_bits(v) << 1 != 0) ? warp_sum(v) : 0.0;
-}
 __device__ __forceinline__ double warp_max_run(double v) {
     for (int o = 16; o > 0; o >>= 1) v = f64_max_run(v, __shfl_down_sync(0xffffffffu, v, o));
     return v;
