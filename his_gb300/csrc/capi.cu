@@ -500,9 +500,10 @@ int32_t his_net_create(const his_solver_cfg* cfg, int32_t n_members, const his_n
     if (n_members <= 0 || !nets) return bad("need at least one network member");
     Arena ar;
     struct Offs { size_t kind, gsrc, fl, fr, gsign, ls, li, rs, ri, z, n, dx, b, m, yb, ts, fb, fm, fyb, fts;
+                  size_t ab, b2, m4, sp, rdx, fab, fib, fbh, fm3, gh;
                   size_t zf, dxf, bf, mf, ybf, tsf, nf, gsf, fbf, fmf, fybf, ftsf; };
     std::vector<Offs> offs(n_members);
-    size_t smem = 0, smem_f32 = 0;
+    size_t smem = 0, smem_f32 = 0, limit = 0;
     for (int mb = 0; mb < n_members; ++mb) {
         const his_net_desc& d = nets[mb];
         std::string who = "network " + std::to_string(mb) + ": ";
@@ -538,6 +539,30 @@ int32_t his_net_create(const his_solver_cfg* cfg, int32_t n_members, const his_n
         o.z = ar.add(d.z, C); o.n = ar.add(d.manning, C); o.dx = ar.add(d.dx, C);
         o.b = ar.add(d.b, C); o.m = ar.add(d.m, C); o.yb = ar.add(d.yb, C); o.ts = ar.add(d.ts, C);
         o.fb = ar.add(d.fb, F); o.fm = ar.add(d.fm, F); o.fyb = ar.add(d.fyb, F); o.fts = ar.add(d.fts, F);
+        // products of the sections' constants (Net)
+        auto cells = [&](auto f) {
+            std::vector<double> v(d.n_cells);
+            for (int i = 0; i < d.n_cells; ++i) v[i] = f(i);
+            return ar.add(v.data(), C);
+        };
+        auto faces = [&](auto f) {
+            std::vector<double> v(d.n_faces);
+            for (int i = 0; i < d.n_faces; ++i) v[i] = f(i);
+            return ar.add(v.data(), F);
+        };
+        o.ab = cells([&](int i) { return d.yb[i] * (d.b[i] + d.m[i] * d.yb[i]); });
+        o.b2 = cells([&](int i) { return d.b[i] * d.b[i]; });
+        o.m4 = cells([&](int i) { return 4.0 * d.m[i]; });
+        o.sp = cells([&](int i) { return std::sqrt(1.0 + d.m[i] * d.m[i]); });
+        o.rdx = cells([&](int i) { return 1.0 / d.dx[i]; });
+        o.fab = faces([&](int f) { return d.fyb[f] * (d.fb[f] + d.fm[f] * d.fyb[f]); });
+        o.fib = faces([&](int f) { return d.fyb[f] * d.fyb[f] * (d.fb[f] / 2.0 + d.fm[f] / 3.0 * d.fyb[f]); });
+        o.fbh = faces([&](int f) { return d.fb[f] / 2.0; });
+        o.fm3 = faces([&](int f) { return d.fm[f] / 3.0; });
+        std::vector<int> gh;
+        for (int i = 0; i < d.n_cells; ++i)
+            if (d.kind[i] >= 2) gh.push_back(i);
+        o.gh = ar.add(gh.data(), sizeof(int) * gh.size());
         // float32 copies of the static geometry for the production form's exchange and
         // network substeps
         auto addf = [&](const double* a, int n) {
@@ -550,9 +575,11 @@ int32_t his_net_create(const his_solver_cfg* cfg, int32_t n_members, const his_n
         o.fbf = addf(d.fb, d.n_faces); o.fmf = addf(d.fm, d.n_faces); o.fybf = addf(d.fyb, d.n_faces);
         o.ftsf = addf(d.fts, d.n_faces);
         smem = std::max(smem, net_smem_bytes(d.n_cells, d.n_faces));
+        // (the largest network accepted is one whose state once took seven values per cell)
+        limit = std::max(limit, net_smem_bytes(d.n_cells, d.n_faces) + 2 * sizeof(double) * (size_t)d.n_cells);
         smem_f32 = std::max(smem_f32, net_smem_bytes_f32(d.n_cells, d.n_faces));
     }
-    if (smem > 200 * 1024 || smem_f32 > 200 * 1024)
+    if (limit > 200 * 1024 || smem_f32 > 200 * 1024)
         return bad("network too large for one thread block's shared memory");
     his_net* N = new his_net();
     N->c = to_consts(cfg);
@@ -584,6 +611,13 @@ int32_t his_net_create(const his_solver_cfg* cfg, int32_t n_members, const his_n
         n.yb = (const double*)(base + o.yb); n.ts = (const double*)(base + o.ts);
         n.fb = (const double*)(base + o.fb); n.fm = (const double*)(base + o.fm);
         n.fyb = (const double*)(base + o.fyb); n.fts = (const double*)(base + o.fts);
+        n.ab = (const double*)(base + o.ab); n.b2 = (const double*)(base + o.b2);
+        n.m4 = (const double*)(base + o.m4); n.sp = (const double*)(base + o.sp);
+        n.rdx = (const double*)(base + o.rdx);
+        n.fab = (const double*)(base + o.fab); n.fib = (const double*)(base + o.fib);
+        n.fbh = (const double*)(base + o.fbh); n.fm3 = (const double*)(base + o.fm3);
+        n.ghosts = (const int*)(base + o.gh);
+        n.n_ghosts = (int)std::count_if(d.kind, d.kind + d.n_cells, [](int k) { return k >= 2; });
         n.zf = (const float*)(base + o.zf); n.dxf = (const float*)(base + o.dxf);
         n.bf = (const float*)(base + o.bf); n.mf = (const float*)(base + o.mf);
         n.ybf = (const float*)(base + o.ybf); n.tsf = (const float*)(base + o.tsf);

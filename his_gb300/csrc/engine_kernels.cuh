@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_p
             if (nets)
                 for (int i = tid; i < s_N.n_cells; i += ENG_EXCH_THREADS) {
                     const CellLevel<R> o = cell_level(s_N, i, K.g, K.h_dry, true);
-                    if (o.wet) rate = rate > o.rate ? rate : o.rate;
+                    if (o.wet) rate = o.rate > rate ? o.rate : rate;
                 }
             for (int o = 16; o > 0; o >>= 1) {
                 const R w = __shfl_xor_sync(0xffffffffu, rate, o);

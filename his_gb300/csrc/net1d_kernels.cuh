@@ -30,6 +30,12 @@ struct Net {
     const double *z, *nman, *dx;
     const double *b, *m, *yb, *ts;                 // cell sections
     const double *fb, *fm, *fyb, *fts;             // face sections
+    // products of the sections' constants: area at the bank, b^2, 4 m, sqrt(1 + m^2) and
+    // 1 / dx of the cells; area and first moment at the bank, b / 2 and m / 3 of the faces
+    const double *ab, *b2, *m4, *sp, *rdx;
+    const double *fab, *fib, *fbh, *fm3;
+    const int* ghosts;                             // the ghost cells (kinds 2 and up)
+    int n_ghosts, pad;
     const float *zf, *dxf, *bf, *mf, *ybf, *tsf;   // float32 copies of z, dx and the cell sections
     const float *nmanf, *gsignf;                   // float32 roughness and ghost signs
     const float *fbf, *fmf, *fybf, *ftsf;          // float32 face sections
@@ -49,66 +55,86 @@ struct Lnk {
 };
 
 // ---------------------------------------------------------------- sections (swe1d.py:51-84)
-struct Sec {
-    const double *b, *m, *yb, *ts;
-};
+// Float64 geometry in few FP64 instructions (f64_ops.cuh): the products of a section's
+// constants come from tables, and the wall above the bank is a branch that water below the
+// bank does not take.  (Every quantity is >= 0, so comparisons are on the bit patterns.)
+__device__ __forceinline__ bool f64_le(double a, double b) { return f64_bits(a) <= f64_bits(b); }   // a, b >= +0
 
-__device__ __forceinline__ double sec_area(const Sec& s, int i, double y) {
-    double yt = fmin(y, s.yb[i]);
-    double at = yt * (s.b[i] + s.m[i] * yt);
-    return at + s.ts[i] * clamp0(y - s.yb[i]);
+__device__ __forceinline__ double cell_depth(const Net& N, int i, double A) {
+    A = f64_clamp0(A);
+    if (f64_bits(A) == 0) return 0.0;
+    const double ab = N.ab[i];
+    if (f64_le(A, ab)) return 2.0 * A / (N.b[i] + sqrt(fma(N.m4[i], A, N.b2[i])));
+    return N.yb[i] + (A - ab) / N.ts[i];
 }
-__device__ __forceinline__ double sec_top(const Sec& s, int i, double y) {
-    return y <= s.yb[i] ? s.b[i] + 2.0 * s.m[i] * y : s.ts[i];
+__device__ __forceinline__ double cell_area(const Net& N, int i, double y) {
+    const double yb = N.yb[i];
+    return f64_le(y, yb) ? y * fma(N.m[i], y, N.b[i]) : fma(N.ts[i], y - yb, N.ab[i]);
 }
-__device__ __forceinline__ double sec_i1(const Sec& s, int i, double y) {
-    double yt = fmin(y, s.yb[i]);
-    double above = clamp0(y - s.yb[i]);
-    double it = s.b[i] * yt * yt / 2.0 + s.m[i] * (yt * yt * yt) / 3.0;
-    double at = yt * (s.b[i] + s.m[i] * yt);
-    return it + at * above + s.ts[i] * above * above / 2.0;
+__device__ __forceinline__ double cell_top(const Net& N, int i, double y) {
+    return f64_le(y, N.yb[i]) ? fma(2.0 * N.m[i], y, N.b[i]) : N.ts[i];
 }
-__device__ __forceinline__ double sec_perim(const Sec& s, int i, double y) {
-    double yt = fmin(y, s.yb[i]);
-    return s.b[i] + 2.0 * yt * sqrt(1.0 + s.m[i] * s.m[i]);
+__device__ __forceinline__ double cell_velocity(const Consts& c, double y, double A, double Q) {
+    return f64_ge_pos(y, c.h_dry) ? Q / (f64_ge_pos(A, 1e-12) ? A : 1e-12) : 0.0;
 }
-__device__ __forceinline__ double sec_bank_area(const Sec& s, int i) { return s.yb[i] * (s.b[i] + s.m[i] * s.yb[i]); }
-__device__ __forceinline__ double sec_depth(const Sec& s, int i, double A) {
-    A = clamp0(A);
-    double ab = sec_bank_area(s, i);
-    double b = s.b[i];
-    double y_t = 2.0 * A / (b + sqrt(b * b + 4.0 * s.m[i] * A));
-    return A <= ab ? y_t : s.yb[i] + (A - ab) / s.ts[i];
-}
-__device__ __forceinline__ double vel1d(const Consts& c, const Sec& s, int i, double A, double Q) {
-    double y = sec_depth(s, i, A);
-    return y >= c.h_dry ? Q / fmax(A, 1e-12) : 0.0;
+
+// One side of a face: area, hydrostatic force and wave speed at depth y of its section
+struct FaceSide {
+    double A, p, c;
+};
+__device__ __forceinline__ FaceSide face_side(const Net& N, int f, double g, double y) {
+    if (f64_bits(y) == 0) return FaceSide{0.0, 0.0, 0.0};
+    const double yb = N.fyb[f], b = N.fb[f], m = N.fm[f];
+    double A, I, top;
+    if (f64_le(y, yb)) {
+        A = y * fma(m, y, b);
+        I = y * y * fma(N.fm3[f], y, N.fbh[f]);
+        top = fma(2.0 * m, y, b);
+    } else {
+        const double above = y - yb, ts = N.fts[f], ab = N.fab[f];
+        A = fma(ts, above, ab);
+        I = N.fib[f] + above * fma(0.5 * ts, above, ab);
+        top = ts;
+    }
+    return FaceSide{A, g * I, sqrt(g * A / top)};
 }
 
 // HLL flux of the 1-D equations (swe1d.py:87-107)
-__device__ __forceinline__ void hll_1d(double AL, double QL, double pL, double cL, double AR, double QR, double pR,
-                                       double cR, double uL, double uR, double& F1o, double& F2o) {
+__device__ __forceinline__ void hll_1d(const FaceSide& L, double uL, const FaceSide& R, double uR, double& F1,
+                                       double& F2) {
     const double tiny = 1e-14;
-    bool dryL = AL <= tiny, dryR = AR <= tiny;
-    double SL = rmin(uL - cL, uR - cR);
-    double SR = rmax(uL + cL, uR + cR);
-    if (dryL) { SL = uR - 2.0 * cR; SR = uR + cR; }
-    if (dryR) { SL = uL - cL; SR = uL + 2.0 * cL; }
-    double FL1 = QL, FR1 = QR;
-    double FL2 = QL * uL + pL, FR2 = QR * uR + pR;
-    double den = SR - SL;
-    if (fabs(den) < tiny) den = 1.0;
-    bool left = SL >= 0.0, right = SR <= 0.0;
-    double F1, F2;
-    if (left) { F1 = FL1; F2 = FL2; }
-    else if (right) { F1 = FR1; F2 = FR2; }
+    const bool dryL = f64_le(L.A, tiny), dryR = f64_le(R.A, tiny);
+    F1 = F2 = 0.0;
+    if (dryL && dryR) return;
+    double SL, SR;
+    if (dryL) { SL = fma(-2.0, R.c, uR); SR = uR + R.c; }
+    else if (dryR) { SL = uL - L.c; SR = fma(2.0, L.c, uL); }
     else {
-        F1 = (SR * FL1 - SL * FR1 + SL * SR * (AR - AL)) / den;
-        F2 = (SR * FL2 - SL * FR2 + SL * SR * (QR - QL)) / den;
+        SL = f64_min(uL - L.c, uR - R.c);
+        SR = f64_max(uL + L.c, uR + R.c);
     }
-    if (dryL && dryR) { F1 = 0.0; F2 = 0.0; }
-    F1o = F1;
-    F2o = F2;
+    const double QL = L.A * uL, QR = R.A * uR;
+    if (f64_plus(SL)) {
+        F1 = QL;
+        F2 = fma(QL, uL, L.p);
+    } else if (f64_minus(SR)) {
+        F1 = QR;
+        F2 = fma(QR, uR, R.p);
+    } else {
+        double den = SR - SL;
+        if (f64_mag_lt(den, tiny)) den = 1.0;
+        const double r = __drcp_rn(den), SS = SL * SR;
+        const double mL = fma(QL, uL, L.p), mR = fma(QR, uR, R.p);
+        F1 = fma(SS, R.A - L.A, fma(-SL, QR, SR * QL)) * r;
+        F2 = fma(SS, QR - QL, fma(-SL, mR, SR * mL)) * r;
+    }
+}
+
+// Largest wave rate (|u| + c) / dx of a wet interior cell, or -1 (swe1d.py:253-262)
+__device__ __forceinline__ double cell_rate_1d(const Net& N, const Consts& c, int i, double y, double A, double Q) {
+    if (N.kind[i] > 1 || !f64_ge_pos(y, c.h_dry) || f64_bits(y) == f64_bits(c.h_dry)) return -1.0;
+    const double cc = sqrt(c.g * A / cell_top(N, i, y));
+    return f64_div(fabs(cell_velocity(c, y, A, Q)) + cc, N.dx[i], N.rdx[i]);
 }
 
 // Deterministic block sum of NV doubles; result valid in thread 0.
@@ -116,149 +142,188 @@ template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
-    for (int j = 0; j < NV; ++j) v[j] = warp_sum(v[j]);
+    for (int j = 0; j < NV; ++j) v[j] = warp_sum_sparse(v[j]);
     if (lane == 0)
         for (int j = 0; j < NV; ++j) red[warp * NV + j] = v[j];
     __syncthreads();
     if (threadIdx.x == 0)
         for (int j = 0; j < NV; ++j) {
             double a = red[j];
-            for (int w = 1; w < nw; ++w) a += red[w * NV + j];
+            for (int w = 1; w < nw; ++w) {
+                const double b = red[w * NV + j];
+                if (f64_bits(b) << 1 != 0) a += b;
+            }
             v[j] = a;
         }
     __syncthreads();
 }
 
 __host__ __device__ inline size_t net_smem_bytes(int n_cells, int n_faces) {
-    return sizeof(double) * (7 * (size_t)n_cells + 4 * (size_t)n_faces + 32 * 4);
+    return sizeof(double) * (5 * (size_t)n_cells + 4 * (size_t)n_faces + 32 * 4);
 }
 
-// n_sub substeps of dt/n_sub each for the network N, run by the whole CTA.
+// Threads of a float64 network CTA: a warp for the ghosts beside those of the cells
+constexpr int NET64_THREADS = 256;
+
+// n_sub substeps of dt/n_sub each for the network N, run by the whole CTA (NET64_THREADS).
 // forcing: per substep (inflow, stage).  vols (thread 0, if non-NULL): bnd_in,
 // bnd_out, clip summed over the substeps.  sm: net_smem_bytes() of shared memory.
+//
+// Bound by one SM's FP64 pipe and by the length of the per-substep chain: ghosts, faces,
+// limiter, update, with a barrier between.  The depth a cell's update needs for its
+// friction is kept as the next substep's, the limiter's factors are applied where the
+// fluxes are summed, and the tallies are summed once per call.  3170 -> 950 FP64 warp
+// instructions per substep of 161 cells; two substeps 130 -> 48 us.
 __device__ __forceinline__ void net_substeps_dev(const Net& N, const Consts& c, double dt_total, int n_sub,
                                                  const double* __restrict__ forcing, double* vols, double* sm,
                                                  float* snap_eta = nullptr, float* snap_q = nullptr,
                                                  double* snap_v1d = nullptr) {
     const int nc = N.n_cells, nf = N.n_faces, tid = threadIdx.x, nt = blockDim.x;
-    double *A = sm, *Q = A + nc, *Ag = Q + nc, *Qg = Ag + nc, *yv = Qg + nc, *uv = yv + nc, *th = uv + nc;
+    // A, Q: state, with the ghosts filled at the start of a substep; y, u: depth and velocity
+    double *A = sm, *Q = A + nc, *yv = Q + nc, *uv = yv + nc, *th = uv + nc;
     double *F1 = th + nc, *F2 = F1 + nf, *pL = F2 + nf, *pR = pL + nf, *red = pR + nf;
-    const Sec s{N.b, N.m, N.yb, N.ts}, fs{N.fb, N.fm, N.fyb, N.fts};
     const double g = c.g, dt = dt_total / n_sub;
-    for (int i = tid; i < nc; i += nt) { A[i] = N.A[i]; Q[i] = N.Q[i]; }
+    for (int i = tid; i < nc; i += nt) {
+        const double a = N.A[i], q = N.Q[i];
+        A[i] = a;
+        Q[i] = q;
+        if (N.kind[i] < 2) {
+            const double y = cell_depth(N, i, a);
+            yv[i] = y;
+            uv[i] = cell_velocity(c, y, a, q);
+        }
+    }
     __syncthreads();
-    double tot_in = 0.0, tot_out = 0.0, tot_clip = 0.0;
+    double bsum[3] = {0.0, 0.0, 0.0};
     for (int k = 0; k < n_sub; ++k) {
         const double q_in = forcing[2 * k + 0];
         const double eta = forcing[2 * k + 1];
         // ghost cells from the interior neighbour (swe1d.py:265-294)
-        for (int i = tid; i < nc; i += nt) {
-            const int kd = N.kind[i];
-            if (kd < 2) { Ag[i] = A[i]; Qg[i] = Q[i]; continue; }
-            const int src = N.gsrc[i];
+        for (int j = tid; j < N.n_ghosts; j += nt) {
+            const int i = N.ghosts[j], kd = N.kind[i], src = N.gsrc[i];
             const double As = A[src], Qs = Q[src], sg = N.gsign[i];
-            const double ys = sec_depth(s, i, As);
-            const double un = sg * vel1d(c, s, i, As, Qs);
-            const bool wet_i = ys >= c.h_dry;
-            double An, Qn;
+            const double ys = cell_depth(N, i, As);
+            const bool wet_i = f64_ge_pos(ys, c.h_dry);
+            double An, Qn, y;
             if (kd == 3) {
-                double yst = clamp0(eta - N.z[i]);
-                double Ast = sec_area(s, i, yst);
-                double ci = sqrt(g * As / sec_top(s, i, ys));
-                double cg = sqrt(g * Ast / sec_top(s, i, yst));
-                double un_st = wet_i ? un + 2.0 * (ci - cg) : 0.0;
-                if (wet_i && (un > ci)) { un_st = un; Ast = As; }
-                if (!(sec_depth(s, i, Ast) >= c.h_dry)) un_st = 0.0;
+                const double un = sg * cell_velocity(c, ys, As, Qs);
+                const double yst = f64_clamp0(eta - N.z[i]);
+                double Ast = cell_area(N, i, yst), un_st = 0.0;
+                y = cell_depth(N, i, Ast);
+                if (wet_i) {
+                    const double ci = sqrt(g * As / cell_top(N, i, ys));
+                    const double cg = f64_bits(Ast) == 0 ? 0.0 : sqrt(g * Ast / cell_top(N, i, yst));
+                    un_st = fma(2.0, ci - cg, un);
+                    if (un > ci) {
+                        un_st = un;
+                        Ast = As;
+                        y = ys;
+                    }
+                }
+                if (!f64_ge_pos(y, c.h_dry)) un_st = 0.0;
                 An = Ast;
                 Qn = sg * Ast * un_st;
             } else if (kd == 2) {
-                double yc = fmax(pow(q_in * q_in / (g * N.b[i] * N.b[i]), 1.0 / 3.0), c.h_dry);
-                An = wet_i ? As : sec_area(s, i, yc);
+                An = As;
+                y = ys;
+                if (!wet_i) {
+                    const double yc = fmax(cbrt(q_in * q_in / (g * N.b[i] * N.b[i])), c.h_dry);
+                    An = cell_area(N, i, yc);
+                    y = cell_depth(N, i, An);
+                }
                 Qn = -sg * q_in;
             } else {
                 An = As;
+                y = ys;
                 Qn = -Qs;
             }
-            Ag[i] = An;
-            Qg[i] = Qn;
-        }
-        __syncthreads();
-        for (int i = tid; i < nc; i += nt) {
-            yv[i] = sec_depth(s, i, Ag[i]);
-            uv[i] = vel1d(c, s, i, Ag[i], Qg[i]);
+            A[i] = An;
+            Q[i] = Qn;
+            yv[i] = y;
+            uv[i] = cell_velocity(c, y, An, Qn);
         }
         __syncthreads();
         // face fluxes with hydrostatic reconstruction (swe1d.py:326-336)
         for (int f = tid; f < nf; f += nt) {
             const int l = N.fl[f], r = N.fr[f];
-            const double zL = N.z[l], zR = N.z[r], zf = rmax(zL, zR);
-            const double yL = clamp0(zL + yv[l] - zf), yR = clamp0(zR + yv[r] - zf);
-            const double AL = sec_area(fs, f, yL), AR = sec_area(fs, f, yR);
-            const double uL = uv[l], uR = uv[r];
-            pL[f] = g * sec_i1(fs, f, yL);
-            pR[f] = g * sec_i1(fs, f, yR);
-            const double cL = sqrt(g * AL / sec_top(fs, f, yL));
-            const double cR = sqrt(g * AR / sec_top(fs, f, yR));
-            hll_1d(AL, AL * uL, pL[f], cL, AR, AR * uR, pR[f], cR, uL, uR, F1[f], F2[f]);
+            const double zL = N.z[l], zR = N.z[r], zf = f64_max(zL, zR);
+            const FaceSide L = face_side(N, f, g, f64_clamp0(zL + yv[l] - zf));
+            const FaceSide R = face_side(N, f, g, f64_clamp0(zR + yv[r] - zf));
+            pL[f] = L.p;
+            pR[f] = R.p;
+            hll_1d(L, uv[l], R, uv[r], F1[f], F2[f]);
         }
         __syncthreads();
         // outflow limiter; ghosts unlimited (swe1d.py:337-344)
         for (int i = tid; i < nc; i += nt) {
-            double out = 0.0;
-            for (int j = N.lstart[i]; j < N.lstart[i + 1]; ++j) out += relu(F1[N.lidx[j]]);
-            for (int j = N.rstart[i]; j < N.rstart[i + 1]; ++j) out += relu(-F1[N.ridx[j]]);
-            const double vol = Ag[i] * N.dx[i];
-            const double need = out * dt;
-            const double t = need > vol ? vol / (need > 0.0 ? need : 1.0) : 1.0;
-            th[i] = N.kind[i] >= 2 ? 1.0 : t;
+            double out = 0.0, t = 1.0;
+            if (N.kind[i] < 2) {
+                for (int j = N.lstart[i]; j < N.lstart[i + 1]; ++j) out += f64_relu(F1[N.lidx[j]]);
+                for (int j = N.rstart[i]; j < N.rstart[i + 1]; ++j) out += f64_relu(-F1[N.ridx[j]]);
+                const double vol = A[i] * N.dx[i], need = out * dt;
+                if (need > vol) t = vol / (need > 0.0 ? need : 1.0);
+            }
+            th[i] = t;
         }
         __syncthreads();
-        double bsum[3] = {0.0, 0.0, 0.0};
-        for (int f = tid; f < nf; f += nt) {
-            const double sc = F1[f] > 0.0 ? th[N.fl[f]] : th[N.fr[f]];
-            const double Fs = F1[f] * sc;
-            F1[f] = Fs;
-            if (N.kind[N.fl[f]] >= 2) { bsum[0] += relu(Fs); bsum[1] += relu(-Fs); }
-            if (N.kind[N.fr[f]] >= 2) { bsum[0] += relu(-Fs); bsum[1] += relu(Fs); }
-        }
-        __syncthreads();
-        // update, clip, semi-implicit friction; ghosts keep their filled state (swe1d.py:345-368)
+        // update with the limited fluxes, clip, semi-implicit friction; ghosts keep their filled
+        // state, and their faces carry the boundary volumes (swe1d.py:345-368)
         for (int i = tid; i < nc; i += nt) {
+            const bool ghost = N.kind[i] >= 2;
             double dA = 0.0, dQ = 0.0;
-            for (int j = N.lstart[i]; j < N.lstart[i + 1]; ++j) dA += -F1[N.lidx[j]];
-            for (int j = N.rstart[i]; j < N.rstart[i + 1]; ++j) dA += F1[N.ridx[j]];
-            for (int j = N.lstart[i]; j < N.lstart[i + 1]; ++j) { int f = N.lidx[j]; dQ += -(F2[f] - pL[f]); }
-            for (int j = N.rstart[i]; j < N.rstart[i + 1]; ++j) { int f = N.ridx[j]; dQ += F2[f] - pR[f]; }
-            const int kd = N.kind[i];
-            double A1 = Ag[i] + dt * dA / N.dx[i];
-            double Q1 = Qg[i] + dt * dQ / N.dx[i];
-            const double neg = clamp0(-A1);
-            bsum[2] += neg * N.dx[i] * (kd >= 2 ? 0.0 : 1.0);
-            A1 = A1 + neg;
-            const double y1 = sec_depth(s, i, A1);
-            const double Ac = fmax(A1, 1e-12);
-            const double R = Ac / sec_perim(s, i, y1);
-            const double nm = N.nman[i];
-            const double denom = 1.0 + dt * g * (nm * nm) * fabs(Q1) / (Ac * pow(fmax(R, c.h_dry), 4.0 / 3.0));
-            Q1 = Q1 / denom;
-            if (!((y1 >= c.h_dry) && kd != 1)) Q1 = 0.0;
-            if (kd >= 2) { A1 = Ag[i]; Q1 = Qg[i]; }
+            auto limited = [&](int f) {
+                const double F = F1[f], t = th[f64_pos(F) ? N.fl[f] : N.fr[f]];
+                return f64_bits(t) == f64_bits(1.0) ? F : F * t;
+            };
+            for (int j = N.lstart[i]; j < N.lstart[i + 1]; ++j) {
+                const int f = N.lidx[j];
+                const double F = limited(f);
+                if (ghost) { bsum[0] += f64_relu(F); bsum[1] += f64_relu(-F); continue; }
+                dA -= F;
+                dQ -= F2[f] - pL[f];
+            }
+            for (int j = N.rstart[i]; j < N.rstart[i + 1]; ++j) {
+                const int f = N.ridx[j];
+                const double F = limited(f);
+                if (ghost) { bsum[0] += f64_relu(-F); bsum[1] += f64_relu(F); continue; }
+                dA += F;
+                dQ += F2[f] - pR[f];
+            }
+            if (ghost) continue;
+            const double dx = N.dx[i], rdx = N.rdx[i];
+            double A1 = A[i] + f64_div(dt * dA, dx, rdx);
+            double Q1 = Q[i] + f64_div(dt * dQ, dx, rdx);
+            if (f64_neg(A1)) {
+                bsum[2] -= A1 * dx;
+                A1 = 0.0;
+            }
+            const double y1 = cell_depth(N, i, A1);
+            if (f64_ge_pos(y1, c.h_dry) && N.kind[i] != 1) {
+                if (f64_bits(Q1) << 1 != 0) {
+                    // Q / (1 + dt g n^2 |Q| / (A R^(4/3))), as one quotient
+                    const double yb = N.yb[i], Ac = f64_ge_pos(A1, 1e-12) ? A1 : 1e-12;
+                    const double R = Ac / fma(2.0 * (f64_le(y1, yb) ? y1 : yb), N.sp[i], N.b[i]);
+                    const double nm = N.nman[i], X = Ac * f64_pow43(f64_ge_pos(R, c.h_dry) ? R : c.h_dry);
+                    Q1 = Q1 * (X / fma(dt * g * (nm * nm), fabs(Q1), X));
+                }
+            } else {
+                Q1 = 0.0;
+            }
             A[i] = A1;
             Q[i] = Q1;
+            yv[i] = y1;
+            uv[i] = cell_velocity(c, y1, A1, Q1);
         }
-        block_sum<3>(bsum, red);
-        if (tid == 0) {
-            tot_in += bsum[0] * dt;
-            tot_out += bsum[1] * dt;
-            tot_clip += bsum[2];
-        }
+        __syncthreads();
     }
-    __syncthreads();
+    bsum[0] *= dt;
+    bsum[1] *= dt;
+    block_sum<3>(bsum, red);
     for (int i = tid; i < nc; i += nt) { N.A[i] = A[i]; N.Q[i] = Q[i]; }
     if (snap_eta) {                         // output: level z + depth and discharge (coupling.py:229-242)
         double v1 = 0.0;
         for (int i = tid; i < nc; i += nt) {
-            snap_eta[i] = (float)(N.z[i] + sec_depth(s, i, A[i]));
+            snap_eta[i] = (float)(N.z[i] + yv[i]);
             snap_q[i] = (float)Q[i];
             if (N.kind[i] <= 1) v1 += A[i] * N.dx[i];
         }
@@ -269,9 +334,9 @@ __device__ __forceinline__ void net_substeps_dev(const Net& N, const Consts& c, 
         }
     }
     if (tid == 0 && vols) {
-        vols[0] = tot_in;
-        vols[1] = tot_out;
-        vols[2] = tot_clip;
+        vols[0] = bsum[0];
+        vols[1] = bsum[1];
+        vols[2] = bsum[2];
     }
 }
 
@@ -373,7 +438,6 @@ __device__ __forceinline__ void net_substeps_f32_dev(const Net& N, const Consts&
         lix[f] = N.lidx[f]; rix[f] = N.ridx[f];
     }
     const SecF s{bs, ms, ybs, tss}, fs{fbs, fms, fybs, ftss};
-    const Sec sd{N.b, N.m, N.yb, N.ts};
     __shared__ float s_k[3];
     if (tid == 0) {
         s_k[0] = (float)c.g;
@@ -427,7 +491,7 @@ __device__ __forceinline__ void net_substeps_f32_dev(const Net& N, const Consts&
         __syncthreads();
         // depth and velocity; a junction's level-pool depth in float64
         for (int i = tid; i < nc; i += nt) {
-            const float y = kind[i] == 1 ? (float)sec_depth(sd, i, Ag[i]) : secf_depth(s, i, Af[i]);
+            const float y = kind[i] == 1 ? (float)cell_depth(N, i, Ag[i]) : secf_depth(s, i, Af[i]);
             yv[i] = y;
             uv[i] = y >= h_dry ? (float)Qg[i] / fmaxf(Af[i], 1e-12f) : 0.0f;
         }
@@ -506,7 +570,7 @@ __device__ __forceinline__ void net_substeps_f32_dev(const Net& N, const Consts&
     if (snap_eta) {                         // output: level z + depth and discharge (coupling.py:229-242)
         double v1 = 0.0;
         for (int i = tid; i < nc; i += nt) {
-            snap_eta[i] = (float)(N.z[i] + sec_depth(sd, i, A[i]));
+            snap_eta[i] = (float)(N.z[i] + cell_depth(N, i, A[i]));
             snap_q[i] = (float)Q[i];
             if (kind[i] <= 1) v1 += A[i] * N.dx[i];
         }
@@ -557,14 +621,13 @@ __device__ __forceinline__ CellLevel<float> cell_level(const Net& N, int i, floa
 }
 __device__ __forceinline__ CellLevel<double> cell_level(const Net& N, int i, double g, double h_dry, bool rate) {
     CellLevel<double> o;
-    const Sec s{N.b, N.m, N.yb, N.ts};
     const double A = N.A[i], dx = N.dx[i];
-    const double y = sec_depth(s, i, A), top = sec_top(s, i, y);
+    const double y = cell_depth(N, i, A), top = cell_top(N, i, y);
     o.eta = N.z[i] + y;
     o.plan = top * dx;
-    o.avail = clamp0(A - sec_bank_area(s, i)) * dx;
-    o.wet = rate && N.kind[i] <= 1 && y > h_dry;
-    o.rate = o.wet ? (fabs(N.Q[i] / fmax(A, 1e-12)) + sqrt(g * A / top)) / dx : 0.0;
+    o.avail = f64_clamp0(A - N.ab[i]) * dx;
+    o.wet = rate && N.kind[i] <= 1 && f64_ge_pos(y, h_dry) && f64_bits(y) != f64_bits(h_dry);
+    o.rate = o.wet ? f64_div(fabs(N.Q[i] / (f64_ge_pos(A, 1e-12) ? A : 1e-12)) + sqrt(g * A / top), dx, N.rdx[i]) : 0.0;
     return o;
 }
 
@@ -673,7 +736,7 @@ __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const G
         const CellLevel<R> o = cell_level(N, i, K.g, K.h_dry, s_rate != nullptr);
         eta1[i] = o.eta;
         rp[i] = gd.rarea + R(1) / o.plan;
-        if (o.wet) rate = rate > o.rate ? rate : o.rate;
+        if (o.wet) rate = o.rate > rate ? o.rate : rate;
     }
     if (s_rate) {
         for (int o = 16; o > 0; o >>= 1) {
