@@ -173,7 +173,8 @@ constexpr int NET64_THREADS = 256;
 // limiter, update, with a barrier between.  The depth a cell's update needs for its
 // friction is kept as the next substep's, the limiter's factors are applied where the
 // fluxes are summed, and the tallies are summed once per call.  3170 -> 950 FP64 warp
-// instructions per substep of 161 cells; two substeps 130 -> 48 us.
+// instructions per substep of 161 cells (two substeps with their CFL reduction through
+// the solver class 299 -> 173 us).
 __device__ __forceinline__ void net_substeps_dev(const Net& N, const Consts& c, double dt_total, int n_sub,
                                                  const double* __restrict__ forcing, double* vols, double* sm,
                                                  float* snap_eta = nullptr, float* snap_q = nullptr,

@@ -61,12 +61,12 @@ struct StripGeom {
     }
 };
 
-// Centred bed source of one cell along one axis (swe2d.py:220), from the cell's own
-// reconstruction: -g/2 (H- + H+)(Z+ - Z-), with Z+ - Z- replaced by the in-cell surface
-// slope sE (the hydrostatic part of the face momentum fluxes is carried by riemann_wb).
-// The row loop computes it where the reconstruction is formed and carries it in
-// registers to the update of that cell.
-__device__ __forceinline__ float bed_term(const KC<float>& c, const Recon& r) { return c.nhg * (r.Hm + r.Hp) * r.sE; }
+// Centred bed source of one cell along one axis (swe2d.py:220): -g/2 (H- + H+)(Z+ - Z-)
+// with Z+ - Z- replaced by the in-cell surface slope (the hydrostatic part of the face
+// momentum fluxes is carried by riemann_wb) and H- + H+ = 2 h.  The row loop computes it
+// where the reconstruction is formed and carries it in registers to the update of that
+// cell.
+__device__ __forceinline__ float bed_term(const KC<float>& c, const Recon& r) { return -2.0f * c.g * r.h0 * r.sE; }
 
 // One halo position: an interior cell, or the ghost that the x-sweep (outside in x)
 // or the y-sweep (outside in y) would see (boundaries.py:81-128), in two parts for
@@ -404,27 +404,31 @@ struct StripPipe {
         const R thW = s_th[k3 + ts - 1], thE = s_th[k3 + ts + 1];
         const Q4<R> xw = s_xf[xp + ts], xe = s_xf[xp + ts + 1], ys = s_yf[k3 + ts];
         const R h3 = s_cell[k3 + ts].a;
-        const R Fw = xw.a, Fe = xe.a, Gs = ys.a, Gn = yn.a;
-        const R sw = Fw > R(0) ? thW : thC, se = Fe > R(0) ? thC : thE;
-        const R ss = Gs > R(0) ? thS : thC, sn = Gn > R(0) ? thC : thN;
-        const R F1w = Fw * sw, F1e = Fe * se, G1s = Gs * ss, G1n = Gn * sn;
-        R a1 = per_len(-(F1e - F1w), rdx, idx);
-        R a2 = per_len(-(xe.b - xw.c), rdx, idx);
-        R a3 = per_len(-(xe.d * se - xw.d * sw), rdx, idx);
-        R b1 = per_len(-(G1n - G1s), rdy, idy);
-        R b2 = per_len(-(yn.b - ys.c), rdy, idy);
-        R b3 = per_len(-(yn.d * sn - ys.d * ss), rdy, idy);
+        R Fw = xw.a, Fe = xe.a, Gs = ys.a, Gn = yn.a, Tw = xw.d, Te = xe.d, Ts = ys.d, Tn = yn.d;
+        // donor scaling, where any cell near this warp's is limited
+        if (__any_sync(0xffffffffu, fminf(fminf(fminf(thC, thW), fminf(thE, thS)), thN) < 1.0f)) {
+            const R sw = Fw > R(0) ? thW : thC, se = Fe > R(0) ? thC : thE;
+            const R ss = Gs > R(0) ? thS : thC, sn = Gn > R(0) ? thC : thN;
+            Fw *= sw; Tw *= sw; Fe *= se; Te *= se;
+            Gs *= ss; Ts *= ss; Gn *= sn; Tn *= sn;
+        }
+        R a1 = per_len(Fw - Fe, rdx, idx);
+        R a2 = per_len(xw.c - xe.b, rdx, idx);
+        R a3 = per_len(Tw - Te, rdx, idx);
+        R b1 = per_len(Gs - Gn, rdy, idy);
+        R b2 = per_len(ys.c - yn.b, rdy, idy);
+        R b3 = per_len(Ts - Tn, rdy, idy);
         if (c.order == 2) {
             a2 = a2 + per_len(bx1, rdx, idx);
             b2 = b2 + per_len(by2, rdy, idy);
         }
         const R dh = a1 + b1, dhu = a2 + b3, dhv = a3 + b2;
         if (!do_out) return;
-        if (west) { xin += relu(F1w); xout += relu(-F1w); }
-        if (east) { xin += relu(-F1e); xout += relu(F1e); }
+        if (west) { xin += relu(Fw); xout += relu(-Fw); }
+        if (east) { xin += relu(-Fe); xout += relu(Fe); }
         if (!FULL) {
-            if (orow == 0) { yin += relu(G1s); yout += relu(-G1s); }
-            if (orow == ny - 1) { yin += relu(-G1n); yout += relu(G1n); }
+            if (orow == 0) { yin += relu(Gs); yout += relu(-Gs); }
+            if (orow == ny - 1) { yin += relu(-Gn); yout += relu(Gn); }
         }
         const unsigned i = (unsigned)orow * (unsigned)nx + (unsigned)cx;
         R hn, hun, hvn;
