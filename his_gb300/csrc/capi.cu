@@ -472,10 +472,12 @@ int32_t his_grid_step_rate_async(his_grid* g, double* rate, void* stream) {
 
 int32_t his_grid_max_rate(his_grid* g, double* rate, void* stream) {
     if (!g || !rate) return bad("grid and rate are required");
+    // the reduction stores into the pinned buffer itself: no copy to wait for
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = g->prec == HIS_PREC_F64 ? grid_reduce_f64(g, s, nullptr, true) : grid_reduce_f32(g, s, nullptr, true);
-    if (rc || (rc = fetch_out(g, s))) return rc;
-    for (int m = 0; m < g->n; ++m) rate[m] = g->h_out[m * 8 + 5];
+    int rc = g->prec == HIS_PREC_F64 ? grid_reduce_f64(g, s, g->h_out, true) : grid_reduce_f32(g, s, g->h_out, true);
+    if (rc) return rc;
+    HIS_CK(cudaStreamSynchronize(s));
+    std::memcpy(rate, g->h_out, sizeof(double) * g->n);
     return HIS_OK;
 }
 
@@ -716,29 +718,27 @@ int32_t his_net_max_rate_async(his_net* N, double* rate_wet, void* stream) {
     return HIS_OK;
 }
 
-static int net_reduce(his_net* N, cudaStream_t s) {
-    int rc = net_reduce_launch(N, s);
-    if (rc) return rc;
-    HIS_CK(cudaMemcpyAsync(N->h_out, N->d_out, sizeof(double) * 3 * N->n, cudaMemcpyDeviceToHost, s));
-    HIS_CK(cudaStreamSynchronize(s));
-    return HIS_OK;
-}
-
 int32_t his_net_max_rate(his_net* N, double* rate, int32_t* any_wet, void* stream) {
     if (!N || !rate || !any_wet) return bad("network, rate and any_wet are required");
-    int rc = net_reduce(N, (cudaStream_t)stream);
+    // the reduction stores into the pinned buffer itself: no copy to wait for
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc = net_reduce_launch(N, s, N->h_out);
     if (rc) return rc;
+    HIS_CK(cudaStreamSynchronize(s));
     for (int m = 0; m < N->n; ++m) {
-        rate[m] = N->h_out[m * 3 + 0];
-        any_wet[m] = N->h_out[m * 3 + 1] > 0.0 ? 1 : 0;
+        rate[m] = N->h_out[m * 2 + 0];
+        any_wet[m] = N->h_out[m * 2 + 1] > 0.0 ? 1 : 0;
     }
     return HIS_OK;
 }
 
 int32_t his_net_volume(his_net* N, double* vol, void* stream) {
     if (!N || !vol) return bad("network and vol are required");
-    int rc = net_reduce(N, (cudaStream_t)stream);
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc = net_reduce_launch(N, s);
     if (rc) return rc;
+    HIS_CK(cudaMemcpyAsync(N->h_out, N->d_out, sizeof(double) * 3 * N->n, cudaMemcpyDeviceToHost, s));
+    HIS_CK(cudaStreamSynchronize(s));
     for (int m = 0; m < N->n; ++m) vol[m] = N->h_out[m * 3 + 2];
     return HIS_OK;
 }
