@@ -252,6 +252,8 @@ int32_t his_grid_destroy(his_grid* g) {
     cudaFree(g->d_partials);
     cudaFree(g->d_out);
     cudaFree(g->d_scratch);
+    cudaFree(g->d_face_planes);
+    cudaFree(g->d_faces);
     if (g->h_out) cudaFreeHost(g->h_out);
     stage_free(g->params_stage);
     for (int k = 0; k < his_grid::MAX_PARTS - 1; ++k) {

@@ -38,6 +38,8 @@ struct his_grid {
     size_t scratch_bytes = 0;
     size_t table_bytes = 0;
     size_t stage_smem = 0;                   // dynamic shared memory of a stage CTA
+    void *d_face_planes = nullptr, *d_faces = nullptr;   // float64: faces of every member, their table
+    size_t cell_smem = 0;                    // and the cell kernel's shared memory
     HostStage params_stage;                  // his_grid_step_async parameters
     // The 2-D stages of a grid step run as n_parts launches over whole members' tiles
     // [part_t[k], part_t[k + 1]), part 0 on the caller's stream and part k >= 1 on

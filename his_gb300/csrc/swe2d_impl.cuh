@@ -13,15 +13,31 @@
 
 namespace his {
 
+// How a grid's stages are launched: dynamic shared memory of the stage kernel, and for
+// float64 sets with room for their faces the faces' table and the cell kernel's shared
+// memory (NULL faces: the fused kernel).
+struct StagePlan {
+    size_t smem;
+    const void* faces;
+    size_t smem_cell;
+};
+
 // Launch of one stage over `count` strip-chunks: float32 marches strips with NT threads,
-// float64 works off sub-tiles (`smem` bytes each, stage_smem).
+// float64 works off sub-tiles, faces and cells in two kernels or fused.
 template <class R, int NT, int STAGE>
 void launch_stage(const Grid<R>* grids, const StripRef* strips, const StepParams* params, const KC<R>& kc, double* part,
-                  int count, size_t smem, cudaStream_t s) {
-    if constexpr (sizeof(R) == 8)
-        tile64_kernel<STAGE><<<count, TILE64_THREADS, smem, s>>>(grids, strips, params, kc, part);
-    else
-        strip_kernel<R, NT, STAGE><<<count, NT, smem, s>>>(grids, strips, params, kc, part);
+                  int count, const StagePlan& plan, cudaStream_t s) {
+    if constexpr (sizeof(R) == 8) {
+        if (plan.faces) {
+            auto* faces = reinterpret_cast<const Faces64*>(plan.faces);
+            face64_kernel<STAGE><<<count, TILE64_THREADS, plan.smem, s>>>(grids, faces, strips, params, kc);
+            cell64_kernel<STAGE><<<count, TILE64_THREADS, plan.smem_cell, s>>>(grids, faces, strips, params, kc, part);
+        } else {
+            tile64_kernel<STAGE><<<count, TILE64_THREADS, plan.smem, s>>>(grids, strips, params, kc, part);
+        }
+    } else {
+        strip_kernel<R, NT, STAGE><<<count, NT, plan.smem, s>>>(grids, strips, params, kc, part);
+    }
 }
 
 // Strip-chunk of a member whose full chunks are w x rows cells.
@@ -43,6 +59,10 @@ int set_stage_attrs() {
         HIS_CK(cudaFuncSetAttribute(tile64_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
         HIS_CK(cudaFuncSetAttribute(tile64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
         HIS_CK(cudaFuncSetAttribute(tile64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        const int face = (int)face64_smem(TILE64_W, TILE64_H, true);
+        HIS_CK(cudaFuncSetAttribute(face64_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, face));
+        HIS_CK(cudaFuncSetAttribute(face64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, face));
+        HIS_CK(cudaFuncSetAttribute(face64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, face));
     } else {
         const int bytes = (int)StripGeom<R, NT>::smem_bytes;
         HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -51,6 +71,8 @@ int set_stage_attrs() {
     }
     return HIS_OK;
 }
+
+inline StagePlan stage_plan(const his_grid* g) { return StagePlan{g->stage_smem, g->d_faces, g->cell_smem}; }
 
 // The 2-D stages of one step on stream s (no finalize), over tiles [t0, t0 + count)
 // (default: all); a tile's partials sit at its global index.
@@ -63,10 +85,10 @@ int launch_stages(his_grid* g, cudaStream_t s, int t0 = 0, int count = -1) {
     auto* strips = reinterpret_cast<const StripRef*>(g->d_tiles) + t0;
     double* part = g->d_partials + (size_t)t0 * NPART;
     if (g->c.order == 2) {
-        launch_stage<R, NT, 1>(grids, strips, g->d_params, kc, part, count, g->stage_smem, s);
-        launch_stage<R, NT, 2>(grids, strips, g->d_params, kc, part, count, g->stage_smem, s);
+        launch_stage<R, NT, 1>(grids, strips, g->d_params, kc, part, count, stage_plan(g), s);
+        launch_stage<R, NT, 2>(grids, strips, g->d_params, kc, part, count, stage_plan(g), s);
     } else {
-        launch_stage<R, NT, 0>(grids, strips, g->d_params, kc, part, count, g->stage_smem, s);
+        launch_stage<R, NT, 0>(grids, strips, g->d_params, kc, part, count, stage_plan(g), s);
         stage_copy_kernel<R><<<count, CHUNK_THREADS, 0, s>>>(grids, strips, g->d_params);
     }
     HIS_CK(cudaGetLastError());
@@ -128,6 +150,44 @@ int launch_reduce(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
         return HIS_ERR_BAD_ARG;                                  \
     } while (0)
 
+// Face planes and bed terms of a float64 set's members and their table.  A set whose faces
+// would take more than FACES_MOST, or more than the device can give, does without (the
+// fused kernel), and so does one of fewer than FACES_LEAST cells, for which two launches more
+// cost what the faces saved would (100 x 81: 120 us per call with its CFL rate fused, 131
+// split; 163 x 201 even; 400 x 325 331 against 309).
+constexpr size_t FACES_MOST = (size_t)4 << 30, FACES_LEAST = 40000;
+inline int faces_alloc(his_grid* g) {
+    size_t total = 0, cells = 0;
+    std::vector<size_t> off(g->n);
+    auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+    for (int m = 0; m < g->n; ++m) {
+        const size_t ny = g->desc[m].ny, nx = g->desc[m].nx;
+        off[m] = total;
+        total += up(32 * ny * (nx + 1)) + up(32 * (ny + 1) * nx) + up(16 * ny * nx);
+        cells += ny * nx;
+    }
+    if (total > FACES_MOST || cells < FACES_LEAST) return HIS_OK;
+    if (cudaMalloc(&g->d_face_planes, total) != cudaSuccess) {
+        cudaGetLastError();
+        g->d_face_planes = nullptr;
+        return HIS_OK;
+    }
+    std::vector<Faces64> F(g->n);
+    for (int m = 0; m < g->n; ++m) {
+        const size_t ny = g->desc[m].ny, nx = g->desc[m].nx;
+        char* p = (char*)g->d_face_planes + off[m];
+        F[m].fx = (Q4<double>*)p;
+        p += up(32 * ny * (nx + 1));
+        F[m].fy = (Q4<double>*)p;
+        p += up(32 * (ny + 1) * nx);
+        F[m].bed = (double2*)p;
+    }
+    HIS_CK(cudaMalloc(&g->d_faces, sizeof(Faces64) * g->n));
+    HIS_CK(cudaMemcpy(g->d_faces, F.data(), sizeof(Faces64) * g->n, cudaMemcpyHostToDevice));
+    g->scratch_bytes += total;
+    return HIS_OK;
+}
+
 // Strip decomposition of every member: columns in ceil(nx / (NT - 6)) strips of equal
 // width, rows in chunks of `ty` rows; the work units are listed member by member.
 template <class R>
@@ -157,6 +217,7 @@ int grid_init_impl(his_grid* g) {
     g->scratch_bytes = total;
     HIS_CK(cudaMalloc(&g->d_scratch, total > 0 ? total : 256));
     const int wmax = g->tx;
+    int sub_w = 1, sub_h = 1;
     for (int m = 0; m < n; ++m) {
         const his_grid_desc& d = g->desc[m];
         Grid<R>& G = H[m];
@@ -180,8 +241,10 @@ int grid_init_impl(his_grid* g) {
         G.tiles_x = ns;
         G.tiles_y = nch;
         G.n_tiles = ns * nch;
-        if constexpr (sizeof(R) == 8)
-            g->stage_smem = std::max(g->stage_smem, stage_smem<R, 0>(w, hch, g->c.order));
+        if constexpr (sizeof(R) == 8) {
+            sub_w = std::max(sub_w, tile64_part(w, TILE64_W));
+            sub_h = std::max(sub_h, tile64_part(hch, TILE64_H));
+        }
         G.tile0 = (int)strips.size();
         g->tile0[m] = G.tile0;
         g->ntile[m] = G.n_tiles;
@@ -199,7 +262,12 @@ int grid_init_impl(his_grid* g) {
         G.pk = (R*)d.peak_h; G.ps = (R*)d.peak_speed;
     }
     g->n_tiles = (int)strips.size();
-    if constexpr (sizeof(R) == 4)
+    if constexpr (sizeof(R) == 8) {
+        if ((rc = faces_alloc(g)) != HIS_OK) return rc;
+        const bool second = g->c.order == 2;
+        g->stage_smem = g->d_faces ? face64_smem(sub_w, sub_h, second) : tile64_smem(sub_w, sub_h, second);
+        g->cell_smem = cell64_smem(sub_w, sub_h);
+    } else
         g->stage_smem = g->nt == 64 ? stage_smem<R, 64>(0, 0, 0) : g->nt == 128 ? stage_smem<R, 128>(0, 0, 0)
                       : g->nt == 224 ? stage_smem<R, 224>(0, 0, 0) : stage_smem<R, 352>(0, 0, 0);
     HIS_CK(cudaMalloc(&g->d_grids, sizeof(Grid<R>) * n));
@@ -312,12 +380,12 @@ int eng_profile_nt(his_grid* g, his_engine* E, int n_steps, double* ms) {
             cudaEventRecord(ev[5], E->s1);
         }
         if (g->c.order == 2) {
-            launch_stage<R, NT, 1>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, g->stage_smem, E->s0);
+            launch_stage<R, NT, 1>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, stage_plan(g), E->s0);
             cudaEventRecord(ev[2], E->s0);
-            launch_stage<R, NT, 2>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, g->stage_smem, E->s0);
+            launch_stage<R, NT, 2>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, stage_plan(g), E->s0);
         } else {
             cudaEventRecord(ev[2], E->s0);
-            launch_stage<R, NT, 0>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, g->stage_smem, E->s0);
+            launch_stage<R, NT, 0>(grids, strips, g->d_params, kc, g->d_partials, g->n_tiles, stage_plan(g), E->s0);
             stage_copy_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, E->s0>>>(grids, strips, g->d_params);
         }
         cudaEventRecord(ev[3], E->s0);
@@ -413,7 +481,7 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
     auto* part = reinterpret_cast<double*>(base + L.o_part);
     auto* out = reinterpret_cast<double*>(base + L.o_out);
     const KC<R> kc = make_kc<R>(c);
-    const size_t smem = stage_smem<R, NT>(L.w, L.hch, c.order);
+    const StagePlan smem{stage_smem<R, NT>(L.w, L.hch, c.order), nullptr, 0};
     if (c.order == 2) {
         launch_stage<R, NT, 1>(grid, strips, params, kc, part, L.n_strips, smem, s);
         launch_stage<R, NT, 2>(grid, strips, params, kc, part, L.n_strips, smem, s);

@@ -19,6 +19,9 @@
 // update with, in the last stage, rain, infiltration, retention, friction, CFL rate and
 // peaks (swe2d.py:305-371).
 //
+// This kernel does a stage in one launch; face64_kernel and cell64_kernel below do it in two
+// with each face computed once, and serve every set with room for its faces.
+//
 // Measured (one member, 400 x 325 cells, infiltration and retention on, 58 x 16 chunks):
 // 1340 us per step with the row-marching kernel this replaces, at 2000 FP64 instructions
 // per cell and one warp on half of the schedulers; 250 us here, at 780 per cell with the
@@ -123,6 +126,222 @@ __device__ __forceinline__ double warp_max_run(double v) {
     return v;
 }
 
+// Constants of a member's step, the same for all its cells
+struct Step64 {
+    double dt, lamx, lamy, rdt, dtg, tt;
+    unsigned feat;
+    const StepParams& pr;
+    __device__ __forceinline__ Step64(const KC<double>& c, const Grid<double>& gd, const StepParams& p, int stage)
+        : dt(p.dt), lamx(p.dt / gd.dx), lamy(p.dt / gd.dy), rdt(p.rain * p.dt), dtg(p.dt * c.g),
+          tt(clamp0(p.t - gd.rt0)), feat(grid_features(gd) | (stage != 1 && p.snap_h ? FEAT_SNAP : 0u)), pr(p) {}
+};
+
+// Running sums of one thread's cells
+struct Acc64 {
+    double clip = 0, xin = 0, xout = 0, yin = 0, yout = 0, infil = 0, rainw = 0, rate = 0, hsum = 0, ssum = 0, hmax = 0;
+};
+
+struct Pos64 {
+    int gx, gy;
+};
+
+// Limiter of one cell inside the grid from its faces' mass fluxes (swe2d.py:259-264)
+__device__ __forceinline__ double theta64(const Step64& k, double h, double Fw, double Fe, double Fs, double Fn) {
+    const double need = fma(k.lamx, f64_relu(Fe) + f64_relu(-Fw), k.lamy * (f64_relu(Fn) + f64_relu(-Fs)));
+    return f64_pos(need) && f64_key(need) > f64_key(h) ? h / need : 1.0;
+}
+
+// Update of cell j from its faces, the limiters around it, its depth hc and the bed terms
+// (slope of h + z less slope of h, in x and y) (swe2d.py:305-371)
+template <int STAGE>
+__device__ __forceinline__ void update64(const KC<double>& c, const Grid<double>& gd, const Step64& k, Acc64& acc, Pos64 p,
+                                         unsigned j, double hc, Q4<double> W, Q4<double> E, Q4<double> S, Q4<double> N,
+                                         double thC, double thW, double thE, double thS, double thN, double bx,
+                                         double by) {
+    const unsigned long long one = f64_bits(1.0);
+    if (((f64_bits(thC) ^ one) | (f64_bits(thW) ^ one) | (f64_bits(thE) ^ one) | (f64_bits(thS) ^ one) |
+         (f64_bits(thN) ^ one)) != 0ull) {
+        const double sw = f64_pos(W.a) ? thW : thC, se = f64_pos(E.a) ? thC : thE;
+        const double ss = f64_pos(S.a) ? thS : thC, sn = f64_pos(N.a) ? thC : thN;
+        W.a *= sw; W.d *= sw; E.a *= se; E.d *= se;
+        S.a *= ss; S.d *= ss; N.a *= sn; N.d *= sn;
+    }
+    if (p.gx == 0) { acc.xin += f64_relu(W.a); acc.xout += f64_relu(-W.a); }
+    if (p.gx == gd.nx - 1) { acc.xin += f64_relu(-E.a); acc.xout += f64_relu(E.a); }
+    if (p.gy == 0) { acc.yin += f64_relu(S.a); acc.yout += f64_relu(-S.a); }
+    if (p.gy == gd.ny - 1) { acc.yin += f64_relu(-N.a); acc.yout += f64_relu(N.a); }
+    double px = W.c - E.b, py = S.c - N.b;
+    if (STAGE != 0) {
+        // bed source -g/2 (H- + H+)(Z+ - Z-) = -g h (slope of h + z less slope of h)
+        const double gh = -(c.g * hc);
+        px = fma(gh, bx, px);
+        py = fma(gh, by, py);
+    }
+    const double dh = fma(k.lamx, W.a - E.a, k.lamy * (S.a - N.a));
+    const double dhu = fma(k.lamx, px, k.lamy * (S.d - N.d));
+    const double dhv = fma(k.lamx, W.d - E.d, k.lamy * py);
+    double hn, hun, hvn;
+    if (STAGE == 2) {
+        hn = 0.5 * (gd.h[j] + (hc + dh));
+        hun = 0.5 * (gd.hu[j] + (gd.hu1[j] + dhu));
+        hvn = 0.5 * (gd.hv[j] + (gd.hv1[j] + dhv));
+    } else {
+        hn = hc + dh;
+        hun = gd.hu[j] + dhu;
+        hvn = gd.hv[j] + dhv;
+    }
+    if (f64_neg(hn)) { acc.clip -= hn; hn = 0.0; }
+    if (STAGE == 1) {
+        gd.h1[j] = hn; gd.hu1[j] = hun; gd.hv1[j] = hvn;
+        return;
+    }
+    // ---- rain, Horton infiltration, retention store (swe2d.py:330-360)
+    if (k.feat & FEAT_RAINW) {
+        const double add = k.rdt * gd.rw[j];
+        hn = hn + add;
+        acc.rainw += add;
+    } else {
+        hn = hn + k.rdt;
+    }
+    const double hp = hn;              // depth the momentum belongs to
+    double sf = 0.0;
+    if (k.feat & FEAT_STORE) sf = gd.sf[j];
+    if (k.feat & FEAT_HORTON) {
+        const double fc = gd.fc[j];
+        const double pot = fma(gd.f0[j] - fc, exp(-gd.k[j] * k.tt), fc) * k.dt;
+        const double take = f64_min(pot, hn);
+        hn = hn - take;
+        double taken = take;
+        if (k.feat & FEAT_STORE) {
+            const double tks = f64_min(pot - take, sf);
+            sf = sf - tks;
+            taken = taken + tks;
+        }
+        acc.infil += taken;
+        gd.ic[j] = gd.ic[j] + taken;
+    }
+    if (k.feat & FEAT_STORE) {
+        const double fill = f64_min(f64_clamp0(gd.S[j] - sf), hn);
+        hn = hn - fill;
+        sf = sf + fill;
+        gd.sf[j] = sf;
+        acc.ssum += sf;
+    }
+    // ---- semi-implicit Manning friction (swe2d.py:362-370).  Water lost takes its
+    // momentum along, so the velocity is that before the losses; dry cells rest
+    double u2 = 0.0, v2 = 0.0;
+    if (f64_ge_pos(hn, c.h_dry)) {
+        const double r = __drcp_rn(hn);
+        const bool plain = f64_ge_pos(hn, c.h_kp);
+        double u, v;
+        if (plain) {
+            const double rp = f64_bits(hp) == f64_bits(hn) ? r : __drcp_rn(hp);
+            u = f64_div(hun, hp, rp);
+            v = f64_div(hvn, hp, rp);
+        } else {
+            const double keep = f64_pos(hp) ? hn / hp : 0.0;
+            kp_velocity(c, hn, hun * keep, hvn * keep, u, v);
+        }
+        const double sq = fma(u, u, v * v);
+        if (f64_pos(sq)) {             // water at rest has no friction (nor a fast root)
+            const double nm = gd.n[j];
+            const double p43 = f64_pow43(hn);
+            const double fac = p43 / fma(k.dtg * nm * nm, sqrt(sq), p43);
+            u = u * fac;
+            v = v * fac;
+        }
+        hun = hn * u;
+        hvn = hn * v;
+        // KP velocities of the new state, for the CFL rate of the next step, the running
+        // peak speed and the outputs (swe2d.py:161-167, coupling.py:229-242)
+        if (plain) {
+            u2 = f64_div(hun, hn, r);
+            v2 = f64_div(hvn, hn, r);
+        } else {
+            kp_velocity(c, hn, hun, hvn, u2, v2);
+        }
+    } else {
+        hun = 0.0;
+        hvn = 0.0;
+    }
+    if (STAGE == 2) {
+        gd.h[j] = hn; gd.hu[j] = hun; gd.hv[j] = hvn;
+    } else {
+        gd.h1[j] = hn; gd.hu1[j] = hun; gd.hv1[j] = hvn;
+    }
+    if (k.feat & FEAT_PEAK) gd.pk[j] = f64_max_run(gd.pk[j], hn);
+    if (k.feat & FEAT_PSPEED) gd.ps[j] = f64_max_run(gd.ps[j], sqrt(fma(u2, u2, v2 * v2)));
+    if (k.feat & FEAT_SNAP) {
+        k.pr.snap_h[j] = (float)hn;
+        k.pr.snap_u[j] = (float)u2;
+        k.pr.snap_v[j] = (float)v2;
+    }
+    if (f64_ge_pos(hn, c.h_dry) && f64_bits(hn) != f64_bits(c.h_dry))
+        acc.rate = f64_max_run(acc.rate, rate64(c, hn, u2, v2, gd.rdx, gd.rdy, gd.idx, gd.idy));
+    acc.hsum += hn;
+    acc.hmax = f64_max_run(acc.hmax, hn);
+}
+
+// Partial sums of a strip-chunk: lanes, then warps in order
+template <int STAGE>
+__device__ __forceinline__ void store_acc64(const Acc64& acc, double* out) {
+    constexpr int NT = TILE64_THREADS, NV = STAGE == 1 ? 5 : 11;
+    __shared__ double red[NT / 32][NV];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double v[NV] = {warp_sum_sparse(acc.clip), warp_sum_sparse(acc.xin), warp_sum_sparse(acc.xout),
+                    warp_sum_sparse(acc.yin), warp_sum_sparse(acc.yout)};
+    if constexpr (STAGE != 1) {
+        v[5] = warp_sum_sparse(acc.infil);
+        v[6] = warp_sum_sparse(acc.rainw);
+        v[7] = warp_max_run(acc.rate);
+        v[8] = warp_sum_sparse(acc.hsum);
+        v[9] = warp_sum_sparse(acc.ssum);
+        v[10] = warp_max_run(acc.hmax);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) red[warp][q] = v[q];
+    }
+    __syncthreads();
+    if (tid < NV) {
+        double a = red[0][tid];
+        if (tid == 7 || tid == 10) {
+            for (int w = 1; w < NT / 32; ++w) a = f64_max_run(a, red[w][tid]);
+        } else {
+            for (int w = 1; w < NT / 32; ++w) a += red[w][tid];
+        }
+        const int b = STAGE == 2 ? P_CLIP2 : P_CLIP1;
+        out[tid < 5 ? b + tid : P_INFIL + (tid - 5)] = a;
+    }
+}
+
+// Slopes of the middle cell o of three {h, u, v, e} along an axis; zero beside dry cells
+// (swe2d.py:205-219)
+__device__ __forceinline__ Q4<double> slope64(const KC<double>& c, const Q4<double>& m, const Q4<double>& o,
+                                              const Q4<double>& q) {
+    Q4<double> s{0.0, 0.0, 0.0, 0.0};
+    if (f64_ge_pos(m.a, c.h_dry) && f64_ge_pos(o.a, c.h_dry) && f64_ge_pos(q.a, c.h_dry)) {
+        s.a = f64_minmod(o.a - m.a, q.a - o.a);
+        s.b = f64_minmod(o.b - m.b, q.b - o.b);
+        s.c = f64_minmod(o.c - m.c, q.c - o.c);
+        s.d = f64_minmod(o.d - m.d, q.d - o.d);
+    }
+    return s;
+}
+
+// The face's flux along y: normal velocity first
+template <bool SECOND>
+__device__ __forceinline__ Q4<double> face64_along(bool alongx, const KC<double>& c, Q4<double> L, Q4<double> R,
+                                                   Q4<double> sl, Q4<double> sr) {
+    if (!alongx) {
+        double t = L.b; L.b = L.c; L.c = t;
+        t = R.b; R.b = R.c; R.c = t;
+        t = sl.b; sl.b = sl.c; sl.c = t;
+        t = sr.b; sr.b = sr.c; sr.c = t;
+    }
+    return face64<SECOND>(c, L, R, sl, sr);
+}
+
 // STAGE: 0 = first-order full step (into the stage buffers), 1 = RK stage 1, 2 = RK stage
 // 2 and sources, as strip_kernel's.
 template <int STAGE>
@@ -131,11 +350,10 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
                                                                    const StepParams* __restrict__ params,
                                                                    const KC<double> kc, double* __restrict__ partials) {
     constexpr bool SECOND = STAGE != 0;
-    constexpr int NT = TILE64_THREADS, NV = STAGE == 1 ? 5 : 11;
+    constexpr int NT = TILE64_THREADS;
     extern __shared__ __align__(32) unsigned char smem_raw[];
     __shared__ Grid<double> gd;
     __shared__ double bcv[4];
-    __shared__ double red[NT / 32][NV];
     KC<double> c = kc;
     c.order = SECOND ? 2 : 1;
     const StripRef sr = strips[blockIdx.x];
@@ -153,11 +371,8 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
     const double* __restrict__ HU = STAGE == 2 ? gd.hu1 : gd.hu;
     const double* __restrict__ HV = STAGE == 2 ? gd.hv1 : gd.hv;
     const int nx = gd.nx, ny = gd.ny;
-    const double dt = pr.dt, lamx = dt / gd.dx, lamy = dt / gd.dy;
-    const unsigned feat = grid_features(gd) | (STAGE != 1 && pr.snap_h ? FEAT_SNAP : 0u);
-    const double rdt = pr.rain * dt, dtg = dt * c.g;
-    const double tt = clamp0(pr.t - gd.rt0);
-    double clip = 0, xin = 0, xout = 0, yin = 0, yout = 0, infil = 0, rainw = 0, rate = 0, hsum = 0, ssum = 0, hmax = 0;
+    const Step64 k(c, gd, pr, STAGE);
+    Acc64 acc;
 
     // parts of at most the member's sub-tile, which the launch's shared memory is sized for
     const int cw = tile64_part(sr.w, sr.sub_w), ch = tile64_part(sr.y1 - sr.y0, sr.sub_h);
@@ -196,9 +411,9 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
                 for (int i = tid; i < n; i += NT) {
                     const bool alongx = i < nsx32;
                     if (alongx && i >= nsx) continue;
-                    const int k = alongx ? i : i - nsx32;
-                    const int iy = alongx ? bx.quot(k) : by.quot(k);
-                    const int x = alongx ? k - iy * LX - 2 : k - iy * LY - 1, y = iy - (alongx ? 1 : 2);
+                    const int e = alongx ? i : i - nsx32;
+                    const int iy = alongx ? bx.quot(e) : by.quot(e);
+                    const int x = alongx ? e - iy * LX - 2 : e - iy * LY - 1, y = iy - (alongx ? 1 : 2);
                     // on the cells of the faces below, within the rows (columns) of the grid
                     if (alongx) {
                         if ((unsigned)(Y0 + y) >= (unsigned)ny || ((y < 0 || y >= h) && (x < -1 || x > w))) continue;
@@ -207,15 +422,9 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
                     }
                     const int p = (y + 3) * LC + x + 3, d = alongx ? 1 : LC;
                     const Q4<double> m = s_c[p - d], o = s_c[p], q = s_c[p + d];
-                    Q4<double> s{0.0, 0.0, 0.0, 0.0};
-                    if (f64_ge_pos(m.a, c.h_dry) && f64_ge_pos(o.a, c.h_dry) && f64_ge_pos(q.a, c.h_dry)) {
-                        s.a = f64_minmod(o.a - m.a, q.a - o.a);
-                        s.b = f64_minmod(o.b - m.b, q.b - o.b);
-                        s.c = f64_minmod(o.c - m.c, q.c - o.c);
-                        s.d = f64_minmod(o.d - m.d, q.d - o.d);
-                    }
-                    if (alongx) s_sx[k] = s;
-                    else s_sy[k] = s;
+                    const Q4<double> s = slope64(c, m, o, q);
+                    if (alongx) s_sx[e] = s;
+                    else s_sy[e] = s;
                 }
                 __syncthreads();
             }
@@ -225,9 +434,9 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
                 for (int i = tid; i < n; i += NT) {
                     const bool alongx = i < nfx32;
                     if (alongx && i >= nfx) continue;
-                    const int k = alongx ? i : i - nfx32;
-                    const int iy = alongx ? bx.quot(k) : by.quot(k);
-                    const int x = k - iy * (alongx ? LF : LG) - 1, y = iy - 1;
+                    const int e = alongx ? i : i - nfx32;
+                    const int iy = alongx ? bx.quot(e) : by.quot(e);
+                    const int x = e - iy * (alongx ? LF : LG) - 1, y = iy - 1;
                     // the faces of the sub-tile's cells and of their four neighbours inside the grid
                     if (alongx) {
                         if ((unsigned)(Y0 + y) >= (unsigned)ny || (unsigned)(X0 + x) > (unsigned)nx ||
@@ -237,22 +446,15 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
                             ((x < 0 || x >= w) && (y < 0 || y > h))) continue;
                     }
                     const int p = (y + 3) * LC + x + 3;
-                    Q4<double> L = s_c[p - (alongx ? 1 : LC)], R = s_c[p];
                     Q4<double> sl{}, sr_{};
                     if (SECOND) {
                         const Q4<double>* s = alongx ? s_sx + (y + 1) * LX + x + 2 : s_sy + (y + 2) * LY + x + 1;
                         sl = s[alongx ? -1 : -LY];
                         sr_ = s[0];
                     }
-                    if (!alongx) {                 // normal velocity first
-                        double t = L.b; L.b = L.c; L.c = t;
-                        t = R.b; R.b = R.c; R.c = t;
-                        t = sl.b; sl.b = sl.c; sl.c = t;
-                        t = sr_.b; sr_.b = sr_.c; sr_.c = t;
-                    }
-                    const Q4<double> f = face64<SECOND>(c, L, R, sl, sr_);
-                    if (alongx) s_fx[k] = f;
-                    else s_fy[k] = f;
+                    const Q4<double> f = face64_along<SECOND>(alongx, c, s_c[p - (alongx ? 1 : LC)], s_c[p], sl, sr_);
+                    if (alongx) s_fx[e] = f;
+                    else s_fy[e] = f;
                 }
             }
             __syncthreads();
@@ -262,13 +464,11 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
                     const int iy = by.quot(i), y = iy - 1, x = i - iy * LT - 1;
                     const bool xi = x >= 0 && x < w, yi = y >= 0 && y < h;
                     if (!xi && !yi) continue;
-                    double th = 1.0;               // swe2d.py:259-264; 1 outside the grid
+                    double th = 1.0;               // outside the grid
                     if ((unsigned)(X0 + x) < (unsigned)nx && (unsigned)(Y0 + y) < (unsigned)ny) {
                         const int fx = (y + 1) * LF + x + 1, fy = (y + 1) * LG + x + 1;
-                        const double need = fma(lamx, f64_relu(s_fx[fx + 1].a) + f64_relu(-s_fx[fx].a),
-                                                lamy * (f64_relu(s_fy[fy + LG].a) + f64_relu(-s_fy[fy].a)));
-                        const double hh = s_c[(y + 3) * LC + x + 3].a;
-                        if (f64_pos(need) && f64_key(need) > f64_key(hh)) th = hh / need;
+                        th = theta64(k, s_c[(y + 3) * LC + x + 3].a, s_fx[fx].a, s_fx[fx + 1].a, s_fy[fy].a,
+                                     s_fy[fy + LG].a);
                     }
                     s_th[i] = th;
                 }
@@ -278,165 +478,201 @@ __global__ void __launch_bounds__(TILE64_THREADS, 1) tile64_kernel(const Grid<do
             for (int i = tid; i < w * h; i += NT) {
                 const int y = by.quot(i), x = i - y * w, gx = X0 + x, gy = Y0 + y;
                 const int fx = (y + 1) * LF + x + 1, fy = (y + 1) * LG + x + 1, t0 = (y + 1) * LT + x + 1;
-                Q4<double> W = s_fx[fx], E = s_fx[fx + 1], S = s_fy[fy], N = s_fy[fy + LG];
-                const double thC = s_th[t0], thW = s_th[t0 - 1], thE = s_th[t0 + 1], thS = s_th[t0 - LT],
-                             thN = s_th[t0 + LT];
-                const unsigned long long one = f64_bits(1.0);
-                if (((f64_bits(thC) ^ one) | (f64_bits(thW) ^ one) | (f64_bits(thE) ^ one) | (f64_bits(thS) ^ one) |
-                     (f64_bits(thN) ^ one)) != 0ull) {
-                    const double sw = f64_pos(W.a) ? thW : thC, se = f64_pos(E.a) ? thC : thE;
-                    const double ss = f64_pos(S.a) ? thS : thC, sn = f64_pos(N.a) ? thC : thN;
-                    W.a *= sw; W.d *= sw; E.a *= se; E.d *= se;
-                    S.a *= ss; S.d *= ss; N.a *= sn; N.d *= sn;
-                }
-                if (gx == 0) { xin += f64_relu(W.a); xout += f64_relu(-W.a); }
-                if (gx == nx - 1) { xin += f64_relu(-E.a); xout += f64_relu(E.a); }
-                if (gy == 0) { yin += f64_relu(S.a); yout += f64_relu(-S.a); }
-                if (gy == ny - 1) { yin += f64_relu(-N.a); yout += f64_relu(N.a); }
-                const double hc = s_c[(y + 3) * LC + x + 3].a;
-                double px = W.c - E.b, py = S.c - N.b;
+                double ex = 0.0, ey = 0.0;
                 if (SECOND) {
-                    // bed source -g/2 (H- + H+)(Z+ - Z-) = -g h (slope of h + z less slope of h)
                     const Q4<double> sx = s_sx[(y + 1) * LX + x + 2], sy = s_sy[(y + 2) * LY + x + 1];
-                    const double gh = -(c.g * hc);
-                    px = fma(gh, sx.d - sx.a, px);
-                    py = fma(gh, sy.d - sy.a, py);
+                    ex = sx.d - sx.a;
+                    ey = sy.d - sy.a;
                 }
-                const double dh = fma(lamx, W.a - E.a, lamy * (S.a - N.a));
-                const double dhu = fma(lamx, px, lamy * (S.d - N.d));
-                const double dhv = fma(lamx, W.d - E.d, lamy * py);
-                const unsigned j = (unsigned)gy * (unsigned)nx + (unsigned)gx;
-                double hn, hun, hvn;
-                if (STAGE == 2) {
-                    hn = 0.5 * (gd.h[j] + (hc + dh));
-                    hun = 0.5 * (gd.hu[j] + (gd.hu1[j] + dhu));
-                    hvn = 0.5 * (gd.hv[j] + (gd.hv1[j] + dhv));
-                } else {
-                    hn = hc + dh;
-                    hun = gd.hu[j] + dhu;
-                    hvn = gd.hv[j] + dhv;
-                }
-                if (f64_neg(hn)) { clip -= hn; hn = 0.0; }
-                if (STAGE == 1) {
-                    gd.h1[j] = hn; gd.hu1[j] = hun; gd.hv1[j] = hvn;
-                    continue;
-                }
-                // ---- rain, Horton infiltration, retention store (swe2d.py:330-360)
-                if (feat & FEAT_RAINW) {
-                    const double add = rdt * gd.rw[j];
-                    hn = hn + add;
-                    rainw += add;
-                } else {
-                    hn = hn + rdt;
-                }
-                const double hp = hn;              // depth the momentum belongs to
-                double sf = 0.0;
-                if (feat & FEAT_STORE) sf = gd.sf[j];
-                if (feat & FEAT_HORTON) {
-                    const double fc = gd.fc[j];
-                    const double pot = fma(gd.f0[j] - fc, exp(-gd.k[j] * tt), fc) * dt;
-                    const double take = f64_min(pot, hn);
-                    hn = hn - take;
-                    double taken = take;
-                    if (feat & FEAT_STORE) {
-                        const double tks = f64_min(pot - take, sf);
-                        sf = sf - tks;
-                        taken = taken + tks;
-                    }
-                    infil += taken;
-                    gd.ic[j] = gd.ic[j] + taken;
-                }
-                if (feat & FEAT_STORE) {
-                    const double fill = f64_min(f64_clamp0(gd.S[j] - sf), hn);
-                    hn = hn - fill;
-                    sf = sf + fill;
-                    gd.sf[j] = sf;
-                    ssum += sf;
-                }
-                // ---- semi-implicit Manning friction (swe2d.py:362-370).  Water lost takes its
-                // momentum along, so the velocity is that before the losses; dry cells rest
-                double u2 = 0.0, v2 = 0.0;
-                if (f64_ge_pos(hn, c.h_dry)) {
-                    const double r = __drcp_rn(hn);
-                    const bool plain = f64_ge_pos(hn, c.h_kp);
-                    double u, v;
-                    if (plain) {
-                        const double rp = f64_bits(hp) == f64_bits(hn) ? r : __drcp_rn(hp);
-                        u = f64_div(hun, hp, rp);
-                        v = f64_div(hvn, hp, rp);
-                    } else {
-                        const double keep = f64_pos(hp) ? hn / hp : 0.0;
-                        kp_velocity(c, hn, hun * keep, hvn * keep, u, v);
-                    }
-                    const double sq = fma(u, u, v * v);
-                    if (f64_pos(sq)) {             // water at rest has no friction (nor a fast root)
-                        const double nm = gd.n[j];
-                        const double p43 = f64_pow43(hn);
-                        const double fac = p43 / fma(dtg * nm * nm, sqrt(sq), p43);
-                        u = u * fac;
-                        v = v * fac;
-                    }
-                    hun = hn * u;
-                    hvn = hn * v;
-                    // KP velocities of the new state, for the CFL rate of the next step, the running
-                    // peak speed and the outputs (swe2d.py:161-167, coupling.py:229-242)
-                    if (plain) {
-                        u2 = f64_div(hun, hn, r);
-                        v2 = f64_div(hvn, hn, r);
-                    } else {
-                        kp_velocity(c, hn, hun, hvn, u2, v2);
-                    }
-                } else {
-                    hun = 0.0;
-                    hvn = 0.0;
-                }
-                if (STAGE == 2) {
-                    gd.h[j] = hn; gd.hu[j] = hun; gd.hv[j] = hvn;
-                } else {
-                    gd.h1[j] = hn; gd.hu1[j] = hun; gd.hv1[j] = hvn;
-                }
-                if (feat & FEAT_PEAK) gd.pk[j] = f64_max_run(gd.pk[j], hn);
-                if (feat & FEAT_PSPEED) gd.ps[j] = f64_max_run(gd.ps[j], sqrt(fma(u2, u2, v2 * v2)));
-                if (feat & FEAT_SNAP) {
-                    pr.snap_h[j] = (float)hn;
-                    pr.snap_u[j] = (float)u2;
-                    pr.snap_v[j] = (float)v2;
-                }
-                if (f64_ge_pos(hn, c.h_dry) && f64_bits(hn) != f64_bits(c.h_dry))
-                    rate = f64_max_run(rate, rate64(c, hn, u2, v2, gd.rdx, gd.rdy, gd.idx, gd.idy));
-                hsum += hn;
-                hmax = f64_max_run(hmax, hn);
+                update64<STAGE>(c, gd, k, acc, Pos64{gx, gy}, (unsigned)gy * (unsigned)nx + (unsigned)gx,
+                                s_c[(y + 3) * LC + x + 3].a, s_fx[fx], s_fx[fx + 1], s_fy[fy], s_fy[fy + LG], s_th[t0],
+                                s_th[t0 - 1], s_th[t0 + 1], s_th[t0 - LT], s_th[t0 + LT], ex, ey);
             }
         }
+    store_acc64<STAGE>(acc, partials + (size_t)blockIdx.x * NPART);
+}
 
-    // partial sums of the strip-chunk: lanes, then warps in order
-    const int lane = tid & 31, warp = tid >> 5;
-    double v[NV] = {warp_sum_sparse(clip), warp_sum_sparse(xin), warp_sum_sparse(xout), warp_sum_sparse(yin),
-                    warp_sum_sparse(yout)};
-    if constexpr (STAGE != 1) {
-        v[5] = warp_sum_sparse(infil);
-        v[6] = warp_sum_sparse(rainw);
-        v[7] = warp_max_run(rate);
-        v[8] = warp_sum_sparse(hsum);
-        v[9] = warp_sum_sparse(ssum);
-        v[10] = warp_max_run(hmax);
+// ------------------------------------------------ faces and cells in two kernels
+// The sub-tile above computes the faces around its cells' neighbours as well, 2.4 to 3.3
+// faces per cell, because the limiter of a neighbour enters a cell's update.  With room for
+// the faces in memory, one kernel computes each face once and a second one limits and
+// updates from them: 2 faces per cell, 220 FP64 instructions per cell in stage 1 against 330,
+// for 80 bytes per cell written and about 200 read (mostly from L2) per stage, which a kernel
+// at 2 FP64 lanes per cycle and SM hardly notices.  The cells' arithmetic and the order of
+// their sums are the fused kernel's: the same bits.  A step of 400 x 325 cells 249 -> 228 us,
+// of four such members 901 -> 752, of 16 of 100 x 81 273 -> 236; 100 x 81 alone 55 -> 52.
+// (512 threads per CTA: faces 72 -> 69 us, cells 52 -> 55 and 17 -> 18.)
+struct Faces64 {
+    Q4<double>*fx, *fy;              // west faces (ny x (nx + 1)) and south faces ((ny + 1) x nx)
+    double2* bed;                    // per cell: slope of h + z less slope of h, in x and y
+};
+// Shared memory of the face kernel over a w x h sub-tile (cells with a two-cell halo, slopes)
+__host__ __device__ constexpr size_t face64_smem(int w, int h, bool second) {
+    return 32 * ((size_t)(w + 4) * (h + 4) + (second ? (size_t)(w + 2) * h + (size_t)w * (h + 2) : 0));
+}
+__host__ __device__ constexpr size_t cell64_smem(int w, int h) { return 8 * (size_t)(w + 2) * (h + 2); }
+
+template <int STAGE>
+__global__ void __launch_bounds__(TILE64_THREADS, 2) face64_kernel(const Grid<double>* __restrict__ grids,
+                                                                   const Faces64* __restrict__ faces,
+                                                                   const StripRef* __restrict__ strips,
+                                                                   const StepParams* __restrict__ params,
+                                                                   const KC<double> kc) {
+    constexpr bool SECOND = STAGE != 0;
+    constexpr int NT = TILE64_THREADS;
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    __shared__ Grid<double> gd;
+    __shared__ double bcv[4];
+    KC<double> c = kc;
+    c.order = SECOND ? 2 : 1;
+    const StripRef sr = strips[blockIdx.x];
+    const StepParams& pr = params[sr.member];
+    if (!pr.active) return;
+    const int tid = threadIdx.x;
+    {
+        const unsigned* src = reinterpret_cast<const unsigned*>(grids + sr.member);
+        unsigned* dst = reinterpret_cast<unsigned*>(&gd);
+        for (int k = tid; k < (int)(sizeof(Grid<double>) / 4); k += NT) dst[k] = src[k];
     }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) red[warp][k] = v[k];
-    }
+    if (tid < 4) bcv[tid] = par_bc<double>(pr, STAGE == 2, tid);
+    const Faces64 out = faces[sr.member];
     __syncthreads();
-    if (tid < NV) {
-        double a = red[0][tid];
-        if (tid == 7 || tid == 10) {
-            for (int k = 1; k < NT / 32; ++k) a = f64_max_run(a, red[k][tid]);
-        } else {
-            for (int k = 1; k < NT / 32; ++k) a += red[k][tid];
+    const double* __restrict__ H = STAGE == 2 ? gd.h1 : gd.h;
+    const double* __restrict__ HU = STAGE == 2 ? gd.hu1 : gd.hu;
+    const double* __restrict__ HV = STAGE == 2 ? gd.hv1 : gd.hv;
+    const int nx = gd.nx, ny = gd.ny;
+    const int cw = tile64_part(sr.w, sr.sub_w), ch = tile64_part(sr.y1 - sr.y0, sr.sub_h);
+    for (int Y0 = sr.y0; Y0 < sr.y1; Y0 += ch)
+        for (int X0 = sr.x0; X0 < sr.x0 + sr.w; X0 += cw) {
+            const int w = min(cw, sr.x0 + sr.w - X0), h = min(ch, sr.y1 - Y0);
+            // the grid's last column and row carry the faces beyond them as well
+            const int xe = X0 + w == nx, ye = Y0 + h == ny;
+            // cells at (x + 2, y + 2), x-slopes (x + 1, y), y-slopes (x, y + 1) of cell (x, y)
+            const int LC = w + 4, LX = w + 2;
+            Q4<double>* s_c = reinterpret_cast<Q4<double>*>(smem_raw);
+            Q4<double>* s_sx = s_c + LC * (h + 4);
+            Q4<double>* s_sy = s_sx + LX * h;
+            __syncthreads();                       // the last sub-tile's readers are done
+            {
+                const Div20 by(LC);
+                for (int i = tid; i < LC * (h + 4); i += NT) {
+                    const int iy = by.quot(i), y = iy - 2, x = i - iy * LC - 2;
+                    const bool xin = x >= 0 && x < w, yin = y >= 0 && y < h;
+                    if (!(yin && x <= w + xe) && !(xin && y <= h + ye)) continue;
+                    const HaloRaw<double> a = halo_fetch(c, gd, H, HU, HV, X0 + x, Y0 + y);
+                    Q4<double> q;
+                    halo_build(c, gd, bcv, a, X0 + x, Y0 + y, q.a, q.b, q.c, q.d);
+                    q.d = q.a + q.d;
+                    s_c[i] = q;
+                }
+            }
+            __syncthreads();
+            if (SECOND) {
+                // x-slopes of columns -1 .. w - 1 (+ 1), y-slopes of rows -1 .. h - 1 (+ 1)
+                const int wx = w + 1 + xe, hy = h + 1 + ye;
+                const Div20 bx(wx), by(w);
+                const int nsx = wx * h, nsx32 = (nsx + 31) & ~31, n = nsx32 + w * hy;
+                for (int i = tid; i < n; i += NT) {
+                    const bool alongx = i < nsx32;
+                    if (alongx && i >= nsx) continue;
+                    const int e = alongx ? i : i - nsx32, iy = alongx ? bx.quot(e) : by.quot(e);
+                    const int x = alongx ? e - iy * wx - 1 : e - iy * w, y = alongx ? iy : iy - 1;
+                    const int p = (y + 2) * LC + x + 2, d = alongx ? 1 : LC;
+                    const Q4<double> s = slope64(c, s_c[p - d], s_c[p], s_c[p + d]);
+                    if (alongx) s_sx[y * LX + x + 1] = s;
+                    else s_sy[(y + 1) * w + x] = s;
+                }
+                __syncthreads();
+            }
+            const int wx = w + xe, hy = h + ye;
+            const Div20 bx(wx), by(w);
+            const int nfx = wx * h, nfx32 = (nfx + 31) & ~31, n = nfx32 + w * hy;
+            for (int i = tid; i < n; i += NT) {
+                const bool alongx = i < nfx32;
+                if (alongx && i >= nfx) continue;
+                const int e = alongx ? i : i - nfx32, y = alongx ? bx.quot(e) : by.quot(e);
+                const int x = e - y * (alongx ? wx : w);
+                const int p = (y + 2) * LC + x + 2;
+                Q4<double> sl{}, sr_{};
+                if (SECOND) {
+                    const Q4<double>* s = alongx ? s_sx + y * LX + x + 1 : s_sy + (y + 1) * w + x;
+                    sl = s[alongx ? -1 : -w];
+                    sr_ = s[0];
+                }
+                const Q4<double> f = face64_along<SECOND>(alongx, c, s_c[p - (alongx ? 1 : LC)], s_c[p], sl, sr_);
+                if (alongx) out.fx[(size_t)(Y0 + y) * (nx + 1) + (X0 + x)] = f;
+                else out.fy[(size_t)(Y0 + y) * nx + (X0 + x)] = f;
+            }
+            if (SECOND) {
+                const Div20 bw(w);
+                for (int i = tid; i < w * h; i += NT) {
+                    const int y = bw.quot(i), x = i - y * w;
+                    const Q4<double> sx = s_sx[y * LX + x + 1], sy = s_sy[(y + 1) * w + x];
+                    out.bed[(size_t)(Y0 + y) * nx + (X0 + x)] = double2{sx.d - sx.a, sy.d - sy.a};
+                }
+            }
         }
-        const int b = STAGE == 2 ? P_CLIP2 : P_CLIP1;
-        const int slot = tid < 5 ? b + tid : P_INFIL + (tid - 5);
-        partials[(size_t)blockIdx.x * NPART + slot] = a;
+}
+
+template <int STAGE>
+__global__ void __launch_bounds__(TILE64_THREADS, STAGE == 1 ? 2 : 1)
+cell64_kernel(const Grid<double>* __restrict__ grids, const Faces64* __restrict__ faces,
+              const StripRef* __restrict__ strips, const StepParams* __restrict__ params, const KC<double> kc,
+              double* __restrict__ partials) {
+    constexpr int NT = TILE64_THREADS;
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    __shared__ Grid<double> gd;
+    KC<double> c = kc;
+    c.order = STAGE != 0 ? 2 : 1;
+    const StripRef sr = strips[blockIdx.x];
+    const StepParams& pr = params[sr.member];
+    if (!pr.active) return;
+    const int tid = threadIdx.x;
+    {
+        const unsigned* src = reinterpret_cast<const unsigned*>(grids + sr.member);
+        unsigned* dst = reinterpret_cast<unsigned*>(&gd);
+        for (int k = tid; k < (int)(sizeof(Grid<double>) / 4); k += NT) dst[k] = src[k];
     }
+    const Faces64 in = faces[sr.member];
+    __syncthreads();
+    const double* __restrict__ H = STAGE == 2 ? gd.h1 : gd.h;
+    const Q4<double>* __restrict__ fx = in.fx;
+    const Q4<double>* __restrict__ fy = in.fy;
+    const int nx = gd.nx, ny = gd.ny;
+    const Step64 k(c, gd, pr, STAGE);
+    Acc64 acc;
+    const int cw = tile64_part(sr.w, sr.sub_w), ch = tile64_part(sr.y1 - sr.y0, sr.sub_h);
+    double* s_th = reinterpret_cast<double*>(smem_raw);
+    for (int Y0 = sr.y0; Y0 < sr.y1; Y0 += ch)
+        for (int X0 = sr.x0; X0 < sr.x0 + sr.w; X0 += cw) {
+            const int w = min(cw, sr.x0 + sr.w - X0), h = min(ch, sr.y1 - Y0), LT = w + 2;
+            __syncthreads();                       // the last sub-tile's readers are done
+            {
+                const Div20 by(LT);
+                for (int i = tid; i < LT * (h + 2); i += NT) {
+                    const int iy = by.quot(i), y = iy - 1, x = i - iy * LT - 1;
+                    if (!(x >= 0 && x < w) && !(y >= 0 && y < h)) continue;
+                    const int gx = X0 + x, gy = Y0 + y;
+                    double th = 1.0;               // outside the grid
+                    if ((unsigned)gx < (unsigned)nx && (unsigned)gy < (unsigned)ny) {
+                        const size_t jx = (size_t)gy * (nx + 1) + gx, j = (size_t)gy * nx + gx;
+                        th = theta64(k, H[j], fx[jx].a, fx[jx + 1].a, fy[j].a, fy[j + nx].a);
+                    }
+                    s_th[i] = th;
+                }
+            }
+            __syncthreads();
+            const Div20 by(w);
+            for (int i = tid; i < w * h; i += NT) {
+                const int y = by.quot(i), x = i - y * w, gx = X0 + x, gy = Y0 + y, t0 = (y + 1) * LT + x + 1;
+                const size_t jx = (size_t)gy * (nx + 1) + gx, j = (size_t)gy * nx + gx;
+                double2 bed{0.0, 0.0};
+                if (STAGE != 0) bed = in.bed[j];
+                update64<STAGE>(c, gd, k, acc, Pos64{gx, gy}, (unsigned)j, H[j], fx[jx], fx[jx + 1], fy[j], fy[j + nx],
+                                s_th[t0], s_th[t0 - 1], s_th[t0 + 1], s_th[t0 - LT], s_th[t0 + LT], bed.x, bed.y);
+            }
+        }
+    store_acc64<STAGE>(acc, partials + (size_t)blockIdx.x * NPART);
 }
 
 }  // namespace his

@@ -174,13 +174,14 @@ class Member:
 
     def nbytes(self) -> int:
         """Device bytes held by this member (state, fields, peaks, network), plus the
-        stage scratch and tables a grid set allocates for it."""
+        stage scratch (float64: and face planes) and tables a grid set allocates for it."""
         ts = [self.z, self.n, self.S, self.f0, self.fc, self.k, self.h, self.hu, self.hv, self.s_filled,
               self.infil_cum, self.peak_h, self.peak_speed, self.A, self.Q]
         if self.n_out:
             ts += [self.snap_h, self.snap_u, self.snap_v, self.snap_t, self.snap_eta, self.snap_q, self.snap_ledger]
         held = sum(t.numel() * t.element_size() for t in ts if t is not None)
-        return held + 3 * self.h.numel() * self.h.element_size() + 64 * 1024
+        faces = 80 * self.h.numel() if self.dtype == torch.float64 else 0
+        return held + 3 * self.h.numel() * self.h.element_size() + faces + 64 * 1024
 
     # ---------------------------------------------------------------- descriptors
     def _build_network(self):

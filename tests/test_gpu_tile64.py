@@ -59,3 +59,37 @@ def test_float64_step_at_sub_tile_edges(ny, nx, tile, order, flux, h_dry):
             d = H.max_abs(getattr(a, name).cpu().numpy(), getattr(o, name)[0])
             assert d <= 1e-12, f"{name} differs from the oracle by {d}"
         assert torch.allclose(va.table, vb.table, rtol=1e-12, atol=1e-12)
+
+
+def test_float64_faces_in_their_own_kernel_give_the_fused_kernel_s_bits():
+    """A set with room for its faces (40,000 cells and more) computes each face once, in two
+    kernels per stage; a smaller set, and the allocation-free step at any size, in one fused
+    kernel.  A 205 x 199 grid in 58 x 16 chunks against the allocation-free step's twin of it
+    and against a batch of three such members: state and totals bit for bit."""
+    import ctypes as C
+    from his_gb300 import _lib
+    from his_gb300.infiltration import Horton
+    from his_gb300.swe2d import SWE2D
+    f, bcs, cfg = _case(205, 199, 2, "hllc", 1e-3)
+    mk = lambda B: SWE2D(f["z"], f["n"], 9.0, cfg, bcs, storage=f["S"], horton=Horton(*f["horton"]), rain_weight=f["rw"],
+                         dy=11.0, batch=B)
+    one, many = mk(None), mk(3)
+    one.set_state(f["h"], f["hu"], f["hv"])
+    many.set_state(f["h"], f["hu"], f["hv"])
+    names = ("h", "hu", "hv", "s_filled", "infil_cum")
+    twin = {k: getattr(one, k).clone() for k in names}
+    d = _lib.GridDesc.from_buffer_copy(one._descs[0])
+    d.h, d.hu, d.hv, d.s_filled, d.infil_cum = (twin[k].data_ptr() for k in names)
+    ccfg, t = _lib.solver_cfg(cfg), 0.0
+    for _ in range(3):
+        dt = 0.8 * one.max_dt()
+        v = one.step(dt, t, 2e-5)
+        many.step(dt, t, 2e-5)
+        got = np.zeros(5)
+        _lib.check(one._lib.his_grid_step_noalloc(one.prec, C.byref(ccfg), C.byref(d), one.step_params(dt, t, 2e-5),
+                                                  _lib.as_p(got), _lib.stream_handle()), "his_grid_step_noalloc")
+        t += dt
+        assert np.array_equal(got, v.table[0].cpu().numpy())
+        for k in names:
+            assert torch.equal(getattr(one, k), twin[k]), k
+            assert all(torch.equal(getattr(many, k)[b], twin[k]) for b in range(3)), k
