@@ -1,6 +1,7 @@
 // C ABI of the flood-engine step (include/his_gb300.h): argument checks, device
 // tables, host<->device parameter and result movement, precision dispatch.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -754,9 +755,11 @@ int32_t his_links_create(his_grid* grid, his_net* net, int32_t n_members, const 
     if (n_members != grid->n || n_members != net->n)
         return bad("links, grid and network must have the same number of members");
     Arena ar;
-    struct Offs { size_t c1, inv, uq, orig, zb, len, z2, us, ui, uf, cs, zbf, lenf, z2f; };
+    struct Offs { size_t c1, c2, orig, zb, len, z2, cs, peer, ms, mi, zbf, lenf, z2f; };
     std::vector<Offs> offs(n_members);
     size_t smem = 0, smem64 = 0, smem32 = 0;
+    std::vector<std::array<int, EXCH_SLICES + 1>> slices(n_members);
+    std::vector<int> n_multi(n_members);
     int total = 0;
     for (int mb = 0; mb < n_members; ++mb) {
         const his_links_desc& d = links[mb];
@@ -778,10 +781,30 @@ int32_t his_links_create(his_grid* grid, his_net* net, int32_t n_members, const 
         std::vector<int> us, ui, cs, ci;
         build_csr(d.inv, d.n_links, d.n_unique, us, ui);
         build_csr(d.cell1d, d.n_links, nc, cs, ci);
-        // links in the order of their 1-D cell; a 2-D cell's links keep the caller's order
-        std::vector<int> pos(d.n_links);
+        // links in the order of their 1-D cell; the links of a shared 2-D cell keep the caller's
+        // order
+        std::vector<int> pos(d.n_links), peer(d.n_links, -1), c2(d.n_links), ms(1, 0), mi;
         for (int p = 0; p < d.n_links; ++p) pos[ci[p]] = p;
-        for (int& l : ui) l = pos[l];
+        for (int p = 0; p < d.n_links; ++p) c2[p] = uq[d.inv[ci[p]]];
+        for (int k = 0; k < d.n_unique; ++k) {
+            if (us[k + 1] - us[k] < 2) continue;
+            for (int j = us[k]; j < us[k + 1]; ++j) {
+                peer[pos[ui[j]]] = (int)ms.size() - 1;
+                mi.push_back(pos[ui[j]]);
+            }
+            ms.push_back((int)mi.size());
+        }
+        // slices of the cells with about equal numbers of links
+        int* slice = slices[mb].data();
+        slice[0] = 0;
+        for (int k = 1; k < EXCH_SLICES; ++k) {
+            int i = slice[k - 1];
+            while (i < nc && (int64_t)cs[i] * EXCH_SLICES < (int64_t)d.n_links * k) ++i;
+            slice[k] = i;
+        }
+        slice[EXCH_SLICES] = nc;
+        for (int k = 0; k < EXCH_SLICES; ++k)
+            smem64 = std::max(smem64, exchange_smem_bytes(cs[slice[k + 1]] - cs[slice[k]], slice[k + 1] - slice[k], 8));
         auto by_cell = [&](const auto* a) {
             std::vector<std::decay_t<decltype(*a)>> v(d.n_links);
             for (int p = 0; p < d.n_links; ++p) v[p] = a[ci[p]];
@@ -791,18 +814,15 @@ int32_t his_links_create(his_grid* grid, his_net* net, int32_t n_members, const 
         auto put_f = [&](const std::vector<double>& v) { return put(std::vector<float>(v.begin(), v.end())); };
         Offs& o = offs[mb];
         const std::vector<double> zb = by_cell(d.zbank), len = by_cell(d.length), z2 = by_cell(d.z2);
-        o.c1 = put(by_cell(d.cell1d)); o.inv = put(by_cell(d.inv));
-        o.uq = put(uq); o.orig = put(ci);
+        o.c1 = put(by_cell(d.cell1d)); o.c2 = put(c2); o.orig = put(ci);
         o.zb = put(zb); o.len = put(len); o.z2 = put(z2);
         o.zbf = put_f(zb); o.lenf = put_f(len); o.z2f = put_f(z2);
-        std::vector<int> uf(d.n_unique);
-        for (int k = 0; k < d.n_unique; ++k) uf[k] = us[k + 1] - us[k] == 1 ? ui[us[k]] : -1;
-        o.us = put(us); o.ui = put(ui); o.uf = put(uf); o.cs = put(cs);
-        // (links per member are limited by one block's shared memory, as they were when sign
-        // and volume of a link were separate)
+        o.cs = put(cs); o.peer = put(peer); o.ms = put(ms); o.mi = put(mi);
+        n_multi[mb] = (int)mi.size();
+        // (links per member are limited by one block's shared memory, as they were when all of
+        // a member's tables were in it)
         smem = std::max(smem, sizeof(double) * (2 * (size_t)d.n_links + 2 * (size_t)d.n_unique + (size_t)nc + 64));
-        smem64 = std::max(smem64, exchange_smem_bytes(d.n_links, d.n_unique, nc, 8));
-        smem32 = std::max(smem32, exchange_smem_bytes(d.n_links, d.n_unique, nc, 4));
+        smem32 = std::max(smem32, exchange_smem_bytes(d.n_links, nc, 4));
         total += d.n_links;
     }
     if (smem > 200 * 1024) return bad("too many links for one thread block's shared memory");
@@ -820,23 +840,26 @@ int32_t his_links_create(his_grid* grid, his_net* net, int32_t n_members, const 
         const his_links_desc& d = links[mb];
         const Offs& o = offs[mb];
         Lnk& L = H[mb];
-        L.n_links = d.n_links; L.n_unique = d.n_unique; L.v_offset = voff;
+        L.n_links = d.n_links; L.n_multi = n_multi[mb]; L.v_offset = voff;
         voff += d.n_links;
-        L.cell1d = (const int*)(base + o.c1); L.inv = (const int*)(base + o.inv); L.uniq = (const int*)(base + o.uq);
+        L.cell1d = (const int*)(base + o.c1); L.cell2d = (const int*)(base + o.c2);
+        L.orig = (const int*)(base + o.orig);
         L.zbank = (const double*)(base + o.zb); L.length = (const double*)(base + o.len);
         L.z2 = (const double*)(base + o.z2);
         L.zbank_f = (const float*)(base + o.zbf); L.length_f = (const float*)(base + o.lenf);
         L.z2_f = (const float*)(base + o.z2f);
-        L.ustart = (const int*)(base + o.us); L.uidx = (const int*)(base + o.ui);
-        L.ufirst = (const int*)(base + o.uf);
-        L.cstart = (const int*)(base + o.cs); L.orig = (const int*)(base + o.orig);
+        L.cstart = (const int*)(base + o.cs);
+        L.peer = (const int*)(base + o.peer); L.mstart = (const int*)(base + o.ms);
+        L.midx = (const int*)(base + o.mi);
+        std::copy(slices[mb].begin(), slices[mb].end(), L.slice);
     }
     e = cudaMalloc(&Lk->d_links, sizeof(Lnk) * n_members);
     if (e == cudaSuccess) e = cudaMemcpy(Lk->d_links, H.data(), sizeof(Lnk) * n_members, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&Lk->d_V, sizeof(double) * std::max(total, 1));
-    if (e == cudaSuccess) e = cudaMallocHost(&Lk->h_V, sizeof(double) * std::max(total, 2 * n_members));
-    if (e == cudaSuccess) e = cudaMalloc(&Lk->d_exch, sizeof(double) * 2 * n_members);
-    if (e == cudaSuccess) e = cudaMemset(Lk->d_exch, 0, sizeof(double) * 2 * n_members);
+    if (e == cudaSuccess) e = cudaMalloc(&Lk->d_Vpos, sizeof(double) * std::max(total, 1));
+    if (e == cudaSuccess) e = cudaMallocHost(&Lk->h_V, sizeof(double) * std::max(total, 2 * EXCH_SLICES * n_members));
+    if (e == cudaSuccess) e = cudaMalloc(&Lk->d_exch, sizeof(double) * 2 * EXCH_SLICES * n_members);
+    if (e == cudaSuccess) e = cudaMemset(Lk->d_exch, 0, sizeof(double) * 2 * EXCH_SLICES * n_members);
     if (e != cudaSuccess) return fail(e, "his_links_create: allocation");
     *out = Lk;
     return HIS_OK;
@@ -847,14 +870,14 @@ int32_t his_links_destroy(his_links* L) {
     cudaFree(L->d_arena);
     cudaFree(L->d_links);
     cudaFree(L->d_V);
+    cudaFree(L->d_Vpos);
     cudaFree(L->d_exch);
     if (L->h_V) cudaFreeHost(L->h_V);
     delete L;
     return HIS_OK;
 }
 
-int32_t his_exchange(his_links* L, const his_solver_cfg* cfg, double dt, double* V, void* stream) {
-    if (!L) return bad("links are required");
+static int exchange(his_links* L, const his_solver_cfg* cfg, double dt, double* V, cudaStream_t s) {
     if (!std::isfinite(dt) || !(dt >= 0)) return bad("dt must be finite and >= 0");
     Consts c = L->grid->c;
     if (cfg) {
@@ -862,8 +885,13 @@ int32_t his_exchange(his_links* L, const his_solver_cfg* cfg, double dt, double*
         c.exchange_limit = cfg->exchange_limit;
         c.exchange_relax = cfg->exchange_relax;
     }
+    return L->grid->prec == HIS_PREC_F64 ? exchange_f64(L, c, dt, V, s) : exchange_f32(L, c, dt, V, s);
+}
+
+int32_t his_exchange(his_links* L, const his_solver_cfg* cfg, double dt, double* V, void* stream) {
+    if (!L) return bad("links are required");
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = L->grid->prec == HIS_PREC_F64 ? exchange_f64(L, c, dt, s) : exchange_f32(L, c, dt, s);
+    int rc = exchange(L, cfg, dt, V ? L->d_V : nullptr, s);
     if (rc || !V) return rc;
     HIS_CK(cudaMemcpyAsync(L->h_V, L->d_V, sizeof(double) * std::max(L->total_links, 1), cudaMemcpyDeviceToHost, s));
     HIS_CK(cudaStreamSynchronize(s));
@@ -876,7 +904,10 @@ int32_t his_exchange_async(his_links* L, const his_solver_cfg* cfg, double dt, d
     bool direct = false;
     int rc = V ? check_async_out(V, "V", &direct) : HIS_OK;
     if (rc) return rc;
-    if ((rc = his_exchange(L, cfg, dt, nullptr, stream)) || !V || L->total_links == 0) return rc;
+    // the kernel writes the caller's volumes itself where the device can store there
+    if ((rc = exchange(L, cfg, dt, V ? (direct ? V : L->d_V) : nullptr, (cudaStream_t)stream)) || !V || direct ||
+        L->total_links == 0)
+        return rc;
     HIS_CK(cudaMemcpyAsync(V, L->d_V, sizeof(double) * L->total_links, cudaMemcpyDefault, (cudaStream_t)stream));
     return HIS_OK;
 }
@@ -884,10 +915,16 @@ int32_t his_exchange_async(his_links* L, const his_solver_cfg* cfg, double dt, d
 int32_t his_links_exchanged(his_links* L, double* totals, int32_t reset, void* stream) {
     if (!L || !totals) return bad("links and totals are required");
     cudaStream_t s = (cudaStream_t)stream;
-    HIS_CK(cudaMemcpyAsync(L->h_V, L->d_exch, sizeof(double) * 2 * L->n, cudaMemcpyDeviceToHost, s));
+    const size_t bytes = sizeof(double) * 2 * EXCH_SLICES * L->n;
+    HIS_CK(cudaMemcpyAsync(L->h_V, L->d_exch, bytes, cudaMemcpyDeviceToHost, s));
     HIS_CK(cudaStreamSynchronize(s));
-    std::memcpy(totals, L->h_V, sizeof(double) * 2 * L->n);
-    if (reset) HIS_CK(cudaMemsetAsync(L->d_exch, 0, sizeof(double) * 2 * L->n, s));
+    for (int m = 0; m < L->n; ++m)
+        for (int j = 0; j < 2; ++j) {
+            double sum = 0.0;
+            for (int k = 0; k < EXCH_SLICES; ++k) sum += L->h_V[(m * EXCH_SLICES + k) * 2 + j];
+            totals[m * 2 + j] = sum;
+        }
+    if (reset) HIS_CK(cudaMemsetAsync(L->d_exch, 0, bytes, s));
     return HIS_OK;
 }
 

@@ -17,48 +17,71 @@
 
 namespace his {
 
-// The per-member pre-step CTA: warps 0 .. 13 exchange water with the channel, warp 14 chooses
-// dt and the substep count and evaluates the substep forcing, warp 15 the step's
+// The per-member pre-step CTAs (one, or a cluster of them, pre_ctas): warps 0 .. 13
+// exchange water with the channel, each CTA a slice of it; warp 14 chooses dt and the
+// substep count (every CTA the same) and evaluates the substep forcing, warp 15 the step's
 // parameters, side by side (a float64 cosine or division is a chain of hundreds to
 // thousands of cycles, and the exchange is a chain of load latencies).
+//
+// CTAs per member: float64 8, the exchange being bound by FP64 instructions; float32 4 while
+// the set is small (32 members and fewer; no member's bits depend on it), where spare SMs
+// shorten the chain (16 steps of six served storms 1213 -> 1152 us), else 1 (of 64 storms
+// 5409 us against 5648).
+constexpr int PRE_MEMBERS_F32 = 32;
 constexpr int ENG_PRE_THREADS = 512, ENG_EXCH_THREADS = 448, ENG_EXCH_WARPS = ENG_EXCH_THREADS / 32;
 
-template <class R>
-__global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_pre_kernel(EngMember* __restrict__ em,
-                                                                  StepParams* __restrict__ params,
-                                                                  const Grid<R>* __restrict__ grids,
-                                                                  const Net* __restrict__ nets,
-                                                                  const Lnk* __restrict__ links, Consts c, ExchK<R> K,
-                                                                  double* __restrict__ netf, int max_sub,
-                                                                  double* __restrict__ exch, int m0) {
+template <class R, int G>
+__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1)
+eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params, const Grid<R>* __restrict__ grids,
+               const Net* __restrict__ nets, const Lnk* __restrict__ links, Consts c, ExchK<R> K,
+               double* __restrict__ netf, int max_sub, double* Vg, double* __restrict__ exch, int m0) {
     extern __shared__ double sm[];
     __shared__ Lnk s_L;
     __shared__ Net s_N;
     __shared__ int s_nsub, s_snap;
     __shared__ double s_dt;
-    __shared__ R s_dtr, s_rate[ENG_EXCH_WARPS];
-    const int m = m0 + blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    __shared__ R s_dtr, s_rate[G * ENG_EXCH_WARPS];     // every CTA's rates
+    const int m = m0 + blockIdx.x / G, rank = blockIdx.x % G, tid = threadIdx.x, lane = tid & 31;
     EngMember& E = em[m];
     StepParams& P = params[m];
     if (E.status != ST_RUNNING) {              // (every thread reads it before any barrier)
-        if (tid == 0) P.active = 0;
+        if (rank == 0 && tid == 0) P.active = 0;
         return;
     }
     if (nets) stage_record(&s_N, nets + m);
     if (links) stage_record(&s_L, links + m);
-    // barriers of the whole CTA, reached from the roles' own code
+    // barriers of the CTA and of the member's CTAs, reached from the roles' own code
     auto all = [] { bar_group(1, ENG_PRE_THREADS); };
-    all();
+    auto wide = [] { member_sync<G>(ENG_PRE_THREADS); };
+    wide();                                      // records are staged, every CTA has started
+    const bool multi = links && s_L.n_multi > 0;
     if (tid < ENG_EXCH_THREADS) {
-        auto ready = [&] { all(); return s_dtr; };
+        auto put_rate = [&](R r) {
+            if constexpr (G > 1) {
+                if (lane < G) {
+                    const unsigned here = (unsigned)__cvta_generic_to_shared(&s_rate[rank * ENG_EXCH_WARPS + (tid >> 5)]);
+                    unsigned there;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here), "r"(lane));
+                    if constexpr (sizeof(R) == 8)
+                        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(there), "d"(r) : "memory");
+                    else
+                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there), "f"(r) : "memory");
+                }
+            } else {
+                if (lane == 0) s_rate[tid >> 5] = r;
+            }
+        };
+        auto ready = [&] { wide(); return s_dtr; };
         auto go = [&] { all(); return s_nsub <= max_sub; };
         if (links) {
-            exchange_dev<R>(s_L, s_N, grids[m], K, nullptr, exch, m, sm, tid, ENG_EXCH_THREADS, s_rate,
-                            [] { bar_group(2, ENG_EXCH_THREADS); }, ready, go);
+            const int2 cs = exch_slice<G>(s_L, s_N.n_cells, rank);
+            exchange_dev<R, 1>(s_L, s_N, grids[m], K, nullptr, Vg + s_L.v_offset,
+                            exch + (size_t)(m * EXCH_SLICES + rank) * 2, cs.x, cs.y, sm, tid, ENG_EXCH_THREADS, true,
+                            [] { bar_group(2, ENG_EXCH_THREADS); }, wide, ready, go, put_rate);
         } else {
             R rate = R(-1);
             if (nets)
-                for (int i = tid; i < s_N.n_cells; i += ENG_EXCH_THREADS) {
+                for (int i = rank * ENG_EXCH_THREADS + tid; i < s_N.n_cells; i += G * ENG_EXCH_THREADS) {
                     const CellLevel<R> o = cell_level(s_N, i, K.g, K.h_dry, true);
                     if (o.wet) rate = o.rate > rate ? o.rate : rate;
                 }
@@ -66,7 +89,7 @@ __global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_p
                 const R w = __shfl_xor_sync(0xffffffffu, rate, o);
                 rate = w > rate ? w : rate;
             }
-            if (lane == 0) s_rate[tid >> 5] = rate;
+            put_rate(rate);
             ready();
             go();
         }
@@ -77,7 +100,7 @@ __global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_p
             const double rate = E.rate;
             double dt = rate > 0.0 ? c.cfl / rate : c.dt_max;
             if (dt < c.dt_min || dt > c.dt_max) {
-                if (dt < c.dt_min) E.n_clamped++;
+                if (dt < c.dt_min && rank == 0) E.n_clamped++;
                 dt = fmin(fmax(dt, c.dt_min), c.dt_max);
             }
             // the step ends at the member's end or its next output time (coupling.py:255-262)
@@ -91,12 +114,12 @@ __global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_p
             s_snap = out_on && E.t + dt >= t_next - 1e-9 ? E.k_out : -1;
         }
         __syncwarp();
-        all();                                   // dt is chosen, the channel rates are in s_rate
+        wide();                                  // dt is chosen, the channel rates are in s_rate
         if (lane == 0) {
             int n = 0;
             if (nets) {
                 R r1 = s_rate[0];
-                for (int w = 1; w < ENG_EXCH_WARPS; ++w) r1 = s_rate[w] > r1 ? s_rate[w] : r1;
+                for (int w = 1; w < G * ENG_EXCH_WARPS; ++w) r1 = s_rate[w] > r1 ? s_rate[w] : r1;
                 const double dt1 = r1 >= R(0) ? fmin(c.cfl_1d / (double)r1, c.dt_max) : c.dt_max;
                 const double ns = ceil(s_dt / dt1 - 1e-9);
                 n = ns < 1.0 ? 1 : (ns > (double)max_sub ? max_sub + 1 : (int)ns);
@@ -104,7 +127,10 @@ __global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_p
             s_nsub = n;
         }
         __syncwarp();
+        if (multi)                               // (the exchange's own barriers)
+            for (int k = 0; k < 3; ++k) wide();
         all();                                   // the substep count is known
+        if (rank != 0) return;
         const int n = s_nsub;
         if (n > max_sub) {
             if (lane == 0) {
@@ -121,15 +147,18 @@ __global__ void __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1) eng_p
         }
         return;
     }
-    all();
+    wide();
     const double dt = s_dt;
     // edge values at t by lanes 0..3 and at t + dt by lanes 4..7, rain by lane 8
     double v = 0.0;
-    if (lane < 8) v = eng_edge(E, lane & 3, lane < 4 ? E.t : E.t + dt);
+    if (rank != 0) v = 0.0;
+    else if (lane < 8) v = eng_edge(E, lane & 3, lane < 4 ? E.t : E.t + dt);
     else if (lane == 8) v = eng_rain(E, E.t);
     __syncwarp();
+    if (multi)
+        for (int k = 0; k < 3; ++k) wide();
     all();
-    if (s_nsub > max_sub) return;
+    if (rank != 0 || s_nsub > max_sub) return;
     if (lane < 4) {
         P.bc0[lane] = v;
         P.bc0_f[lane] = (float)v;

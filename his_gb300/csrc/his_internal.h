@@ -85,7 +85,8 @@ struct his_links {
     void* d_arena = nullptr;
     double* d_V = nullptr;
     double* h_V = nullptr;
-    double* d_exch = nullptr;                // n x 2 running exchange totals
+    double* d_Vpos = nullptr;                // volume per link by position, for shared 2-D cells
+    double* d_exch = nullptr;                // running exchange totals: n x EXCH_SLICES x 2
     size_t smem64 = 0, smem32 = 0;           // shared memory of one member's exchange, by precision
     size_t smem_of(size_t size) const { return size == 8 ? smem64 : smem32; }
 };
@@ -178,8 +179,9 @@ int grid_step_f64(his_grid* g, cudaStream_t s, double* ext = nullptr, double* le
 int grid_step_f32(his_grid* g, cudaStream_t s, double* ext = nullptr, double* ledger = nullptr);
 int grid_reduce_f64(his_grid* g, cudaStream_t s, double* ext = nullptr, bool rate_only = false);
 int grid_reduce_f32(his_grid* g, cudaStream_t s, double* ext = nullptr, bool rate_only = false);
-int exchange_f64(his_links* l, const Consts& c, double dt, cudaStream_t s);
-int exchange_f32(his_links* l, const Consts& c, double dt, cudaStream_t s);
+// V: optional device-writable volume per link, by member in the caller's link order
+int exchange_f64(his_links* l, const Consts& c, double dt, double* V, cudaStream_t s);
+int exchange_f32(his_links* l, const Consts& c, double dt, double* V, cudaStream_t s);
 
 // n_steps engine steps of chain `chain` on its own streams
 int engine_enqueue_f64(his_engine* e, int chain, int n_steps);

@@ -42,16 +42,24 @@ struct Net {
     double *A, *Q;
 };
 
+// CTAs that share the float64 exchange of one member
+constexpr int EXCH_SLICES = 8;
+
 struct Lnk {
     // Links in the order of their 1-D cell (within a cell in the caller's order), so that a
-    // cell's links are contiguous; orig: the caller's index
-    int n_links, n_unique, v_offset, pad;
-    const int *cell1d, *inv, *uniq, *orig;
+    // cell's links are contiguous; orig: the caller's index; cell2d: the 2-D cell
+    int n_links, n_multi, v_offset, pad;
+    const int *cell1d, *cell2d, *orig;
     const double *zbank, *length, *z2;
     const float *zbank_f, *length_f, *z2_f;        // float32 copies for the production form
-    const int *ustart, *uidx;                      // unique 2-D cell -> links (caller's order)
-    const int *ufirst;                             // its link where it has exactly one, else -1
-    const int *cstart;                             // 1-D cell -> its links
+    const int* cstart;                             // 1-D cell -> its links
+    // Links that share their 2-D cell with others (n_multi of them): peer[l] is -1 for a link
+    // alone on its cell, else the cell's entry in mstart, whose links midx lists in the caller's
+    // order
+    const int *peer, *mstart, *midx;
+    // Slices of the 1-D cells (and with them of the links) for the CTAs of a cluster, of about
+    // equal numbers of links
+    int slice[EXCH_SLICES + 1], pad2;
 };
 
 // ---------------------------------------------------------------- sections (swe1d.py:51-84)
@@ -588,10 +596,10 @@ __device__ __forceinline__ void net_substeps_f32_dev(const Net& N, const Consts&
     }
 }
 
-// Shared memory the exchange of one member uses: volumes per link, depth and limit per
-// unique 2-D cell, level (then limit) and storage per 1-D cell, and the reductions.
-__host__ __device__ inline size_t exchange_smem_bytes(int n_links, int n_unique, int n_cells, size_t size) {
-    return sizeof(double) * 96 + size * ((size_t)n_links + 2 * (size_t)n_unique + 2 * (size_t)n_cells);
+// Shared memory of the exchange of one slice: volumes per link, level (then limit) and
+// storage per 1-D cell.
+__host__ __device__ inline size_t exchange_smem_bytes(int n_links, int n_cells, size_t size) {
+    return sizeof(double) * 64 + size * ((size_t)n_links + 2 * (size_t)n_cells);
 }
 
 // Barrier `id` among n threads (whole warps) of a CTA
@@ -683,129 +691,152 @@ __device__ __forceinline__ void stage_record(T* dst, const T* src) {
         reinterpret_cast<unsigned*>(dst)[k] = reinterpret_cast<const unsigned*>(src)[k];
 }
 
-// Weir exchange of one member by nt threads (whole warps, this one tid) of a CTA
-// (coupling.py:73-124), with the 1-D CFL rate of the same cells.  float64 plain method;
-// float32 in the production form (GB300's float64 pipe runs at a small fraction of the
-// float32 rate), with the 1-D area update and the tallies in float64.
+// Weir exchange of one member by nt threads (whole warps, this one tid) of a CTA, or of a
+// slice of its 1-D cells and their links by one CTA of a cluster (coupling.py:73-124), with
+// the 1-D CFL rate of the same cells.  float64 plain method; float32 in the production form
+// (GB300's float64 pipe runs at a small fraction of the float32 rate), with the 1-D area
+// update and the tallies in float64.
 //
-// It is a chain of dependent phases on one SM, bound by the latency of their loads.  So
-// every static table entry and 2-D depth a thread needs is fetched before the first
-// barrier, for EXCH_SLOTS links and 2-D cells per thread at once (more in a loop), and the
-// later phases run from registers and shared memory; links lie in the order of their 1-D
-// cell, so a cell's sum walks contiguous shared memory.  Measured with the pre kernel
-// below, a step of six served storms in float32 89 -> 78 us, one of a 400 x 325 storm in
-// float64 444 -> 313 us.
+// In float32 it is a chain of dependent phases bound by the latency of their loads: what a
+// thread needs of its links is fetched before the first barrier, for SLOTS links at
+// once (more in a loop), a link alone on its 2-D cell limits and moves that cell's water
+// itself, and a 1-D cell's sums walk its contiguous links in shared memory.  In float64 it is
+// bound by FP64 instructions (powers, roots and quotients of every link that overtops; 4800
+// per 400 x 325 member, 47 us of one SM's pipe), so EXCH_SLICES CTAs share a member: the
+// pre-step of such a member 73 -> 25 us, a resident step of it 296 -> 253 us.
 //
-// sync: barrier of the nt threads.  ready(): barrier with whoever chooses dt; returns it.
-//  go(): barrier before the states are changed; false leaves them as they are.
-// s_rate (optional): per warp the largest rate of a wet cell, -1 where none is wet.
-constexpr int EXCH_SLOTS = 3;
-template <class R, class Sync, class Ready, class Go>
+// sync: barrier of the nt threads.  wide: barrier of every thread of the member's CTAs.
+// ready(): barrier with whoever chooses dt; returns it.  go(): barrier before the states are
+// changed; false leaves them as they are.  Vg: volumes by position in global memory.
+// put_rate (optional): takes each warp's largest rate of a wet cell, -1 where none is wet.
+// SLOTS: links per thread fetched ahead (each costs registers).
+template <class R, int SLOTS, class Sync, class Wide, class Ready, class Go, class Rate>
 __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const Grid<R>& gd, const ExchK<R>& K,
-                                             double* __restrict__ Vout, double* __restrict__ exch, int mb, double* sm,
-                                             int tid, int nt, R* s_rate, Sync sync, Ready ready, Go go) {
-    constexpr int S = EXCH_SLOTS;
+                                             double* __restrict__ Vout, double* Vg, double* __restrict__ tally,
+                                             int c0, int c1, double* sm, int tid, int nt, bool rates, Sync sync,
+                                             Wide wide, Ready ready, Go go, Rate put_rate) {
+    constexpr int S = SLOTS;
     constexpr bool F32 = sizeof(R) == 4;
-    const int nl = L.n_links, nu = L.n_unique, nc = N.n_cells;
+    const int l0 = L.cstart[c0], nl = L.cstart[c1] - l0, nc = c1 - c0;
     const R area = R(gd.area);
-    double* red = sm;                                   // 64 doubles used
-    R* V = reinterpret_cast<R*>(sm + 96);
-    R *hq = V + nl, *f2 = hq + nu, *eta1 = f2 + nu, *rp = eta1 + nc, *f1 = eta1;
+    double* red = sm;                                   // 64 doubles
+    R* V = reinterpret_cast<R*>(sm + 64);
+    R *eta1 = V + nl, *rp = eta1 + nc, *f1 = eta1;
     auto zbank = [&](int l) -> R { if constexpr (F32) return L.zbank_f[l]; else return L.zbank[l]; };
     auto length = [&](int l) -> R { if constexpr (F32) return L.length_f[l]; else return L.length[l]; };
     auto z2 = [&](int l) -> R { if constexpr (F32) return L.z2_f[l]; else return L.z2[l]; };
 
-    int c1[S], q2[S], cell[S], u0[S];
-    R zb[S], len[S], zz[S];
+    const bool multi = L.n_multi > 0;
+    int cell[S], at[S], peer[S];
+    R zb[S], len[S], zz[S], hq[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) {
-        const int k = tid + j * nt;
-        cell[j] = u0[j] = 0;
-        if (k < nu) { cell[j] = L.uniq[k]; u0[j] = L.ufirst[k]; }
-        c1[j] = q2[j] = 0;
-        zb[j] = len[j] = zz[j] = R(0);
-        if (k < nl) { c1[j] = L.cell1d[k]; q2[j] = L.inv[k]; zb[j] = zbank(k); len[j] = length(k); zz[j] = z2(k); }
+        const int k = tid + j * nt, l = l0 + k;
+        cell[j] = at[j] = 0;
+        peer[j] = -1;
+        zb[j] = len[j] = zz[j] = hq[j] = R(0);
+        if (k < nl) {
+            cell[j] = L.cell1d[l] - c0;
+            at[j] = L.cell2d[l];
+            if (multi) peer[j] = L.peer[l];
+            zb[j] = zbank(l);
+            len[j] = length(l);
+            zz[j] = z2(l);
+        }
     }
 #pragma unroll
-    for (int j = 0; j < S; ++j) {
-        const int k = tid + j * nt;
-        if (k < nu) hq[k] = gd.h[cell[j]];
-    }
-    for (int k = tid + S * nt; k < nu; k += nt) hq[k] = gd.h[L.uniq[k]];
+    for (int j = 0; j < S; ++j)
+        if (tid + j * nt < nl) hq[j] = gd.h[at[j]];
     R rate = R(-1);
     for (int i = tid; i < nc; i += nt) {
-        const CellLevel<R> o = cell_level(N, i, K.g, K.h_dry, s_rate != nullptr);
+        const CellLevel<R> o = cell_level(N, c0 + i, K.g, K.h_dry, rates);
         eta1[i] = o.eta;
         rp[i] = gd.rarea + R(1) / o.plan;
         if (o.wet) rate = o.rate > rate ? o.rate : rate;
     }
-    if (s_rate) {
+    if (rates) {
         for (int o = 16; o > 0; o >>= 1) {
             const R w = __shfl_xor_sync(0xffffffffu, rate, o);
             rate = w > rate ? w : rate;
         }
-        if ((tid & 31) == 0) s_rate[tid >> 5] = rate;
+        put_rate(rate);
     }
     const R dt = ready();
-#pragma unroll
-    for (int j = 0; j < S; ++j) {
-        const int l = tid + j * nt;
-        if (l < nl) V[l] = link_volume(eta1[c1[j]], zz[j] + hq[q2[j]], zb[j], len[j], rp[c1[j]], dt, K.cw, K.relax);
-    }
-    for (int l = tid + S * nt; l < nl; l += nt) {
-        const int c = L.cell1d[l];
-        V[l] = link_volume(eta1[c], z2(l) + hq[L.inv[l]], zbank(l), length(l), rp[c], dt, K.cw, K.relax);
-    }
-    sync();
-    // donor limits, aggregated per donor in the caller's link order (coupling.py:98-107)
-    auto limit2 = [&](int k, int one) {
-        R tot = R(0);
-        if (one >= 0) tot = pos_part(V[one]);
-        else
-            for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) tot += pos_part(V[L.uidx[j]]);
-        const R avail = K.limit * hq[k] * area;
-        f2[k] = tot > avail ? avail / (tot > R(0) ? tot : R(1)) : R(1);
+    // volumes before the limits
+    auto volume = [&](int k, int c, R h, R zbk, R ln, R zk, int p) {
+        const R v = link_volume(eta1[c], zk + h, zbk, ln, rp[c], dt, K.cw, K.relax);
+        V[k] = v;
+        if (p >= 0) Vg[l0 + k] = (double)v;
     };
 #pragma unroll
     for (int j = 0; j < S; ++j)
-        if (tid + j * nt < nu) limit2(tid + j * nt, u0[j]);
-    for (int k = tid + S * nt; k < nu; k += nt) limit2(k, L.ufirst[k]);
+        if (tid + j * nt < nl) volume(tid + j * nt, cell[j], hq[j], zb[j], len[j], zz[j], peer[j]);
+    for (int k = tid + S * nt; k < nl; k += nt) {
+        const int l = l0 + k;
+        volume(k, L.cell1d[l] - c0, gd.h[L.cell2d[l]], zbank(l), length(l), z2(l), L.peer[l]);
+    }
+    if (multi) wide();
+    sync();
+    // donor limits, aggregated per donor in the caller's link order (coupling.py:98-107); a
+    // 2-D donor's limit is formed by each of its links
     for (int i = tid; i < nc; i += nt) {
         R tot = R(0);
-        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) tot += pos_part(-V[j]);
-        const R avail = K.limit * (tot > R(0) ? cell_level(N, i, K.g, K.h_dry, false).avail : R(0));
+        for (int j = L.cstart[c0 + i] - l0; j < L.cstart[c0 + i + 1] - l0; ++j) tot += pos_part(-V[j]);
+        const R avail = K.limit * (tot > R(0) ? cell_level(N, c0 + i, K.g, K.h_dry, false).avail : R(0));
         f1[i] = tot > avail ? avail / (tot > R(0) ? tot : R(1)) : R(1);
     }
+    auto limit2 = [&](R v, R h, int p) -> R {
+        R tot = pos_part(v);
+        if (p >= 0) {
+            tot = R(0);
+            for (int j = L.mstart[p]; j < L.mstart[p + 1]; ++j) tot += pos_part((R)Vg[L.midx[j]]);
+        }
+        const R avail = K.limit * h * area;
+        return tot > avail ? v * (avail / (tot > R(0) ? tot : R(1))) : v;
+    };
     sync();
     R ex0 = R(0), ex1 = R(0);
-    auto settle = [&](int l, int k, int c) {
-        const R v0 = V[l], v = v0 > R(0) ? v0 * f2[k] : v0 * f1[c];
-        V[l] = v;
-        if (Vout) Vout[L.v_offset + L.orig[l]] = (double)v;
+    auto settle = [&](int k, int c, R h, int p) {
+        R v = V[k];
+        v = v > R(0) ? limit2(v, h, p) : v * f1[c];
+        return v;
+    };
+    auto keep_v = [&](int k, R v, int p) {
+        V[k] = v;
+        if (p >= 0) Vg[l0 + k] = (double)v;
+        if (Vout) Vout[L.v_offset + L.orig[l0 + k]] = (double)v;
         ex0 += pos_part(v);
         ex1 += pos_part(-v);
     };
+    R vs[S];
 #pragma unroll
     for (int j = 0; j < S; ++j)
-        if (tid + j * nt < nl) settle(tid + j * nt, q2[j], c1[j]);
-    for (int l = tid + S * nt; l < nl; l += nt) settle(l, L.inv[l], L.cell1d[l]);
+        if (tid + j * nt < nl) vs[j] = settle(tid + j * nt, cell[j], hq[j], peer[j]);
+    for (int k = tid + S * nt; k < nl; k += nt) V[k] = settle(k, L.cell1d[l0 + k] - c0, gd.h[L.cell2d[l0 + k]], L.peer[l0 + k]);
+    if (multi) wide();                                  // shared volumes are read before they change
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+        if (tid + j * nt < nl) keep_v(tid + j * nt, vs[j], peer[j]);
+    for (int k = tid + S * nt; k < nl; k += nt) keep_v(k, V[k], L.peer[l0 + k]);
+    if (multi) wide();
     if (!go()) return;
-    // apply: 2-D through the unique cells, momentum kept only for water that stays (a cell
-    // that gains and loses nothing keeps what it has)
-    auto apply = [&](int k, int idx, int one) {
-        R d = R(0);
-        if (one >= 0) d = V[one];
-        else
-            for (int j = L.ustart[k]; j < L.ustart[k + 1]; ++j) d += V[L.uidx[j]];
-        const R h0 = hq[k];
+    // apply: 2-D cells, momentum kept only for water that stays (a cell that gains and loses
+    // nothing keeps what it has); a shared cell by the first of its links
+    auto mine = [&](int k, int p) { return p < 0 || L.midx[L.mstart[p]] == l0 + k; };
+    auto apply = [&](int k, int idx, int p, R h0) {
+        R d = V[k];
+        if (p >= 0) {
+            d = R(0);
+            for (int j = L.mstart[p]; j < L.mstart[p + 1]; ++j) d += (R)Vg[L.midx[j]];
+        }
         if (d == R(0) && h0 > R(0)) return;
         R hn, keep;
         if constexpr (F32) {
             hn = h0 - d * gd.rarea;
             keep = h0 > 0.0f ? fminf(hn / h0, 1.0f) : 0.0f;
         } else {
-            hn = h0 - d / area;
-            keep = h0 > 0.0 ? fmin(hn / h0, 1.0) : 0.0;
+            hn = h0 - f64_div(d, area, gd.rarea);
+            keep = h0 > 0.0 ? f64_min(hn / h0, 1.0) : 0.0;
         }
         gd.h[idx] = hn;
         gd.hu[idx] = gd.hu[idx] * keep;
@@ -813,17 +844,21 @@ __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const G
     };
 #pragma unroll
     for (int j = 0; j < S; ++j)
-        if (tid + j * nt < nu) apply(tid + j * nt, cell[j], u0[j]);
-    for (int k = tid + S * nt; k < nu; k += nt) apply(k, L.uniq[k], L.ufirst[k]);
+        if (tid + j * nt < nl && mine(tid + j * nt, peer[j])) apply(tid + j * nt, at[j], peer[j], hq[j]);
+    for (int k = tid + S * nt; k < nl; k += nt) {
+        const int p = L.peer[l0 + k], idx = L.cell2d[l0 + k];
+        if (mine(k, p)) apply(k, idx, p, gd.h[idx]);
+    }
     for (int i = tid; i < nc; i += nt) {
+        const int c = c0 + i;
         R d = R(0);
-        for (int j = L.cstart[i]; j < L.cstart[i + 1]; ++j) d += V[j];
+        for (int j = L.cstart[c] - l0; j < L.cstart[c + 1] - l0; ++j) d += V[j];
         if (d != R(0)) {
-            if constexpr (F32) N.A[i] = N.A[i] + (double)(d / N.dxf[i]);
-            else N.A[i] = N.A[i] + d / N.dx[i];
+            if constexpr (F32) N.A[c] = N.A[c] + (double)(d / N.dxf[c]);
+            else N.A[c] = N.A[c] + f64_div(d, N.dx[c], N.rdx[c]);
         }
     }
-    if (!exch) return;
+    if (!tally) return;
     // tallies in float64: lanes, then warps in order
     const double e0 = warp_sum_sparse((double)ex0), e1 = warp_sum_sparse((double)ex1);
     if ((tid & 31) == 0) {
@@ -837,29 +872,47 @@ __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const G
             const double b = red[2 * w + tid];
             if (f64_bits(b) << 1 != 0) a += b;
         }
-        if (f64_bits(a) << 1 != 0) exch[mb * 2 + tid] += a;
+        if (f64_bits(a) << 1 != 0) tally[tid] += a;
     }
 }
 
-// One CTA of EXCHANGE_THREADS per member.  The drop-in step runs it alone between
-// its CFL wait and the 2-D stages.
+// Slice of the cells of CTA `rank` of G
+template <int G>
+__device__ __forceinline__ int2 exch_slice(const Lnk& L, int n_cells, int rank) {
+    static_assert(EXCH_SLICES % G == 0, "whole slices per CTA");
+    if constexpr (G == 1) return int2{0, n_cells};
+    else return int2{L.slice[rank * (EXCH_SLICES / G)], L.slice[(rank + 1) * (EXCH_SLICES / G)]};
+}
+// Barrier of every thread of a member's CTAs
+template <int G>
+__device__ __forceinline__ void member_sync(int threads) {
+    if constexpr (G > 1) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else {
+        bar_group(1, threads);
+    }
+}
+
+// The drop-in step runs the exchange alone between its CFL wait and the 2-D stages.
 constexpr int EXCHANGE_THREADS = 512;
 
-template <class R>
-__global__ void __launch_bounds__(EXCHANGE_THREADS, sizeof(R) == 4 ? 2 : 1) exchange_kernel(const Lnk* __restrict__ links,
-                                                                    const Net* __restrict__ nets,
-                                                                    const Grid<R>* __restrict__ grids, ExchK<R> K, R dt,
-                                                                    double* __restrict__ Vout,
-                                                                    double* __restrict__ exch) {
+template <class R, int G>
+__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(EXCHANGE_THREADS, sizeof(R) == 4 ? 2 : 1)
+exchange_kernel(const Lnk* __restrict__ links, const Net* __restrict__ nets, const Grid<R>* __restrict__ grids,
+                ExchK<R> K, R dt, double* __restrict__ Vout, double* Vg, double* __restrict__ exch) {
     extern __shared__ double sm[];
     __shared__ Lnk L;
     __shared__ Net N;
-    const int mb = blockIdx.x;
+    const int mb = blockIdx.x / G, slice = blockIdx.x % G;
     stage_record(&L, links + mb);
     stage_record(&N, nets + mb);
     __syncthreads();
-    exchange_dev<R>(L, N, grids[mb], K, Vout, exch, mb, sm, threadIdx.x, EXCHANGE_THREADS, nullptr,
-                    [] { __syncthreads(); }, [&] { __syncthreads(); return dt; }, [] { __syncthreads(); return true; });
+    const int2 cs = exch_slice<G>(L, N.n_cells, slice);
+    auto sync = [] { __syncthreads(); };
+    exchange_dev<R, G == 1 ? 3 : 1>(L, N, grids[mb], K, Vout, Vg + L.v_offset, exch + (size_t)(mb * EXCH_SLICES + slice) * 2, cs.x, cs.y, sm,
+                    threadIdx.x, EXCHANGE_THREADS, false, sync, [] { member_sync<G>(EXCHANGE_THREADS); },
+                    [&] { __syncthreads(); return dt; }, [] { __syncthreads(); return true; }, [](R) {});
 }
 
 }  // namespace his

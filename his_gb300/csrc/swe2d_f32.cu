@@ -10,7 +10,9 @@ int grid_step_f32(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
 int grid_reduce_f32(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
     return grid_reduce_impl<float>(g, s, ext, rate_only);
 }
-int exchange_f32(his_links* l, const Consts& c, double dt, cudaStream_t s) { return exchange_impl<float>(l, c, dt, s); }
+int exchange_f32(his_links* l, const Consts& c, double dt, double* V, cudaStream_t s) {
+    return exchange_impl<float>(l, c, dt, V, s);
+}
 int engine_enqueue_f32(his_engine* e, int chain, int n) { return engine_enqueue_impl<float>(e, chain, n); }
 int engine_take_rate_f32(his_engine* e) { return engine_take_rate_impl<float>(e); }
 int engine_profile_f32(his_engine* e, int n, double* ms) { return engine_profile_impl<float>(e, n, ms); }

@@ -291,15 +291,34 @@ int grid_reduce_impl(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
 }
 
 template <class R>
-int exchange_impl(his_links* l, const Consts& c, double dt, cudaStream_t s) {
+int exchange_impl(his_links* l, const Consts& c, double dt, double* V, cudaStream_t s) {
+    constexpr int G = sizeof(R) == 8 ? EXCH_SLICES : 1;
     const size_t smem = l->smem_of(sizeof(R));
     if (smem > 48 * 1024)
-        HIS_CK(cudaFuncSetAttribute(exchange_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    exchange_kernel<R><<<l->n, EXCHANGE_THREADS, smem, s>>>(l->d_links, l->net->d_nets,
-                                                            reinterpret_cast<const Grid<R>*>(l->grid->d_grids),
-                                                            make_exch_k<R>(c), (R)dt, l->d_V, l->d_exch);
+        HIS_CK(cudaFuncSetAttribute(exchange_kernel<R, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    exchange_kernel<R, G><<<l->n * G, EXCHANGE_THREADS, smem, s>>>(l->d_links, l->net->d_nets,
+                                                                   reinterpret_cast<const Grid<R>*>(l->grid->d_grids),
+                                                                   make_exch_k<R>(c), (R)dt, V, l->d_Vpos, l->d_exch);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
+}
+
+// The pre-step of members [m0, m0 + mc), with the set's number of CTAs per member.
+template <class R>
+void launch_pre(his_engine* E, const Grid<R>* grids, int m0, int mc, cudaStream_t s) {
+    his_grid* g = E->grid;
+    const Net* nets = E->net ? E->net->d_nets : nullptr;
+    const Lnk* links = E->links ? E->links->d_links : nullptr;
+    double* exch = E->links ? E->links->d_exch : nullptr;
+    double* vpos = E->links ? E->links->d_Vpos : nullptr;
+    auto launch = [&](auto kernel, int ctas) {
+        kernel<<<mc * ctas, ENG_PRE_THREADS, E->pre_smem, s>>>(E->d_em, g->d_params, grids, nets, links, g->c,
+                                                               make_exch_k<R>(g->c), E->d_netf, E->max_sub, vpos, exch,
+                                                               m0);
+    };
+    if constexpr (sizeof(R) == 8) launch(eng_pre_kernel<R, EXCH_SLICES>, EXCH_SLICES);
+    else if (E->n <= PRE_MEMBERS_F32) launch(eng_pre_kernel<R, 4>, 4);
+    else launch(eng_pre_kernel<R, 1>, 1);
 }
 
 // One device-resident step for every member of one chain (see engine_kernels.cuh)
@@ -308,18 +327,13 @@ int exchange_impl(his_links* l, const Consts& c, double dt, cudaStream_t s) {
 template <class R, int NT>
 int eng_enqueue_nt(his_grid* g, his_engine* E, int chain, int n_steps) {
     auto* grids = reinterpret_cast<const Grid<R>*>(g->d_grids);
-    const Net* nets = E->net ? E->net->d_nets : nullptr;
-    const Lnk* links = E->links ? E->links->d_links : nullptr;
-    double* exch = E->links ? E->links->d_exch : nullptr;
     const int m0 = E->chain_m[chain], mc = E->chain_m[chain + 1] - m0;
     const int t0 = E->chain_t[chain], tc = E->chain_t[chain + 1] - t0;
     cudaStream_t s_main = E->main_of(chain), s_side = E->side_of(chain);
     cudaEvent_t fork = E->fork_of(chain), join = E->join_of(chain);
     if (mc == 0) return HIS_OK;
     for (int k = 0; k < n_steps; ++k) {
-        eng_pre_kernel<R><<<mc, ENG_PRE_THREADS, E->pre_smem, s_main>>>(E->d_em, g->d_params, grids, nets, links, g->c,
-                                                                        make_exch_k<R>(g->c), E->d_netf, E->max_sub,
-                                                                        exch, m0);
+        launch_pre<R>(E, grids, m0, mc, s_main);
         if (E->net) {
             HIS_CK(cudaEventRecord(fork, s_main));
             HIS_CK(cudaStreamWaitEvent(s_side, fork, 0));
@@ -346,8 +360,17 @@ int engine_enqueue_impl(his_engine* E, int chain, int n_steps) {
 template <class R>
 int engine_take_rate_impl(his_engine* E) {
     // kernel attributes are set here, outside any stream capture
-    if (E->pre_smem > 48 * 1024)
-        HIS_CK(cudaFuncSetAttribute(eng_pre_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E->pre_smem));
+    if (E->pre_smem > 48 * 1024) {
+        if constexpr (sizeof(R) == 8) {
+            HIS_CK(cudaFuncSetAttribute(eng_pre_kernel<R, EXCH_SLICES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)E->pre_smem));
+        } else {
+            HIS_CK(cudaFuncSetAttribute(eng_pre_kernel<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)E->pre_smem));
+            HIS_CK(cudaFuncSetAttribute(eng_pre_kernel<R, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)E->pre_smem));
+        }
+    }
     int rc = grid_reduce_impl<R>(E->grid, E->s0, nullptr, false);
     if (rc) return rc;
     eng_take_rate_kernel<<<(E->n + 127) / 128, 128, 0, E->s0>>>(E->d_em, E->grid->d_out, E->n);
@@ -360,9 +383,6 @@ int engine_take_rate_impl(his_engine* E) {
 template <class R, int NT>
 int eng_profile_nt(his_grid* g, his_engine* E, int n_steps, double* ms) {
     auto* grids = reinterpret_cast<const Grid<R>*>(g->d_grids);
-    const Net* nets = E->net ? E->net->d_nets : nullptr;
-    const Lnk* links = E->links ? E->links->d_links : nullptr;
-    double* exch = E->links ? E->links->d_exch : nullptr;
     const KC<R> kc = make_kc<R>(g->c);
     auto* strips = reinterpret_cast<const StripRef*>(g->d_tiles);
     cudaEvent_t ev[7];
@@ -370,8 +390,7 @@ int eng_profile_nt(his_grid* g, his_engine* E, int n_steps, double* ms) {
     int rc = HIS_OK;
     for (int k = 0; k < n_steps && rc == HIS_OK; ++k) {
         cudaEventRecord(ev[0], E->s0);
-        eng_pre_kernel<R><<<E->n, ENG_PRE_THREADS, E->pre_smem, E->s0>>>(E->d_em, g->d_params, grids, nets, links, g->c,
-                                                             make_exch_k<R>(g->c), E->d_netf, E->max_sub, exch, 0);
+        launch_pre<R>(E, grids, 0, E->n, E->s0);
         cudaEventRecord(ev[1], E->s0);
         if (E->net) {
             cudaStreamWaitEvent(E->s1, ev[1], 0);
