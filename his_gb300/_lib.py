@@ -7,6 +7,7 @@ CUDA failures to ``RuntimeError``.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import threading
 
@@ -107,6 +108,8 @@ SIGNATURES = {
     "his_exchange": (C.c_int32, [_H, C.POINTER(SolverCfg), C.c_double, _F64P, C.c_void_p]),
     "his_exchange_async": (C.c_int32, [_H, C.POINTER(SolverCfg), C.c_double, C.c_void_p, C.c_void_p]),
     "his_links_exchanged": (C.c_int32, [_H, _F64P, C.c_int32, C.c_void_p]),
+    "his_coupled_step_async": (C.c_int32, [_H, _H, C.c_double, C.c_int32, C.POINTER(StepParams), _F64P, C.c_void_p,
+                                           C.c_void_p, C.c_void_p, C.c_void_p]),
     "his_engine_create": (C.c_int32, [_H, _H, _H, C.c_int32, C.POINTER(ForcingDesc), C.c_int32, C.c_int32,
                                       C.POINTER(_H)]),
     "his_engine_destroy": (C.c_int32, [_H]),
@@ -184,13 +187,15 @@ def as_p(a: np.ndarray):
     raise TypeError(a.dtype)
 
 
+_HERE = contextlib.nullcontext()
+
+
 def on_device(device):
     """Make ``device`` (a torch.device with an index) current for a block; no switch
     when it already is, which is the common case on the step's hot path."""
-    import contextlib
     import torch
     if device.index == torch.cuda.current_device():
-        return contextlib.nullcontext()
+        return _HERE
     return torch.cuda.device(device)
 
 

@@ -178,7 +178,6 @@ class CoupledEngine:
         self._rates = torch.zeros(3 * two.B, dtype=torch.float64, pin_memory=True)
         # the 1-D substeps overlap the 2-D step (disjoint state once the exchange is done)
         self._side = torch.cuda.Stream(two.device) if one is not None else None
-        self._exchanged = torch.cuda.Event() if one is not None else None
         # the step kernels add their volume terms straight into the mass balance's device
         # ledger: no copy and no extra kernel per step
         self._ledger = self.mb.device_ledger(two.device)
@@ -267,9 +266,9 @@ class CoupledEngine:
         ms = main.cuda_stream
         if wait:
             self._enqueue_rates(dt is None, need1, ms)
-        # forcing at t does not depend on dt: evaluated while the GPU reduces
-        rain_t = self.rain(t)
-        edges_t = edge_values(two.bcs, t)
+        # forcing at t does not depend on dt: evaluated and laid out while the GPU works
+        two.params_at(t, self.rain(t), edge_values(two.bcs, t))
+        first = one.forcing(t) if one is not None else None
         if wait:
             r2, r1, wet1 = self._wait_rates(main)
         dt = min(two.dt_from_rate(r2) if dt is None else dt, t_limit - t)
@@ -277,21 +276,25 @@ class CoupledEngine:
             if n_sub is None:
                 n_sub = max(1, math.ceil(dt / one.dt_from_rate(r1, wet1) - 1e-9))
             exchange(one, two, self.links, dt, self.cfg, volumes=False, stream=ms)
-            self._exchanged.record(main)
-        two.step_ledger(dt, t, rain_t, edges_t, self._ledger.data_ptr(), ms)
-        self._rates2_at = two.state_version()        # its last stage formed the new state's rates
-        if one is not None:
-            # after the 2-D launch, so the host prepares the substeps while it runs;
-            # the next step's 1-D rates are reduced right behind them, beside the 2-D
-            side = self._side
-            side.wait_event(self._exchanged)
-            one.substeps_ledger(dt, t, n_sub, self._ledger.data_ptr(), side.cuda_stream)
-            one.rates_async(self._rates[two.B:], side.cuda_stream)
+        params = two.params_until(dt, t)
+        if one is None:
+            two.ledger_call(params, self._ledger.data_ptr(), ms)
+        else:
+            # one call: the 2-D step on this stream; beside it, on the side stream, the 1-D
+            # substeps and the next step's 1-D rates; the two joined.  Issued one by one from
+            # here the side stream's part came 50 us late: 156 -> 138 us a step for one small
+            # float64 storm, whose GPU work is 100 us
+            f = one.substep_forcing(dt, t, n_sub, first)
+            one._kernel_writes += 1
+            with _lib.on_device(two.device):
+                _lib.check(two._lib.his_coupled_step_async(two._handle, one._handle, float(dt), int(n_sub), params,
+                                                           _lib.as_p(f), self._ledger.data_ptr(),
+                                                           self._rates[two.B:].data_ptr(), ms,
+                                                           self._side.cuda_stream), "his_coupled_step_async")
             self._rates1_at = one.state_version()
-        if one is not None:
-            main.wait_stream(self._side)
             self.log.n_sub_max = max(self.log.n_sub_max, n_sub)
             self._last_n_sub = n_sub
+        self._rates2_at = two.state_version()        # its last stage formed the new state's rates
         self.log.steps += 1
         self._last_dt = dt
         self.log.dt_min = min(self.log.dt_min, dt)

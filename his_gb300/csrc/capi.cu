@@ -266,6 +266,7 @@ int32_t his_grid_destroy(his_grid* g) {
     }
     if (g->pev_fork) cudaEventDestroy(g->pev_fork);
     if (g->ledger_exec) cudaGraphExecDestroy(g->ledger_exec);
+    if (g->stage_exec) cudaGraphExecDestroy(g->stage_exec);
     if (g->cap_stream) cudaStreamDestroy(g->cap_stream);
     delete g;
     return HIS_OK;
@@ -369,6 +370,45 @@ int32_t his_grid_step(his_grid* g, const his_step_params* params, double* vols, 
     return HIS_OK;
 }
 
+// The stage launches of a set in parts (their forks and joins: about five calls per part),
+// captured once; the finalize follows it, as its output differs from call to call.
+static int capture_stages(his_grid* g) {
+    if (!g->cap_stream) HIS_CK(cudaStreamCreateWithFlags(&g->cap_stream, cudaStreamNonBlocking));
+    HIS_CK(cudaStreamBeginCapture(g->cap_stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = g->prec == HIS_PREC_F64 ? grid_stages_f64(g, g->cap_stream) : grid_stages_f32(g, g->cap_stream);
+    cudaGraph_t graph = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(g->cap_stream, &graph);
+    if (rc || e != cudaSuccess) {
+        if (graph) cudaGraphDestroy(graph);
+        return rc ? rc : cuda_fail(e, "cudaStreamEndCapture");
+    }
+    const cudaError_t ei = cudaGraphInstantiate(&g->stage_exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (ei != cudaSuccess) g->stage_exec = nullptr;
+    HIS_CK(ei);
+    return HIS_OK;
+}
+
+// A step's kernels on s: from the stage graph where the set runs in parts and the caller is
+// not capturing, else launched one by one.
+static int step_kernels(his_grid* g, double* ext, cudaStream_t s) {
+    const bool f64 = g->prec == HIS_PREC_F64;
+    if (g->n_parts > 1 && !g->stage_graph_off) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        HIS_CK(cudaStreamIsCapturing(s, &cs));
+        if (cs == cudaStreamCaptureStatusNone) {
+            if (!g->stage_exec && capture_stages(g) != HIS_OK) {
+                cudaGetLastError();
+                g->stage_graph_off = true;
+            } else {
+                HIS_CK(cudaGraphLaunch(g->stage_exec, s));
+                return f64 ? grid_finalize_f64(g, s, ext) : grid_finalize_f32(g, s, ext);
+            }
+        }
+    }
+    return f64 ? grid_step_f64(g, s, ext) : grid_step_f32(g, s, ext);
+}
+
 int32_t his_grid_step_async(his_grid* g, const his_step_params* params, double* vols, void* stream) {
     if (!g || !params) return bad("grid and params are required");
     if (!g->n_parts) {
@@ -381,7 +421,7 @@ int32_t his_grid_step_async(his_grid* g, const his_step_params* params, double* 
     cudaStream_t s = (cudaStream_t)stream;
     if ((rc = upload_params_pinned(g, params, s))) return rc;
     double* ext = direct ? vols : nullptr;
-    rc = g->prec == HIS_PREC_F64 ? grid_step_f64(g, s, ext) : grid_step_f32(g, s, ext);
+    rc = step_kernels(g, ext, s);
     if (rc || !vols || direct) return rc;
     HIS_CK(cudaMemcpy2DAsync(vols, 5 * sizeof(double), g->d_out, 8 * sizeof(double), 5 * sizeof(double), g->n,
                              cudaMemcpyDefault, s));
@@ -648,6 +688,8 @@ int32_t his_net_destroy(his_net* N) {
     cudaFree(N->d_forcing);
     cudaFree(N->d_out);
     if (N->h_out) cudaFreeHost(N->h_out);
+    if (N->ev_fork) cudaEventDestroy(N->ev_fork);
+    if (N->ev_join) cudaEventDestroy(N->ev_join);
     stage_free(N->forcing_stage);
     delete N;
     return HIS_OK;
@@ -909,6 +951,25 @@ int32_t his_exchange_async(his_links* L, const his_solver_cfg* cfg, double dt, d
         L->total_links == 0)
         return rc;
     HIS_CK(cudaMemcpyAsync(V, L->d_V, sizeof(double) * L->total_links, cudaMemcpyDefault, (cudaStream_t)stream));
+    return HIS_OK;
+}
+
+int32_t his_coupled_step_async(his_grid* g, his_net* N, double dt, int32_t n_sub, const his_step_params* params,
+                               const double* forcing, double* ledger, double* rate_wet, void* stream, void* side) {
+    if (!g || !N || !params || !forcing || !ledger || !rate_wet)
+        return bad("grid, network, params, forcing, ledger and rate_wet are required");
+    cudaStream_t s = (cudaStream_t)stream, s1 = (cudaStream_t)side;
+    for (cudaEvent_t* ev : {&N->ev_fork, &N->ev_join})
+        if (!*ev) HIS_CK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+    HIS_CK(cudaEventRecord(N->ev_fork, s));
+    int rc = his_grid_step_ledger_async(g, params, ledger, stream);
+    if (rc) return rc;
+    // after the 2-D launch, so that the host prepares the substeps while it runs
+    HIS_CK(cudaStreamWaitEvent(s1, N->ev_fork, 0));
+    if ((rc = his_net_step_ledger_async(N, dt, n_sub, forcing, ledger, side))) return rc;
+    if ((rc = his_net_max_rate_async(N, rate_wet, side))) return rc;
+    HIS_CK(cudaEventRecord(N->ev_join, s1));
+    HIS_CK(cudaStreamWaitEvent(s, N->ev_join, 0));
     return HIS_OK;
 }
 

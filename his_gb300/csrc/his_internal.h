@@ -58,6 +58,9 @@ struct his_grid {
     double* ledger_exec_for = nullptr;      // the ledger ledger_exec adds into
     double* ledger_checked = nullptr;       // the last ledger found to be device memory
     bool ledger_graph_off = false;          // capture failed once: plain launches from then on
+    // his_grid_step_async of a set in parts: the stage launches as one graph
+    cudaGraphExec_t stage_exec = nullptr;
+    bool stage_graph_off = false;
 };
 
 struct his_net {
@@ -74,6 +77,7 @@ struct his_net {
     size_t smem = 0;
     size_t smem_f32 = 0;                     // the float32 substeps (staged geometry)
     HostStage forcing_stage;                 // his_net_step_async forcing
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;    // his_coupled_step_async
     double* ledger_checked = nullptr;        // the last ledger found to be device memory
 };
 
@@ -177,6 +181,11 @@ int grid_init_f32(his_grid* g);
 // ledger: optional device 8 x n float64 ledger the step's volume terms are added into
 int grid_step_f64(his_grid* g, cudaStream_t s, double* ext = nullptr, double* ledger = nullptr);
 int grid_step_f32(his_grid* g, cudaStream_t s, double* ext = nullptr, double* ledger = nullptr);
+// the stages alone (in the set's parts), and the finalize that follows them
+int grid_stages_f64(his_grid* g, cudaStream_t s);
+int grid_stages_f32(his_grid* g, cudaStream_t s);
+int grid_finalize_f64(his_grid* g, cudaStream_t s, double* ext);
+int grid_finalize_f32(his_grid* g, cudaStream_t s, double* ext);
 int grid_reduce_f64(his_grid* g, cudaStream_t s, double* ext = nullptr, bool rate_only = false);
 int grid_reduce_f32(his_grid* g, cudaStream_t s, double* ext = nullptr, bool rate_only = false);
 // V: optional device-writable volume per link, by member in the caller's link order

@@ -94,6 +94,29 @@ class Sections:
         return torch.where(A <= full, in_trapezoid, self.yb + (A - full) / self.ts)
 
 
+class _TableVolumes1D(Step1DVolumes):
+    """Step1DVolumes over the (B, 3) table the substeps filled, its columns taken when
+    asked for."""
+
+    @classmethod
+    def over(cls, table: torch.Tensor, batched: bool):
+        self = cls.__new__(cls)
+        self.table, self._batched = table, batched
+        return self
+
+    def __getattr__(self, name):
+        # only reached for a column not taken yet
+        if name not in _COLUMNS:
+            raise AttributeError(name)
+        k = _COLUMNS.index(name)
+        col = self.table[:, k] if self._batched else self.table[0, k]
+        setattr(self, name, col)
+        return col
+
+
+_COLUMNS = ("bnd_in", "bnd_out", "clip")
+
+
 class SWE1D:
     SHARED = ("kind", "reach_of", "ghost_src", "ghost_sign", "face_l", "face_r", "n", "m", "zbank", "dx", "x", "y",
               "chain")
@@ -198,13 +221,15 @@ class SWE1D:
         y = (sec or self.sec).depth(A)
         return torch.where(y >= self.cfg.h_dry, Q / torch.clamp(A, min=1e-12), torch.zeros_like(Q))
 
-    def member_rates(self):
-        rate = np.zeros(self.B)
-        wet = np.zeros(self.B, dtype=np.int32)
+    def _rates(self):
+        rate, wet = (C.c_double * self.B)(), (C.c_int32 * self.B)()
         with _lib.on_device(self.device):
-            _lib.check(self._lib.his_net_max_rate(self._handle, _lib.as_p(rate), _lib.as_p(wet),
-                                                  _lib.stream_handle()), "his_net_max_rate")
+            _lib.check(self._lib.his_net_max_rate(self._handle, rate, wet, _lib.stream_handle()), "his_net_max_rate")
         return rate, wet
+
+    def member_rates(self):
+        rate, wet = self._rates()
+        return np.array(rate), np.array(wet, dtype=np.int32)
 
     def rates_async(self, out: torch.Tensor, stream: int | None = None) -> None:
         """Enqueue per-member (rate, wet) into ``out`` (B x 2 float64, device or pinned
@@ -215,8 +240,8 @@ class SWE1D:
                        "his_net_max_rate_async")
 
     def max_dt(self) -> float:
-        rate, wet = self.member_rates()
-        return self.dt_from_rate(float(rate.max()), bool(wet.any()))
+        rate, wet = self._rates()
+        return self.dt_from_rate(float(np.frombuffer(rate).max()), any(wet))
 
     def dt_from_rate(self, rate: float, any_wet: bool) -> float:
         """The 1-D CFL choice of swe1d.py:253-262 from the batch's largest rate."""
@@ -235,15 +260,21 @@ class SWE1D:
         (coupling.py:216-221), in one launch."""
         vols = torch.empty((self.B, 3), dtype=torch.float64, device=self.device)
         self.substeps_into(dt, t, n_sub, vols.data_ptr())
-        cols = vols.t().unbind(0) if self.bshape else vols[0].unbind(0)
-        return Step1DVolumes(*cols, table=vols)
+        return _TableVolumes1D.over(vols, bool(self.bshape))
+
+    def substep_forcing(self, dt: float, t: float, n_sub: int, first=None) -> np.ndarray:
+        """(B, n_sub, 2) inflow and stage at the start of each substep (coupling.py:216-221);
+        ``first``: forcing(t), where the caller has it already."""
+        f = self.forcing(t) if first is None else first
+        if n_sub > 1:
+            sub = dt / n_sub
+            f = np.stack([f] + [self.forcing(t + k * sub) for k in range(1, n_sub)], axis=1)
+        return np.ascontiguousarray(f, dtype=np.float64)
 
     def substeps_into(self, dt: float, t: float, n_sub: int, vols_ptr: int, stream: int | None = None) -> None:
         """The substeps with their (B, 3) float64 volumes written to ``vols_ptr`` (device
         or page-locked memory) on ``stream`` (default: the current stream)."""
-        sub = dt / n_sub
-        f = self.forcing(t) if n_sub == 1 else np.stack([self.forcing(t + k * sub) for k in range(n_sub)], axis=1)
-        f = np.ascontiguousarray(f, dtype=np.float64)
+        f = self.substep_forcing(dt, t, n_sub)
         self._kernel_writes += 1
         with _lib.on_device(self.device):
             _lib.check(self._lib.his_net_step_async(self._handle, float(dt), int(n_sub), _lib.as_p(f), vols_ptr,
@@ -253,9 +284,7 @@ class SWE1D:
     def substeps_ledger(self, dt: float, t: float, n_sub: int, ledger_ptr: int, stream: int | None = None) -> None:
         """The substeps with their boundary volumes and clip added into an 8 x B float64
         device ledger (``MassBalance.device_ledger``) on ``stream``."""
-        sub = dt / n_sub
-        f = self.forcing(t) if n_sub == 1 else np.stack([self.forcing(t + k * sub) for k in range(n_sub)], axis=1)
-        f = np.ascontiguousarray(f, dtype=np.float64)
+        f = self.substep_forcing(dt, t, n_sub)
         self._kernel_writes += 1
         with _lib.on_device(self.device):
             _lib.check(self._lib.his_net_step_ledger_async(self._handle, float(dt), int(n_sub), _lib.as_p(f),

@@ -38,6 +38,29 @@ class StepVolumes:
     TERMS = ("bnd2d_in", "bnd2d_out", "rain", "infiltration", "clip")
 
 
+class _TableVolumes(StepVolumes):
+    """StepVolumes over the (B, 5) table a step filled, its columns taken when asked for
+    (five views cost the host as much as the step's launches)."""
+
+    @classmethod
+    def over(cls, table: torch.Tensor, batched: bool):
+        self = cls.__new__(cls)
+        self.table, self._batched = table, batched
+        return self
+
+    def __getattr__(self, name):
+        # only reached for a column not taken yet
+        if name not in _COLUMNS:
+            raise AttributeError(name)
+        k = _COLUMNS.index(name)
+        col = self.table[:, k] if self._batched else self.table[0, k]
+        setattr(self, name, col)
+        return col
+
+
+_COLUMNS = ("bnd_in", "bnd_out", "rain", "infil", "clip")
+
+
 def cuda_device(device=None) -> torch.device:
     if not torch.cuda.is_available():
         raise RuntimeError("his_gb300 runs its time step on a CUDA GPU and none is available")
@@ -138,6 +161,8 @@ class SWE2D:
         tx, ty = tile if tile is not None else (0, 0)
         self._params_rec = np.zeros(self.B, dtype=_STEP_DTYPE)
         self._params_ptr = self._params_rec.ctypes.data_as(C.POINTER(_lib.StepParams))
+        # the records as rows of float64: dt, t, rain, four edge values at t, four at t + dt
+        self._params_cols = self._params_rec.view(np.float64).reshape(self.B, 11)
         cfgc = _lib.solver_cfg(cfg)
         with _lib.on_device(self.device):
             _lib.check(self._lib.his_grid_create(self.prec, C.byref(cfgc), self.B, descs, int(tx), int(ty),
@@ -203,12 +228,14 @@ class SWE2D:
         return self._sf.to(torch.float64).sum(dim=(-2, -1)) * self.area
 
     # -------------------------------------------------------------- time step
-    def member_rates(self) -> np.ndarray:
-        out = np.zeros(self.B)
+    def _rates(self):
+        out = (C.c_double * self.B)()
         with _lib.on_device(self.device):
-            _lib.check(self._lib.his_grid_max_rate(self._handle, _lib.as_p(out), _lib.stream_handle()),
-                       "his_grid_max_rate")
+            _lib.check(self._lib.his_grid_max_rate(self._handle, out, _lib.stream_handle()), "his_grid_max_rate")
         return out
+
+    def member_rates(self) -> np.ndarray:
+        return np.array(self._rates())
 
     def rates_async(self, out: torch.Tensor, stream: int | None = None) -> None:
         """Enqueue the per-member CFL rates into ``out`` (B float64, device or pinned
@@ -234,7 +261,8 @@ class SWE2D:
 
     def max_dt(self) -> float:
         """CFL step over the whole batch (the reference shares one dt across members)."""
-        return self.dt_from_rate(float(self.member_rates().max()))
+        out = self._rates()
+        return self.dt_from_rate(out[0] if self.B == 1 else float(np.frombuffer(out).max()))
 
     def dt_from_rate(self, m: float) -> float:
         """The CFL choice of swe2d.py:186-193 from the batch's largest rate."""
@@ -253,11 +281,24 @@ class SWE2D:
         The records live in one buffer per solver, refilled by every call: the pointer
         returned is valid until the next call (the C entry points copy the records
         before returning)."""
-        at_t = edge_values(self.bcs, t) if edges_t is None else edges_t
-        pm = per_member([rain_rate] + at_t + edge_values(self.bcs, t + dt), self.B)
-        a = self._params_rec
-        a["dt"], a["t"], a["rain"] = float(dt), float(t), pm[0]
-        a["bc_t"], a["bc_t_dt"] = pm[1:5].T, pm[5:9].T
+        self.params_at(t, rain_rate, edge_values(self.bcs, t) if edges_t is None else edges_t)
+        return self.params_until(dt, t)
+
+    def _fill_columns(self, k: int, values: list) -> None:
+        if all(isinstance(v, (float, int)) for v in values):
+            self._params_cols[:, k:k + len(values)] = values
+        else:
+            self._params_cols[:, k:k + len(values)] = per_member(values, self.B).T
+
+    def params_at(self, t: float, rain_rate, edges_t: list) -> None:
+        """The records' values at t, which do not wait for the step's dt."""
+        self._fill_columns(1, [float(t), rain_rate, *edges_t])
+
+    def params_until(self, dt: float, t: float):
+        """The records' dt and edge values at t + dt, behind ``params_at``; the pointer
+        ``step_params`` returns."""
+        self._params_cols[:, 0] = float(dt)
+        self._fill_columns(7, edge_values(self.bcs, t + dt))
         return self._params_ptr
 
     def step(self, dt: float, t: float, rain_rate=0.0, edges_t=None) -> StepVolumes:
@@ -265,8 +306,7 @@ class SWE2D:
         volumes are float64 device tensors, as the reference's are."""
         vols = torch.empty((self.B, 5), dtype=torch.float64, device=self.device)
         self.step_into(dt, t, rain_rate, edges_t, vols.data_ptr())
-        cols = vols.t().unbind(0) if self.bshape else vols[0].unbind(0)
-        return StepVolumes(*cols, table=vols)
+        return _TableVolumes.over(vols, bool(self.bshape))
 
     def step_into(self, dt: float, t: float, rain_rate, edges_t, vols_ptr: int, stream: int | None = None) -> None:
         """The step with its (B, 5) float64 volumes written to ``vols_ptr`` (device or
@@ -280,7 +320,10 @@ class SWE2D:
     def step_ledger(self, dt: float, t: float, rain_rate, edges_t, ledger_ptr: int, stream: int | None = None) -> None:
         """The step with its volume terms added into an 8 x B float64 device ledger
         (``MassBalance.device_ledger``) by the step's own finalize kernel, on ``stream``."""
-        params = self.step_params(dt, t, rain_rate, edges_t)
+        self.ledger_call(self.step_params(dt, t, rain_rate, edges_t), ledger_ptr, stream)
+
+    def ledger_call(self, params, ledger_ptr: int, stream: int | None = None) -> None:
+        """``step_ledger`` of records laid out already."""
         with _lib.on_device(self.device):
             _lib.check(self._lib.his_grid_step_ledger_async(self._handle, params, ledger_ptr,
                                                             _lib.stream_handle() if stream is None else stream),
