@@ -222,12 +222,6 @@ template <class R> __device__ __forceinline__ R clamp0(R x) {
     if constexpr (sizeof(R) == 4) return fmaxf(x, 0.0f);
     else return x < R(0) ? R(0) : x;
 }
-// x / d for a cell spacing d: float64 divides as the reference does; float32
-// multiplies by the reciprocal formed once on the host.
-template <class R> __device__ __forceinline__ R per_len(R x, R d, R inv_d) {
-    if constexpr (sizeof(R) == 4) return x * inv_d;
-    else return x / d;
-}
 
 __device__ __forceinline__ double dsqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float dsqrt(float x) { return sqrtf(x); }
@@ -243,11 +237,12 @@ template <class R>
 __device__ __forceinline__ void kp_velocity(const KC<R>& c, R h, R hu, R hv, R& u, R& v) {
     const R SQRT2 = R(1.4142135623730951);
     if constexpr (sizeof(R) == 4) {
-        const float h2 = h * h, h4 = h2 * h2;
+        // (_rn: products the compiler must not fuse into a sum in one kernel and not another)
+        const float h2 = h * h, h4 = __fmul_rn(h2, h2);
         const float s = SQRT2 * h * rsqrtf(h4 + fmaxf(h4, c.kp_eps));
         const bool wet = h >= c.h_dry;
-        u = wet ? hu * s : 0.0f;
-        v = wet ? hv * s : 0.0f;
+        u = wet ? __fmul_rn(hu, s) : 0.0f;
+        v = wet ? __fmul_rn(hv, s) : 0.0f;
     } else {
         u = v = 0.0;
         if (!f64_ge_pos(h, c.h_dry)) return;
@@ -377,7 +372,7 @@ __device__ __forceinline__ void riemann_wb(const KC<float>& c, float hL, float u
     SL = fminf(SL, 0.0f);
     SR = fmaxf(SR, 0.0f);
     const float inv = dryL && dryR ? 0.0f : 1.0f / (SR - SL);
-    const float qL = hL * uL, qR = hR * uR;
+    const float qL = __fmul_rn(hL, uL), qR = __fmul_rn(hR, uR);
     const float dp = c.hg * jump * (hR + hL);
     const float wL = SL * inv, wR = SR * inv, ww = wL * SR;
     const float F1 = fmaf(ww, jump, fmaf(-wL, qR, wR * qL));
@@ -389,7 +384,7 @@ __device__ __forceinline__ void riemann_wb(const KC<float>& c, float hL, float u
         const float num = fmaf(SL, hR * (uR - SR), -(SR * (hL * (uL - SL))));
         F3o = F1 * (num <= 0.0f ? vL : vR);
     } else {
-        F3o = fmaf(ww, hR * vR - hL * vL, fmaf(-wL, qR * vR, wR * (qL * vL)));
+        F3o = fmaf(ww, fmaf(hR, vR, -__fmul_rn(hL, vL)), fmaf(-wL, qR * vR, wR * (qL * vL)));
     }
 }
 

@@ -15,12 +15,39 @@ namespace his {
 
 // How a grid's stages are launched: dynamic shared memory of the stage kernel, and for
 // float64 sets with room for their faces the faces' table and the cell kernel's shared
-// memory (NULL faces: the fused kernel).
+// memory (NULL faces: the fused kernel); for float32 sets the segments a chunk is marched in.
 struct StagePlan {
     size_t smem;
     const void* faces;
     size_t smem_cell;
+    int seg;
 };
+
+// Segments (1, 2 or 4) the rows of a float32 strip-chunk are marched in side by side: the
+// least estimated time for `tiles` chunks of at most `rows` rows, by default_tile's model of
+// the march ((rows + 6) row times, a row 1.6 us while an SM holds few marches and 0.4 + 0.28 us
+// x marches per SM beyond), where all of an SM's chunks stay resident.  Strips of up to 58
+// columns only.  Measured, us per step in 1, 2 and 4 segments, second order with sources:
+// 400 x 325 in 58 x 16, 147 chunks 57, 45 and 37; 294 58, 46 and 45; 441 58, 52 and 70; 588
+// 62, 69 and 69; in 58 x 48 (49 chunks) 107, 70 and 57; 1601 x 1301 in 58 x 48 (784) 146,
+// 330 and 235.
+inline int strip_segments(int nt, int tiles, int rows) {
+    if (nt != 64) return 1;
+    using G = StripGeom<float, 64>;
+    const double per_sm = tiles / 152.0;
+    int best = 1;
+    double least = INFINITY;
+    for (int seg = 1; seg <= 4; seg *= 2) {
+        const int part = (rows + seg - 1) / seg;
+        if (seg > 1 && std::ceil(per_sm) * (double)(G::seg_smem(seg, rows) + 2048) > 227 * 1024.0) break;
+        const double t = (part + 6) * std::max(1.6, 0.4 + 0.28 * seg * per_sm);
+        if (t < 0.9 * least) {
+            least = t;
+            best = seg;
+        }
+    }
+    return best;
+}
 
 // Launch of one stage over `count` strip-chunks: float32 marches strips with NT threads,
 // float64 works off sub-tiles, faces and cells in two kernels or fused.
@@ -36,7 +63,17 @@ void launch_stage(const Grid<R>* grids, const StripRef* strips, const StepParams
             tile64_kernel<STAGE><<<count, TILE64_THREADS, plan.smem, s>>>(grids, strips, params, kc, part);
         }
     } else {
-        strip_kernel<R, NT, STAGE><<<count, NT, plan.smem, s>>>(grids, strips, params, kc, part);
+        if constexpr (NT == 64) {
+            if (plan.seg == 4) {
+                strip_kernel<R, NT, STAGE, 4><<<count, 4 * NT, plan.smem, s>>>(grids, strips, params, kc, part);
+                return;
+            }
+            if (plan.seg == 2) {
+                strip_kernel<R, NT, STAGE, 2><<<count, 2 * NT, plan.smem, s>>>(grids, strips, params, kc, part);
+                return;
+            }
+        }
+        strip_kernel<R, NT, STAGE, 1><<<count, NT, plan.smem, s>>>(grids, strips, params, kc, part);
     }
 }
 
@@ -45,11 +82,27 @@ inline StripRef strip_ref(int member, int x0, int wc, int y0, int y1, int w, int
     return StripRef{member, x0, wc, y0, y1, (short)tile64_part(w, TILE64_W), (short)tile64_part(rows, TILE64_H)};
 }
 
-// Dynamic shared memory of a stage CTA over strip-chunks of at most w x rows cells.
+// Dynamic shared memory of a stage CTA over strip-chunks of at most w x rows cells
+// (float32: marched in seg segments).
 template <class R, int NT>
-size_t stage_smem(int w, int rows, int order) {
+size_t stage_smem(int w, int rows, int order, int seg) {
     if constexpr (sizeof(R) == 8) return tile64_smem(tile64_part(w, TILE64_W), tile64_part(rows, TILE64_H), order == 2);
-    else return StripGeom<R, NT>::smem_bytes;
+    else return seg > 1 ? StripGeom<R, NT>::seg_smem(seg, rows) : StripGeom<R, NT>::smem_bytes;
+}
+
+// Shared memory limits of one stage's strip kernels.
+template <class R, int NT, int STAGE>
+int set_strip_attrs() {
+    constexpr int MOST = 227 * 1024;
+    HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)StripGeom<R, NT>::smem_bytes));
+    if constexpr (NT == 64) {
+        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    MOST - 1024));
+        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    MOST - 1024));
+    }
+    return HIS_OK;
 }
 
 template <class R, int NT>
@@ -64,15 +117,14 @@ int set_stage_attrs() {
         HIS_CK(cudaFuncSetAttribute(face64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, face));
         HIS_CK(cudaFuncSetAttribute(face64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, face));
     } else {
-        const int bytes = (int)StripGeom<R, NT>::smem_bytes;
-        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        int rc;
+        if ((rc = set_strip_attrs<R, NT, 0>()) || (rc = set_strip_attrs<R, NT, 1>()) || (rc = set_strip_attrs<R, NT, 2>()))
+            return rc;
     }
     return HIS_OK;
 }
 
-inline StagePlan stage_plan(const his_grid* g) { return StagePlan{g->stage_smem, g->d_faces, g->cell_smem}; }
+inline StagePlan stage_plan(const his_grid* g) { return StagePlan{g->stage_smem, g->d_faces, g->cell_smem, g->seg}; }
 
 // The 2-D stages of one step on stream s (no finalize), over tiles [t0, t0 + count)
 // (default: all); a tile's partials sit at its global index.
@@ -221,7 +273,7 @@ int grid_init_impl(his_grid* g) {
     g->scratch_bytes = total;
     HIS_CK(cudaMalloc(&g->d_scratch, total > 0 ? total : 256));
     const int wmax = g->tx;
-    int sub_w = 1, sub_h = 1;
+    int sub_w = 1, sub_h = 1, rows = 1;
     for (int m = 0; m < n; ++m) {
         const his_grid_desc& d = g->desc[m];
         Grid<R>& G = H[m];
@@ -245,6 +297,7 @@ int grid_init_impl(his_grid* g) {
         G.tiles_x = ns;
         G.tiles_y = nch;
         G.n_tiles = ns * nch;
+        rows = std::max(rows, hch);
         if constexpr (sizeof(R) == 8) {
             sub_w = std::max(sub_w, tile64_part(w, TILE64_W));
             sub_h = std::max(sub_h, tile64_part(hch, TILE64_H));
@@ -271,9 +324,11 @@ int grid_init_impl(his_grid* g) {
         const bool second = g->c.order == 2;
         g->stage_smem = g->d_faces ? face64_smem(sub_w, sub_h, second) : tile64_smem(sub_w, sub_h, second);
         g->cell_smem = cell64_smem(sub_w, sub_h);
-    } else
-        g->stage_smem = g->nt == 64 ? stage_smem<R, 64>(0, 0, 0) : g->nt == 128 ? stage_smem<R, 128>(0, 0, 0)
-                      : g->nt == 224 ? stage_smem<R, 224>(0, 0, 0) : stage_smem<R, 352>(0, 0, 0);
+    } else {
+        g->seg = strip_segments(g->nt, g->n_tiles, rows);
+        g->stage_smem = g->nt == 64 ? stage_smem<R, 64>(0, rows, 0, g->seg) : g->nt == 128 ? stage_smem<R, 128>(0, 0, 0, 1)
+                      : g->nt == 224 ? stage_smem<R, 224>(0, 0, 0, 1) : stage_smem<R, 352>(0, 0, 0, 1);
+    }
     HIS_CK(cudaMalloc(&g->d_grids, sizeof(Grid<R>) * n));
     HIS_CK(cudaMemcpy(g->d_grids, H.data(), sizeof(Grid<R>) * n, cudaMemcpyHostToDevice));
     HIS_CK(cudaMalloc(&g->d_tiles, sizeof(StripRef) * strips.size()));
@@ -509,7 +564,8 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
     auto* part = reinterpret_cast<double*>(base + L.o_part);
     auto* out = reinterpret_cast<double*>(base + L.o_out);
     const KC<R> kc = make_kc<R>(c);
-    const StagePlan smem{stage_smem<R, NT>(L.w, L.hch, c.order), nullptr, 0};
+    const int seg = sizeof(R) == 8 ? 1 : strip_segments(NT, L.n_strips, L.hch);
+    const StagePlan smem{stage_smem<R, NT>(L.w, L.hch, c.order, seg), nullptr, 0, seg};
     if (c.order == 2) {
         launch_stage<R, NT, 1>(grid, strips, params, kc, part, L.n_strips, smem, s);
         launch_stage<R, NT, 2>(grid, strips, params, kc, part, L.n_strips, smem, s);

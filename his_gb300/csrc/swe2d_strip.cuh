@@ -55,9 +55,18 @@ struct StripGeom {
     static constexpr size_t scalars = (size_t)(1 + RING) * P;
     static_assert((size_t)4 * RING * P >= (size_t)(NT / 32) * NRED, "reduction scratch must fit in the cell ring");
     static constexpr size_t smem_bytes = sizeof(Q4<R>) * quads + sizeof(R) * scalars;
-    // resident CTAs per SM the kernels are register-capped for
-    static constexpr int min_ctas(int stage) {
-        return (stage == 1 ? 768 : 640) / NT > 0 ? (stage == 1 ? 768 : 640) / NT : 1;
+    // resident CTAs per SM the kernels are register-capped for (a chunk marched in segments:
+    // few of them share an SM)
+    static constexpr int min_ctas(int stage, int seg) {
+        const int threads = seg > 1 ? 512 : stage == 1 ? 768 : 640;
+        return threads / (NT * seg) > 0 ? threads / (NT * seg) : 1;
+    }
+    // a chunk marched in segments: each segment's rings, then every row's sums per thread
+    // (SegSums) and every segment's maxima
+    static constexpr int NSUM = 9, NMAX = 2;
+    static constexpr size_t seg_stride = (smem_bytes + 31) / 32 * 32;
+    static constexpr size_t seg_smem(int seg, int rows) {
+        return seg * seg_stride + sizeof(R) * NT * ((size_t)rows * NSUM + (size_t)seg * NMAX);
     }
 };
 
@@ -212,7 +221,7 @@ __device__ __forceinline__ void block_reduce_store(T (&v)[NV], const bool* is_ma
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nthreads >> 5;
 #pragma unroll
     for (int j = 0; j < NV; ++j) v[j] = is_max[j] ? warp_max_t(v[j]) : warp_sum_t(v[j]);
-    if (lane == 0) {
+    if (lane == 0 && warp < nw) {
 #pragma unroll
         for (int j = 0; j < NV; ++j) red[warp * NV + j] = v[j];
     }
@@ -264,7 +273,12 @@ __device__ __forceinline__ Q4<float> side_flux(const KC<float>& c, const Side& L
 // row<true> is the steady state: every row touched lies inside the grid, so the
 // range tests, y-ghosts and domain-edge terms drop out; row<false> handles the
 // pipeline fill at the chunk's start, the drain at its end and the grid's edges.
-template <class R, int NT, int STAGE>
+//
+// SEG > 1: the chunk's rows are dealt to SEG groups of NT threads, which march side by side,
+// each with its own rings and barrier; the rows' contributions to the partial sums are kept
+// per row and thread and added up in row order at the end, so that the sums are those of one
+// march over all rows, bit for bit.
+template <class R, int NT, int STAGE, int SEG>
 struct StripPipe {
     static_assert(sizeof(R) == 4, "the float64 step is tile64_kernel's");
     using G = StripGeom<R, NT>;
@@ -283,16 +297,43 @@ struct StripPipe {
     const R* __restrict__ H;
     const R* __restrict__ HU;
     const R* __restrict__ HV;
-    int ts, cx, cxc, nx, ny, y0, y1, scol, xside, xkind;
+    int ts, cx, cxc, nx, ny, cy0, y0, y1, scol, xside, xkind;      // cy0: the chunk's first row; [y0, y1) this march
     unsigned feat;                     // FEAT_* bits of the member's optional fields
     bool col_in, do_out, west, east;
-    R dt, rdx, rdy, idx, idy, rdt, tt;
+    R dt, idx, idy, rdt, tt;
     // carried state of this thread's column
     HaloRaw<R> ra;                     // raw row r (prefetched one row ahead)
     Side ylow;                      // plus side of the y-reconstruction of row r-2
     R by1, by2, bx1;                   // bed terms: y of rows r-2, r-3; x of row r-3
     CellIn<R> cin;
     R acc_clip, xin, xout, yin, yout, infil, rainw, rate, hsum, ssum, hmax;
+    R* sums;                           // SEG > 1: this thread's entry of the chunk's first row
+    int bar;                           // and its segment's barrier
+
+    // Barrier among the NT threads of one march
+    __device__ __forceinline__ void sync() const {
+        if (SEG == 1) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NT) : "memory");
+    }
+    // Row's contributions to the sums, put aside (SEG > 1)
+    __device__ __forceinline__ void put_sums(int row) {
+        R* s = sums + (size_t)row * (G::NSUM * NT);
+        R* const v[G::NSUM] = {&acc_clip, &xin, &xout, &yin, &yout, &infil, &rainw, &hsum, &ssum};
+#pragma unroll
+        for (int k = 0; k < (STAGE == 1 ? 5 : G::NSUM); ++k) {
+            s[k * NT] = *v[k];
+            *v[k] = R(0);
+        }
+    }
+    // All rows' contributions added in row order
+    __device__ __forceinline__ void take_sums(int rows) {
+        R* const v[G::NSUM] = {&acc_clip, &xin, &xout, &yin, &yout, &infil, &rainw, &hsum, &ssum};
+        for (int j = 0; j < rows; ++j) {
+            const R* s = sums + (size_t)j * (G::NSUM * NT);
+#pragma unroll
+            for (int k = 0; k < (STAGE == 1 ? 5 : G::NSUM); ++k) *v[k] += s[k * NT];
+        }
+    }
 
     // Raw values of an interior row at this thread's source column (its own column, or
     // the layer an x-ghost copies)
@@ -359,7 +400,7 @@ struct StripPipe {
             xm = side_minus(xr);
             if (c.order == 2) bx0 = bed_term(c, xr);
         }
-        __syncthreads();
+        sync();
         // ---- B: y-face between rows r-2 and r-1; x-face between columns cx-1 and cx of row r-2
         Q4<R> yf0{R(0), R(0), R(0), R(0)};
         if (yact) {
@@ -374,7 +415,7 @@ struct StripPipe {
             xf0 = side_flux(c, L, cl.d, cl.a, xm, c2.d, c2.a);
             s_xf[xo + ts] = xf0;
         }
-        __syncthreads();
+        sync();
         // ---- C: theta of row r-2 (swe2d.py:259-264); 1 outside the grid
         R th0 = R(1);
         Q4<R> yn{R(0), R(0), R(0), R(0)};          // y-face r-2: south of row r-2, north of row r-3
@@ -382,8 +423,8 @@ struct StripPipe {
             yn = s_yf[k2 + ts];
             if (FULL || (unsigned)row < (unsigned)ny) {
                 const R Fw = xf0.a, Fe = s_xf[xo + ts + 1].a, Gs = yn.a, Gn = yf0.a;
-                const R out = per_len(relu(Fe) + relu(-Fw), rdx, idx) + per_len(relu(Gn) + relu(-Gs), rdy, idy);
-                const R need = out * dt;
+                const R out = fmaf(relu(Gn) + relu(-Gs), idy, __fmul_rn(relu(Fe) + relu(-Fw), idx));
+                const R need = __fmul_rn(out, dt);
                 const R hh = c2.a;
                 const R th = need > hh ? hh / (need > R(0) ? need : R(1)) : R(1);
                 th0 = col_in ? th : R(1);
@@ -391,7 +432,10 @@ struct StripPipe {
             s_th[k2 + ts] = th0;
         }
         // ---- D: update of row r-3
-        if (upd) update<FULL>(orow, xp, k3, k4, th0, yn);
+        if (upd) {
+            update<FULL>(orow, xp, k3, k4, th0, yn);
+            if (SEG > 1) put_sums(orow - cy0);
+        }
         by2 = by1;
         by1 = by0;
         bx1 = bx0;
@@ -409,20 +453,19 @@ struct StripPipe {
         if (__any_sync(0xffffffffu, fminf(fminf(fminf(thC, thW), fminf(thE, thS)), thN) < 1.0f)) {
             const R sw = Fw > R(0) ? thW : thC, se = Fe > R(0) ? thC : thE;
             const R ss = Gs > R(0) ? thS : thC, sn = Gn > R(0) ? thC : thN;
-            Fw *= sw; Tw *= sw; Fe *= se; Te *= se;
-            Gs *= ss; Ts *= ss; Gn *= sn; Tn *= sn;
+            Fw = __fmul_rn(Fw, sw); Tw = __fmul_rn(Tw, sw); Fe = __fmul_rn(Fe, se); Te = __fmul_rn(Te, se);
+            Gs = __fmul_rn(Gs, ss); Ts = __fmul_rn(Ts, ss); Gn = __fmul_rn(Gn, sn); Tn = __fmul_rn(Tn, sn);
         }
-        R a1 = per_len(Fw - Fe, rdx, idx);
-        R a2 = per_len(xw.c - xe.b, rdx, idx);
-        R a3 = per_len(Tw - Te, rdx, idx);
-        R b1 = per_len(Gs - Gn, rdy, idy);
-        R b2 = per_len(ys.c - yn.b, rdy, idy);
-        R b3 = per_len(Ts - Tn, rdy, idy);
+        // which product of a sum is fused is written out: a cell's bits must not depend on the
+        // instantiation that updates it
+        const R dh = fmaf(Gs - Gn, idy, __fmul_rn(Fw - Fe, idx));
+        R dhu = __fmul_rn(xw.c - xe.b, idx), dhv = __fmul_rn(ys.c - yn.b, idy);
         if (c.order == 2) {
-            a2 = a2 + per_len(bx1, rdx, idx);
-            b2 = b2 + per_len(by2, rdy, idy);
+            dhu = fmaf(bx1, idx, dhu);
+            dhv = fmaf(by2, idy, dhv);
         }
-        const R dh = a1 + b1, dhu = a2 + b3, dhv = a3 + b2;
+        dhu = fmaf(Ts - Tn, idy, dhu);
+        dhv = fmaf(Tw - Te, idx, dhv);
         if (!do_out) return;
         if (west) { xin += relu(Fw); xout += relu(-Fw); }
         if (east) { xin += relu(-Fe); xout += relu(Fe); }
@@ -433,13 +476,13 @@ struct StripPipe {
         const unsigned i = (unsigned)orow * (unsigned)nx + (unsigned)cx;
         R hn, hun, hvn;
         if (STAGE == 2) {
-            hn = R(0.5) * (cin.h0 + h3 + dt * dh);
-            hun = R(0.5) * (cin.hu0 + cin.hu1 + dt * dhu);
-            hvn = R(0.5) * (cin.hv0 + cin.hv1 + dt * dhv);
+            hn = R(0.5) * fmaf(dt, dh, cin.h0 + h3);
+            hun = R(0.5) * fmaf(dt, dhu, cin.hu0 + cin.hu1);
+            hvn = R(0.5) * fmaf(dt, dhv, cin.hv0 + cin.hv1);
         } else {
-            hn = h3 + dt * dh;
-            hun = cin.hu0 + dt * dhu;
-            hvn = cin.hv0 + dt * dhv;
+            hn = fmaf(dt, dh, h3);
+            hun = fmaf(dt, dhu, cin.hu0);
+            hvn = fmaf(dt, dhv, cin.hv0);
         }
         const R neg = clamp0(-hn);
         acc_clip += neg;
@@ -451,15 +494,15 @@ struct StripPipe {
         // ---- rain, Horton infiltration, retention store (swe2d.py:330-360)
         R sf = cin.sf;
         if (feat & FEAT_RAINW) {
-            const R add = rdt * cin.rw;
+            const R add = __fmul_rn(rdt, cin.rw);
             hn = hn + add;
             rainw += add;
         } else {
             hn = hn + rdt;
         }
         if (feat & FEAT_HORTON) {
-            const R rate_f = cin.fc + (cin.f0 - cin.fc) * expf(-cin.k * tt);
-            const R pot = rate_f * dt;
+            const R rate_f = fmaf(cin.f0 - cin.fc, expf(-cin.k * tt), cin.fc);
+            const R pot = __fmul_rn(rate_f, dt);
             const R take = rmin(pot, hn);
             const R safe = hn > R(0) ? hn : R(1);
             const R scale = hn > R(0) ? (hn - take) / safe : R(0);
@@ -488,13 +531,13 @@ struct StripPipe {
         }
         // ---- semi-implicit Manning friction (swe2d.py:362-370)
         // KP factor of the new depth, kept for the CFL velocity below
-        const R h2 = hn * hn, h4 = h2 * h2;
+        const R h2 = hn * hn, h4 = __fmul_rn(h2, h2);
         const R ks = hn >= c.h_dry ? 1.4142135623730951f * hn * rsqrtf(h4 + fmaxf(h4, c.kp_eps)) : 0.0f;
         R u = hun * ks, v = hvn * ks;
-        const R speed = dsqrt(u * u + v * v);
+        const R speed = dsqrt(fmaf(u, u, __fmul_rn(v, v)));
         const R hf = rmax(hn, c.h_dry);
         const R nm = cin.n;
-        const R denom = R(1) + dt * c.g * nm * nm * speed / powf(hf, 4.0f / 3.0f);
+        const R denom = __fadd_rn(1.0f, dt * c.g * nm * nm * speed / powf(hf, 4.0f / 3.0f));
         u = u / denom;
         v = v / denom;
         const bool wet = hn >= c.h_dry;
@@ -510,14 +553,14 @@ struct StripPipe {
         const R u2 = hun * ks, v2 = hvn * ks;
         // running peak speed and output use the KP velocities of the new state, as the
         // reference's snapshots do (swe2d.py:161-167, coupling.py:229-242)
-        if (feat & FEAT_PSPEED) gd.ps[i] = rmax(gd.ps[i], dsqrt(u2 * u2 + v2 * v2));
+        if (feat & FEAT_PSPEED) gd.ps[i] = rmax(gd.ps[i], dsqrt(fmaf(u2, u2, __fmul_rn(v2, v2))));
         if (feat & FEAT_SNAP) {
             s_snap[0][i] = (float)hn;
             s_snap[1][i] = (float)u2;
             s_snap[2][i] = (float)v2;
         }
         const R cw = dsqrt(c.g * hn);
-        const R rr = hn > c.h_dry ? per_len(fabs(u2) + cw, rdx, idx) + per_len(fabs(v2) + cw, rdy, idy) : R(0);
+        const R rr = hn > c.h_dry ? fmaf(__fadd_rn(fabsf(v2), cw), idy, __fmul_rn(__fadd_rn(fabsf(u2), cw), idx)) : R(0);
         rate = rmax(rate, rr);
         hsum += hn;
         ssum += sf;
@@ -546,8 +589,12 @@ __device__ __forceinline__ int ghost_source_column(const KC<R>& c, const Grid<R>
 // state.  The first-order step reads the state in its halo, so it writes its result
 // to the stage buffers and stage_copy_kernel moves it back (no CTA overwrites cells
 // that another CTA may still read).
-template <class R, int NT, int STAGE>
-__global__ void __launch_bounds__(NT, StripGeom<R, NT>::min_ctas(STAGE)) strip_kernel(const Grid<R>* __restrict__ grids,
+//
+// With few chunks a march is bound by its latency: 1.6 us a row, rows + 6 of them, two warps
+// on an SM.  SEG = 2 and 4 march parts of the chunk side by side (strip_segments): one served
+// storm of 400 x 325 cells in 58 x 16 took 71.5 us a step in one march, 59.7 in four.
+template <class R, int NT, int STAGE, int SEG>
+__global__ void __launch_bounds__(NT * SEG, StripGeom<R, NT>::min_ctas(STAGE, SEG)) strip_kernel(const Grid<R>* __restrict__ grids,
                                                     const StripRef* __restrict__ strips,
                                                     const StepParams* __restrict__ params, const KC<R> kc,
                                                     double* __restrict__ partials) {
@@ -567,31 +614,32 @@ __global__ void __launch_bounds__(NT, StripGeom<R, NT>::min_ctas(STAGE)) strip_k
     const StripRef sr = strips[blockIdx.x];
     const StepParams& pr = params[sr.member];
     if (!pr.active) return;
-    const int t = threadIdx.x;
+    const int t = SEG == 1 ? threadIdx.x : threadIdx.x % NT, seg = SEG == 1 ? 0 : threadIdx.x / NT;
     {
         static_assert(sizeof(Grid<R>) % 4 == 0, "record copied as 32-bit words");
         const unsigned* src = reinterpret_cast<const unsigned*>(grids + sr.member);
         unsigned* dst = reinterpret_cast<unsigned*>(&s_gd);
-        for (int k = t; k < (int)(sizeof(Grid<R>) / 4); k += NT) dst[k] = src[k];
+        for (int k = threadIdx.x; k < (int)(sizeof(Grid<R>) / 4); k += NT * SEG) dst[k] = src[k];
     }
-    if (t < 4) bcv[t] = par_bc<R>(pr, STAGE == 2, t);
-    if (t == 0) {
+    if (threadIdx.x < 4) bcv[t] = par_bc<R>(pr, STAGE == 2, t);
+    if (threadIdx.x == 0) {
         s_snap[0] = STAGE != 1 ? pr.snap_h : nullptr;
         s_snap[1] = pr.snap_u;
         s_snap[2] = pr.snap_v;
     }
     __syncthreads();
     const Grid<R>& gd = s_gd;
-    Q4<R>* s_cell = reinterpret_cast<Q4<R>*>(smem_raw);
+    Q4<R>* s_cell = reinterpret_cast<Q4<R>*>(smem_raw + seg * G::seg_stride);
     Q4<R>* s_rp = s_cell + G::RING * P;
     Q4<R>* s_xf = s_rp + P;
     Q4<R>* s_yf = s_xf + 2 * P;
     R* s_rs = reinterpret_cast<R*>(s_yf + G::RING * P);
     R* s_th = s_rs + P;
-    StripPipe<R, NT, STAGE> pp{s_cell, s_rp, s_xf, s_yf, s_rs, s_th, gd, c, bcv, s_snap,
+    StripPipe<R, NT, STAGE, SEG> pp{s_cell, s_rp, s_xf, s_yf, s_rs, s_th, gd, c, bcv, s_snap,
                                STAGE == 2 ? gd.h1 : gd.h, STAGE == 2 ? gd.hu1 : gd.hu, STAGE == 2 ? gd.hv1 : gd.hv};
     const int nx = gd.nx, ny = gd.ny;
-    const int x0 = sr.x0, W = sr.w, y0 = sr.y0, y1 = sr.y1;
+    const int x0 = sr.x0, W = sr.w, rows = (sr.y1 - sr.y0 + SEG - 1) / SEG;
+    const int y0 = SEG == 1 ? sr.y0 : min(sr.y0 + seg * rows, sr.y1), y1 = SEG == 1 ? sr.y1 : min(y0 + rows, sr.y1);
     const int cx = x0 - 3 + t;                        // this thread's column
     const int q = cx - x0;                            // column relative to the strip
     pp.ts = t + 1;
@@ -600,8 +648,13 @@ __global__ void __launch_bounds__(NT, StripGeom<R, NT>::min_ctas(STAGE)) strip_k
     pp.cxc = cx < 0 ? 0 : (cx > nx - 1 ? nx - 1 : cx);
     pp.nx = nx;
     pp.ny = ny;
+    pp.cy0 = sr.y0;
     pp.y0 = y0;
     pp.y1 = y1;
+    R* const s_sum = reinterpret_cast<R*>(smem_raw + SEG * G::seg_stride);
+    R* const s_max = s_sum + (sr.y1 - sr.y0) * (G::NSUM * NT);
+    pp.sums = s_sum + t;
+    pp.bar = seg + 1;
     pp.col_in = (unsigned)cx < (unsigned)nx;
     pp.do_out = q >= 0 && q < W && pp.col_in;
     pp.west = cx == 0;
@@ -610,28 +663,40 @@ __global__ void __launch_bounds__(NT, StripGeom<R, NT>::min_ctas(STAGE)) strip_k
     pp.xside = cx < 0 ? EDGE_W : EDGE_E;
     pp.xkind = pp.col_in ? -1 : gd.bc[pp.xside];
     pp.dt = par_dt<R>(pr);
-    pp.rdx = gd.rdx;
-    pp.rdy = gd.rdy;
     pp.idx = gd.idx;
     pp.idy = gd.idy;
-    pp.rdt = par_rain<R>(pr) * pp.dt;
+    pp.rdt = __fmul_rn(par_rain<R>(pr), pp.dt);
     pp.tt = clamp0(par_t<R>(pr) - gd.rt0);
     pp.acc_clip = pp.xin = pp.xout = pp.yin = pp.yout = pp.infil = pp.rainw = pp.rate = pp.hsum = pp.ssum = R(0);
     pp.hmax = R(0);
     pp.by1 = pp.by2 = pp.bx1 = R(0);
     // software pipeline: raw rows are fetched one row ahead
-    pp.ra = halo_fetch(c, gd, pp.H, pp.HU, pp.HV, cx, y0 - 3);
+    if (SEG == 1 || y0 < y1) pp.ra = halo_fetch(c, gd, pp.H, pp.HU, pp.HV, cx, y0 - 3);
     static_assert((G::RING & (G::RING - 1)) == 0, "ring slots are row & (RING - 1)");
     // steady-state rows: every row touched (r-4 .. r+1) inside the grid, the update row
     // neither the first nor the last row of the grid
     const int r_lo = max(y0 + 3, 4), r_hi = min(y1 + 2, ny - 2);
-    int r = y0 - 3;
+    int r = SEG == 1 || y0 < y1 ? y0 - 3 : y1 + 3;     // a segment without rows marches none
     for (; r <= y1 + 2 && r < r_lo; ++r) pp.template row<false>(r);
     // (not unrolled: four copies of the row body ran 1.75x slower, the hot loop no
     // longer fitting the instruction cache beside the other member chains' kernels)
     for (; r <= r_hi; ++r) pp.template row<true>(r);
     for (; r <= y1 + 2; ++r) pp.template row<false>(r);
+    if (SEG > 1 && STAGE != 1) {
+        s_max[(seg * G::NMAX + 0) * NT + t] = pp.rate;
+        s_max[(seg * G::NMAX + 1) * NT + t] = pp.hmax;
+    }
     __syncthreads();
+    if (SEG > 1 && seg == 0) {
+        pp.take_sums(sr.y1 - sr.y0);
+        if (STAGE != 1) {
+#pragma unroll
+            for (int k = 1; k < SEG; ++k) {
+                pp.rate = rmax(pp.rate, s_max[(k * G::NMAX + 0) * NT + t]);
+                pp.hmax = rmax(pp.hmax, s_max[(k * G::NMAX + 1) * NT + t]);
+            }
+        }
+    }
     R* red = reinterpret_cast<R*>(smem_raw);
     double* out = partials + (size_t)blockIdx.x * NPART;
     if (STAGE == 1) {
@@ -684,7 +749,7 @@ __device__ __forceinline__ float cell_rate(const KC<float>& c, float h, float hu
     float u, v;
     kp_velocity(c, h, hu, hv, u, v);
     const float cw = sqrtf(c.g * h);
-    return h > c.h_dry ? per_len(fabsf(u) + cw, gd.rdx, gd.idx) + per_len(fabsf(v) + cw, gd.rdy, gd.idy) : 0.0f;
+    return h > c.h_dry ? fmaf(__fadd_rn(fabsf(v), cw), gd.idy, __fmul_rn(__fadd_rn(fabsf(u), cw), gd.idx)) : 0.0f;
 }
 __device__ __forceinline__ double rate64(const KC<double>& c, double h, double u, double v, double dx, double dy,
                                          double idx, double idy) {
