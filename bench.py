@@ -37,7 +37,14 @@ sys.path.insert(0, str(ROOT))
 
 ALG_BYTES_F32 = 64      # per member-cell-step: 11 fields read + 5 written, float32
 ALG_BYTES_F64 = 128
-LAUNCHES_PER_STEP = 5   # pre, stage 1, stage 2, 1-D substeps, post: per member chain
+# pre, stage 1, stage 2, 1-D substeps, post: per member chain.  Up to 32 members a step's post
+# and the next one's pre are one kernel inside a graph of 16 steps.
+LAUNCHES_PER_STEP = 5
+
+
+def launches(members: int, chains: int, steps: int) -> int:
+    per_chain = LAUNCHES_PER_STEP * steps if members > 32 else (LAUNCHES_PER_STEP - 1) * steps + -(-steps // 16)
+    return per_chain * chains
 
 
 def parse():
@@ -467,7 +474,7 @@ def run_ours(args, world, rank, local):
            "vs_baseline": None, "dtype": "f32 (f64 accumulators, 1-D channel state and junction depths)",
            "data": "synthetic (seeded terrain, forcing and networks)",
            "config": workload_config(members),
-           "gpu_launches": LAUNCHES_PER_STEP * eng.chains * args.steps, "tile": list(eng.tile), "chains": eng.chains,
+           "gpu_launches": launches(members, eng.chains, args.steps), "tile": list(eng.tile), "chains": eng.chains,
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                         "frac": achieved / hbm, "peak_kind": peak_kind,
                         "traffic": traffic * cells if traffic is not None else None,

@@ -11,6 +11,9 @@
 //                                                         (coupling.py:216-221)
 //   eng_post  (one CTA per member)  step volumes summed in tile order into the
 //             float64 accumulators, t += dt, plausibility (coupling.py:213-227, :169-192)
+//
+// Where a member's pre-step has several CTAs, a step's eng_post and the next one's eng_pre
+// are one kernel (TURN below).
 #pragma once
 #include "net1d_kernels.cuh"
 #include "swe2d_strip.cuh"
@@ -30,16 +33,26 @@ namespace his {
 constexpr int PRE_MEMBERS_F32 = 32;
 constexpr int ENG_PRE_THREADS = 512, ENG_EXCH_THREADS = 448, ENG_EXCH_WARPS = ENG_EXCH_THREADS / 32;
 
-template <class R, int G>
-__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 ? 2 : 1)
+//
+// TURN: the last step's eng_post in front, spread over warps 14 and 15 of the member's CTAs:
+// every CTA's take the clock, the rate and the status they need, side by side with the
+// exchange's loads and water levels; rank 0's write them, and those of ranks 1 to 3 add up the
+// volumes.  eng_post's chain (partial sums, then a division) and one launch leave the step:
+// six served storms 60 -> 57 us a step, one float64 storm of 400 x 325 cells 252 -> 248.
+// A member that ended or failed leaves at the substep count (s_nsub), as one that needs too
+// many substeps does: after the barriers, before any state is written.
+template <class R, int G, bool TURN>
+__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(ENG_PRE_THREADS, sizeof(R) == 4 && G == 1 ? 2 : 1)
 eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params, const Grid<R>* __restrict__ grids,
                const Net* __restrict__ nets, const Lnk* __restrict__ links, Consts c, ExchK<R> K,
-               double* __restrict__ netf, int max_sub, double* Vg, double* __restrict__ exch, int m0) {
+               double* __restrict__ netf, int max_sub, double* Vg, double* __restrict__ exch, int m0,
+               const double* __restrict__ partials, const double* __restrict__ vol1d, double* __restrict__ out) {
+    static_assert(!TURN || G >= 4, "the volumes are added up by three CTAs beside the first");
     extern __shared__ double sm[];
     __shared__ Lnk s_L;
     __shared__ Net s_N;
-    __shared__ int s_nsub, s_snap;
-    __shared__ double s_dt;
+    __shared__ int s_nsub, s_snap, s_status;
+    __shared__ double s_dt, s_t;
     __shared__ R s_dtr, s_rate[G * ENG_EXCH_WARPS];     // every CTA's rates
     const int m = m0 + blockIdx.x / G, rank = blockIdx.x % G, tid = threadIdx.x, lane = tid & 31;
     EngMember& E = em[m];
@@ -48,6 +61,81 @@ eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params, cons
         if (rank == 0 && tid == 0) P.active = 0;
         return;
     }
+    // what the last step left, the clock and the output counter one step on (volatile: every
+    // CTA reads it before the first barrier, behind which another CTA writes it)
+    struct { double t, dt, rate, rain; int k_out, snap, n_sub; double* ledger; } last{};
+    if (tid >= ENG_EXCH_THREADS) {
+        const volatile EngMember& Ev = E;
+        const volatile StepParams& Pv = P;
+        last.t = Ev.t;
+        last.rate = Ev.rate;
+        last.k_out = Ev.k_out;
+        if (TURN) {
+            last.dt = Ev.dt;
+            last.t += last.dt;
+            last.rain = Pv.rain;
+            last.snap = Pv.snap_k;
+            last.n_sub = Ev.n_sub;
+            if (last.snap >= 0) {
+                last.k_out = last.snap + 1;
+                last.ledger = Pv.snap_ledger;
+            }
+        }
+    }
+    // TURN: step volumes into the accumulators, by warp 14 (w = 0) and 15 (w = 1) of ranks 1 to 3
+    auto add_volumes = [&](int w) {
+        if (rank > 3) return;
+        const Grid<R>& gd = grids[m];
+        double* o = out + (size_t)m * 8;
+        double* L = last.ledger;
+        const bool net = vol1d && last.n_sub > 0;
+        double S[NPART];
+        auto take = [&](auto... q) {
+            const int j[sizeof...(q)] = {(int)q...};
+            double s[sizeof...(q)];
+            sum_columns<sizeof...(q)>(partials, gd.tile0, gd.n_tiles, j, s);
+            int k = 0;
+            ((S[q] = s[k++]), ...);
+        };
+        auto account = [&](int term, int a, double more) {
+            const double v = step_term(term, gd, last.dt, last.rain, c.order, S);
+            if (lane != 0) return;
+            o[term] = v;
+            double acc = E.acc[a] + v;
+            if (term == 4 && net) acc += more;
+            E.acc[a] = acc;
+            if (L) L[L_RAIN + a] = acc;
+        };
+        if (rank == 1 && w == 0) {
+            take(P_XIN1, P_YIN1, P_XIN2, P_YIN2);
+            account(0, 2, 0.0);
+        } else if (rank == 1) {
+            take(P_XOUT1, P_YOUT1, P_XOUT2, P_YOUT2);
+            account(1, 3, 0.0);
+        } else if (rank == 2 && w == 0) {
+            take(P_RAINW, P_INFIL);
+            account(2, 0, 0.0);
+            account(3, 1, 0.0);
+        } else if (rank == 2) {
+            take(P_CLIP1, P_CLIP2);
+            account(4, 6, net ? vol1d[m * 3 + 2] : 0.0);
+        } else if (w == 0) {
+            take(P_HSUM, P_SSUM);
+            if (lane == 0) {
+                const double v2 = S[P_HSUM] * gd.area, vs = S[P_SSUM] * gd.area;
+                o[6] = v2;
+                o[7] = vs;
+                if (L) {
+                    L[L_V2D] = v2;
+                    L[L_STORE] = vs;
+                }
+            }
+        } else if (lane < 2) {
+            const double acc = net ? E.acc[4 + lane] + vol1d[m * 3 + lane] : E.acc[4 + lane];
+            E.acc[4 + lane] = acc;
+            if (L) L[L_BND1_IN + lane] = acc;
+        }
+    };
     if (nets) stage_record(&s_N, nets + m);
     if (links) stage_record(&s_L, links + m);
     // barriers of the CTA and of the member's CTAs, reached from the roles' own code
@@ -95,23 +183,33 @@ eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params, cons
         }
         return;
     }
+    const Grid<R>& gd = grids[m];
     if (tid < ENG_EXCH_THREADS + 32) {
+        double rate = last.rate;
+        if (TURN) {
+            const int j[1] = {P_RATE};
+            double s[1];
+            sum_columns<1>(partials, gd.tile0, gd.n_tiles, j, s);
+            rate = s[0];
+        }
+        const double t = last.t;
+        bool clamped = false;
         if (lane == 0) {
-            const double rate = E.rate;
             double dt = rate > 0.0 ? c.cfl / rate : c.dt_max;
             if (dt < c.dt_min || dt > c.dt_max) {
-                if (dt < c.dt_min && rank == 0) E.n_clamped++;
+                clamped = dt < c.dt_min;
                 dt = fmin(fmax(dt, c.dt_min), c.dt_max);
             }
             // the step ends at the member's end or its next output time (coupling.py:255-262)
             double limit = E.t_end;
-            const bool out_on = E.n_out > 0 && E.k_out < E.n_out;
-            const double t_next = out_on ? E.out_dt * E.k_out : 0.0;
+            const bool out_on = E.n_out > 0 && last.k_out < E.n_out;
+            const double t_next = out_on ? E.out_dt * last.k_out : 0.0;
             if (out_on) limit = fmin(limit, t_next);
-            dt = fmin(dt, limit - E.t);
+            dt = fmin(dt, limit - t);
             s_dt = dt;
             s_dtr = (R)dt;
-            s_snap = out_on && E.t + dt >= t_next - 1e-9 ? E.k_out : -1;
+            s_t = t;
+            s_snap = out_on && t + dt >= t_next - 1e-9 ? last.k_out : -1;
         }
         __syncwarp();
         wide();                                  // dt is chosen, the channel rates are in s_rate
@@ -124,41 +222,78 @@ eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params, cons
                 const double ns = ceil(s_dt / dt1 - 1e-9);
                 n = ns < 1.0 ? 1 : (ns > (double)max_sub ? max_sub + 1 : (int)ns);
             }
-            s_nsub = n;
+            const bool run = !TURN || s_status == ST_RUNNING;
+            s_nsub = run ? n : max_sub + 1;
+            if (rank == 0) {
+                if (run && clamped) E.n_clamped++;
+                if (TURN) {
+                    out[(size_t)m * 8 + 5] = rate;
+                    E.rate = rate;
+                    E.t = t;
+                    if (last.snap >= 0) {
+                        E.snap_t[last.snap] = t;
+                        E.k_out = last.k_out;
+                    }
+                    E.steps += 1;
+                    E.n_sub_max = max(E.n_sub_max, last.n_sub);
+                    E.dt_min = fmin(E.dt_min, last.dt);
+                    E.dt_max = fmax(E.dt_max, last.dt);
+                }
+            }
         }
         __syncwarp();
         if (multi)                               // (the exchange's own barriers)
             for (int k = 0; k < 3; ++k) wide();
         all();                                   // the substep count is known
-        if (rank != 0) return;
+        if (rank != 0) {
+            if (TURN) add_volumes(0);
+            return;
+        }
         const int n = s_nsub;
         if (n > max_sub) {
             if (lane == 0) {
-                E.status = ST_SUBSTEPS;
+                if (!TURN || s_status == ST_RUNNING) E.status = ST_SUBSTEPS;
                 P.active = 0;
             }
             return;
         }
         const double sub = s_dt / n;
         for (int k = lane; k < n; k += 32) {
-            const double tk = E.t + k * sub;
+            const double tk = s_t + k * sub;
             netf[((size_t)m * max_sub + k) * 2 + 0] = eng_inflow(E, tk);
             netf[((size_t)m * max_sub + k) * 2 + 1] = eng_tide(E, tk);
         }
         return;
+    }
+    if (TURN) {
+        const int j[3] = {P_HSUM, P_RATE, P_HMAX};
+        double s[3];
+        sum_columns<3>(partials, gd.tile0, gd.n_tiles, j, s);
+        if (lane == 0) {
+            int st = ST_RUNNING;
+            if (!isfinite(s[0]) || !isfinite(s[1])) st = ST_NONFINITE;
+            else if (s[2] > MAX_PLAUSIBLE_DEPTH_2D) st = ST_IMPLAUSIBLE;
+            else if (last.t >= E.t_end - 1e-9) st = ST_DONE;
+            s_status = st;
+            if (rank == 0) E.status = st;
+        }
     }
     wide();
     const double dt = s_dt;
     // edge values at t by lanes 0..3 and at t + dt by lanes 4..7, rain by lane 8
     double v = 0.0;
     if (rank != 0) v = 0.0;
-    else if (lane < 8) v = eng_edge(E, lane & 3, lane < 4 ? E.t : E.t + dt);
-    else if (lane == 8) v = eng_rain(E, E.t);
+    else if (lane < 8) v = eng_edge(E, lane & 3, lane < 4 ? s_t : s_t + dt);
+    else if (lane == 8) v = eng_rain(E, s_t);
     __syncwarp();
     if (multi)
         for (int k = 0; k < 3; ++k) wide();
     all();
-    if (rank != 0 || s_nsub > max_sub) return;
+    if (rank != 0) {
+        if (TURN) add_volumes(1);
+        return;
+    }
+    if (s_nsub > max_sub) return;
     if (lane < 4) {
         P.bc0[lane] = v;
         P.bc0_f[lane] = (float)v;
@@ -170,9 +305,9 @@ eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params, cons
         P.rain_f = (float)v;
     } else if (lane == 9) {
         P.dt = dt;
-        P.t = E.t;
+        P.t = s_t;
         P.dt_f = (float)dt;
-        P.t_f = (float)E.t;
+        P.t_f = (float)s_t;
         E.dt = dt;
         E.n_sub = s_nsub;
         P.active = 1;
@@ -207,7 +342,7 @@ __global__ void __launch_bounds__(FIN_THREADS) eng_post_kernel(EngMember* __rest
     double* L = pr.snap_k >= 0 ? pr.snap_ledger : nullptr;      // the 1-D kernel writes L[L_V1D]
     const bool net = vol1d && E.n_sub > 0;
     if (warp <= 4) {
-        const double v = step_term(warp, gd, pr, c.order, S);
+        const double v = step_term(warp, gd, pr.dt, pr.rain, c.order, S);
         o[warp] = v;
         const int a = warp == 0 ? 2 : warp == 1 ? 3 : warp == 2 ? 0 : warp == 3 ? 1 : 6;
         double acc = E.acc[a] + v;

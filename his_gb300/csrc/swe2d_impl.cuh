@@ -367,9 +367,14 @@ int exchange_impl(his_links* l, const Consts& c, double dt, double* V, cudaStrea
     return HIS_OK;
 }
 
-// The pre-step of members [m0, m0 + mc), with the set's number of CTAs per member.
+// CTAs per member of a set's pre-steps (see eng_pre_kernel).
 template <class R>
-void launch_pre(his_engine* E, const Grid<R>* grids, int m0, int mc, cudaStream_t s) {
+int pre_ctas(const his_engine* E) { return sizeof(R) == 8 ? EXCH_SLICES : E->n <= PRE_MEMBERS_F32 ? 4 : 1; }
+
+// The pre-step of members [m0, m0 + mc), with the set's number of CTAs per member; turn: behind
+// the accounting of the step before it (pre_ctas > 1).
+template <class R>
+void launch_pre(his_engine* E, const Grid<R>* grids, int m0, int mc, cudaStream_t s, bool turn = false) {
     his_grid* g = E->grid;
     const Net* nets = E->net ? E->net->d_nets : nullptr;
     const Lnk* links = E->links ? E->links->d_links : nullptr;
@@ -378,11 +383,13 @@ void launch_pre(his_engine* E, const Grid<R>* grids, int m0, int mc, cudaStream_
     auto launch = [&](auto kernel, int ctas) {
         kernel<<<mc * ctas, ENG_PRE_THREADS, E->pre_smem, s>>>(E->d_em, g->d_params, grids, nets, links, g->c,
                                                                make_exch_k<R>(g->c), E->d_netf, E->max_sub, vpos, exch,
-                                                               m0);
+                                                               m0, g->d_partials, E->net ? E->d_vol1d : nullptr,
+                                                               g->d_out);
     };
-    if constexpr (sizeof(R) == 8) launch(eng_pre_kernel<R, EXCH_SLICES>, EXCH_SLICES);
-    else if (E->n <= PRE_MEMBERS_F32) launch(eng_pre_kernel<R, 4>, 4);
-    else launch(eng_pre_kernel<R, 1>, 1);
+    constexpr int G = sizeof(R) == 8 ? EXCH_SLICES : 4;
+    if (sizeof(R) == 4 && pre_ctas<R>(E) == 1) launch(eng_pre_kernel<R, sizeof(R) == 4 ? 1 : G, false>, 1);
+    else if (turn) launch(eng_pre_kernel<R, G, true>, G);
+    else launch(eng_pre_kernel<R, G, false>, G);
 }
 
 // One device-resident step for every member of one chain (see engine_kernels.cuh)
@@ -396,8 +403,9 @@ int eng_enqueue_nt(his_grid* g, his_engine* E, int chain, int n_steps) {
     cudaStream_t s_main = E->main_of(chain), s_side = E->side_of(chain);
     cudaEvent_t fork = E->fork_of(chain), join = E->join_of(chain);
     if (mc == 0) return HIS_OK;
+    const bool turns = pre_ctas<R>(E) > 1;
     for (int k = 0; k < n_steps; ++k) {
-        launch_pre<R>(E, grids, m0, mc, s_main);
+        if (k == 0 || !turns) launch_pre<R>(E, grids, m0, mc, s_main);
         if (E->net) {
             HIS_CK(cudaEventRecord(fork, s_main));
             HIS_CK(cudaStreamWaitEvent(s_side, fork, 0));
@@ -408,7 +416,8 @@ int eng_enqueue_nt(his_grid* g, his_engine* E, int chain, int n_steps) {
         int rc = launch_stages<R, NT>(g, s_main, t0, tc);
         if (rc) return rc;
         if (E->net) HIS_CK(cudaStreamWaitEvent(s_main, join, 0));
-        eng_post_kernel<R><<<mc, FIN_THREADS, 0, s_main>>>(E->d_em, g->d_params, grids, g->c, g->d_partials,
+        if (turns && k + 1 < n_steps) launch_pre<R>(E, grids, m0, mc, s_main, true);
+        else eng_post_kernel<R><<<mc, FIN_THREADS, 0, s_main>>>(E->d_em, g->d_params, grids, g->c, g->d_partials,
                                                   E->net ? E->d_vol1d : nullptr, g->d_out, m0);
         HIS_CK(cudaGetLastError());
     }
@@ -425,15 +434,9 @@ template <class R>
 int engine_take_rate_impl(his_engine* E) {
     // kernel attributes are set here, outside any stream capture
     if (E->pre_smem > 48 * 1024) {
-        if constexpr (sizeof(R) == 8) {
-            HIS_CK(cudaFuncSetAttribute(eng_pre_kernel<R, EXCH_SLICES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)E->pre_smem));
-        } else {
-            HIS_CK(cudaFuncSetAttribute(eng_pre_kernel<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)E->pre_smem));
-            HIS_CK(cudaFuncSetAttribute(eng_pre_kernel<R, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)E->pre_smem));
-        }
+        constexpr int G = sizeof(R) == 8 ? EXCH_SLICES : 4;
+        for (auto kernel : {eng_pre_kernel<R, sizeof(R) == 4 ? 1 : G, false>, eng_pre_kernel<R, G, false>, eng_pre_kernel<R, G, true>})
+            HIS_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E->pre_smem));
     }
     int rc = grid_reduce_impl<R>(E->grid, E->s0, nullptr, false);
     if (rc) return rc;

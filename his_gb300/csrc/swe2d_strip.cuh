@@ -805,47 +805,57 @@ __global__ void __launch_bounds__(CHUNK_THREADS) strip_rate_kernel(const Grid<R>
     block_reduce_store<1>(v, mx, red, partials + (size_t)blockIdx.x * NPART, sl, CHUNK_THREADS);
 }
 
-// Sums (and the rate's and depth's maxima) of a member's strip-chunk partials into
-// S[NPART], in a fixed order: warp w takes the quantities w, w + FIN_WARPS, ..., lane l the
-// tiles l, l + 32, ..., then the lanes by a shuffle tree.  Eight warps instead of one: a
-// float64 add costs a warp 64 cycles, and one warp spent 16 quantities x (tiles / 32 + 5)
-// of them in a row (1601 x 1301 float32 step with its reduction 261 -> 244 us, 225 -> 212
-// with four loads in flight and votes instead of adds of zeros; six served
-// storms 94.7 -> 89.1 us per step).
-constexpr int FIN_THREADS = 256, FIN_WARPS = FIN_THREADS / 32;
-__device__ __forceinline__ void sum_partials(const double* __restrict__ partials, int tile0, int n_tiles, double* S) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    static_assert(NPART == 2 * FIN_WARPS, "two quantities per warp");
-    const int ja = warp, jb = warp + FIN_WARPS;
-    const bool ma = ja == P_RATE || ja == P_HMAX, mb = jb == P_RATE || jb == P_HMAX;
-    double a = 0.0, b = 0.0;
+// N quantities j[] of a member's strip-chunk partials over its tiles, each summed (the rate
+// and the depth: their maximum) in a fixed order by one warp: lane l takes the tiles l,
+// l + 32, ..., then the lanes by a shuffle tree; valid in lane 0.
+template <int N>
+__device__ __forceinline__ void sum_columns(const double* __restrict__ partials, int tile0, int n_tiles,
+                                            const int (&j)[N], double (&s)[N]) {
+    const int lane = threadIdx.x & 31;
+    bool mx[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        mx[q] = j[q] == P_RATE || j[q] == P_HMAX;
+        s[q] = 0.0;
+    }
     // four tiles' loads in flight; a quantity that is zero in every lane's tile (edges, clips,
     // options that are off) costs a vote instead of an add
-    auto add = [](double& s, double v, bool mx) {
-        if (!__any_sync(0xffffffffu, f64_bits(v) << 1 != 0)) return;
-        if (mx) s = fmax(s, v);
-        else s += v;
-    };
     const double* p = partials + (size_t)tile0 * NPART;
     for (int t0 = 0; t0 < n_tiles; t0 += 128) {
-        double pa[4], pb[4];
+        double v[4][N];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int t = t0 + 32 * k + lane;
-            pa[k] = t < n_tiles ? p[(size_t)t * NPART + ja] : 0.0;
-            pb[k] = t < n_tiles ? p[(size_t)t * NPART + jb] : 0.0;
+#pragma unroll
+            for (int q = 0; q < N; ++q) v[k][q] = t < n_tiles ? p[(size_t)t * NPART + j[q]] : 0.0;
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            add(a, pa[k], ma);
-            add(b, pb[k], mb);
-        }
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int q = 0; q < N; ++q) {
+                if (!__any_sync(0xffffffffu, f64_bits(v[k][q]) << 1 != 0)) continue;
+                s[q] = mx[q] ? fmax(s[q], v[k][q]) : s[q] + v[k][q];
+            }
     }
-    a = ma ? warp_max(a) : warp_sum_sparse(a);
-    b = mb ? warp_max(b) : warp_sum_sparse(b);
-    if (lane == 0) {
-        S[ja] = a;
-        S[jb] = b;
+#pragma unroll
+    for (int q = 0; q < N; ++q) s[q] = mx[q] ? warp_max(s[q]) : warp_sum_sparse(s[q]);
+}
+
+// All of them into S[NPART] by a CTA: warp w the quantities w and w + FIN_WARPS.  Eight warps
+// instead of one: a float64 add costs a warp 64 cycles, and one warp spent 16 quantities x
+// (tiles / 32 + 5) of them in a row (1601 x 1301 float32 step with its reduction 261 -> 244 us,
+// 225 -> 212 with four loads in flight and votes instead of adds of zeros; six served
+// storms 94.7 -> 89.1 us per step).
+constexpr int FIN_THREADS = 256, FIN_WARPS = FIN_THREADS / 32;
+__device__ __forceinline__ void sum_partials(const double* __restrict__ partials, int tile0, int n_tiles, double* S) {
+    const int warp = threadIdx.x >> 5;
+    static_assert(NPART == 2 * FIN_WARPS, "two quantities per warp");
+    const int j[2] = {warp, warp + FIN_WARPS};
+    double s[2];
+    sum_columns<2>(partials, tile0, n_tiles, j, s);
+    if ((threadIdx.x & 31) == 0) {
+        S[j[0]] = s[0];
+        S[j[1]] = s[1];
     }
     __syncthreads();
 }
@@ -854,9 +864,9 @@ __device__ __forceinline__ void sum_partials(const double* __restrict__ partials
 // warps, so that their float64 chains run side by side.  term: 0 boundary in, 1 boundary
 // out, 2 rain, 3 infiltration, 4 clip.
 template <class R>
-__device__ __forceinline__ double step_term(int term, const Grid<R>& gd, const StepParams& pr, int order,
+__device__ __forceinline__ double step_term(int term, const Grid<R>& gd, double dt_, double rain, int order,
                                             const double* S) {
-    const double dt = (double)R(pr.dt);
+    const double dt = (double)R(dt_);
     if (term <= 1) {
         double q = S[term ? P_XOUT1 : P_XIN1] * gd.dy + S[term ? P_YOUT1 : P_YIN1] * gd.dx;
         if (order == 2) q = 0.5 * (q + (S[term ? P_XOUT2 : P_XIN2] * gd.dy + S[term ? P_YOUT2 : P_YIN2] * gd.dx));
@@ -864,7 +874,7 @@ __device__ __forceinline__ double step_term(int term, const Grid<R>& gd, const S
     }
     if (term == 2)
         return gd.rw ? S[P_RAINW] * gd.area
-                     : (double)(R(pr.rain) * R(pr.dt)) * ((double)((long long)gd.nx * gd.ny) * gd.area);
+                     : (double)(R(rain) * R(dt_)) * ((double)((long long)gd.nx * gd.ny) * gd.area);
     if (term == 3) return S[P_INFIL] * gd.area;
     const double clip = S[P_CLIP1] * gd.area;
     return order == 2 ? clip + S[P_CLIP2] * gd.area : clip;
@@ -914,7 +924,7 @@ __global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const Grid<R>* __
     } else if (warp == 7) {
         o[7] = S[P_SSUM] * gd.area;
     } else if (mode == 0) {
-        const double v = step_term(warp, gd, params[m], c.order, S);
+        const double v = step_term(warp, gd, params[m].dt, params[m].rain, c.order, S);
         o[warp] = v;
         if (ext) ext[(size_t)m * 5 + warp] = v;
         if (ledger) {
