@@ -266,7 +266,8 @@ int32_t his_grid_destroy(his_grid* g) {
     }
     if (g->pev_fork) cudaEventDestroy(g->pev_fork);
     if (g->ledger_exec) cudaGraphExecDestroy(g->ledger_exec);
-    if (g->stage_exec) cudaGraphExecDestroy(g->stage_exec);
+    if (g->step_graph.exec) cudaGraphExecDestroy(g->step_graph.exec);
+    if (g->rate_graph.exec) cudaGraphExecDestroy(g->rate_graph.exec);
     if (g->cap_stream) cudaStreamDestroy(g->cap_stream);
     delete g;
     return HIS_OK;
@@ -316,7 +317,8 @@ static int grid_parts_setup(his_grid* g) {
     return HIS_OK;
 }
 
-static int fill_params(his_grid* g, const his_step_params* p, StepParams* sp) {
+// vols: where finalize puts the members' volumes for the caller, or NULL
+static int fill_params(his_grid* g, const his_step_params* p, StepParams* sp, double* vols = nullptr) {
     for (int m = 0; m < g->n; ++m) {
         const his_step_params& q = p[m];
         sp[m] = StepParams{};
@@ -324,6 +326,7 @@ static int fill_params(his_grid* g, const his_step_params* p, StepParams* sp) {
         if (!std::isfinite(q.dt) || !(q.dt >= 0) || !std::isfinite(q.t) || !std::isfinite(q.rain))
             return bad("member " + std::to_string(m) + ": dt, t and rain must be finite (dt >= 0)");
         sp[m] = step_params_from(q);
+        if (vols) sp[m].vols = vols + 5 * (size_t)m;
     }
     return HIS_OK;
 }
@@ -337,11 +340,11 @@ static int upload_params(his_grid* g, const his_step_params* p, cudaStream_t s) 
     return HIS_OK;
 }
 
-static int upload_params_pinned(his_grid* g, const his_step_params* p, cudaStream_t s) {
+static int upload_params_pinned(his_grid* g, const his_step_params* p, cudaStream_t s, double* vols = nullptr) {
     int slot = 0;
     auto* sp = (StepParams*)stage_acquire(g->params_stage, sizeof(StepParams) * g->n, &slot);
     if (!sp) return HIS_ERR_CUDA;
-    int rc = fill_params(g, p, sp);
+    int rc = fill_params(g, p, sp, vols);
     if (rc) return rc;
     HIS_CK(cudaMemcpyAsync(g->d_params, sp, sizeof(StepParams) * g->n, cudaMemcpyHostToDevice, s));
     return stage_release(g->params_stage, slot, s);
@@ -370,43 +373,48 @@ int32_t his_grid_step(his_grid* g, const his_step_params* params, double* vols, 
     return HIS_OK;
 }
 
-// The stage launches of a set in parts (their forks and joins: about five calls per part),
-// captured once; the finalize follows it, as its output differs from call to call.
-static int capture_stages(his_grid* g) {
+static int capture_launches(his_grid* g, int (*launches)(his_grid*, cudaStream_t), cudaGraphExec_t* exec) {
     if (!g->cap_stream) HIS_CK(cudaStreamCreateWithFlags(&g->cap_stream, cudaStreamNonBlocking));
     HIS_CK(cudaStreamBeginCapture(g->cap_stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = g->prec == HIS_PREC_F64 ? grid_stages_f64(g, g->cap_stream) : grid_stages_f32(g, g->cap_stream);
+    const int rc = launches(g, g->cap_stream);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(g->cap_stream, &graph);
     if (rc || e != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return rc ? rc : cuda_fail(e, "cudaStreamEndCapture");
     }
-    const cudaError_t ei = cudaGraphInstantiate(&g->stage_exec, graph, 0);
+    const cudaError_t ei = cudaGraphInstantiate(exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (ei != cudaSuccess) g->stage_exec = nullptr;
+    if (ei != cudaSuccess) *exec = nullptr;
     HIS_CK(ei);
     return HIS_OK;
 }
 
-// A step's kernels on s: from the stage graph where the set runs in parts and the caller is
-// not capturing, else launched one by one.
-static int step_kernels(his_grid* g, double* ext, cudaStream_t s) {
-    const bool f64 = g->prec == HIS_PREC_F64;
-    if (g->n_parts > 1 && !g->stage_graph_off) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        HIS_CK(cudaStreamIsCapturing(s, &cs));
-        if (cs == cudaStreamCaptureStatusNone) {
-            if (!g->stage_exec && capture_stages(g) != HIS_OK) {
-                cudaGetLastError();
-                g->stage_graph_off = true;
-            } else {
-                HIS_CK(cudaGraphLaunch(g->stage_exec, s));
-                return f64 ? grid_finalize_f64(g, s, ext) : grid_finalize_f32(g, s, ext);
-            }
+// launches(g, s), from the second call on as a graph, unless the caller is capturing s.
+static int launch_graph(his_grid* g, LaunchGraph& G, cudaStream_t s, int (*launches)(his_grid*, cudaStream_t)) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    HIS_CK(cudaStreamIsCapturing(s, &cs));
+    if (cs != cudaStreamCaptureStatusNone || G.off || (!G.exec && G.calls++ == 0)) return launches(g, s);
+    if (!G.exec) {
+        // relaxed: another thread may be capturing streams of its own meanwhile
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        HIS_CK(cudaThreadExchangeStreamCaptureMode(&mode));
+        const int rc = capture_launches(g, launches, &G.exec);
+        HIS_CK(cudaThreadExchangeStreamCaptureMode(&mode));
+        if (rc != HIS_OK) {
+            cudaGetLastError();
+            G.off = true;
+            return launches(g, s);
         }
     }
-    return f64 ? grid_step_f64(g, s, ext) : grid_step_f32(g, s, ext);
+    HIS_CK(cudaGraphLaunch(G.exec, s));
+    return HIS_OK;
+}
+static int step_launches(his_grid* g, cudaStream_t s) {
+    return g->prec == HIS_PREC_F64 ? grid_step_f64(g, s) : grid_step_f32(g, s);
+}
+static int rate_launches(his_grid* g, cudaStream_t s) {
+    return g->prec == HIS_PREC_F64 ? grid_reduce_f64(g, s, g->h_out, true) : grid_reduce_f32(g, s, g->h_out, true);
 }
 
 int32_t his_grid_step_async(his_grid* g, const his_step_params* params, double* vols, void* stream) {
@@ -419,9 +427,8 @@ int32_t his_grid_step_async(his_grid* g, const his_step_params* params, double* 
     int rc = vols ? check_async_out(vols, "vols", &direct) : HIS_OK;
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if ((rc = upload_params_pinned(g, params, s))) return rc;
-    double* ext = direct ? vols : nullptr;
-    rc = step_kernels(g, ext, s);
+    if ((rc = upload_params_pinned(g, params, s, direct ? vols : nullptr))) return rc;
+    rc = launch_graph(g, g->step_graph, s, step_launches);
     if (rc || !vols || direct) return rc;
     HIS_CK(cudaMemcpy2DAsync(vols, 5 * sizeof(double), g->d_out, 8 * sizeof(double), 5 * sizeof(double), g->n,
                              cudaMemcpyDefault, s));
@@ -449,8 +456,8 @@ static int capture_ledger_step(his_grid* g, double* ledger) {
         g->ledger_exec_for = nullptr;
     }
     HIS_CK(cudaStreamBeginCapture(g->cap_stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = g->prec == HIS_PREC_F64 ? grid_step_f64(g, g->cap_stream, nullptr, ledger)
-                                           : grid_step_f32(g, g->cap_stream, nullptr, ledger);
+    const int rc = g->prec == HIS_PREC_F64 ? grid_step_f64(g, g->cap_stream, ledger)
+                                           : grid_step_f32(g, g->cap_stream, ledger);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(g->cap_stream, &graph);
     if (rc || e != cudaSuccess) {
@@ -484,7 +491,7 @@ int32_t his_grid_step_ledger_async(his_grid* g, const his_step_params* params, d
         g->ledger_graph_off = true;
     }
     if (cs != cudaStreamCaptureStatusNone || g->ledger_graph_off)
-        return g->prec == HIS_PREC_F64 ? grid_step_f64(g, s, nullptr, ledger) : grid_step_f32(g, s, nullptr, ledger);
+        return g->prec == HIS_PREC_F64 ? grid_step_f64(g, s, ledger) : grid_step_f32(g, s, ledger);
     HIS_CK(cudaGraphLaunch(g->ledger_exec, s));
     return HIS_OK;
 }
@@ -517,7 +524,7 @@ int32_t his_grid_max_rate(his_grid* g, double* rate, void* stream) {
     if (!g || !rate) return bad("grid and rate are required");
     // the reduction stores into the pinned buffer itself: no copy to wait for
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = g->prec == HIS_PREC_F64 ? grid_reduce_f64(g, s, g->h_out, true) : grid_reduce_f32(g, s, g->h_out, true);
+    int rc = launch_graph(g, g->rate_graph, s, rate_launches);
     if (rc) return rc;
     HIS_CK(cudaStreamSynchronize(s));
     std::memcpy(rate, g->h_out, sizeof(double) * g->n);

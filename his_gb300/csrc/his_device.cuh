@@ -132,6 +132,7 @@ struct StepParams {
     // this step's snapshot slots (NULL: no output at the end of this step)
     float *snap_h, *snap_u, *snap_v, *snap_eta, *snap_q;
     double* snap_ledger;
+    double* vols;                    // the member's 5 step volumes for the caller (finalize), or NULL
 };
 
 __host__ __device__ inline void params_set_f32(StepParams& p) {

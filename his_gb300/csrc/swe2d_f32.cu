@@ -4,11 +4,7 @@
 
 namespace his {
 int grid_init_f32(his_grid* g) { return grid_init_impl<float>(g); }
-int grid_step_f32(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
-    return grid_step_impl<float>(g, s, ext, ledger);
-}
-int grid_stages_f32(his_grid* g, cudaStream_t s) { return grid_stages_impl<float>(g, s); }
-int grid_finalize_f32(his_grid* g, cudaStream_t s, double* ext) { return launch_finalize<float>(g, s, ext, nullptr); }
+int grid_step_f32(his_grid* g, cudaStream_t s, double* ledger) { return grid_step_impl<float>(g, s, ledger); }
 int grid_reduce_f32(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
     return grid_reduce_impl<float>(g, s, ext, rate_only);
 }

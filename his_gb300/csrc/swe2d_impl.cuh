@@ -166,18 +166,14 @@ int launch_stages_parted(his_grid* g, cudaStream_t s) {
     return HIS_OK;
 }
 
-template <class R>
-int launch_finalize(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
+template <class R, int NT>
+int launch_step_nt(his_grid* g, cudaStream_t s, double* ledger) {
+    int rc = launch_stages_parted<R, NT>(g, s);
+    if (rc) return rc;
     finalize_kernel<R><<<g->n, FIN_THREADS, 0, s>>>(reinterpret_cast<const Grid<R>*>(g->d_grids), g->d_params, g->c,
-                                           g->d_partials, g->d_out, 0, ext, ledger);
+                                           g->d_partials, g->d_out, 0, nullptr, ledger);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
-}
-
-template <class R, int NT>
-int launch_step_nt(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
-    int rc = launch_stages_parted<R, NT>(g, s);
-    return rc ? rc : launch_finalize<R>(g, s, ext, ledger);
 }
 
 template <class R>
@@ -340,13 +336,8 @@ int grid_init_impl(his_grid* g) {
 }
 
 template <class R>
-int grid_step_impl(his_grid* g, cudaStream_t s, double* ext, double* ledger) {
-    HIS_NT_DISPATCH(launch_step_nt, R, g, s, ext, ledger);
-}
-
-template <class R>
-int grid_stages_impl(his_grid* g, cudaStream_t s) {
-    HIS_NT_DISPATCH(launch_stages_parted, R, g, s);
+int grid_step_impl(his_grid* g, cudaStream_t s, double* ledger) {
+    HIS_NT_DISPATCH(launch_step_nt, R, g, s, ledger);
 }
 
 template <class R>

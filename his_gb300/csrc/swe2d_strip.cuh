@@ -883,8 +883,8 @@ __device__ __forceinline__ double step_term(int term, const Grid<R>& gd, double 
 // Per-member totals from the strip-chunk partials, in a fixed order.  out: 8 per
 // member = bnd_in, bnd_out, rain, infil, clip (m^3), rate (1/s), surface and retained
 // volume.  mode 0: after a step; mode 1: rate and volumes only; mode 2: rate only
-// (after strip_rate_kernel).  ext (optional, device-writable): mode 0 the 5 volumes,
-// modes 1 and 2 the rate, per member.  ledger (optional, mode 0): an 8 x n_members
+// (after strip_rate_kernel).  For the caller (device-writable, optional): mode 0 the 5 volumes
+// at StepParams::vols, modes 1 and 2 the rates at ext.  ledger (optional, mode 0): an 8 x n_members
 // float64 ledger (rows LG_*) the step's rain, infiltration, boundary and clip volumes
 // are added into.
 template <class R>
@@ -892,7 +892,7 @@ __global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const Grid<R>* __
                                                                const StepParams* __restrict__ params, Consts c,
                                                                const double* __restrict__ partials,
                                                                double* __restrict__ out, int mode,
-                                                               double* __restrict__ ext,
+                                                               double* __restrict__ ext = nullptr,
                                                                double* __restrict__ ledger = nullptr) {
     __shared__ double S[NPART];
     const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const Grid<R>* __
     } else if (mode == 0) {
         const double v = step_term(warp, gd, params[m].dt, params[m].rain, c.order, S);
         o[warp] = v;
-        if (ext) ext[(size_t)m * 5 + warp] = v;
+        if (params[m].vols) params[m].vols[warp] = v;
         if (ledger) {
             const int row = warp == 0 ? LG_BND2_IN : warp == 1 ? LG_BND2_OUT : warp == 2 ? LG_RAIN
                           : warp == 3 ? LG_INFIL : LG_CLIP2;
