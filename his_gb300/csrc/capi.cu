@@ -1,6 +1,7 @@
 // C ABI of the flood-engine step (include/his_gb300.h): argument checks, device
 // tables, host<->device parameter and result movement, precision dispatch.
 #include <algorithm>
+#include <atomic>
 #include <array>
 #include <cmath>
 #include <cstring>
@@ -245,6 +246,12 @@ int32_t his_grid_create(int32_t precision, const his_solver_cfg* cfg, int32_t n_
     return HIS_OK;
 }
 
+static void graph_drop(LaunchGraph& G) {
+    if (G.exec) cudaGraphExecDestroy(G.exec);
+    G.exec = nullptr;
+    G.calls = 0;
+}
+
 int32_t his_grid_destroy(his_grid* g) {
     if (!g) return HIS_OK;
     cudaFree(g->d_grids);
@@ -265,9 +272,8 @@ int32_t his_grid_destroy(his_grid* g) {
         if (g->pev_join[k]) cudaEventDestroy(g->pev_join[k]);
     }
     if (g->pev_fork) cudaEventDestroy(g->pev_fork);
-    if (g->ledger_exec) cudaGraphExecDestroy(g->ledger_exec);
-    if (g->step_graph.exec) cudaGraphExecDestroy(g->step_graph.exec);
-    if (g->rate_graph.exec) cudaGraphExecDestroy(g->rate_graph.exec);
+    for (LaunchGraph* G : {&g->step_graph, &g->rate_graph, &g->ledger_graph, &g->coupled_graph}) graph_drop(*G);
+    if (g->cap_side) cudaStreamDestroy(g->cap_side);
     if (g->cap_stream) cudaStreamDestroy(g->cap_stream);
     delete g;
     return HIS_OK;
@@ -390,6 +396,7 @@ static int capture_launches(his_grid* g, int (*launches)(his_grid*, cudaStream_t
     return HIS_OK;
 }
 
+// (graph_drop: for other arguments; its next call is a first one again)
 // launches(g, s), from the second call on as a graph, unless the caller is capturing s.
 static int launch_graph(his_grid* g, LaunchGraph& G, cudaStream_t s, int (*launches)(his_grid*, cudaStream_t)) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -435,65 +442,35 @@ int32_t his_grid_step_async(his_grid* g, const his_step_params* params, double* 
     return HIS_OK;
 }
 
-// The caller's ledger must be device memory (the finalize kernel adds into it).
-static int check_ledger(double* ledger) {
+// The caller's ledger must be device memory (the step kernels add into it); *checked: the last
+// one found to be.
+static int ledger_device(double** checked, double* ledger) {
+    if (ledger == *checked) return HIS_OK;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, ledger) != cudaSuccess || a.type != cudaMemoryTypeDevice) {
         cudaGetLastError();
         return bad("ledger must be device memory");
     }
+    *checked = ledger;
     return HIS_OK;
 }
 
-// The ledger step's launches (stages of every part, finalize) captured once per ledger:
-// the same kernels with the same arguments every step (the step parameters are read
-// from the grid's device buffer, uploaded before the graph runs).
-static int capture_ledger_step(his_grid* g, double* ledger) {
-    if (!g->cap_stream) HIS_CK(cudaStreamCreateWithFlags(&g->cap_stream, cudaStreamNonBlocking));
-    if (g->ledger_exec) {
-        HIS_CK(cudaGraphExecDestroy(g->ledger_exec));
-        g->ledger_exec = nullptr;
-        g->ledger_exec_for = nullptr;
-    }
-    HIS_CK(cudaStreamBeginCapture(g->cap_stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = g->prec == HIS_PREC_F64 ? grid_step_f64(g, g->cap_stream, ledger)
-                                           : grid_step_f32(g, g->cap_stream, ledger);
-    cudaGraph_t graph = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(g->cap_stream, &graph);
-    if (rc || e != cudaSuccess) {
-        if (graph) cudaGraphDestroy(graph);
-        return rc ? rc : cuda_fail(e, "cudaStreamEndCapture");
-    }
-    const cudaError_t ei = cudaGraphInstantiate(&g->ledger_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    HIS_CK(ei);
-    g->ledger_exec_for = ledger;
-    return HIS_OK;
+static int ledger_launches(his_grid* g, cudaStream_t s) {
+    return g->prec == HIS_PREC_F64 ? grid_step_f64(g, s, g->ledger_for) : grid_step_f32(g, s, g->ledger_for);
 }
 
 int32_t his_grid_step_ledger_async(his_grid* g, const his_step_params* params, double* ledger, void* stream) {
     if (!g || !params || !ledger) return bad("grid, params and ledger are required");
-    int rc = HIS_OK;
-    if (ledger != g->ledger_checked) {
-        if ((rc = check_ledger(ledger))) return rc;
-        g->ledger_checked = ledger;
-    }
+    int rc = ledger_device(&g->ledger_checked, ledger);
+    if (rc) return rc;
     if (!g->n_parts && (rc = grid_parts_setup(g))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if ((rc = upload_params_pinned(g, params, s))) return rc;
-    // a caller capturing its own graph gets the launches themselves, and so does every
-    // step once a capture has failed (a capture the thread cannot open, for one)
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    HIS_CK(cudaStreamIsCapturing(s, &cs));
-    if (cs == cudaStreamCaptureStatusNone && !g->ledger_graph_off && g->ledger_exec_for != ledger &&
-        capture_ledger_step(g, ledger) != HIS_OK) {
-        cudaGetLastError();
-        g->ledger_graph_off = true;
+    if (g->ledger_for != ledger) {
+        graph_drop(g->ledger_graph);
+        g->ledger_for = ledger;
     }
-    if (cs != cudaStreamCaptureStatusNone || g->ledger_graph_off)
-        return g->prec == HIS_PREC_F64 ? grid_step_f64(g, s, ledger) : grid_step_f32(g, s, ledger);
-    HIS_CK(cudaGraphLaunch(g->ledger_exec, s));
-    return HIS_OK;
+    return launch_graph(g, g->ledger_graph, s, ledger_launches);
 }
 
 int32_t his_grid_max_rate_async(his_grid* g, double* rate, void* stream) {
@@ -639,6 +616,8 @@ int32_t his_net_create(const his_solver_cfg* cfg, int32_t n_members, const his_n
     N->smem = smem;
     N->smem_f32 = smem_f32;
     N->max_sub = 256;
+    static std::atomic<long long> made{0};
+    N->id = ++made;
     cudaGetDevice(&N->device);
     auto fail = [&](cudaError_t e, const char* w) { int r = cuda_fail(e, w); his_net_destroy(N); return r; };
     cudaError_t e = cudaMalloc(&N->d_arena, ar.host.size() ? ar.host.size() : 256);
@@ -680,7 +659,7 @@ int32_t his_net_create(const his_solver_cfg* cfg, int32_t n_members, const his_n
     }
     e = cudaMalloc(&N->d_nets, sizeof(Net) * n_members);
     if (e == cudaSuccess) e = cudaMemcpy(N->d_nets, N->h_nets.data(), sizeof(Net) * n_members, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&N->d_forcing, sizeof(double) * 2 * N->max_sub * n_members);
+    if (e == cudaSuccess) e = cudaMalloc(&N->d_forcing, sizeof(double) * (2 + 2 * (size_t)N->max_sub * n_members));
     if (e == cudaSuccess) e = cudaMalloc(&N->d_out, sizeof(double) * 3 * n_members);
     if (e == cudaSuccess) e = cudaMallocHost(&N->h_out, sizeof(double) * 3 * n_members);
     if (e != cudaSuccess) return fail(e, "his_net_create: allocation");
@@ -702,13 +681,31 @@ int32_t his_net_destroy(his_net* N) {
     return HIS_OK;
 }
 
-int32_t his_net_step(his_net* N, double dt, int32_t n_sub, const double* forcing, double* vols, void* stream) {
-    if (!N || !forcing) return bad("network and forcing are required");
+static int check_substeps(const his_net* N, double dt, int32_t n_sub) {
     if (n_sub < 1 || n_sub > N->max_sub) return bad("n_sub must be in [1, 256]");
     if (!std::isfinite(dt) || !(dt >= 0)) return bad("dt must be finite and >= 0");
+    return HIS_OK;
+}
+
+// dt, the substep count and the forcing to the device, through pinned staging
+static int upload_forcing(his_net* N, double dt, int32_t n_sub, const double* forcing, cudaStream_t s) {
+    const size_t count = 2 * (size_t)n_sub * N->n;
+    int slot = 0;
+    auto* pin = (double*)stage_acquire(N->forcing_stage, sizeof(double) * (2 + count), &slot);
+    if (!pin) return HIS_ERR_CUDA;
+    pin[0] = dt;
+    pin[1] = (double)n_sub;
+    std::memcpy(pin + 2, forcing, sizeof(double) * count);
+    HIS_CK(cudaMemcpyAsync(N->d_forcing, pin, sizeof(double) * (2 + count), cudaMemcpyHostToDevice, s));
+    return stage_release(N->forcing_stage, slot, s);
+}
+
+int32_t his_net_step(his_net* N, double dt, int32_t n_sub, const double* forcing, double* vols, void* stream) {
+    if (!N || !forcing) return bad("network and forcing are required");
     cudaStream_t s = (cudaStream_t)stream;
-    HIS_CK(cudaMemcpyAsync(N->d_forcing, forcing, sizeof(double) * 2 * n_sub * N->n, cudaMemcpyHostToDevice, s));
-    int rc = net_step_launch(N, dt, n_sub, s);
+    int rc = check_substeps(N, dt, n_sub);
+    if (rc || (rc = upload_forcing(N, dt, n_sub, forcing, s))) return rc;
+    rc = net_step_launch(N, s);
     if (rc || !vols) return rc;
     HIS_CK(cudaMemcpyAsync(N->h_out, N->d_out, sizeof(double) * 3 * N->n, cudaMemcpyDeviceToHost, s));
     HIS_CK(cudaStreamSynchronize(s));
@@ -719,20 +716,13 @@ int32_t his_net_step(his_net* N, double dt, int32_t n_sub, const double* forcing
 int32_t his_net_step_async(his_net* N, double dt, int32_t n_sub, const double* forcing, double* vols,
                            void* stream) {
     if (!N || !forcing) return bad("network and forcing are required");
-    if (n_sub < 1 || n_sub > N->max_sub) return bad("n_sub must be in [1, 256]");
-    if (!std::isfinite(dt) || !(dt >= 0)) return bad("dt must be finite and >= 0");
-    bool direct = false;
-    int rc = vols ? check_async_out(vols, "vols", &direct) : HIS_OK;
+    int rc = check_substeps(N, dt, n_sub);
     if (rc) return rc;
+    bool direct = false;
+    if (vols && (rc = check_async_out(vols, "vols", &direct))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    size_t bytes = sizeof(double) * 2 * n_sub * N->n;
-    int slot = 0;
-    void* pin = stage_acquire(N->forcing_stage, bytes, &slot);
-    if (!pin) return HIS_ERR_CUDA;
-    std::memcpy(pin, forcing, bytes);
-    HIS_CK(cudaMemcpyAsync(N->d_forcing, pin, bytes, cudaMemcpyHostToDevice, s));
-    if ((rc = stage_release(N->forcing_stage, slot, s))) return rc;
-    if ((rc = net_step_launch(N, dt, n_sub, s, direct ? vols : nullptr)) || !vols || direct) return rc;
+    if ((rc = upload_forcing(N, dt, n_sub, forcing, s))) return rc;
+    if ((rc = net_step_launch(N, s, direct ? vols : nullptr)) || !vols || direct) return rc;
     HIS_CK(cudaMemcpyAsync(vols, N->d_out, sizeof(double) * 3 * N->n, cudaMemcpyDefault, s));
     return HIS_OK;
 }
@@ -740,22 +730,11 @@ int32_t his_net_step_async(his_net* N, double dt, int32_t n_sub, const double* f
 int32_t his_net_step_ledger_async(his_net* N, double dt, int32_t n_sub, const double* forcing, double* ledger,
                                   void* stream) {
     if (!N || !forcing || !ledger) return bad("network, forcing and ledger are required");
-    if (n_sub < 1 || n_sub > N->max_sub) return bad("n_sub must be in [1, 256]");
-    if (!std::isfinite(dt) || !(dt >= 0)) return bad("dt must be finite and >= 0");
-    int rc = HIS_OK;
-    if (ledger != N->ledger_checked) {
-        if ((rc = check_ledger(ledger))) return rc;
-        N->ledger_checked = ledger;
-    }
+    int rc = check_substeps(N, dt, n_sub);
+    if (rc || (rc = ledger_device(&N->ledger_checked, ledger))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    size_t bytes = sizeof(double) * 2 * n_sub * N->n;
-    int slot = 0;
-    void* pin = stage_acquire(N->forcing_stage, bytes, &slot);
-    if (!pin) return HIS_ERR_CUDA;
-    std::memcpy(pin, forcing, bytes);
-    HIS_CK(cudaMemcpyAsync(N->d_forcing, pin, bytes, cudaMemcpyHostToDevice, s));
-    if ((rc = stage_release(N->forcing_stage, slot, s))) return rc;
-    return net_step_launch(N, dt, n_sub, s, nullptr, ledger);
+    if ((rc = upload_forcing(N, dt, n_sub, forcing, s))) return rc;
+    return net_step_launch(N, s, nullptr, ledger);
 }
 
 int32_t his_net_max_rate_async(his_net* N, double* rate_wet, void* stream) {
@@ -961,23 +940,48 @@ int32_t his_exchange_async(his_links* L, const his_solver_cfg* cfg, double dt, d
     return HIS_OK;
 }
 
+// A coupled step's kernels: the 2-D step on s, the 1-D substeps and the rates of the state
+// they leave beside it on the side stream, joined.
+static int coupled_launches(his_grid* g, cudaStream_t s, cudaStream_t side) {
+    his_net* N = g->coupled.net;
+    HIS_CK(cudaEventRecord(N->ev_fork, s));
+    HIS_CK(cudaStreamWaitEvent(side, N->ev_fork, 0));
+    int rc = g->prec == HIS_PREC_F64 ? grid_step_f64(g, s, g->coupled.ledger) : grid_step_f32(g, s, g->coupled.ledger);
+    if (rc || (rc = net_step_launch(N, side, nullptr, g->coupled.ledger))) return rc;
+    if ((rc = net_reduce_launch(N, side, g->coupled.rate_wet))) return rc;
+    HIS_CK(cudaEventRecord(N->ev_join, side));
+    HIS_CK(cudaStreamWaitEvent(s, N->ev_join, 0));
+    return HIS_OK;
+}
+static int coupled_capture(his_grid* g, cudaStream_t s) {
+    if (!g->cap_side) HIS_CK(cudaStreamCreateWithFlags(&g->cap_side, cudaStreamNonBlocking));
+    return coupled_launches(g, s, g->cap_side);
+}
+
 int32_t his_coupled_step_async(his_grid* g, his_net* N, double dt, int32_t n_sub, const his_step_params* params,
                                const double* forcing, double* ledger, double* rate_wet, void* stream, void* side) {
     if (!g || !N || !params || !forcing || !ledger || !rate_wet)
         return bad("grid, network, params, forcing, ledger and rate_wet are required");
-    cudaStream_t s = (cudaStream_t)stream, s1 = (cudaStream_t)side;
+    cudaStream_t s = (cudaStream_t)stream;
+    bool direct = false;
+    int rc = check_substeps(N, dt, n_sub);
+    if (rc || (rc = ledger_device(&g->ledger_checked, ledger))) return rc;
+    if ((rc = check_async_out(rate_wet, "rate_wet", &direct))) return rc;
+    if (!direct) return bad("rate_wet must be memory the device can write");
+    if (!g->n_parts && (rc = grid_parts_setup(g))) return rc;
     for (cudaEvent_t* ev : {&N->ev_fork, &N->ev_join})
         if (!*ev) HIS_CK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
-    HIS_CK(cudaEventRecord(N->ev_fork, s));
-    int rc = his_grid_step_ledger_async(g, params, ledger, stream);
-    if (rc) return rc;
-    // after the 2-D launch, so that the host prepares the substeps while it runs
-    HIS_CK(cudaStreamWaitEvent(s1, N->ev_fork, 0));
-    if ((rc = his_net_step_ledger_async(N, dt, n_sub, forcing, ledger, side))) return rc;
-    if ((rc = his_net_max_rate_async(N, rate_wet, side))) return rc;
-    HIS_CK(cudaEventRecord(N->ev_join, s1));
-    HIS_CK(cudaStreamWaitEvent(s, N->ev_join, 0));
-    return HIS_OK;
+    if (g->coupled.net_id != N->id || g->coupled.ledger != ledger || g->coupled.rate_wet != rate_wet) {
+        graph_drop(g->coupled_graph);
+        g->coupled = {N, N->id, ledger, rate_wet};
+    }
+    if ((rc = upload_params_pinned(g, params, s))) return rc;
+    if ((rc = upload_forcing(N, dt, n_sub, forcing, s))) return rc;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    HIS_CK(cudaStreamIsCapturing(s, &cs));
+    if (cs != cudaStreamCaptureStatusNone || g->coupled_graph.off || g->coupled_graph.calls++ == 0)
+        return coupled_launches(g, s, (cudaStream_t)side);
+    return launch_graph(g, g->coupled_graph, s, coupled_capture);
 }
 
 int32_t his_links_exchanged(his_links* L, double* totals, int32_t reset, void* stream) {

@@ -60,26 +60,28 @@ struct his_grid {
     int part_t[MAX_PARTS + 1] = {};
     cudaStream_t ps[MAX_PARTS - 1] = {};
     cudaEvent_t pev_fork = nullptr, pev_join[MAX_PARTS - 1] = {};
-    // his_grid_step_ledger_async: the stage launches (all parts, forked and joined)
-    // and the finalize as one graph, captured on cap_stream on the first call for a
-    // ledger and launched on the caller's stream after the parameter upload
-    cudaStream_t cap_stream = nullptr;
-    cudaGraphExec_t ledger_exec = nullptr;
-    double* ledger_exec_for = nullptr;      // the ledger ledger_exec adds into
+    // the graphs' capture streams: all launches, and beside them a coupled step's 1-D side
+    cudaStream_t cap_stream = nullptr, cap_side = nullptr;
     double* ledger_checked = nullptr;       // the last ledger found to be device memory
-    bool ledger_graph_off = false;          // capture failed once: plain launches from then on
+    // his_grid_step_ledger_async: the step's kernels for the ledger they add into
+    LaunchGraph ledger_graph;
+    double* ledger_for = nullptr;
+    // his_coupled_step_async: both models' kernels, for one network, ledger and rate buffer
+    LaunchGraph coupled_graph;
+    struct { struct his_net* net; long long net_id; double *ledger, *rate_wet; } coupled{};
     // his_grid_step_async and his_grid_max_rate: their kernels as graphs from the second call on
     LaunchGraph step_graph, rate_graph;
 };
 
 struct his_net {
+    long long id = 0;                        // of all networks of the process
     his::Consts c{};
     int n = 0, device = 0;
     std::vector<his::Net> h_nets;
     his::Net* d_nets = nullptr;
     void* d_arena = nullptr;
     size_t arena_bytes = 0;
-    double* d_forcing = nullptr;
+    double* d_forcing = nullptr;             // dt, substeps, then the substeps' forcing
     int max_sub = 0;
     double* d_out = nullptr;                 // n x 3
     double* h_out = nullptr;
@@ -206,7 +208,7 @@ int engine_profile_f32(his_engine* e, int n_steps, double* ms);
 
 // net1d.cu
 // vols / rate_wet: optional device-writable outputs (3 per member; rate and wet per member)
-int net_step_launch(his_net* n, double dt, int n_sub, cudaStream_t s, double* vols = nullptr, double* ledger = nullptr);
+int net_step_launch(his_net* n, cudaStream_t s, double* vols = nullptr, double* ledger = nullptr);
 int net_reduce_launch(his_net* n, cudaStream_t s, double* rate_wet = nullptr);
 int net_engine_launch(his_engine* e, cudaStream_t s, int m0, int count);
 int net_engine_prepare(his_engine* e);

@@ -5,16 +5,17 @@
 
 namespace his {
 
-// n_sub substeps of dt/n_sub each for every member; forcing: per member, per
+// n_sub substeps of dt/n_sub each for every member; forcing: dt, n_sub, then per member, per
 // substep (inflow, stage); vols: 3 per member.
 // ledger (optional): 8 x members float64 ledger; the substeps' boundary volumes and
 // clip are added into its 1-D rows.
-__global__ void __launch_bounds__(NET64_THREADS, 1) net_step_kernel(const Net* __restrict__ nets, Consts c, double dt_total, int n_sub,
+__global__ void __launch_bounds__(NET64_THREADS, 1) net_step_kernel(const Net* __restrict__ nets, Consts c,
                                 const double* __restrict__ forcing, double* __restrict__ vols,
                                 double* __restrict__ ledger) {
     extern __shared__ double sm[];
     __shared__ double v[3];
-    net_substeps_dev(nets[blockIdx.x], c, dt_total, n_sub, forcing + (size_t)blockIdx.x * n_sub * 2,
+    const int n_sub = (int)forcing[1];
+    net_substeps_dev(nets[blockIdx.x], c, forcing[0], n_sub, forcing + 2 + (size_t)blockIdx.x * n_sub * 2,
                      (vols || ledger) ? v : nullptr, sm);
     if (threadIdx.x == 0) {
         if (vols)
@@ -91,10 +92,10 @@ int net_engine_launch(his_engine* e, cudaStream_t s, int m0, int count) {
     return HIS_OK;
 }
 
-int net_step_launch(his_net* n, double dt, int n_sub, cudaStream_t s, double* vols, double* ledger) {
+int net_step_launch(his_net* n, cudaStream_t s, double* vols, double* ledger) {
     if (n->smem > 48 * 1024)
         HIS_CK(cudaFuncSetAttribute(net_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n->smem));
-    net_step_kernel<<<n->n, NET64_THREADS, n->smem, s>>>(n->d_nets, n->c, dt, n_sub, n->d_forcing,
+    net_step_kernel<<<n->n, NET64_THREADS, n->smem, s>>>(n->d_nets, n->c, n->d_forcing,
                                                vols ? vols : (ledger ? nullptr : n->d_out), ledger);
     HIS_CK(cudaGetLastError());
     return HIS_OK;

@@ -257,10 +257,11 @@ int32_t his_exchange_async(his_links* links, const his_solver_cfg* cfg, double d
 int32_t his_links_exchanged(his_links* links, double* totals, int32_t reset, void* stream);
 
 /* The step of both models behind an exchange already queued on `stream`, without waiting:
- * there the 2-D step of his_grid_step_ledger_async (params: its records), and beside it on
- * `side`, once the exchange is done, the n_sub substeps of his_net_step_ledger_async and the
- * CFL rates of the 1-D state they leave (his_net_max_rate_async into rate_wet, 2 per
- * member); `stream` then waits for `side`.
+ * the 2-D step of his_grid_step_ledger_async (params: its records) and beside it the n_sub
+ * substeps of his_net_step_ledger_async and the CFL rates of the 1-D state they leave
+ * (his_net_max_rate_async into rate_wet, 2 per member: device or mapped page-locked memory).
+ * `side` is a second stream for the 1-D part where the kernels are not launched as a graph
+ * (a first call, a caller that captures `stream`); `stream` waits for it.
  * Replaces the body of hydrointel/solver/coupling.py:212-227 (CoupledEngine.step). */
 int32_t his_coupled_step_async(his_grid* grid, his_net* net, double dt, int32_t n_sub, const his_step_params* params,
                                const double* forcing, double* ledger, double* rate_wet, void* stream, void* side);
