@@ -237,6 +237,14 @@ __device__ __forceinline__ void block_reduce_store(T (&v)[NV], const bool* is_ma
     }
 }
 
+// *p = max(*p, v) of a running peak (v >= 0, or NaN, which leaves it) without waiting for the
+// old value: floats compare as their bits here.  A load and a store left the row waiting for
+// the load: 16 steps of six served storms with running peaks 906 -> 858 us, of 64 storms 5411
+// -> 5341.
+__device__ __forceinline__ void raise_peak(float* p, float v) {
+    atomicMax(reinterpret_cast<int*>(p), __float_as_int(fmaxf(v, 0.0f)));
+}
+
 // One side of a reconstructed cell as a face sees it: depth, normal and tangential
 // velocity, X = the in-cell bed slope d and S = the in-cell surface slope sE.  The cell's
 // own bed z and depth h0 (the flux's difference form) come with the cell record.
@@ -548,12 +556,12 @@ struct StripPipe {
         } else {
             gd.h1[i] = hn; gd.hu1[i] = hun; gd.hv1[i] = hvn;
         }
-        if (feat & FEAT_PEAK) gd.pk[i] = rmax(gd.pk[i], hn);
+        if (feat & FEAT_PEAK) raise_peak(gd.pk + i, hn);
         // ---- CFL rate of the new state for the next step (swe2d.py:179-184)
         const R u2 = hun * ks, v2 = hvn * ks;
         // running peak speed and output use the KP velocities of the new state, as the
         // reference's snapshots do (swe2d.py:161-167, coupling.py:229-242)
-        if (feat & FEAT_PSPEED) gd.ps[i] = rmax(gd.ps[i], dsqrt(fmaf(u2, u2, __fmul_rn(v2, v2))));
+        if (feat & FEAT_PSPEED) raise_peak(gd.ps + i, dsqrt(fmaf(u2, u2, __fmul_rn(v2, v2))));
         if (feat & FEAT_SNAP) {
             s_snap[0][i] = (float)hn;
             s_snap[1][i] = (float)u2;
