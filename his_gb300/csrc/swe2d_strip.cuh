@@ -308,7 +308,7 @@ struct StripPipe {
     int ts, cx, cxc, nx, ny, cy0, y0, y1, scol, xside, xkind;      // cy0: the chunk's first row; [y0, y1) this march
     unsigned feat;                     // FEAT_* bits of the member's optional fields
     bool col_in, do_out, west, east;
-    R dt, idx, idy, rdt, tt;
+    R dt, hdt, idx, idy, rdt, tt;
     // carried state of this thread's column
     HaloRaw<R> ra;                     // raw row r (prefetched one row ahead)
     Side ylow;                      // plus side of the y-reconstruction of row r-2
@@ -431,8 +431,9 @@ struct StripPipe {
             yn = s_yf[k2 + ts];
             if (FULL || (unsigned)row < (unsigned)ny) {
                 const R Fw = xf0.a, Fe = s_xf[xo + ts + 1].a, Gs = yn.a, Gn = yf0.a;
-                const R out = fmaf(relu(Gn) + relu(-Gs), idy, __fmul_rn(relu(Fe) + relu(-Fw), idx));
-                const R need = __fmul_rn(out, dt);
+                const R out = fmaf((Gn + fabsf(Gn)) + (fabsf(Gs) - Gs), idy,
+                                   __fmul_rn((Fe + fabsf(Fe)) + (fabsf(Fw) - Fw), idx));      // twice the outflow
+                const R need = __fmul_rn(out, hdt);
                 const R hh = c2.a;
                 const R th = need > hh ? hh / (need > R(0) ? need : R(1)) : R(1);
                 th0 = col_in ? th : R(1);
@@ -671,6 +672,7 @@ __global__ void __launch_bounds__(NT * SEG, StripGeom<R, NT>::min_ctas(STAGE, SE
     pp.xside = cx < 0 ? EDGE_W : EDGE_E;
     pp.xkind = pp.col_in ? -1 : gd.bc[pp.xside];
     pp.dt = par_dt<R>(pr);
+    pp.hdt = R(0.5) * pp.dt;
     pp.idx = gd.idx;
     pp.idy = gd.idy;
     pp.rdt = __fmul_rn(par_rain<R>(pr), pp.dt);
