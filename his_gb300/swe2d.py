@@ -292,6 +292,8 @@ class SWE2D:
 
     def params_at(self, t: float, rain_rate, edges_t: list) -> None:
         """The records' values at t, which do not wait for the step's dt."""
+        if len(edges_t) < 4:
+            raise ValueError(f"expected the values of four edges, got {len(edges_t)}")
         self._fill_columns(1, [float(t), rain_rate, *edges_t])
 
     def params_until(self, dt: float, t: float):

@@ -38,3 +38,16 @@ def test_one_call_equals_the_separate_calls(dtype, n_sub):
     got = a._rates[a.two.B:].numpy().copy()
     rate, wet = b.one.member_rates()
     assert np.array_equal(got.reshape(-1, 2)[:, 0], rate) and np.array_equal(got.reshape(-1, 2)[:, 1] > 0, wet > 0)
+
+
+def test_too_few_edge_values_are_refused():
+    # records are laid out once and refilled: a short list must not leave old edge values in
+    from his_gb300 import workloads as W
+    from his_gb300.assembly import build_engine
+    two = build_engine(W.plain_small(), dtype=torch.float32).two
+    before = two.h.clone()
+    for edges in ([], [0.0, 0.0, 0.0]):
+        with pytest.raises(ValueError):
+            two.step(0.1, 0.0, 0.0, edges)
+    torch.cuda.synchronize()
+    assert torch.equal(two.h, before)
