@@ -509,15 +509,12 @@ struct StripPipe {
         } else {
             hn = hn + rdt;
         }
+        const R hp = hn;                   // depth the momentum belongs to
         if (feat & FEAT_HORTON) {
             const R rate_f = fmaf(cin.f0 - cin.fc, expf(-cin.k * tt), cin.fc);
             const R pot = __fmul_rn(rate_f, dt);
             const R take = rmin(pot, hn);
-            const R safe = hn > R(0) ? hn : R(1);
-            const R scale = hn > R(0) ? (hn - take) / safe : R(0);
             hn = hn - take;
-            hun = hun * scale;
-            hvn = hvn * scale;
             R taken = take;
             if (feat & FEAT_STORE) {
                 const R tks = rmin(pot - take, sf);
@@ -530,13 +527,14 @@ struct StripPipe {
         if (feat & FEAT_STORE) {
             const R room = clamp0(cin.S - sf);
             const R fill = rmin(room, hn);
-            const R safe = hn > R(0) ? hn : R(1);
-            const R scale = hn > R(0) ? (hn - fill) / safe : R(0);
             hn = hn - fill;
-            hun = hun * scale;
-            hvn = hvn * scale;
             sf = sf + fill;
             gd.sf[i] = sf;
+        }
+        if (feat & (FEAT_HORTON | FEAT_STORE)) {       // water lost takes its momentum along
+            const R keep = hp > R(0) ? hn / hp : R(0);
+            hun = hun * keep;
+            hvn = hvn * keep;
         }
         // ---- semi-implicit Manning friction (swe2d.py:362-370)
         // KP factor of the new depth, kept for the CFL velocity below
@@ -544,11 +542,10 @@ struct StripPipe {
         const R ks = hn >= c.h_dry ? 1.4142135623730951f * hn * rsqrtf(h4 + fmaxf(h4, c.kp_eps)) : 0.0f;
         R u = hun * ks, v = hvn * ks;
         const R speed = dsqrt(fmaf(u, u, __fmul_rn(v, v)));
-        const R hf = rmax(hn, c.h_dry);
         const R nm = cin.n;
-        const R denom = __fadd_rn(1.0f, dt * c.g * nm * nm * speed / powf(hf, 4.0f / 3.0f));
-        u = u / denom;
-        v = v / denom;
+        const R slow = 1.0f / __fadd_rn(1.0f, dt * c.g * nm * nm * speed * powf(hn, -4.0f / 3.0f));
+        u = u * slow;
+        v = v * slow;
         const bool wet = hn >= c.h_dry;
         hun = wet ? hn * u : R(0);
         hvn = wet ? hn * v : R(0);
