@@ -166,12 +166,22 @@ int launch_stages_parted(his_grid* g, cudaStream_t s) {
     return HIS_OK;
 }
 
+// finalize_kernel over n members of n_tiles tiles in all
+template <class R>
+void finalize_launch(const Grid<R>* grids, const StepParams* params, const Consts& c, const double* partials, double* out,
+                     int mode, double* ext, double* ledger, int n, int n_tiles, cudaStream_t s) {
+    if (mode != 2 && n_tiles / n >= FIN_SPLIT)
+        finalize_kernel<R, true><<<n * FIN_OUT, 32 * FIN_COLUMNS, 0, s>>>(grids, params, c, partials, out, mode, ext, ledger);
+    else
+        finalize_kernel<R, false><<<n, FIN_THREADS, 0, s>>>(grids, params, c, partials, out, mode, ext, ledger);
+}
+
 template <class R, int NT>
 int launch_step_nt(his_grid* g, cudaStream_t s, double* ledger) {
     int rc = launch_stages_parted<R, NT>(g, s);
     if (rc) return rc;
-    finalize_kernel<R><<<g->n, FIN_THREADS, 0, s>>>(reinterpret_cast<const Grid<R>*>(g->d_grids), g->d_params, g->c,
-                                           g->d_partials, g->d_out, 0, nullptr, ledger);
+    finalize_launch(reinterpret_cast<const Grid<R>*>(g->d_grids), g->d_params, g->c, g->d_partials, g->d_out, 0, nullptr,
+                    ledger, g->n, g->n_tiles, s);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
 }
@@ -184,8 +194,7 @@ int launch_reduce(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
         strip_rate_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
     else
         strip_reduce_kernel<R><<<g->n_tiles, CHUNK_THREADS, 0, s>>>(grids, strips, make_kc<R>(g->c), g->d_partials);
-    finalize_kernel<R><<<g->n, FIN_THREADS, 0, s>>>(grids, g->d_params, g->c, g->d_partials, g->d_out, rate_only ? 2 : 1,
-                                           ext);
+    finalize_launch(grids, g->d_params, g->c, g->d_partials, g->d_out, rate_only ? 2 : 1, ext, nullptr, g->n, g->n_tiles, s);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
 }
@@ -567,7 +576,7 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
         launch_stage<R, NT, 0>(grid, strips, params, kc, part, L.n_strips, smem, s);
         stage_copy_kernel<R><<<L.n_strips, CHUNK_THREADS, 0, s>>>(grid, strips, params);
     }
-    finalize_kernel<R><<<1, FIN_THREADS, 0, s>>>(grid, params, c, part, out, 0, nullptr);
+    finalize_launch<R>(grid, params, c, part, out, 0, nullptr, nullptr, 1, L.n_strips, s);
     HIS_CK(cudaGetLastError());
     return HIS_OK;
 }

@@ -894,7 +894,15 @@ __device__ __forceinline__ double step_term(int term, const Grid<R>& gd, double 
 // at StepParams::vols, modes 1 and 2 the rates at ext.  ledger (optional, mode 0): an 8 x n_members
 // float64 ledger (rows LG_*) the step's rain, infiltration, boundary and clip volumes
 // are added into.
-template <class R>
+//
+// SPLIT: a CTA of FIN_COLUMNS warps for each of a member's FIN_OUT outputs instead of one for all
+// (modes 0 and 1).  One SM takes an FP64 instruction per 19 cycles and a column's loads touch
+// a line per tile, so one CTA takes 18 us for the 16 columns of 1148 tiles, eight 12 (a
+// 1601 x 1301 float32 step with its CFL rate 186 -> 180 us).  From FIN_SPLIT tiles per member on:
+// with 42 for each of 64 members, 512 CTAs cost more than they save (a coupled step 480 us in
+// one CTA per member, 487 in eight).  Same order of summation, same bits.
+constexpr int FIN_OUT = 8, FIN_COLUMNS = 4, FIN_SPLIT = 512;
+template <class R, bool SPLIT>
 __global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const Grid<R>* __restrict__ grids,
                                                                const StepParams* __restrict__ params, Consts c,
                                                                const double* __restrict__ partials,
@@ -902,7 +910,8 @@ __global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const Grid<R>* __
                                                                double* __restrict__ ext = nullptr,
                                                                double* __restrict__ ledger = nullptr) {
     __shared__ double S[NPART];
-    const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m = SPLIT ? blockIdx.x / FIN_OUT : blockIdx.x, k = SPLIT ? blockIdx.x % FIN_OUT : warp;
     const Grid<R>& gd = grids[m];
     if (mode == 0 && !params[m].active) return;
     double* o = out + (size_t)m * 8;
@@ -921,23 +930,40 @@ __global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const Grid<R>* __
         }
         return;
     }
-    sum_partials(partials, gd.tile0, gd.n_tiles, S);
-    if (lane != 0) return;
-    if (warp == 5) {
+    if constexpr (SPLIT) {
+        // a warp per column that the CTA's output needs
+        constexpr int COLUMNS[FIN_OUT][FIN_COLUMNS] = {{P_XIN1, P_YIN1, P_XIN2, P_YIN2},
+                                                       {P_XOUT1, P_YOUT1, P_XOUT2, P_YOUT2},
+                                                       {P_RAINW, -1, -1, -1}, {P_INFIL, -1, -1, -1},
+                                                       {P_CLIP1, P_CLIP2, -1, -1}, {P_RATE, -1, -1, -1},
+                                                       {P_HSUM, -1, -1, -1}, {P_SSUM, -1, -1, -1}};
+        if (mode == 1 && k < 5) return;
+        const int j[1] = {COLUMNS[k][warp]};
+        if (j[0] >= 0) {
+            double s[1];
+            sum_columns<1>(partials, gd.tile0, gd.n_tiles, j, s);
+            if (lane == 0) S[j[0]] = s[0];
+        }
+        __syncthreads();
+        if (threadIdx.x != 0) return;
+    } else {
+        sum_partials(partials, gd.tile0, gd.n_tiles, S);
+        if (lane != 0) return;
+    }
+    if (k == 5) {
         o[5] = S[P_RATE];
         if (mode != 0 && ext) ext[m] = S[P_RATE];
-    } else if (warp == 6) {
+    } else if (k == 6) {
         o[6] = S[P_HSUM] * gd.area;
-    } else if (warp == 7) {
+    } else if (k == 7) {
         o[7] = S[P_SSUM] * gd.area;
     } else if (mode == 0) {
-        const double v = step_term(warp, gd, params[m].dt, params[m].rain, c.order, S);
-        o[warp] = v;
-        if (params[m].vols) params[m].vols[warp] = v;
+        const double v = step_term(k, gd, params[m].dt, params[m].rain, c.order, S);
+        o[k] = v;
+        if (params[m].vols) params[m].vols[k] = v;
         if (ledger) {
-            const int row = warp == 0 ? LG_BND2_IN : warp == 1 ? LG_BND2_OUT : warp == 2 ? LG_RAIN
-                          : warp == 3 ? LG_INFIL : LG_CLIP2;
-            ledger[row * (size_t)gridDim.x + m] += v;
+            const int row = k == 0 ? LG_BND2_IN : k == 1 ? LG_BND2_OUT : k == 2 ? LG_RAIN : k == 3 ? LG_INFIL : LG_CLIP2;
+            ledger[row * (size_t)(SPLIT ? gridDim.x / FIN_OUT : gridDim.x) + m] += v;
         }
     }
 }

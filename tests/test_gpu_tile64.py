@@ -119,3 +119,23 @@ def test_float64_contact_side_on_closed_thin_films(ny, nx, order):
         for name in ("h", "hu", "hv"):
             d = H.max_abs(getattr(s, name).cpu().numpy(), getattr(o, name)[0])
             assert d <= 1e-15, f"{name} differs from the oracle by {d}"
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("nx", [511, 512, 513])
+def test_totals_around_the_split_of_finalize(nx, dtype):
+    # members of 512 chunks and more are totalled by eight CTAs.  The totals of 1 x nx cells in
+    # one-cell and in 58-cell chunks differ by the order of at most 513 float64 adds, and in
+    # float32 by that of a chunk's 58 partial sums
+    from his_gb300.swe2d import SWE2D
+    f, bcs, cfg = _case(1, nx, 2, "hllc", 1e-3)
+    sims = [SWE2D(f["z"], f["n"], 9.0, cfg, bcs, storage=f["S"], rain_weight=f["rw"], dy=11.0, tile=t, dtype=dtype)
+            for t in ((1, 1), (58, 16))]
+    for s in sims:
+        s.set_state(f["h"], f["hu"], f["hv"])
+    assert sims[0].max_dt() == sims[1].max_dt()
+    dt = 0.5 * sims[1].max_dt()
+    a, b = (s.step(dt, 0.0, 2e-5) for s in sims)
+    assert torch.equal(sims[0].h, sims[1].h)
+    rel = 1e-12 if dtype == torch.float64 else 58 * 2.0 ** -24
+    assert torch.allclose(a.table, b.table, rtol=rel, atol=1e-12)
