@@ -43,7 +43,8 @@ __device__ __forceinline__ long long f64_key(double x) {
 }
 __device__ __forceinline__ double f64_max(double a, double b) { return f64_key(a) < f64_key(b) ? b : a; }
 __device__ __forceinline__ double f64_min(double a, double b) { return f64_key(b) < f64_key(a) ? b : a; }
-// Running maximum of values >= +0; a NaN candidate is passed over, as a > comparison does
+// Running maximum of values a >= +0 (bit patterns: a negative a would stay); a NaN candidate is
+// passed over, as a > comparison does
 __device__ __forceinline__ double f64_max_run(double a, double b) {
     const unsigned long long u = f64_bits(b);
     return u > f64_bits(a) && u <= F64_INF ? b : a;

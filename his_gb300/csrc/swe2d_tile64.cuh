@@ -276,8 +276,9 @@ __device__ __forceinline__ void update64(const KC<double>& c, const Grid<double>
     } else {
         gd.h1[j] = hn; gd.hu1[j] = hun; gd.hv1[j] = hvn;
     }
-    if (k.feat & FEAT_PEAK) gd.pk[j] = f64_max_run(gd.pk[j], hn);
-    if (k.feat & FEAT_PSPEED) gd.ps[j] = f64_max_run(gd.ps[j], sqrt(fma(u2, u2, v2 * v2)));
+    // (the caller's fields, of any start: not f64_max_run's)
+    if (k.feat & FEAT_PEAK) gd.pk[j] = rmax(gd.pk[j], hn);
+    if (k.feat & FEAT_PSPEED) gd.ps[j] = rmax(gd.ps[j], sqrt(fma(u2, u2, v2 * v2)));
     if (k.feat & FEAT_SNAP) {
         k.pr.snap_h[j] = (float)hn;
         k.pr.snap_u[j] = (float)u2;
