@@ -48,6 +48,7 @@ struct his_grid {
     size_t table_bytes = 0;
     size_t stage_smem = 0;                   // dynamic shared memory of a stage CTA
     int seg = 1;                             // segments a float32 strip-chunk is marched in
+    bool peaks = false;                      // some member has running peaks
     void *d_face_planes = nullptr, *d_faces = nullptr;   // float64: faces of every member, their table
     size_t cell_smem = 0;                    // and the cell kernel's shared memory
     HostStage params_stage;                  // his_grid_step_async parameters

@@ -21,6 +21,7 @@ struct StagePlan {
     const void* faces;
     size_t smem_cell;
     int seg;
+    bool peaks;                      // some member has running peaks
 };
 
 // Segments (1, 2 or 4) the rows of a float32 strip-chunk are marched in side by side: the
@@ -49,6 +50,22 @@ inline int strip_segments(int nt, int tiles, int rows) {
     return best;
 }
 
+template <class R, int NT, int STAGE, bool PEAKS>
+void launch_strips(const Grid<R>* grids, const StripRef* strips, const StepParams* params, const KC<R>& kc, double* part,
+                   int count, const StagePlan& plan, cudaStream_t s) {
+    if constexpr (NT == 64) {
+        if (plan.seg == 4) {
+            strip_kernel<R, NT, STAGE, 4, PEAKS><<<count, 4 * NT, plan.smem, s>>>(grids, strips, params, kc, part);
+            return;
+        }
+        if (plan.seg == 2) {
+            strip_kernel<R, NT, STAGE, 2, PEAKS><<<count, 2 * NT, plan.smem, s>>>(grids, strips, params, kc, part);
+            return;
+        }
+    }
+    strip_kernel<R, NT, STAGE, 1, PEAKS><<<count, NT, plan.smem, s>>>(grids, strips, params, kc, part);
+}
+
 // Launch of one stage over `count` strip-chunks: float32 marches strips with NT threads,
 // float64 works off sub-tiles, faces and cells in two kernels or fused.
 template <class R, int NT, int STAGE>
@@ -63,17 +80,8 @@ void launch_stage(const Grid<R>* grids, const StripRef* strips, const StepParams
             tile64_kernel<STAGE><<<count, TILE64_THREADS, plan.smem, s>>>(grids, strips, params, kc, part);
         }
     } else {
-        if constexpr (NT == 64) {
-            if (plan.seg == 4) {
-                strip_kernel<R, NT, STAGE, 4><<<count, 4 * NT, plan.smem, s>>>(grids, strips, params, kc, part);
-                return;
-            }
-            if (plan.seg == 2) {
-                strip_kernel<R, NT, STAGE, 2><<<count, 2 * NT, plan.smem, s>>>(grids, strips, params, kc, part);
-                return;
-            }
-        }
-        strip_kernel<R, NT, STAGE, 1><<<count, NT, plan.smem, s>>>(grids, strips, params, kc, part);
+        if (STAGE != 1 && plan.peaks) launch_strips<R, NT, STAGE, STAGE != 1>(grids, strips, params, kc, part, count, plan, s);
+        else launch_strips<R, NT, STAGE, false>(grids, strips, params, kc, part, count, plan, s);
     }
 }
 
@@ -91,17 +99,18 @@ size_t stage_smem(int w, int rows, int order, int seg) {
 }
 
 // Shared memory limits of one stage's strip kernels.
-template <class R, int NT, int STAGE>
+template <class R, int NT, int STAGE, bool PEAKS>
 int set_strip_attrs() {
     constexpr int MOST = 227 * 1024;
-    HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 1, PEAKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)StripGeom<R, NT>::smem_bytes));
     if constexpr (NT == 64) {
-        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 2, PEAKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     MOST - 1024));
-        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HIS_CK(cudaFuncSetAttribute(strip_kernel<R, NT, STAGE, 4, PEAKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     MOST - 1024));
     }
+    if constexpr (STAGE != 1 && !PEAKS) return set_strip_attrs<R, NT, STAGE, true>();
     return HIS_OK;
 }
 
@@ -118,13 +127,14 @@ int set_stage_attrs() {
         HIS_CK(cudaFuncSetAttribute(face64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, face));
     } else {
         int rc;
-        if ((rc = set_strip_attrs<R, NT, 0>()) || (rc = set_strip_attrs<R, NT, 1>()) || (rc = set_strip_attrs<R, NT, 2>()))
+        if ((rc = set_strip_attrs<R, NT, 0, false>()) || (rc = set_strip_attrs<R, NT, 1, false>()) ||
+            (rc = set_strip_attrs<R, NT, 2, false>()))
             return rc;
     }
     return HIS_OK;
 }
 
-inline StagePlan stage_plan(const his_grid* g) { return StagePlan{g->stage_smem, g->d_faces, g->cell_smem, g->seg}; }
+inline StagePlan stage_plan(const his_grid* g) { return StagePlan{g->stage_smem, g->d_faces, g->cell_smem, g->seg, g->peaks}; }
 
 // The 2-D stages of one step on stream s (no finalize), over tiles [t0, t0 + count)
 // (default: all); a tile's partials sit at its global index.
@@ -322,6 +332,7 @@ int grid_init_impl(his_grid* g) {
         G.z = (const R*)d.z; G.n = (const R*)d.manning; G.S = (const R*)d.storage;
         G.f0 = (const R*)d.f0; G.fc = (const R*)d.fc; G.k = (const R*)d.k; G.rw = (const R*)d.rain_weight;
         G.pk = (R*)d.peak_h; G.ps = (R*)d.peak_speed;
+        g->peaks = g->peaks || G.pk || G.ps;
     }
     g->n_tiles = (int)strips.size();
     if constexpr (sizeof(R) == 8) {
@@ -568,7 +579,7 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
     auto* out = reinterpret_cast<double*>(base + L.o_out);
     const KC<R> kc = make_kc<R>(c);
     const int seg = sizeof(R) == 8 ? 1 : strip_segments(NT, L.n_strips, L.hch);
-    const StagePlan smem{stage_smem<R, NT>(L.w, L.hch, c.order, seg), nullptr, 0, seg};
+    const StagePlan smem{stage_smem<R, NT>(L.w, L.hch, c.order, seg), nullptr, 0, seg, G.pk || G.ps};
     if (c.order == 2) {
         launch_stage<R, NT, 1>(grid, strips, params, kc, part, L.n_strips, smem, s);
         launch_stage<R, NT, 2>(grid, strips, params, kc, part, L.n_strips, smem, s);

@@ -50,9 +50,9 @@ struct StripGeom {
     static constexpr int P = NT + 2;               // padded row of entries
     static constexpr int NRED = 11;                // reduced values (the reduction reuses the cell ring)
     // cells [RING][P], x-recon plus side [P], x-faces [2][P], y-faces [RING][P]; then
-    // the plus-side surface slope [P] and theta [RING][P]
+    // the plus-side surface slope [P], theta [RING][P] and two old peaks [2][P]
     static constexpr size_t quads = (size_t)(RING + 1 + 2 + RING) * P;
-    static constexpr size_t scalars = (size_t)(1 + RING) * P;
+    static constexpr size_t scalars = (size_t)(1 + RING + 2) * P;
     static_assert((size_t)4 * RING * P >= (size_t)(NT / 32) * NRED, "reduction scratch must fit in the cell ring");
     static constexpr size_t smem_bytes = sizeof(Q4<R>) * quads + sizeof(R) * scalars;
     // resident CTAs per SM the kernels are register-capped for (a chunk marched in segments:
@@ -164,7 +164,8 @@ struct CellIn {
 // Optional fields of a member, tested once per CTA: the row loop reads a bit of a
 // register instead of re-reading a 64-bit pointer from the shared record and
 // comparing it with null.
-enum : unsigned { FEAT_STORE = 1u, FEAT_HORTON = 2u, FEAT_RAINW = 4u, FEAT_PEAK = 8u, FEAT_PSPEED = 16u, FEAT_SNAP = 32u };
+enum : unsigned { FEAT_STORE = 1u, FEAT_HORTON = 2u, FEAT_RAINW = 4u, FEAT_PEAK = 8u, FEAT_PSPEED = 16u, FEAT_SNAP = 32u,
+                  FEAT_PEAKS = FEAT_PEAK | FEAT_PSPEED };
 template <class R>
 __device__ __forceinline__ unsigned grid_features(const Grid<R>& gd) {
     return (gd.S ? FEAT_STORE : 0u) | (gd.f0 ? FEAT_HORTON : 0u) | (gd.rw ? FEAT_RAINW : 0u) |
@@ -237,13 +238,12 @@ __device__ __forceinline__ void block_reduce_store(T (&v)[NV], const bool* is_ma
     }
 }
 
-// *p = max(*p, v) of a running peak (v >= 0, or NaN, which leaves it) without waiting for the
-// old value: floats compare as their bits here.  A load and a store left the row waiting for
-// the load: 16 steps of six served storms with running peaks 906 -> 858 us, of 64 storms 5411
-// -> 5341.
-__device__ __forceinline__ void raise_peak(float* p, float v) {
-    atomicMax(reinterpret_cast<int*>(p), __float_as_int(fmaxf(v, 0.0f)));
+// A running peak's old value on its way to shared memory, and the wait for it
+__device__ __forceinline__ void peak_fetch(float* s, const float* p) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(p)
+                 : "memory");
 }
+__device__ __forceinline__ void peak_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // One side of a reconstructed cell as a face sees it: depth, normal and tangential
 // velocity, X = the in-cell bed slope d and S = the in-cell surface slope sE.  The cell's
@@ -286,7 +286,10 @@ __device__ __forceinline__ Q4<float> side_flux(const KC<float>& c, const Side& L
 // each with its own rings and barrier; the rows' contributions to the partial sums are kept
 // per row and thread and added up in row order at the end, so that the sums are those of one
 // march over all rows, bit for bit.
-template <class R, int NT, int STAGE, int SEG>
+//
+// PEAKS: some member of the set has running peaks (a kernel without their code takes 5251 us for
+// 16 steps of 64 storms of 400 x 325 cells, one that tests for them in every row 5285).
+template <class R, int NT, int STAGE, int SEG, bool PEAKS>
 struct StripPipe {
     static_assert(sizeof(R) == 4, "the float64 step is tile64_kernel's");
     using G = StripGeom<R, NT>;
@@ -314,6 +317,7 @@ struct StripPipe {
     Side ylow;                      // plus side of the y-reconstruction of row r-2
     R by1, by2, bx1;                   // bed terms: y of rows r-2, r-3; x of row r-3
     CellIn<R> cin;
+    R old_pk, old_ps;                  // PEAKS: row r-3's running peaks
     R acc_clip, xin, xout, yin, yout, infil, rainw, rate, hsum, ssum, hmax;
     R* sums;                           // SEG > 1: this thread's entry of the chunk's first row
     int bar;                           // and its segment's barrier
@@ -343,6 +347,28 @@ struct StripPipe {
         }
     }
 
+    // The running peaks of cell i before this step, fetched with the row's other inputs: into
+    // registers where segments, few warps to an SM, have some to spare, else into shared memory
+    // (16 steps of 64 storms with both peaks 5470 us; loaded by the update 6450; an integer
+    // maximum in L2, which keeps a NaN for good, 5340.  Six served storms: 850
+    // and 850 us by either).
+    __device__ __forceinline__ void peaks_fetch(unsigned i) {
+        if (SEG > 1) {
+            if (feat & FEAT_PEAK) old_pk = gd.pk[i];
+            if (feat & FEAT_PSPEED) old_ps = gd.ps[i];
+        } else {
+            R* s = s_th + G::RING * P + ts;
+            if (feat & FEAT_PEAK) peak_fetch(s, gd.pk + i);
+            if (feat & FEAT_PSPEED) peak_fetch(s + P, gd.ps + i);
+        }
+    }
+    // Raised, from any start (fmaxf: NaN on either side gives way)
+    __device__ __forceinline__ void peaks_raise(unsigned i, R h, R speed) {
+        const R* s = s_th + G::RING * P + ts;
+        if (SEG == 1) peak_wait();
+        if (feat & FEAT_PEAK) gd.pk[i] = fmaxf(SEG > 1 ? old_pk : s[0], h);
+        if (feat & FEAT_PSPEED) gd.ps[i] = fmaxf(SEG > 1 ? old_ps : s[P], speed);
+    }
     // Raw values of an interior row at this thread's source column (its own column, or
     // the layer an x-ghost copies)
     __device__ __forceinline__ HaloRaw<R> fetch_in(int gy) const {
@@ -381,7 +407,11 @@ struct StripPipe {
         }
         s_cell[k0 + ts] = c0;
         ra = FULL ? fetch_in(r + 1) : halo_fetch(c, gd, H, HU, HV, cx, r + 1);
-        if (upd) cin = cell_fetch<R, STAGE>(gd, (unsigned)orow * (unsigned)nx + (unsigned)cxc, feat);
+        if (upd) {
+            const unsigned i = (unsigned)orow * (unsigned)nx + (unsigned)cxc;
+            cin = cell_fetch<R, STAGE>(gd, i, feat);
+            if (PEAKS && (feat & FEAT_PEAKS)) peaks_fetch(i);
+        }
         R by0 = R(0), bx0 = R(0);
         const Q4<R> c2 = s_cell[k2 + ts];           // own cells of rows r-2 and r-1
         const Q4<R> c1 = s_cell[k1 + ts];
@@ -554,12 +584,11 @@ struct StripPipe {
         } else {
             gd.h1[i] = hn; gd.hu1[i] = hun; gd.hv1[i] = hvn;
         }
-        if (feat & FEAT_PEAK) raise_peak(gd.pk + i, hn);
         // ---- CFL rate of the new state for the next step (swe2d.py:179-184)
         const R u2 = hun * ks, v2 = hvn * ks;
         // running peak speed and output use the KP velocities of the new state, as the
         // reference's snapshots do (swe2d.py:161-167, coupling.py:229-242)
-        if (feat & FEAT_PSPEED) raise_peak(gd.ps + i, dsqrt(fmaf(u2, u2, __fmul_rn(v2, v2))));
+        if (PEAKS && (feat & FEAT_PEAKS)) peaks_raise(i, hn, dsqrt(fmaf(u2, u2, __fmul_rn(v2, v2))));
         if (feat & FEAT_SNAP) {
             s_snap[0][i] = (float)hn;
             s_snap[1][i] = (float)u2;
@@ -599,7 +628,7 @@ __device__ __forceinline__ int ghost_source_column(const KC<R>& c, const Grid<R>
 // With few chunks a march is bound by its latency: 1.6 us a row, rows + 6 of them, two warps
 // on an SM.  SEG = 2 and 4 march parts of the chunk side by side (strip_segments): one served
 // storm of 400 x 325 cells in 58 x 16 took 71.5 us a step in one march, 59.7 in four.
-template <class R, int NT, int STAGE, int SEG>
+template <class R, int NT, int STAGE, int SEG, bool PEAKS>
 __global__ void __launch_bounds__(NT * SEG, StripGeom<R, NT>::min_ctas(STAGE, SEG)) strip_kernel(const Grid<R>* __restrict__ grids,
                                                     const StripRef* __restrict__ strips,
                                                     const StepParams* __restrict__ params, const KC<R> kc,
@@ -641,7 +670,7 @@ __global__ void __launch_bounds__(NT * SEG, StripGeom<R, NT>::min_ctas(STAGE, SE
     Q4<R>* s_yf = s_xf + 2 * P;
     R* s_rs = reinterpret_cast<R*>(s_yf + G::RING * P);
     R* s_th = s_rs + P;
-    StripPipe<R, NT, STAGE, SEG> pp{s_cell, s_rp, s_xf, s_yf, s_rs, s_th, gd, c, bcv, s_snap,
+    StripPipe<R, NT, STAGE, SEG, PEAKS> pp{s_cell, s_rp, s_xf, s_yf, s_rs, s_th, gd, c, bcv, s_snap,
                                STAGE == 2 ? gd.h1 : gd.h, STAGE == 2 ? gd.hu1 : gd.hu, STAGE == 2 ? gd.hv1 : gd.hv};
     const int nx = gd.nx, ny = gd.ny;
     const int x0 = sr.x0, W = sr.w, rows = (sr.y1 - sr.y0 + SEG - 1) / SEG;
@@ -663,6 +692,7 @@ __global__ void __launch_bounds__(NT * SEG, StripGeom<R, NT>::min_ctas(STAGE, SE
     pp.bar = seg + 1;
     pp.col_in = (unsigned)cx < (unsigned)nx;
     pp.do_out = q >= 0 && q < W && pp.col_in;
+    if (!pp.do_out) pp.feat &= ~FEAT_PEAKS;           // a halo column's peaks are another strip's
     pp.west = cx == 0;
     pp.east = cx == nx - 1;
     pp.scol = ghost_source_column(c, gd, cx);
@@ -677,6 +707,7 @@ __global__ void __launch_bounds__(NT * SEG, StripGeom<R, NT>::min_ctas(STAGE, SE
     pp.acc_clip = pp.xin = pp.xout = pp.yin = pp.yout = pp.infil = pp.rainw = pp.rate = pp.hsum = pp.ssum = R(0);
     pp.hmax = R(0);
     pp.by1 = pp.by2 = pp.bx1 = R(0);
+    pp.old_pk = pp.old_ps = R(0);
     // software pipeline: raw rows are fetched one row ahead
     if (SEG == 1 || y0 < y1) pp.ra = halo_fetch(c, gd, pp.H, pp.HU, pp.HV, cx, y0 - 3);
     static_assert((G::RING & (G::RING - 1)) == 0, "ring slots are row & (RING - 1)");
