@@ -243,8 +243,11 @@ __device__ __forceinline__ void update64(const KC<double>& c, const Grid<double>
         double u, v;
         if (plain) {
             const double rp = f64_bits(hp) == f64_bits(hn) ? r : __drcp_rn(hp);
-            u = f64_div(hun, hp, rp);
-            v = f64_div(hvn, hp, rp);
+            u = v = 0.0;
+            if (f64_pos(hp)) {             // (infiltration below zero wets dry cells)
+                u = f64_div(hun, hp, rp);
+                v = f64_div(hvn, hp, rp);
+            }
         } else {
             const double keep = f64_pos(hp) ? hn / hp : 0.0;
             kp_velocity(c, hn, hun * keep, hvn * keep, u, v);
