@@ -162,9 +162,11 @@ eng_pre_kernel(EngMember* __restrict__ em, StepParams* __restrict__ params, cons
         auto ready = [&] { wide(); return s_dtr; };
         auto go = [&] { all(); return s_nsub <= max_sub; };
         if (links) {
-            const int2 cs = exch_slice<G>(s_L, s_N.n_cells, rank);
+            constexpr int NS = EXCH_SLICES / G;      // slices of this CTA
+            static_assert(NS * G == EXCH_SLICES && ENG_EXCH_WARPS >= NS, "whole slices, a warp to each");
             exchange_dev<R, 1>(s_L, s_N, grids[m], K, nullptr, Vg + s_L.v_offset,
-                            exch + (size_t)(m * EXCH_SLICES + rank) * 2, cs.x, cs.y, sm, tid, ENG_EXCH_THREADS, true,
+                            exch + (size_t)(m * EXCH_SLICES + rank * NS) * 2, rank * NS, NS, sm, tid,
+                            ENG_EXCH_THREADS, true,
                             [] { bar_group(2, ENG_EXCH_THREADS); }, wide, ready, go, put_rate);
         } else {
             R rate = R(-1);

@@ -599,7 +599,7 @@ __device__ __forceinline__ void net_substeps_f32_dev(const Net& N, const Consts&
 // Shared memory of the exchange of one slice: volumes per link, level (then limit) and
 // storage per 1-D cell.
 __host__ __device__ inline size_t exchange_smem_bytes(int n_links, int n_cells, size_t size) {
-    return sizeof(double) * 64 + size * ((size_t)n_links + 2 * (size_t)n_cells);
+    return size * ((size_t)n_links + 2 * (size_t)n_cells);
 }
 
 // Barrier `id` among n threads (whole warps) of a CTA
@@ -709,18 +709,20 @@ __device__ __forceinline__ void stage_record(T* dst, const T* src) {
 // ready(): barrier with whoever chooses dt; returns it.  go(): barrier before the states are
 // changed; false leaves them as they are.  Vg: volumes by position in global memory.
 // put_rate (optional): takes each warp's largest rate of a wet cell, -1 where none is wet.
-// SLOTS: links per thread fetched ahead (each costs registers).
+// SLOTS: links per thread fetched ahead (each costs registers).  s0, ns: the first of this CTA's
+// slices and their number; tally: 2 values of its first slice.
 template <class R, int SLOTS, class Sync, class Wide, class Ready, class Go, class Rate>
 __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const Grid<R>& gd, const ExchK<R>& K,
                                              double* __restrict__ Vout, double* Vg, double* __restrict__ tally,
-                                             int c0, int c1, double* sm, int tid, int nt, bool rates, Sync sync,
+                                             int s0, int ns, double* sm, int tid, int nt, bool rates, Sync sync,
                                              Wide wide, Ready ready, Go go, Rate put_rate) {
     constexpr int S = SLOTS;
     constexpr bool F32 = sizeof(R) == 4;
-    const int l0 = L.cstart[c0], nl = L.cstart[c1] - l0, nc = c1 - c0;
+    const bool whole = ns == EXCH_SLICES;               // (a constant: this CTA has the whole member)
+    const int c0 = whole ? 0 : L.slice[s0], l0 = whole ? 0 : L.cstart[c0];
+    const int nc = whole ? N.n_cells : L.slice[s0 + ns] - c0, nl = whole ? L.n_links : L.cstart[c0 + nc] - l0;
     const R area = R(gd.area);
-    double* red = sm;                                   // 64 doubles
-    R* V = reinterpret_cast<R*>(sm + 64);
+    R* V = reinterpret_cast<R*>(sm);
     R *eta1 = V + nl, *rp = eta1 + nc, *f1 = eta1;
     auto zbank = [&](int l) -> R { if constexpr (F32) return L.zbank_f[l]; else return L.zbank[l]; };
     auto length = [&](int l) -> R { if constexpr (F32) return L.length_f[l]; else return L.length[l]; };
@@ -795,7 +797,6 @@ __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const G
         return tot > avail ? v * (avail / (tot > R(0) ? tot : R(1))) : v;
     };
     sync();
-    R ex0 = R(0), ex1 = R(0);
     auto settle = [&](int k, int c, R h, int p) {
         R v = V[k];
         v = v > R(0) ? limit2(v, h, p) : v * f1[c];
@@ -805,8 +806,6 @@ __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const G
         V[k] = v;
         if (p >= 0) Vg[l0 + k] = (double)v;
         if (Vout) Vout[L.v_offset + L.orig[l0 + k]] = (double)v;
-        ex0 += pos_part(v);
-        ex1 += pos_part(-v);
     };
     R vs[S];
 #pragma unroll
@@ -858,31 +857,34 @@ __device__ __forceinline__ void exchange_dev(const Lnk& L, const Net& N, const G
             else N.A[c] = N.A[c] + f64_div(d, N.dx[c], N.rdx[c]);
         }
     }
-    if (!tally) return;
-    // tallies in float64: lanes, then warps in order
-    const double e0 = warp_sum_sparse((double)ex0), e1 = warp_sum_sparse((double)ex1);
-    if ((tid & 31) == 0) {
-        red[2 * (tid >> 5)] = e0;
-        red[2 * (tid >> 5) + 1] = e1;
-    }
-    sync();
-    if (tid < 2) {
-        double a = red[tid];
-        for (int w = 1; w < nt / 32; ++w) {
-            const double b = red[2 * w + tid];
-            if (f64_bits(b) << 1 != 0) a += b;
+    // Tallies, a warp to a slice: lane l takes the slice's links l, l + 32, ..., four at a time in R,
+    // then in float64, and the lanes by a shuffle tree, so that a member's totals do not depend
+    // on how many CTAs share it.
+    const int w = tid >> 5, lane = tid & 31;
+    if (w >= ns) return;
+    const int a = L.cstart[L.slice[s0 + w]] - l0, b = L.cstart[L.slice[s0 + w + 1]] - l0;
+    double e0 = 0.0, e1 = 0.0;
+    for (int k = a; k < b; k += 128) {
+        R x0 = R(0), x1 = R(0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int q = k + 32 * j + lane;
+            const R v = q < b ? V[q] : R(0);
+            // (float64: a sum that gets nothing costs a vote)
+            if (F32 || __any_sync(0xffffffffu, pos_part(v) != R(0))) x0 += pos_part(v);
+            if (F32 || __any_sync(0xffffffffu, pos_part(-v) != R(0))) x1 += pos_part(-v);
         }
-        if (f64_bits(a) << 1 != 0) tally[tid] += a;
+        if (__any_sync(0xffffffffu, x0 != R(0))) e0 += (double)x0;
+        if (__any_sync(0xffffffffu, x1 != R(0))) e1 += (double)x1;
+    }
+    e0 = warp_sum_sparse(e0);
+    e1 = warp_sum_sparse(e1);
+    if (lane == 0) {
+        if (f64_bits(e0) << 1 != 0) tally[2 * w] += e0;
+        if (f64_bits(e1) << 1 != 0) tally[2 * w + 1] += e1;
     }
 }
 
-// Slice of the cells of CTA `rank` of G
-template <int G>
-__device__ __forceinline__ int2 exch_slice(const Lnk& L, int n_cells, int rank) {
-    static_assert(EXCH_SLICES % G == 0, "whole slices per CTA");
-    if constexpr (G == 1) return int2{0, n_cells};
-    else return int2{L.slice[rank * (EXCH_SLICES / G)], L.slice[(rank + 1) * (EXCH_SLICES / G)]};
-}
 // Barrier of every thread of a member's CTAs
 template <int G>
 __device__ __forceinline__ void member_sync(int threads) {
@@ -904,14 +906,16 @@ exchange_kernel(const Lnk* __restrict__ links, const Net* __restrict__ nets, con
     extern __shared__ double sm[];
     __shared__ Lnk L;
     __shared__ Net N;
-    const int mb = blockIdx.x / G, slice = blockIdx.x % G;
+    const int mb = blockIdx.x / G, rank = blockIdx.x % G;
     stage_record(&L, links + mb);
     stage_record(&N, nets + mb);
     __syncthreads();
-    const int2 cs = exch_slice<G>(L, N.n_cells, slice);
+    constexpr int NS = EXCH_SLICES / G;             // slices of this CTA
+    static_assert(NS * G == EXCH_SLICES && EXCHANGE_THREADS / 32 >= NS, "whole slices, a warp to each");
     auto sync = [] { __syncthreads(); };
-    exchange_dev<R, G == 1 ? 3 : 1>(L, N, grids[mb], K, Vout, Vg + L.v_offset, exch + (size_t)(mb * EXCH_SLICES + slice) * 2, cs.x, cs.y, sm,
-                    threadIdx.x, EXCHANGE_THREADS, false, sync, [] { member_sync<G>(EXCHANGE_THREADS); },
+    exchange_dev<R, G == 1 ? 3 : 1>(L, N, grids[mb], K, Vout, Vg + L.v_offset,
+                    exch + (size_t)(mb * EXCH_SLICES + rank * NS) * 2, rank * NS, NS, sm, threadIdx.x,
+                    EXCHANGE_THREADS, false, sync, [] { member_sync<G>(EXCHANGE_THREADS); },
                     [&] { __syncthreads(); return dt; }, [] { __syncthreads(); return true; }, [](R) {});
 }
 
