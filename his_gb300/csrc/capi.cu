@@ -962,6 +962,7 @@ int32_t his_coupled_step_async(his_grid* g, his_net* N, double dt, int32_t n_sub
                                const double* forcing, double* ledger, double* rate_wet, void* stream, void* side) {
     if (!g || !N || !params || !forcing || !ledger || !rate_wet)
         return bad("grid, network, params, forcing, ledger and rate_wet are required");
+    if (g->n != N->n) return bad("grid and network must have the same number of members");
     cudaStream_t s = (cudaStream_t)stream;
     bool direct = false;
     int rc = check_substeps(N, dt, n_sub);

@@ -260,6 +260,7 @@ int32_t his_links_exchanged(his_links* links, double* totals, int32_t reset, voi
  * the 2-D step of his_grid_step_ledger_async (params: its records) and beside it the n_sub
  * substeps of his_net_step_ledger_async and the CFL rates of the 1-D state they leave
  * (his_net_max_rate_async into rate_wet, 2 per member: device or mapped page-locked memory).
+ * Grid set and network set have the same members (else HIS_ERR_BAD_ARG, nothing is queued).
  * `side` is a second stream for the 1-D part where the kernels are not launched as a graph
  * (a first call, a caller that captures `stream`); `stream` waits for it.
  * Replaces the body of hydrointel/solver/coupling.py:212-227 (CoupledEngine.step). */
