@@ -442,16 +442,14 @@ int32_t his_grid_step_async(his_grid* g, const his_step_params* params, double* 
     return HIS_OK;
 }
 
-// The caller's ledger must be device memory (the step kernels add into it); *checked: the last
-// one found to be.
-static int ledger_device(double** checked, double* ledger) {
-    if (ledger == *checked) return HIS_OK;
+// The caller's ledger must be device memory (the step kernels add into it).  Asked on every call:
+// memory at an address that was good before may have been freed since.
+static int ledger_device(const double* ledger) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, ledger) != cudaSuccess || a.type != cudaMemoryTypeDevice) {
         cudaGetLastError();
         return bad("ledger must be device memory");
     }
-    *checked = ledger;
     return HIS_OK;
 }
 
@@ -461,7 +459,7 @@ static int ledger_launches(his_grid* g, cudaStream_t s) {
 
 int32_t his_grid_step_ledger_async(his_grid* g, const his_step_params* params, double* ledger, void* stream) {
     if (!g || !params || !ledger) return bad("grid, params and ledger are required");
-    int rc = ledger_device(&g->ledger_checked, ledger);
+    int rc = ledger_device(ledger);
     if (rc) return rc;
     if (!g->n_parts && (rc = grid_parts_setup(g))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
@@ -731,7 +729,7 @@ int32_t his_net_step_ledger_async(his_net* N, double dt, int32_t n_sub, const do
                                   void* stream) {
     if (!N || !forcing || !ledger) return bad("network, forcing and ledger are required");
     int rc = check_substeps(N, dt, n_sub);
-    if (rc || (rc = ledger_device(&N->ledger_checked, ledger))) return rc;
+    if (rc || (rc = ledger_device(ledger))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if ((rc = upload_forcing(N, dt, n_sub, forcing, s))) return rc;
     return net_step_launch(N, s, nullptr, ledger);
@@ -966,7 +964,7 @@ int32_t his_coupled_step_async(his_grid* g, his_net* N, double dt, int32_t n_sub
     cudaStream_t s = (cudaStream_t)stream;
     bool direct = false;
     int rc = check_substeps(N, dt, n_sub);
-    if (rc || (rc = ledger_device(&g->ledger_checked, ledger))) return rc;
+    if (rc || (rc = ledger_device(ledger))) return rc;
     if ((rc = check_async_out(rate_wet, "rate_wet", &direct))) return rc;
     if (!direct) return bad("rate_wet must be memory the device can write");
     if (!g->n_parts && (rc = grid_parts_setup(g))) return rc;

@@ -63,7 +63,6 @@ struct his_grid {
     cudaEvent_t pev_fork = nullptr, pev_join[MAX_PARTS - 1] = {};
     // the graphs' capture streams: all launches, and beside them a coupled step's 1-D side
     cudaStream_t cap_stream = nullptr, cap_side = nullptr;
-    double* ledger_checked = nullptr;       // the last ledger found to be device memory
     // his_grid_step_ledger_async: the step's kernels for the ledger they add into
     LaunchGraph ledger_graph;
     double* ledger_for = nullptr;
@@ -90,7 +89,6 @@ struct his_net {
     size_t smem_f32 = 0;                     // the float32 substeps (staged geometry)
     HostStage forcing_stage;                 // his_net_step_async forcing
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;    // his_coupled_step_async
-    double* ledger_checked = nullptr;        // the last ledger found to be device memory
 };
 
 struct his_links {
