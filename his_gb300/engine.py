@@ -82,6 +82,13 @@ def output_count(t_end: float, interval: float) -> int:
     return int(math.floor(t_end / interval + 1e-9)) + 1
 
 
+def face_bytes(ny: int, nx: int) -> int:
+    """Face planes of a float64 member's grid: 32 bytes per face and 16 per cell, each of
+    the three on a 256-byte boundary; a grid set takes at most 4 GB of them (else none)."""
+    total = 32 * ny * (nx + 1) + 32 * (ny + 1) * nx + 16 * ny * nx + 3 * 256
+    return total if total <= 4 << 30 else 0
+
+
 def _level_1d(topo_z, sec, A):
     """Channel level z + depth(A) of the trapezoid-plus-slot sections (swe1d.py:51-84)."""
     A = np.maximum(A, 0.0)
@@ -180,7 +187,7 @@ class Member:
         if self.n_out:
             ts += [self.snap_h, self.snap_u, self.snap_v, self.snap_t, self.snap_eta, self.snap_q, self.snap_ledger]
         held = sum(t.numel() * t.element_size() for t in ts if t is not None)
-        faces = 80 * self.h.numel() if self.dtype == torch.float64 else 0
+        faces = face_bytes(*self.shape) if self.dtype == torch.float64 else 0
         return held + 3 * self.h.numel() * self.h.element_size() + faces + 64 * 1024
 
     # ---------------------------------------------------------------- descriptors

@@ -29,7 +29,7 @@ import numpy as np
 import torch
 
 from .config import SolverConfig
-from .engine import FloodEngine, FloodResult, Member, MemberResult, output_count
+from .engine import FloodEngine, FloodResult, Member, MemberResult, face_bytes, output_count
 from .records import write_records
 from .swe2d import cuda_device
 from .workloads import Storm, served_requests, uneven_member
@@ -38,11 +38,13 @@ from .workloads import Storm, served_requests, uneven_member
 def estimate_bytes(storm: Storm, dtype: torch.dtype, track_peaks: bool = True,
                    output_interval: float | None = None) -> int:
     """Device bytes a storm needs as a member: 5 state planes, up to 6 field planes,
-    3 stage planes, 2 peak planes, its channel network and tables, and with outputs
-    three float32 planes and two channel rows per output time."""
+    3 stage planes, 2 peak planes, in float64 the grid set's face planes, its channel
+    network and tables, and with outputs three float32 planes and two channel rows per
+    output time."""
     planes = 5 + 2 + 3 + (3 if storm.horton is not None else 0) + (1 if storm.storage is not None else 0) + \
         (2 if track_peaks else 0)
     elem = torch.tensor([], dtype=dtype).element_size()
+    faces = face_bytes(storm.terrain.ny, storm.terrain.nx) if dtype == torch.float64 else 0
     net = cells1d = 0
     if storm.network is not None:
         cells1d = sum(r.n for r in storm.network.reaches) + 8 * len(storm.network.reaches)
@@ -51,7 +53,7 @@ def estimate_bytes(storm: Storm, dtype: torch.dtype, track_peaks: bool = True,
     if output_interval is not None:
         n_out = output_count(float(storm.t_end), float(output_interval))
         out = n_out * (3 * 4 * storm.cells + 2 * 4 * cells1d + 8)
-    return planes * storm.cells * elem + net + out + 64 * 1024
+    return planes * storm.cells * elem + faces + net + out + 64 * 1024
 
 
 @dataclass

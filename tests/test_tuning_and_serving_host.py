@@ -44,6 +44,16 @@ def test_footprint_estimate_covers_the_state():
     assert estimate_bytes(s, torch.float32, track_peaks=False) < b32
 
 
+def test_float64_footprint_covers_the_face_planes():
+    # a float64 grid set keeps 32 bytes per face and 16 per cell beside its 16 planes
+    s = W.uneven_member("fp/1", 2, 3600.0)
+    ny, nx = s.terrain.ny, s.terrain.nx
+    faces = ny * (nx + 1) + (ny + 1) * nx
+    assert estimate_bytes(s, torch.float64) >= (16 * 8 + 16) * s.cells + 32 * faces
+    without = estimate_bytes(s, torch.float64, track_peaks=False)
+    assert without >= (14 * 8 + 16) * s.cells + 32 * faces
+
+
 def test_request_stream_is_seeded():
     a = W.served_requests(2.0, 30.0, key="srv-test")
     b = W.served_requests(2.0, 30.0, key="srv-test")
