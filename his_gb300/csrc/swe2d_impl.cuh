@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "engine_kernels.cuh"
+#include "face_rule.h"
 #include "his_internal.h"
 #include "net1d_kernels.cuh"
 #include "swe2d_strip.cuh"
@@ -221,12 +222,8 @@ int launch_reduce(his_grid* g, cudaStream_t s, double* ext, bool rate_only) {
         return HIS_ERR_BAD_ARG;                                  \
     } while (0)
 
-// Face planes and bed terms of a float64 set's members and their table.  A set whose faces
-// would take more than FACES_MOST, or more than the device can give, does without (the
-// fused kernel), and so does one of fewer than FACES_LEAST cells, for which two launches more
-// cost what the faces saved would (100 x 81: 120 us per call with its CFL rate fused, 131
-// split; 163 x 201 even; 400 x 325 331 against 309).
-constexpr size_t FACES_MOST = (size_t)4 << 30, FACES_LEAST = 40000;
+// Face planes and bed terms of a float64 set's members and their table, where the set takes them
+// (faces_taken) and the device can give them; else the fused kernel runs.
 inline int faces_alloc(his_grid* g) {
     size_t total = 0, cells = 0;
     std::vector<size_t> off(g->n);
@@ -237,7 +234,9 @@ inline int faces_alloc(his_grid* g) {
         total += up(32 * ny * (nx + 1)) + up(32 * (ny + 1) * nx) + up(16 * ny * nx);
         cells += ny * nx;
     }
-    if (total > FACES_MOST || cells < FACES_LEAST) return HIS_OK;
+    size_t free_bytes = 0, all_bytes = 0;
+    HIS_CK(cudaMemGetInfo(&free_bytes, &all_bytes));
+    if (!faces_taken(total, cells, free_bytes)) return HIS_OK;
     if (cudaMalloc(&g->d_face_planes, total) != cudaSuccess) {
         cudaGetLastError();
         g->d_face_planes = nullptr;
