@@ -97,7 +97,8 @@ class FloodServer:
                  graph_steps: int = 16, tile=(58, 16), track_peaks: bool = True, keep_state: bool = False,
                  output_interval: float | None = None, record_dir=None, store_factor: int = 1):
         """hbm_budget: device bytes the members may hold (default: 80 % of the free memory
-        at start).  tile: the one work decomposition every batch uses; short 16-row
+        at start).  tile: the one work decomposition every batch uses ((0, 0): 58 x 48, as
+        the library's own choice follows the batch and a request's totals with it); short 16-row
         chunks by default, because a served batch is small and each step is bound by
         the latency of one CTA's march up its chunk (at 2 requests/s: p50 latency 0.86
         s against 1.66 s with 48-row chunks).  keep_state:
@@ -116,7 +117,7 @@ class FloodServer:
         self.max_members = int(max_members)
         self.chunk_steps = int(chunk_steps)
         self.graph_steps = int(graph_steps)
-        self.tile = tuple(tile)
+        self.tile = tuple(tile) if tuple(tile) != (0, 0) else (58, 48)
         self.track_peaks = track_peaks
         self.keep_state = keep_state
         self.output_interval = output_interval
