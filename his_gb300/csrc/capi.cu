@@ -108,6 +108,11 @@ bool tile_supported(int tx, int ty) { return tx >= 1 && strip_threads(tx) > 0 &&
 //    SM holds few CTAs and 0.4 + 0.28 us x CTAs per SM beyond.  Picks 58 x 2 for 100 x 81
 //    (31 us against 95), 58 x 4 for 400 x 325 (43 against 106), 58 x 8 for 4 members (58
 //    against 107), 58 x 24 to 64 for 16 to 64.
+// It follows the whole set, and a member's totals follow it in their last digits (states and
+// rates do not).  One by the member's own grid alone would keep those, at, us a step: float32
+// 400 x 325, 58 x 4 for any number, 32 members 306 against 196, 64 members 589 against 330
+// (58 x 48 for any: one 48 against 35, eight 101 against 82); float64 100 x 81, 10 x 6, 4
+// members 127 against 84, 24 members 490 against 281.
 void default_tile(int prec, int order, int n, const his_grid_desc* grids, int* tx, int* ty) {
     constexpr double SMS = 152.0;
     const int w64[] = {58, 50, 41, 34, 29, 25, 20, 17, 13, 10, 8}, w32[] = {58};

@@ -20,7 +20,8 @@ enum : int { BC_CLOSED = 0, BC_TRANSMISSIVE = 1, BC_STAGE = 2, BC_DISCHARGE = 3 
 enum : int { EDGE_W = 0, EDGE_E = 1, EDGE_S = 2, EDGE_N = 3 };
 
 // Per-tile partial sums written by the stage kernels (one slot per tile, summed in
-// tile order by the finalize kernel: deterministic and independent of the batch).
+// tile order by the finalize kernel: deterministic, and for a given decomposition
+// independent of the batch).
 enum : int {
     P_CLIP1 = 0, P_XIN1, P_XOUT1, P_YIN1, P_YOUT1,
     P_CLIP2, P_XIN2, P_XOUT2, P_YIN2, P_YOUT2,

@@ -19,7 +19,8 @@
 // reconstruction and theta is computed once.  Per-thread partial sums (clip,
 // boundary flux, infiltration, rain, rate, volumes) are reduced once per strip-chunk
 // into one float64 slot set, summed in a fixed order per member by the finalize
-// kernel, so results do not depend on the batch a member runs in.
+// kernel: states and rates do not depend on the batch a member runs in, its totals only
+// through the decomposition, where that is left to the library (default_tile).
 #pragma once
 #include "his_device.cuh"
 

@@ -81,6 +81,9 @@ const char* his_last_error(void);
 /* Create a set of n_members 2-D grids computed in `precision`.  The stencil kernels
  * work on strips of at most tile_x columns (1..346) in chunks of at most tile_y rows
  * (0, 0 = chosen by the grids' sizes, their number and the precision); the set allocates its own stage scratch.
+ * States and CFL rates do not depend on the tile.  A member's step volumes do in their last digits (they are
+ * summed chunk by chunk, in `precision` within one): for volumes whose bits do not depend on the other members of
+ * the set, give the tile.
  * Replaces hydrointel/solver/swe2d.py:113-146 (SWE2D constructor, batched form). */
 int32_t his_grid_create(int32_t precision, const his_solver_cfg* cfg, int32_t n_members, const his_grid_desc* grids,
                         int32_t tile_x, int32_t tile_y, his_grid** out);
