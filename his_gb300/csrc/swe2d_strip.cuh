@@ -507,8 +507,11 @@ struct StripPipe {
         dhu = fmaf(Ts - Tn, idy, dhu);
         dhv = fmaf(Tw - Te, idx, dhv);
         if (!do_out) return;
-        if (west) { xin += relu(Fw); xout += relu(-Fw); }
-        if (east) { xin += relu(-Fe); xout += relu(Fe); }
+        // (one column is west and east: its two terms are added first, as a segment's row is)
+        if (west || east) {
+            xin += (west ? relu(Fw) : R(0)) + (east ? relu(-Fe) : R(0));
+            xout += (west ? relu(-Fw) : R(0)) + (east ? relu(Fe) : R(0));
+        }
         if (!FULL) {
             if (orow == 0) { yin += relu(Gs); yout += relu(-Gs); }
             if (orow == ny - 1) { yin += relu(-Gn); yout += relu(Gn); }
