@@ -19,6 +19,7 @@ void set_error(const std::string& msg) { g_last_error = msg; }
 
 int cuda_fail(cudaError_t e, const char* what) {
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();                      // reported here, not by the caller's next CUDA call
     return HIS_ERR_CUDA;
 }
 
@@ -27,7 +28,7 @@ void* stage_acquire(HostStage& st, size_t bytes, int* slot) {
     if (bytes > st.bytes) {
         size_t want = (std::max(bytes, size_t(256)) + 4095) & ~size_t(4095);
         for (int k = 0; k < HostStage::SLOTS; ++k) {
-            if (st.done[k]) cudaEventSynchronize(st.done[k]);
+            if (st.done[k] && cudaEventSynchronize(st.done[k]) != cudaSuccess) cudaGetLastError();
             if (st.buf[k]) cudaFreeHost(st.buf[k]);
             st.buf[k] = nullptr;
         }
@@ -61,7 +62,8 @@ int stage_release(HostStage& st, int slot, cudaStream_t s) {
 void stage_free(HostStage& st) {
     for (int k = 0; k < HostStage::SLOTS; ++k) {
         if (st.done[k]) {
-            cudaEventSynchronize(st.done[k]);
+            // (an event that a caller's capture recorded cannot be waited for)
+            if (cudaEventSynchronize(st.done[k]) != cudaSuccess) cudaGetLastError();
             cudaEventDestroy(st.done[k]);
         }
         if (st.buf[k]) cudaFreeHost(st.buf[k]);
