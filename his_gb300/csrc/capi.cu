@@ -27,8 +27,13 @@ void* stage_acquire(HostStage& st, size_t bytes, int* slot) {
     cudaError_t e = cudaSuccess;
     if (bytes > st.bytes) {
         size_t want = (std::max(bytes, size_t(256)) + 4095) & ~size_t(4095);
+        // (a slot that a graph of the caller's copies from stays, and the call is refused)
+        for (int k = 0; k < HostStage::SLOTS; ++k)
+            if (st.done[k] && (e = cudaEventSynchronize(st.done[k])) != cudaSuccess) {
+                cuda_fail(e, "pinned staging buffer: previous copy");
+                return nullptr;
+            }
         for (int k = 0; k < HostStage::SLOTS; ++k) {
-            if (st.done[k] && cudaEventSynchronize(st.done[k]) != cudaSuccess) cudaGetLastError();
             if (st.buf[k]) cudaFreeHost(st.buf[k]);
             st.buf[k] = nullptr;
         }

@@ -35,6 +35,10 @@ def test_a_captured_coupled_step_replays():
             refused += 1
         assert float(torch.ones(4, device="cuda").sum()) == 4.0
     assert refused > 0
+    # nor is it freed for larger ones: 256 substeps' forcing
+    with pytest.raises(RuntimeError):
+        G._in_one(a, a.one, dt, 0.0, la, rate, 256, side)
+    assert float(torch.ones(4, device="cuda").sum()) == 4.0
     del a, g
     gc.collect()
     assert float(torch.ones(4, device="cuda").sum()) == 4.0
