@@ -58,8 +58,9 @@ __device__ __forceinline__ double f64_minmod(double a, double b) {
 }
 
 // a / b from r = 1 / b correctly rounded: the residual step of Markstein's theorem (IBM
-// Journal of Research and Development 34 (1), 1990), which rounds the quotient correctly;
-// 3 FP64 instructions per numerator instead of 7.4.  An infinite quotient is kept.
+// Journal of Research and Development 34 (1), 1990), which rounds the quotient correctly
+// while neither it nor a is subnormal (then within 2 ulp); 3 FP64 instructions per numerator
+// instead of 7.4.  An infinite quotient is kept; a zero loses its sign; an infinite b gives NaN.
 __device__ __forceinline__ double f64_div(double a, double b, double r) {
     const double q = a * r;
     return (f64_bits(q) & ~F64_SIGN) == F64_INF ? q : fma(fma(-q, b, a), r, q);
