@@ -40,10 +40,11 @@ ALG_BYTES_F64 = 128
 # pre, stage 1, stage 2, 1-D substeps, post: per member chain.  Up to 32 members a step's post
 # and the next one's pre are one kernel inside a graph of 16 steps.
 LAUNCHES_PER_STEP = 5
+TURN_MEMBERS = 32       # PRE_MEMBERS_F32 of the engine's kernels
 
 
 def launches(members: int, chains: int, steps: int) -> int:
-    per_chain = LAUNCHES_PER_STEP * steps if members > 32 else (LAUNCHES_PER_STEP - 1) * steps + -(-steps // 16)
+    per_chain = LAUNCHES_PER_STEP * steps if members > TURN_MEMBERS else (LAUNCHES_PER_STEP - 1) * steps + -(-steps // 16)
     return per_chain * chains
 
 

@@ -28,8 +28,10 @@ namespace his {
 //
 // CTAs per member: float64 8, the exchange being bound by FP64 instructions; float32 4 while
 // the set is small (32 members and fewer; no member's bits depend on it), where spare SMs
-// shorten the chain (16 steps of six served storms 1213 -> 1152 us), else 1 (of 64 storms
-// 5409 us against 5648).
+// shorten the chain, else 1.  16 steps in us with one CTA and with four (and TURN): 400 x 325
+// cells in 58 x 48, 8 members 1904 and 1752, 24 2894 and 2802, 32 3238 and 3320, 48 4116 and 4430,
+// 64 5253 and 5635; in 58 x 16, 8 1322 and 1181, 32 3368 and 3298, 64 6253 and 6227; 100 x 81
+// cells, 8 644 and 571, 32 974 and 898, 48 983 and 976, 64 1064 and 1099.
 constexpr int PRE_MEMBERS_F32 = 32;
 constexpr int ENG_PRE_THREADS = 512, ENG_EXCH_THREADS = 448, ENG_EXCH_WARPS = ENG_EXCH_THREADS / 32;
 

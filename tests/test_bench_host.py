@@ -17,6 +17,17 @@ def test_traffic_per_cell_is_read_from_the_stage2_profile():
     assert 64.0 <= v <= 88.0, v
 
 
+def test_launch_counts_follow_the_engine():
+    # from how many members on a step's accounting and the next one's pre-step are apart
+    import re
+    import bench
+    text = (ROOT / "his_gb300" / "csrc" / "engine_kernels.cuh").read_text()
+    assert bench.TURN_MEMBERS == int(re.search(r"constexpr int PRE_MEMBERS_F32 = (\d+);", text).group(1))
+    assert bench.launches(bench.TURN_MEMBERS + 1, 2, 10) == 2 * 10 * 5
+    assert bench.launches(bench.TURN_MEMBERS, 1, 32) == 32 * 4 + 2
+    assert bench.launches(1, 1, 10) == 10 * 4 + 1
+
+
 def test_both_arms_name_the_same_workload():
     import bench
     cfg = bench.workload_config(64)
