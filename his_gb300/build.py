@@ -1,8 +1,8 @@
 """Build ``libhis_gb300.so`` in-tree for sm_103a (GB300) with plain nvcc.
 
 Each translation unit compiles in parallel; the float64 kernels and the 1-D
-network are built with ``-fmad=false`` (products and sums round separately, as in
-the reference's float64 arithmetic), the float32 kernels with fused multiply-add.
+network are built with ``-fmad=false`` (a product and a sum are fused only where the
+code says so), the float32 kernels with fused multiply-add.
 """
 from __future__ import annotations
 

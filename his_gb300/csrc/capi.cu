@@ -258,6 +258,7 @@ int32_t his_grid_create(int32_t precision, const his_solver_cfg* cfg, int32_t n_
     return HIS_OK;
 }
 
+// For other arguments: the next call is a first one again.
 static void graph_drop(LaunchGraph& G) {
     if (G.exec) cudaGraphExecDestroy(G.exec);
     G.exec = nullptr;
@@ -408,7 +409,6 @@ static int capture_launches(his_grid* g, int (*launches)(his_grid*, cudaStream_t
     return HIS_OK;
 }
 
-// (graph_drop: for other arguments; its next call is a first one again)
 // launches(g, s), from the second call on as a graph, unless the caller is capturing s.
 static int launch_graph(his_grid* g, LaunchGraph& G, cudaStream_t s, int (*launches)(his_grid*, cudaStream_t)) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;

@@ -3,9 +3,9 @@
 // host round trip.  The per-member kernels take the first member m0 of the chain
 // they serve (block b works on member m0 + b).  One step is
 //
-//   eng_pre   (one CTA per member)  2-D CFL dt from the rate of the current state,
-//             1-D CFL and substep count, weir exchange, forcing at t, t+dt and at the
-//             1-D substep starts                          (coupling.py:201-212)
+//   eng_pre   (a CTA, or a cluster of four or eight, per member)  2-D CFL dt from the rate
+//             of the current state, 1-D CFL and substep count, weir exchange, forcing at
+//             t, t+dt and the 1-D substep starts          (coupling.py:201-212)
 //   stage 1, stage 2 (tiles of every member)              (swe2d.py:305-371)
 //   net substeps (one CTA per member, concurrent with the 2-D stages)
 //                                                         (coupling.py:216-221)

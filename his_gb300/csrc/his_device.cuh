@@ -4,8 +4,9 @@
 //
 // Everything is templated on the storage/arithmetic type R (double for the plain
 // method, float for the production form).  The float64 translation unit is built
-// with -fmad=false so its arithmetic rounds after every operation, like the
-// reference solver's float64 torch ops (hydrointel/solver/swe2d.py).
+// with -fmad=false, so a product and a sum are fused only where the code says so; its
+// order of rounding is its own (f64_ops.cuh), not that of the reference solver's float64
+// torch ops (hydrointel/solver/swe2d.py).
 #pragma once
 #include <cmath>
 #include <cstdint>

@@ -1,4 +1,5 @@
-// 1-D St. Venant network step and 1-D <-> 2-D weir exchange (one CTA per member).
+// 1-D St. Venant network step (one CTA per member) and 1-D <-> 2-D weir exchange (one CTA per
+// member, or a cluster of them).
 //
 // The channel network is small (10^2 - 10^3 cells): a member's whole network lives
 // in shared memory for all of its substeps.  Scatter-adds of the reference

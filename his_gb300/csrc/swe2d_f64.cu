@@ -1,5 +1,5 @@
-// Plain method: every 2-D kernel instantiated in float64.  Built with -fmad=false so
-// products and sums round separately, as in the reference's float64 torch ops.
+// Plain method: every 2-D kernel instantiated in float64.  Built with -fmad=false, so a
+// product and a sum are fused only where the code says so.
 #include "swe2d_impl.cuh"
 
 namespace his {
