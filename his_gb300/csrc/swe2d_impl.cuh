@@ -3,6 +3,7 @@
 // swe2d_f32.cu.
 #pragma once
 #include <algorithm>
+#include <climits>
 #include <vector>
 
 #include "engine_kernels.cuh"
@@ -33,8 +34,10 @@ struct StagePlan {
 // 400 x 325 in 58 x 16, 147 chunks 57, 45 and 37; 294 58, 46 and 45; 441 58, 52 and 70; 588
 // 62, 69 and 69; in 58 x 48 (49 chunks) 107, 70 and 57; 1601 x 1301 in 58 x 48 (784) 146,
 // 330 and 235.
-inline int strip_segments(int nt, int tiles, int rows) {
-    if (nt != 64) return 1;
+//
+// A set with a member of one column is marched in one, for its totals' sake (StripPipe).
+inline int strip_segments(int nt, int tiles, int rows, int narrowest) {
+    if (nt != 64 || narrowest < 2) return 1;
     using G = StripGeom<float, 64>;
     const double per_sm = tiles / 152.0;
     int best = 1;
@@ -287,7 +290,7 @@ int grid_init_impl(his_grid* g) {
     g->scratch_bytes = total;
     HIS_CK(cudaMalloc(&g->d_scratch, total > 0 ? total : 256));
     const int wmax = g->tx;
-    int sub_w = 1, sub_h = 1, rows = 1;
+    int sub_w = 1, sub_h = 1, rows = 1, narrowest = INT_MAX;
     for (int m = 0; m < n; ++m) {
         const his_grid_desc& d = g->desc[m];
         Grid<R>& G = H[m];
@@ -312,6 +315,7 @@ int grid_init_impl(his_grid* g) {
         G.tiles_y = nch;
         G.n_tiles = ns * nch;
         rows = std::max(rows, hch);
+        narrowest = std::min(narrowest, d.nx);
         if constexpr (sizeof(R) == 8) {
             sub_w = std::max(sub_w, tile64_part(w, TILE64_W));
             sub_h = std::max(sub_h, tile64_part(hch, TILE64_H));
@@ -340,7 +344,7 @@ int grid_init_impl(his_grid* g) {
         g->stage_smem = g->d_faces ? face64_smem(sub_w, sub_h, second) : tile64_smem(sub_w, sub_h, second);
         g->cell_smem = cell64_smem(sub_w, sub_h);
     } else {
-        g->seg = strip_segments(g->nt, g->n_tiles, rows);
+        g->seg = strip_segments(g->nt, g->n_tiles, rows, narrowest);
         g->stage_smem = g->nt == 64 ? stage_smem<R, 64>(0, rows, 0, g->seg) : g->nt == 128 ? stage_smem<R, 128>(0, 0, 0, 1)
                       : g->nt == 224 ? stage_smem<R, 224>(0, 0, 0, 1) : stage_smem<R, 352>(0, 0, 0, 1);
     }
@@ -577,7 +581,7 @@ int noalloc_step_impl(const Consts& c, const his_grid_desc& d, const his_step_pa
     auto* part = reinterpret_cast<double*>(base + L.o_part);
     auto* out = reinterpret_cast<double*>(base + L.o_out);
     const KC<R> kc = make_kc<R>(c);
-    const int seg = sizeof(R) == 8 ? 1 : strip_segments(NT, L.n_strips, L.hch);
+    const int seg = sizeof(R) == 8 ? 1 : strip_segments(NT, L.n_strips, L.hch, G.nx);
     const StagePlan smem{stage_smem<R, NT>(L.w, L.hch, c.order, seg), nullptr, 0, seg, G.pk || G.ps};
     if (c.order == 2) {
         launch_stage<R, NT, 1>(grid, strips, params, kc, part, L.n_strips, smem, s);

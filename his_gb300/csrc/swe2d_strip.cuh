@@ -286,7 +286,9 @@ __device__ __forceinline__ Q4<float> side_flux(const KC<float>& c, const Side& L
 // SEG > 1: the chunk's rows are dealt to SEG groups of NT threads, which march side by side,
 // each with its own rings and barrier; the rows' contributions to the partial sums are kept
 // per row and thread and added up in row order at the end, so that the sums are those of one
-// march over all rows, bit for bit.
+// march over all rows, bit for bit.  (But where a thread adds twice to a sum in a row, the terms
+// of a column that is both the west and the east edge: strip_segments marches sets with such
+// members in one.)
 //
 // PEAKS: some member of the set has running peaks (a kernel without their code takes 5251 us for
 // 16 steps of 64 storms of 400 x 325 cells, one that tests for them in every row 5285).
@@ -507,11 +509,8 @@ struct StripPipe {
         dhu = fmaf(Ts - Tn, idy, dhu);
         dhv = fmaf(Tw - Te, idx, dhv);
         if (!do_out) return;
-        // (one column is west and east: its two terms are added first, as a segment's row is)
-        if (west || east) {
-            xin += (west ? relu(Fw) : R(0)) + (east ? relu(-Fe) : R(0));
-            xout += (west ? relu(-Fw) : R(0)) + (east ? relu(Fe) : R(0));
-        }
+        if (west) { xin += relu(Fw); xout += relu(-Fw); }
+        if (east) { xin += relu(-Fe); xout += relu(Fe); }
         if (!FULL) {
             if (orow == 0) { yin += relu(Gs); yout += relu(-Gs); }
             if (orow == ny - 1) { yin += relu(-Gn); yout += relu(Gn); }
